@@ -79,38 +79,52 @@ int check_body(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, const c
     return CG_OK;
 }
 
-// Precomputed viscosity arrays of a solve (dense Center layout, halo 1, in the field type):
-// [inv_eta], eta_ve, and per shear component the interpolated 1/eta and its eta_ve.
-struct Pre {
+// The coefficients of a loop of FP64 PT iterations (PtCoef): scalars, and with a variable
+// viscosity arrays in scratch slot 2 (dense Center layout, halo 1).
+struct LoopCoef {
+    bool on = false;      // the loop runs stress_loop_kernel and velocity_loop_kernel
     char* base = nullptr;
     long s1 = 0, s2 = 0, count = 0;  // element strides and elements per array
-    int ne = 0;                      // shear components
-    int own_ieta = 0;                // inv_eta computed here (the caller gave only eta)
+    int own_ieta = 0;                // 1/eta computed here (the caller gave only eta)
 };
 
 template <class T>
-DF<T> pre_view(const Pre& pr, int idx) {
+DF<T> coef_view(const LoopCoef& lc, int idx) {
     DF<T> v;
-    v.p = reinterpret_cast<T*>(pr.base) + (long)idx * pr.count + 1 + pr.s1 + pr.s2;
-    v.s1 = pr.s1;
-    v.s2 = pr.s2;
+    v.p = reinterpret_cast<T*>(lc.base) + (long)idx * lc.count + 1 + lc.s1 + lc.s2;
+    v.s1 = lc.s1;
+    v.s2 = lc.s2;
     return v;
 }
 
-template <class T>
-void apply_pre(SV<T>& v, const Pre* pr) {
-    if (!pr || !pr->base) return;
+template <class T, int ND>
+PtCoef<T> loop_coef(const cg_grid* g, const cg_stokes_params* p, const SV<T>& v, const LoopCoef& lc) {
+    PtCoef<T> c;
+    std::memset(&c, 0, sizeof(c));
+    const SP<T> s = scalars<T>(g, p);
+    c.g = s.inv_Gdt;
+    c.third = s.third;
+    for (int d = 0; d < 3; ++d) {
+        c.idx[d] = s.idx[d];
+        c.idx2[d] = T(2) * s.idx[d];
+    }
+    if (!lc.base) {
+        c.ieta_s = T(1) / s.eta;
+        c.cP_s = T(0.5) * (s.eta_ve * s.dtau_Pr);
+        c.cT_s = s.eta_ve * s.dtau_r;
+        c.step_s = s.nu_dtau / s.eta_ve;
+        return c;
+    }
     int idx = 0;
-    if (pr->own_ieta) {
-        v.ieta = pre_view<T>(*pr, idx++);
-        v.has_ieta = 1;
+    c.ieta = lc.own_ieta ? coef_view<T>(lc, idx++) : v.ieta;
+    c.cP = coef_view<T>(lc, idx++);
+    c.cT = coef_view<T>(lc, idx++);
+    for (int e = 0; e < (ND == 2 ? 1 : 3); ++e) {
+        c.ievE[e] = coef_view<T>(lc, idx++);
+        c.cE[e] = coef_view<T>(lc, idx++);
     }
-    v.eveC = pre_view<T>(*pr, idx++);
-    for (int e = 0; e < pr->ne; ++e) {
-        v.ievE[e] = pre_view<T>(*pr, idx++);
-        v.eveE[e] = pre_view<T>(*pr, idx++);
-    }
-    v.has_pre = 1;
+    for (int d = 0; d < ND; ++d) c.step[d] = coef_view<T>(lc, idx++);
+    return c;
 }
 
 template <class T>
@@ -121,31 +135,44 @@ __global__ void inv_kernel(DF<T> dst, DF<T> src, int lo, int e0, int e1, int e2)
     for (int k = e2 < 0 ? 0 : lo; k <= (e2 < 0 ? 0 : e2); ++k) dst(i, j, k) = T(1) / src(i, j, k);
 }
 
-// Fill `pr` for the variable-viscosity field set `f` (scratch slot 2) and run the precompute.
+// Set up `lc` for a loop of PT iterations over the field set `f` and fill its arrays. The loop's
+// kernels run for FP64 from two iterations on: for a single one, filling the arrays costs what
+// they save. FP32 loops are bound by HBM (the arrays would add traffic) and keep stress_kernel and
+// velocity_kernel, as does a loop whose arrays find no room.
 template <class T, int ND>
-int setup_pre(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p, Pre* pr) {
-    const long e0 = g->n[0] + 4, e1 = g->n[1] + 4, e2 = ND > 2 ? g->n[2] + 4 : 1;
-    pr->s1 = e0;
-    pr->s2 = ND > 2 ? e0 * e1 : 0;
-    pr->count = e0 * e1 * e2;
-    pr->ne = ND == 2 ? 1 : 3;
-    pr->own_ieta = !cg_present(f->inv_eta);
-    const int narr = pr->own_ieta + 1 + 2 * pr->ne;
-    int rc = CG_OK;
-    pr->base = static_cast<char*>(cg_scratch(ctx, 2, (size_t)narr * pr->count * sizeof(T), &rc));
-    if (rc) return rc;
-    SV<T> v = views<T>(f, ND);
-    const dim3 block(32, 8);
-    if (pr->own_ieta) {
-        // 1/eta over the whole padded range the kernels read (logical -1 .. n+2)
-        const DF<T> dst = pre_view<T>(*pr, 0);
-        const dim3 gi(cg_div_up(g->n[0] + 4, 32), cg_div_up(g->n[1] + 4, 8));
-        inv_kernel<T><<<gi, block, 0, ctx->stream>>>(dst, v.eta, -1, g->n[0] + 2, g->n[1] + 2, ND > 2 ? g->n[2] + 2 : -1);
-        CG_CHECK_LAUNCH(ctx);
+int setup_coef(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p, int niter, LoopCoef* lc) {
+    *lc = LoopCoef{};
+    if (sizeof(T) != 8 || niter < 2) return CG_OK;
+    if (!cg_present(f->eta) && !cg_present(f->inv_eta)) {
+        lc->on = true;
+        return CG_OK;
     }
-    apply_pre(v, pr);
-    precompute_kernel<T, ND><<<range_grid<ND>(g, block), block, 0, ctx->stream>>>(v, scalars<T>(g, p), g->n[0] + 1,
-                                                                                 g->n[1] + 1);
+    const long e0 = g->n[0] + 4, e1 = g->n[1] + 4, e2 = ND > 2 ? g->n[2] + 4 : 1;
+    lc->s1 = e0;
+    lc->s2 = ND > 2 ? e0 * e1 : 0;
+    lc->count = e0 * e1 * e2;
+    lc->own_ieta = !cg_present(f->inv_eta);
+    const int narr = lc->own_ieta + 2 + 2 * (ND == 2 ? 1 : 3) + ND;
+    int rc = CG_OK;
+    lc->base = static_cast<char*>(cg_scratch(ctx, 2, (size_t)narr * lc->count * sizeof(T), &rc));
+    if (rc) {
+        cudaGetLastError();
+        *lc = LoopCoef{};
+        return CG_OK;
+    }
+    lc->on = true;
+    SV<T> v = views<T>(f, ND);
+    const PtCoef<T> c = loop_coef<T, ND>(g, p, v, *lc);
+    const dim3 block(32, 8);
+    if (lc->own_ieta) {
+        // 1/eta over the whole padded range the kernels read (logical -1 .. n+2)
+        const dim3 gi(cg_div_up(g->n[0] + 4, 32), cg_div_up(g->n[1] + 4, 8));
+        inv_kernel<T><<<gi, block, 0, ctx->stream>>>(c.ieta, v.eta, -1, g->n[0] + 2, g->n[1] + 2, ND > 2 ? g->n[2] + 2 : -1);
+        CG_CHECK_LAUNCH(ctx);
+        v.ieta = c.ieta;
+        v.has_ieta = 1;
+    }
+    coef_kernel<T, ND><<<range_grid<ND>(g, block), block, 0, ctx->stream>>>(v, scalars<T>(g, p), c, g->n[0] + 1, g->n[1] + 1);
     CG_CHECK_LAUNCH(ctx);
     return CG_OK;
 }
@@ -160,35 +187,63 @@ FieldMaskW<T> mask_views(const cg_mask* m) {
     return w;
 }
 
+// update_stress! over [0, n+1]^N with operand reader m, by the loop's kernel where lc is on.
 template <class T, int ND, class M>
-void stress_launch(const cg_grid* g, const SV<T>& v, const SP<T>& s, bool res, const M& m, dim3 block, cudaStream_t st) {
+void stress_launch(const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p, bool res, const LoopCoef* lc,
+                   const M& m, dim3 block, cudaStream_t st) {
+    const SV<T> v = views<T>(f, ND);
+    const dim3 grid = range_grid<ND>(g, block);
+    const int e0 = g->n[0] + 1, e1 = g->n[1] + 1;
+    if constexpr (sizeof(T) == 8) {
+        if (lc && lc->on) {
+            const PtCoef<T> c = loop_coef<T, ND>(g, p, v, *lc);
+            if (lc->base && res) stress_loop_kernel<T, ND, true, true, M><<<grid, block, 0, st>>>(v, c, e0, e1, m);
+            else if (lc->base) stress_loop_kernel<T, ND, false, true, M><<<grid, block, 0, st>>>(v, c, e0, e1, m);
+            else if (res) stress_loop_kernel<T, ND, true, false, M><<<grid, block, 0, st>>>(v, c, e0, e1, m);
+            else stress_loop_kernel<T, ND, false, false, M><<<grid, block, 0, st>>>(v, c, e0, e1, m);
+            return;
+        }
+    }
+    const SP<T> s = scalars<T>(g, p);
     if (res)
-        stress_kernel<T, ND, true, M><<<range_grid<ND>(g, block), block, 0, st>>>(v, s, g->n[0] + 1, g->n[1] + 1, m);
+        stress_kernel<T, ND, true, M><<<grid, block, 0, st>>>(v, s, e0, e1, m);
     else
-        stress_kernel<T, ND, false, M><<<range_grid<ND>(g, block), block, 0, st>>>(v, s, g->n[0] + 1, g->n[1] + 1, m);
+        stress_kernel<T, ND, false, M><<<grid, block, 0, st>>>(v, s, e0, e1, m);
 }
 
 template <class T, int ND, class M>
-void velocity_launch(const cg_grid* g, const SV<T>& v, const SP<T>& s, const BodyFn<T>& bf, bool res, const M& m,
-                     dim3 block, cudaStream_t st) {
+void velocity_launch(const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p, bool res, const LoopCoef* lc,
+                     const M& m, dim3 block, cudaStream_t st) {
+    const SV<T> v = views<T>(f, ND);
+    const BodyFn<T> bf = body_fns<T>(g, p);
+    const dim3 grid = range_grid<ND>(g, block);
+    const int e0 = g->n[0] + 1, e1 = g->n[1] + 1;
+    if constexpr (sizeof(T) == 8) {
+        if (lc && lc->on) {
+            const PtCoef<T> c = loop_coef<T, ND>(g, p, v, *lc);
+            if (lc->base && res) velocity_loop_kernel<T, ND, true, true, M><<<grid, block, 0, st>>>(v, c, bf, e0, e1, m);
+            else if (lc->base) velocity_loop_kernel<T, ND, false, true, M><<<grid, block, 0, st>>>(v, c, bf, e0, e1, m);
+            else if (res) velocity_loop_kernel<T, ND, true, false, M><<<grid, block, 0, st>>>(v, c, bf, e0, e1, m);
+            else velocity_loop_kernel<T, ND, false, false, M><<<grid, block, 0, st>>>(v, c, bf, e0, e1, m);
+            return;
+        }
+    }
+    const SP<T> s = scalars<T>(g, p);
     if (res)
-        velocity_kernel<T, ND, true, M><<<range_grid<ND>(g, block), block, 0, st>>>(v, s, bf, g->n[0] + 1, g->n[1] + 1, m);
+        velocity_kernel<T, ND, true, M><<<grid, block, 0, st>>>(v, s, bf, e0, e1, m);
     else
-        velocity_kernel<T, ND, false, M><<<range_grid<ND>(g, block), block, 0, st>>>(v, s, bf, g->n[0] + 1, g->n[1] + 1, m);
+        velocity_kernel<T, ND, false, M><<<grid, block, 0, st>>>(v, s, bf, e0, e1, m);
 }
 
 // update_stress! over [0, n+1]^N; with `mask`, every strain-rate derivative is the masked
 // operator ∂(V.d, ω, g, I) (src/GridOperators/masked_field_operators.jl:20-57).
 template <class T, int ND>
-cudaError_t stress_any(const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p, bool res, const Pre* pr,
-                       const cg_mask* mask, dim3 block, cudaStream_t st) {
-    SV<T> v = views<T>(f, ND);
-    apply_pre(v, pr);
-    const SP<T> s = scalars<T>(g, p);
+cudaError_t stress_any(const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p, bool res,
+                       const LoopCoef* lc, const cg_mask* mask, dim3 block, cudaStream_t st) {
     if (mask)
-        stress_launch<T, ND>(g, v, s, res, mask_views<T>(mask), block, st);
+        stress_launch<T, ND>(g, f, p, res, lc, mask_views<T>(mask), block, st);
     else
-        stress_launch<T, ND>(g, v, s, res, NoMask<T>{}, block, st);
+        stress_launch<T, ND>(g, f, p, res, lc, NoMask<T>{}, block, st);
     return cudaGetLastError();
 }
 
@@ -196,29 +251,26 @@ cudaError_t stress_any(const cg_grid* g, const cg_stokes_fields* f, const cg_sto
 // masked operators.
 template <class T, int ND>
 cudaError_t velocity_any(const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p, bool res,
-                         const Pre* pr, const cg_mask* mask, dim3 block, cudaStream_t st) {
-    SV<T> v = views<T>(f, ND);
-    apply_pre(v, pr);
-    const SP<T> s = scalars<T>(g, p);
+                         const LoopCoef* lc, const cg_mask* mask, dim3 block, cudaStream_t st) {
     if (mask)
-        velocity_launch<T, ND>(g, v, s, body_fns<T>(g, p), res, mask_views<T>(mask), block, st);
+        velocity_launch<T, ND>(g, f, p, res, lc, mask_views<T>(mask), block, st);
     else
-        velocity_launch<T, ND>(g, v, s, body_fns<T>(g, p), res, NoMask<T>{}, block, st);
+        velocity_launch<T, ND>(g, f, p, res, lc, NoMask<T>{}, block, st);
     return cudaGetLastError();
 }
 
 template <class T, int ND>
 int launch_stress(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p, bool res,
-                  const Pre* pr = nullptr, const cg_mask* mask = nullptr, dim3 block = dim3(32, 8)) {
-    const cudaError_t e = stress_any<T, ND>(g, f, p, res, pr, mask, block, ctx->stream);
+                  const LoopCoef* lc = nullptr, const cg_mask* mask = nullptr, dim3 block = dim3(32, 8)) {
+    const cudaError_t e = stress_any<T, ND>(g, f, p, res, lc, mask, block, ctx->stream);
     if (e != cudaSuccess) return cg_fail(ctx, CG_ERR_CUDA, "update_stress: %s", cudaGetErrorString(e));
     return CG_OK;
 }
 
 template <class T, int ND>
 int launch_velocity(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p, bool res,
-                    const Pre* pr = nullptr, const cg_mask* mask = nullptr, dim3 block = dim3(32, 8)) {
-    const cudaError_t e = velocity_any<T, ND>(g, f, p, res, pr, mask, block, ctx->stream);
+                    const LoopCoef* lc = nullptr, const cg_mask* mask = nullptr, dim3 block = dim3(32, 8)) {
+    const cudaError_t e = velocity_any<T, ND>(g, f, p, res, lc, mask, block, ctx->stream);
     if (e != cudaSuccess) return cg_fail(ctx, CG_ERR_CUDA, "update_velocity: %s", cudaGetErrorString(e));
     return CG_OK;
 }
@@ -235,7 +287,7 @@ size_t padded_span_bytes(const cg_field& f) {
 // and write divV and r_V, so the candidates run on copies of those fields in a temporary
 // allocation, released before the loop's graph is captured; the caller's fields are untouched.
 template <class T, int ND>
-int stokes_blocks(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p, const Pre* pr,
+int stokes_blocks(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p, const LoopCoef* lc,
                   const cg_mask* mask, dim3* bs, dim3* bv) {
     *bs = *bv = dim3(32, 8);
     dim3 forced;
@@ -249,7 +301,7 @@ int stokes_blocks(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, cons
     cg_key_add(base, (int)sizeof(T));
     cg_key_add(base, f->V[0].stride);
     cg_key_add(base, f->tau[0].stride);
-    cg_key_add(base, (int)cg_present(f->eta) + 2 * (int)cg_present(f->inv_eta) + 4 * (pr != nullptr) + 8 * (mask != nullptr));
+    cg_key_add(base, (int)cg_present(f->eta) + 2 * (int)cg_present(f->inv_eta) + 4 * (lc && lc->on) + 8 * (mask != nullptr));
     cg_key_add(base, ctx->num_sms);
     const std::string ks = base + "stress", kv = base + "velocity";
     cg_tune_cfg c1{0, 0}, c2{0, 0};
@@ -289,9 +341,9 @@ int stokes_blocks(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, cons
         upd[a]->data = tmp + off[a];
     }
     *bs = cgk::tune_block("update_stress", ks,
-                          [&](dim3 b) { return stress_any<T, ND>(g, &c, p, true, pr, mask, b, ctx->stream); }, ctx->stream);
+                          [&](dim3 b) { return stress_any<T, ND>(g, &c, p, true, lc, mask, b, ctx->stream); }, ctx->stream);
     *bv = cgk::tune_block("update_velocity", kv,
-                          [&](dim3 b) { return velocity_any<T, ND>(g, &c, p, true, pr, mask, b, ctx->stream); }, ctx->stream);
+                          [&](dim3 b) { return velocity_any<T, ND>(g, &c, p, true, lc, mask, b, ctx->stream); }, ctx->stream);
     cudaStreamSynchronize(ctx->stream);
     cudaFree(tmp);
     return CG_OK;
@@ -390,7 +442,7 @@ int thermal_partner(cg_ctx* ctx, const cg_field& Tf, cg_field* out) {
 // step and bc!(T) (examples/stokes_2d_inc_ve_T.jl:144-152). T alternates with the library's
 // partner buffer and ends in f->T.
 int pt_iterations(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p,
-                  const cg_bc* bc_V, int niter, int dtype, const Pre* pr = nullptr, const cg_bc* bc_T = nullptr,
+                  const cg_bc* bc_V, int niter, int dtype, const LoopCoef* lc = nullptr, const cg_bc* bc_T = nullptr,
                   const cg_mask* mask = nullptr) {
     cg_field Tw;
     std::memset(&Tw, 0, sizeof(Tw));
@@ -406,7 +458,8 @@ int pt_iterations(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, cons
     cg_bc none[3];
     std::memset(none, 0, sizeof(none));
     for (int d = 0; d < g->ndim; ++d) cg_key_add(key, bc_V ? bc_V[d] : none[d]);
-    cg_key_add(key, pr ? pr->base : nullptr);
+    cg_key_add(key, lc ? lc->base : nullptr);
+    cg_key_add(key, lc && lc->on ? 1 : 0);
     cg_key_add(key, bc_T ? 1 : 0);
     if (bc_T) {
         cg_key_add(key, *bc_T);
@@ -416,7 +469,7 @@ int pt_iterations(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, cons
     if (mask) cg_key_add(key, *mask);
     const int nd = g->ndim;
     dim3 bs, bv;
-    int rc0 = SDISPATCH(stokes_blocks, dtype, nd, ctx, g, f, p, pr, mask, &bs, &bv);
+    int rc0 = SDISPATCH(stokes_blocks, dtype, nd, ctx, g, f, p, lc, mask, &bs, &bv);
     if (rc0) return rc0;
     cg_key_add(key, bs);
     cg_key_add(key, bv);
@@ -426,9 +479,9 @@ int pt_iterations(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, cons
         if (bc_T) CG_CUDA(ctx, cudaMemcpyAsync(Tw.data, f->T.data, tbytes, cudaMemcpyDeviceToDevice, st));
         for (int it = 0; it < niter; ++it) {
             const bool last = it == niter - 1;
-            int rc = SDISPATCH(launch_stress, dtype, nd, ctx, g, f, p, last, pr, mask, bs);
+            int rc = SDISPATCH(launch_stress, dtype, nd, ctx, g, f, p, last, lc, mask, bs);
             if (rc) return rc;
-            rc = SDISPATCH(launch_velocity, dtype, nd, ctx, g, f, p, last, pr, mask, bv);
+            rc = SDISPATCH(launch_velocity, dtype, nd, ctx, g, f, p, last, lc, mask, bv);
             if (rc) return rc;
             rc = apply_bc_V(ctx, g, f, bc_V);
             if (rc) return rc;
@@ -442,6 +495,15 @@ int pt_iterations(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, cons
         if (bc_T && (niter & 1)) CG_CUDA(ctx, cudaMemcpyAsync(f->T.data, Tw.data, tbytes, cudaMemcpyDeviceToDevice, st));
         return (int)CG_OK;
     });
+}
+
+// pt_iterations with the loop's coefficients set up for this call.
+int pt_loop(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p, const cg_bc* bc_V,
+            int niter, int dtype, const cg_bc* bc_T, const cg_mask* mask) {
+    LoopCoef lc;
+    const int rc = SDISPATCH(setup_coef, dtype, g->ndim, ctx, g, f, p, niter, &lc);
+    if (rc) return rc;
+    return pt_iterations(ctx, g, f, p, bc_V, niter, dtype, &lc, bc_T, mask);
 }
 
 int residual(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, double tau_scale, double v_scale, double* err,
@@ -530,7 +592,7 @@ extern "C" int cg_stokes_pt_iterations(cg_ctx* ctx, const cg_grid* grid, const c
     if (niter < 0) return cg_fail(ctx, CG_ERR_ARG, "pt_iterations: niter < 0");
     if (niter == 0) return CG_OK;
     cudaSetDevice(ctx->device);
-    return pt_iterations(ctx, grid, f, p, bc_V, niter, dtype);
+    return pt_loop(ctx, grid, f, p, bc_V, niter, dtype, nullptr, nullptr);
 }
 
 extern "C" int cg_stokes_update_stress_masked(cg_ctx* ctx, const cg_grid* grid, const cg_stokes_fields* f,
@@ -568,7 +630,7 @@ extern "C" int cg_stokes_pt_iterations_masked(cg_ctx* ctx, const cg_grid* grid, 
     if (niter < 0) return cg_fail(ctx, CG_ERR_ARG, "pt_iterations_masked: niter < 0");
     if (niter == 0) return CG_OK;
     cudaSetDevice(ctx->device);
-    return pt_iterations(ctx, grid, f, p, bc_V, niter, dtype, nullptr, nullptr, mask);
+    return pt_loop(ctx, grid, f, p, bc_V, niter, dtype, nullptr, mask);
 }
 
 namespace {
@@ -814,17 +876,16 @@ int check_solve(cg_ctx* ctx, const cg_grid* grid, const cg_stokes_fields* f, con
 int solve_fp64(cg_ctx* ctx, const cg_grid* grid, const cg_stokes_fields* f, const cg_stokes_params* p,
                const cg_bc* bc_V, const cg_bc* bc_T, const cg_solve_opts* o, cg_solve_result* res, int dtype) {
     int rc;
-    // variable viscosity: precompute the viscosity terms once for the whole solve
-    Pre pre;
-    const bool var = cg_present(f->eta) || cg_present(f->inv_eta);
-    if (var && (rc = SDISPATCH(setup_pre, dtype, grid->ndim, ctx, grid, f, p, &pre))) return rc;
+    // the loop's coefficients, once for the whole solve
+    LoopCoef lc;
+    if ((rc = SDISPATCH(setup_coef, dtype, grid->ndim, ctx, grid, f, p, o->max_iter, &lc))) return rc;
     std::memset(res, 0, sizeof(*res));
     CG_CUDA(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
     int iter = 0;
     int status = CG_ERR_NOCONV;
     while (iter < o->max_iter) {
         const int chunk = std::min(o->ncheck, o->max_iter - iter);
-        if ((rc = pt_iterations(ctx, grid, f, p, bc_V, chunk, dtype, var ? &pre : nullptr, bc_T))) return rc;
+        if ((rc = pt_iterations(ctx, grid, f, p, bc_V, chunk, dtype, &lc, bc_T))) return rc;
         iter += chunk;
         if (chunk < o->ncheck) break;  // the reference only checks at multiples of ncheck
         int32_t bad = 0;
@@ -898,7 +959,7 @@ extern "C" int cg_stokes_pt_iterations_thermal(cg_ctx* ctx, const cg_grid* grid,
     if (niter < 0) return cg_fail(ctx, CG_ERR_ARG, "pt_iterations_thermal: niter < 0");
     if (niter == 0) return CG_OK;
     cudaSetDevice(ctx->device);
-    return pt_iterations(ctx, grid, f, p, bc_V, niter, dtype, nullptr, bc_T);
+    return pt_loop(ctx, grid, f, p, bc_V, niter, dtype, bc_T, nullptr);
 }
 
 extern "C" int cg_stokes_thermal_step(cg_ctx* ctx, const cg_grid* grid, const cg_stokes_fields* f,

@@ -13,11 +13,7 @@ struct SV {  // device views of the Stokes field set
     // continuity forcing of the defect-correction solve: the pressure update and the divV
     // output use (divV + fP); the deviatoric strain rate uses divV alone
     DF<T> fP;
-    // precomputed viscosity terms of the variable-viscosity form (bit-identical to computing
-    // them in the kernel; saves the FP64 divisions): eta_ve at cells, and per shear component
-    // the interpolated 1/eta and its eta_ve (2D: [0] = xy; 3D: [0..2] = xy, xz, yz)
-    DF<T> eveC, ievE[3], eveE[3];
-    int has_rV, has_divV, has_eta, has_ieta, has_rho[3], has_fP, has_pre;
+    int has_rV, has_divV, has_eta, has_ieta, has_rho[3], has_fP;
     // 1/eta at a cell: the precomputed field when given, else an IEEE division (same bits)
     __device__ __forceinline__ T inv_eta(int i, int j, int k) const {
         return has_ieta ? ieta(i, j, k) : T(1) / eta(i, j, k);
@@ -161,23 +157,6 @@ struct FieldMaskW {
     }
 };
 
-// Viscosity terms used by every PT iteration, computed once per solve over [0, n+1]^N with the
-// stress kernel's own expressions (so the values are bit-identical).
-template <class T, int ND>
-__global__ void precompute_kernel(const SV<T> v, const SP<T> s, int e0, int e1) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = ND > 2 ? blockIdx.z : 0;
-    if (i > e0 || j > e1) return;
-    v.eveC(i, j, k) = T(1) / (v.inv_eta(i, j, k) + s.inv_Gdt);
-    const int pairs[3][2] = {{0, 1}, {0, 2}, {1, 2}};
-    for (int e = 0; e < (ND == 2 ? 1 : 3); ++e) {
-        const T iev = shear_inv_eta(v, i, j, k, pairs[e][0], pairs[e][1]);
-        v.ievE[e](i, j, k) = iev;
-        v.eveE[e](i, j, k) = T(1) / (iev + s.inv_Gdt);
-    }
-}
-
 // update_stress! at one point. Tensor order 2D (xx, yy, xy), 3D (xx, yy, zz, xy, xz, yz).
 // M reads the operands of the strain-rate derivatives (NoMask, or FieldMaskW for the masked
 // operators ∂(V.d, ω, g, I) and divg(V, ω, g, I)); V.d sits at location bits 1 << d.
@@ -204,7 +183,7 @@ __global__ void stress_kernel(const SV<T> v, const SP<T> s, int e0, int e1, cons
     T ieta_c = T(0), eve_c = s.eta_ve;
     if (v.has_eta) {
         ieta_c = v.inv_eta(i, j, k);
-        eve_c = v.has_pre ? v.eveC(i, j, k) : T(1) / (ieta_c + s.inv_Gdt);
+        eve_c = T(1) / (ieta_c + s.inv_Gdt);
     }
     v.P(i, j, k) = v.P(i, j, k) - dvP * eve_c * s.dtau_Pr;
     auto diag = [&](int c, T edd) {
@@ -221,15 +200,8 @@ __global__ void stress_kernel(const SV<T> v, const SP<T> s, int e0, int e1, cons
     auto shear = [&](int c, T eod, int a, int b) {
         const T t = v.tau[c](i, j, k), to = v.tau_old[c](i, j, k);
         if (v.has_eta) {
-            T iev, eve;
-            if (v.has_pre) {
-                const int e = ND == 2 ? 0 : c - 3;
-                iev = v.ievE[e](i, j, k);
-                eve = v.eveE[e](i, j, k);
-            } else {
-                iev = shear_inv_eta(v, i, j, k, a, b);
-                eve = T(1) / (iev + s.inv_Gdt);
-            }
+            const T iev = shear_inv_eta(v, i, j, k, a, b);
+            const T eve = T(1) / (iev + s.inv_Gdt);
             const T r = -(t - to) * s.inv_Gdt - t * iev + T(2.0) * eod;
             v.tau[c](i, j, k) = t + r * eve * s.dtau_r;
         } else {  // examples/stokes_2d_inc_ve_T.jl:30
@@ -314,6 +286,128 @@ __global__ void velocity_kernel(const SV<T> v, const SP<T> s, const BodyFn<T> bf
         v.V[1](i, j, k) = v.V[1](i, j, k) + ry * s.nu_dtau / s.eta_ve;
         if (ND > 2) v.V[2](i, j, k) = v.V[2](i, j, k) + rz * s.nu_dtau / s.eta_ve;
     }
+}
+
+// ---- the two kernels of a loop of FP64 PT iterations ------------------------------------------
+//
+// A loop calls update_stress! and update_velocity! many times with the same viscosity, G, dt and
+// PT parameters. FP64 arithmetic bounds both kernels on GB300 (two FP64 instructions per clock and
+// SM; stress_kernel kept that pipe 84 % busy at 0.41 of the HBM time), so the loop's kernels issue
+// as few of them as the update allows:
+// - what depends on the viscosity alone is computed once per loop (coef_kernel), the 1/eta
+//   interpolation and the reciprocals among it: eta_ve dtau_Pr and eta_ve dtau_r at cells, the
+//   interpolated 1/eta and its eta_ve dtau_r at every shear component, and nu_dtau / eta_ve at the
+//   faces (with one scalar viscosity, the same values as scalars);
+// - strain rates are kept doubled (2 idx is exact), which removes the products by 2 and 1/2;
+// - the stress residual keeps its form (t_old - t)/(G dt) - t/eta + 2 e, evaluated with fused
+//   multiply-adds, and tau += r (eta_ve dtau_r) is one more: the iteration's fixed point is where
+//   the residual itself vanishes, exactly as in stress_kernel.
+// Per 2D cell that leaves 24 + 14 FP64 instructions of 58 + 20 (3D: 48 + 27 of 122 + 36).
+// Measured against a loop of stress_kernel and velocity_kernel: 2D 511^2 stress 29.3 -> 15.2 us,
+// velocity 13.3 -> 10.8 us; 3D 95 x 80 x 112 stress 244 -> 109 us, velocity 90 -> 68 us; 2D 254^2
+// with a scalar viscosity and thermal coupling (the divisions were by scalars) 36.4 -> 23.8 us per
+// iteration.
+template <class T>
+struct PtCoef {
+    DF<T> ieta, cP, cT, ievE[3], cE[3], step[3];  // variable viscosity
+    T g;                                          // 1 / (G dt)
+    T ieta_s, cP_s, cT_s, step_s;                 // scalar viscosity
+    T third, idx[3], idx2[3];
+};
+
+// The viscosity terms over [0, n+1]^N. cP carries a factor 1/2 for the doubled divergence.
+template <class T, int ND>
+__global__ void coef_kernel(const SV<T> v, const SP<T> s, const PtCoef<T> c, int e0, int e1) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int k = ND > 2 ? blockIdx.z : 0;
+    if (i > e0 || j > e1) return;
+    const T ie = v.inv_eta(i, j, k);
+    const T eve = T(1) / (ie + s.inv_Gdt);
+    c.cP(i, j, k) = T(0.5) * (eve * s.dtau_Pr);
+    c.cT(i, j, k) = eve * s.dtau_r;
+    const int pairs[3][2] = {{0, 1}, {0, 2}, {1, 2}};
+    for (int e = 0; e < (ND == 2 ? 1 : 3); ++e) {
+        const T iev = shear_inv_eta(v, i, j, k, pairs[e][0], pairs[e][1]);
+        c.ievE[e](i, j, k) = iev;
+        c.cE[e](i, j, k) = T(1) / (iev + s.inv_Gdt) * s.dtau_r;
+    }
+    for (int d = 0; d < ND; ++d)
+        c.step[d](i, j, k) = s.nu_dtau * (fmin(v.inv_eta(i - (d == 0), j - (d == 1), k - (d == 2)), ie) + s.inv_Gdt);
+}
+
+// update_stress! of a PT loop at one point (VAR: the viscosity varies per cell).
+template <class T, int ND, bool WRITE_RES, bool VAR, class M>
+__global__ void stress_loop_kernel(const SV<T> v, const PtCoef<T> c, int e0, int e1, const M m) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int k = ND > 2 ? blockIdx.z : 0;
+    if (i > e0 || j > e1) return;
+    const DF<T>& Vx = v.V[0];
+    const DF<T>& Vy = v.V[1];
+    const DF<T>& Vz = v.V[2];
+    const T vx = m(1, Vx, i, j, k), vy = m(2, Vy, i, j, k), vz = ND > 2 ? m(4, Vz, i, j, k) : T(0);
+    // doubled strain rates and divergence
+    const T exx = (m(1, Vx, i + 1, j, k) - vx) * c.idx2[0];
+    const T eyy = (m(2, Vy, i, j + 1, k) - vy) * c.idx2[1];
+    T dv = exx + eyy, ezz = T(0);
+    if (ND > 2) {
+        ezz = (m(4, Vz, i, j, k + 1) - vz) * c.idx2[2];
+        dv = dv + ezz;
+    }
+    if (WRITE_RES && v.has_divV) v.divV(i, j, k) = T(0.5) * dv;
+    v.P(i, j, k) = fma(-dv, VAR ? c.cP(i, j, k) : c.cP_s, v.P(i, j, k));
+    auto update = [&](int q, T e2, T ie, T ct) {  // e2 = 2 e
+        const T t = v.tau[q](i, j, k), to = v.tau_old[q](i, j, k);
+        const T r = fma(to - t, c.g, fma(-t, ie, e2));
+        v.tau[q](i, j, k) = fma(r, ct, t);
+    };
+    const T ie = VAR ? c.ieta(i, j, k) : c.ieta_s, ct = VAR ? c.cT(i, j, k) : c.cT_s;
+    update(0, fma(-dv, c.third, exx), ie, ct);
+    update(1, fma(-dv, c.third, eyy), ie, ct);
+    if (ND > 2) update(2, fma(-dv, c.third, ezz), ie, ct);
+    auto shear = [&](int q, int e, T e2) { update(q, e2, VAR ? c.ievE[e](i, j, k) : c.ieta_s, VAR ? c.cE[e](i, j, k) : c.cT_s); };
+    shear(ND == 2 ? 2 : 3, 0, fma(vx - m(1, Vx, i, j - 1, k), c.idx[1], (vy - m(2, Vy, i - 1, j, k)) * c.idx[0]));
+    if (ND > 2) {
+        shear(4, 1, fma(vx - m(1, Vx, i, j, k - 1), c.idx[2], (vz - m(4, Vz, i - 1, j, k)) * c.idx[0]));
+        shear(5, 2, fma(vy - m(2, Vy, i, j, k - 1), c.idx[2], (vz - m(4, Vz, i, j - 1, k)) * c.idx[1]));
+    }
+}
+
+// update_velocity! of a PT loop at one point. The differences of tau_dd and of P are formed
+// separately (each is small against its operands) and share one product by idx.
+template <class T, int ND, bool WRITE_RES, bool VAR, class M>
+__global__ void velocity_loop_kernel(const SV<T> v, const PtCoef<T> c, const BodyFn<T> bf, int e0, int e1, const M m) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int k = ND > 2 ? blockIdx.z : 0;
+    if (i > e0 || j > e1) return;
+    constexpr int XY = ND == 2 ? 2 : 3, XZ = 4, YZ = 5;
+    const int LXY = 3, LXZ = 5, LYZ = 6;  // location bits of the shear components
+    const T p = m(0, v.P, i, j, k);
+    auto normal = [&](int d) {  // d(tau_dd) - d(P) along d
+        const int l = i - (d == 0), r = j - (d == 1), q = k - (d == 2);
+        return ((m(0, v.tau[d], i, j, k) - m(0, v.tau[d], l, r, q)) - (p - m(0, v.P, l, r, q))) * c.idx[d];
+    };
+    auto finish = [&](int d, T r) {
+        if (v.has_rho[d]) r = r - v.rho[d](i, j, k);
+        else if (bf.fn[d].kind) r = r - body_fn(bf, d, ND, i, j, k);
+        if (WRITE_RES && v.has_rV) v.rV[d](i, j, k) = r;
+        v.V[d](i, j, k) = fma(r, VAR ? c.step[d](i, j, k) : c.step_s, v.V[d](i, j, k));
+    };
+    const T xy = m(LXY, v.tau[XY], i, j, k);
+    T rx = fma(m(LXY, v.tau[XY], i, j + 1, k) - xy, c.idx[1], normal(0));
+    T ry = fma(m(LXY, v.tau[XY], i + 1, j, k) - xy, c.idx[0], normal(1));
+    if (ND > 2) {
+        const T xz = m(LXZ, v.tau[XZ], i, j, k), yz = m(LYZ, v.tau[YZ], i, j, k);
+        rx = fma(m(LXZ, v.tau[XZ], i, j, k + 1) - xz, c.idx[2], rx);
+        ry = fma(m(LYZ, v.tau[YZ], i, j, k + 1) - yz, c.idx[2], ry);
+        T rz = fma(m(LXZ, v.tau[XZ], i + 1, j, k) - xz, c.idx[0], normal(2));
+        rz = fma(m(LYZ, v.tau[YZ], i, j + 1, k) - yz, c.idx[1], rz);
+        finish(2, rz);
+    }
+    finish(0, rx);
+    finish(1, ry);
 }
 
 template <class T, int ND>
