@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB)
     const bool lo = w == 0, hi = w == NW - 1;
     const bool own = !lo && !hi && lane >= 1 && lane <= 30 && i <= e0 && j <= e1;
     const bool oldcell_ij = i < 0 || j < 0;  // column or row -1 keeps its old cells
-    const MAt3<T, int, true> at{i, j, s1u, s2u};
+    const MAt3<T, int, kLayOne> at(i, j, MStr{{s1u}, {s2u}});
     const int wu = w + 1 < NW ? w + 1 : NW - 1, wd = w > 0 ? w - 1 : 0;  // in-bounds neighbours
     const int ll = lane > 0 ? lane - 1 : 0;
     const int xs = i0 + xo;  // tensor x of lane 0's column
@@ -239,8 +239,8 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB)
                          : m3_shear(s, m3_rate(vy_c, vyp, s.idx[2], vz_c, vzD, s.idx[1]), iepD, iep, ieD_c, ie_c, tyz0,
                                     tyzo0);
         if (own && ok) {
-            at.st(f.tau_out[4], ks, txz_c);
-            at.st(f.tau_out[5], ks, tyz_c);
+            at.st(1, f.tau_out[4], ks, txz_c);
+            at.st(2, f.tau_out[5], ks, tyz_c);
         }
         ie_p = iep;
     }
@@ -337,24 +337,24 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB)
             if (f.has_rho[0]) rx = rsub(rx, crx);
             if (f.has_rho[1]) ry = rsub(ry, cry);
             if (f.has_rho[2]) rz = rsub(rz, crz);
-            at.st(f.P_out, k, c.P);
-            at.st(f.tau_out[0], k, c.txx);
-            at.st(f.tau_out[1], k, c.tyy);
-            at.st(f.tau_out[2], k, c.tzz);
-            at.st(f.tau_out[3], k, txyn);
+            at.st(0, f.P_out, k, c.P);
+            at.st(0, f.tau_out[0], k, c.txx);
+            at.st(0, f.tau_out[1], k, c.tyy);
+            at.st(0, f.tau_out[2], k, c.tzz);
+            at.st(3, f.tau_out[3], k, txyn);
             if (k + 1 <= ke) {
-                at.st(f.tau_out[4], k + 1, txzn);
-                at.st(f.tau_out[5], k + 1, tyzn);
+                at.st(1, f.tau_out[4], k + 1, txzn);
+                at.st(2, f.tau_out[5], k + 1, tyzn);
             }
             if (WRITE_RES) {
-                at.st(f.divV, k, c.dvP);
-                at.st(f.rV[0], k, rx);
-                at.st(f.rV[1], k, ry);
-                at.st(f.rV[2], k, rz);
+                at.st(0, f.divV, k, c.dvP);
+                at.st(1, f.rV[0], k, rx);
+                at.st(2, f.rV[1], k, ry);
+                at.st(0, f.rV[2], k, rz);
             }
-            at.st(f.V_out[0], k, radd(vx_c, rmul(rx, rmul(s.nu_dtau, radd(fmin(ieL_c, ie_c), s.inv_Gdt)))));
-            at.st(f.V_out[1], k, radd(vy_c, rmul(ry, rmul(s.nu_dtau, radd(fmin(ieD_c, ie_c), s.inv_Gdt)))));
-            at.st(f.V_out[2], k, radd(vz_c, rmul(rz, rmul(s.nu_dtau, radd(fmin(ie_p, ie_c), s.inv_Gdt)))));
+            at.st(1, f.V_out[0], k, radd(vx_c, rmul(rx, rmul(s.nu_dtau, radd(fmin(ieL_c, ie_c), s.inv_Gdt)))));
+            at.st(2, f.V_out[1], k, radd(vy_c, rmul(ry, rmul(s.nu_dtau, radd(fmin(ieD_c, ie_c), s.inv_Gdt)))));
+            at.st(0, f.V_out[2], k, radd(vz_c, rmul(rz, rmul(s.nu_dtau, radd(fmin(ie_p, ie_c), s.inv_Gdt)))));
         }
         // advance one plane
         vx_c = nvx;
@@ -543,9 +543,10 @@ inline cudaError_t launch_march3d_any(const Fused3D<T>& f, const SP<T>& s, int n
     if constexpr (sizeof(T) == 4) {
         if (variant >= kM3TmaFirst) {
             const int h = variant - kM3TmaFirst;
-            long s1 = 0, s2 = 0;
-            if (h < m3t::kHeights && l.dir[h] && l.dir[h]->ok && l.err && march3_uniform(f, &s1, &s2) &&
+            MStr str;
+            if (h < m3t::kHeights && l.dir[h] && l.dir[h]->ok && l.err && march3_layout(f, &str) == kLayOne &&
                 march3_fits_int(f, n0 + 1, n1 + 1, n2 + 1)) {
+                const long s1 = str.s1[0], s2 = str.s2[0];
                 // an ordinary launch (and the bc! launch after it too): with dependent launches around
                 // it, the defect-correction chunk measured 465-486 instead of 457-472 us per 256^3
                 // iteration
@@ -573,19 +574,19 @@ inline cg_tune_cfg tune_march3d(const Fused3D<T>& f, const SP<T>& s, int n0, int
         return best;
     }
     if (!cg_autotune_enabled()) return best;
-    long s1 = 0, s2 = 0;
-    const bool uni = march3_uniform(f, &s1, &s2);
+    MStr str;
+    const int lay = march3_layout(f, &str);
     std::string key = "march3d";
     cg_key_add(key, n0);
     cg_key_add(key, n1);
     cg_key_add(key, n2);
     cg_key_add(key, (int)sizeof(T));
-    cg_key_add(key, uni ? s1 : 0L);
-    cg_key_add(key, uni ? s2 : 0L);
+    cg_key_add(key, lay);
+    cg_key_add(key, str);
     cg_key_add(key, nsm);
     cg_key_add(key, (int)tma);
     if (cg_tune_lookup(key, &best)) return best;
-    const int nvar = (sizeof(T) == 4 && uni) ? (tma ? kM3Variants : 2) : 1;
+    const int nvar = (sizeof(T) == 4 && lay != kLayOwn) ? (tma ? kM3Variants : 2) : 1;
     float tbest = 1e30f;
     for (int v = 0; v < nvar; ++v)
         for (int seg : {0, 16, 32, 64}) {

@@ -604,13 +604,30 @@ struct Fused2D {
 // vertex at lane l needs Vy and 1/eta of lane l-1, so lane 0's vertex is invalid. The owned
 // lanes 1..30 read cells of lanes l-1, l and vertices of lanes l, l+1, all valid.
 // Ix is the element-offset type: int where every offset fits in 32 bits, else long.
-template <class T, class Ix, bool UNI>
-struct MAt {  // column i of a lane; UNI: every array has the row stride s1u
+// LAY says how the arrays' strides are related. kLayOwn: each array has its own; kLayOne: all
+// share one (the defect-correction pool); kLayLoc: arrays at one location share theirs, which is
+// Chmy's dense layout and every layout that pads fields of one location alike. In 2D the location
+// class is 0 for Center along x (P, tau_dd, 1/eta, V.y) and 1 for Vertex along x (V.x, tau_xy). A
+// lane keeps one offset per class; with own strides each access takes its own multiplication and
+// the kernel 114 registers, 4 blocks per SM instead of 8. Measured at 2047 x 1535 FP32 in
+// the dense layout: 51.0 us per iteration with own strides, 39.9 us with class strides.
+constexpr int kLayOwn = 0, kLayOne = 1, kLayLoc = 2;
+struct MStr2 {
+    long s1[2];
+};
+template <class T, class Ix, int LAY>
+struct MAt {  // column i of a lane
     int i;
-    Ix s1u;
-    __device__ __forceinline__ Ix off(const DF<T>& f, int j) const { return (Ix)i + (Ix)j * (UNI ? s1u : (Ix)f.s1); }
-    __device__ __forceinline__ T ld(const DF<T>& f, int j, bool ok) const { return ok ? __ldg(f.p + off(f, j)) : T(0); }
-    __device__ __forceinline__ void st(const DF<T>& f, int j, T v) const { f.p[off(f, j)] = v; }
+    Ix s1[2];
+    __device__ __forceinline__ MAt(int i_, const MStr2& m) : i(i_), s1{(Ix)m.s1[0], (Ix)m.s1[LAY == kLayLoc ? 1 : 0]} {}
+    // c: the array's location class
+    __device__ __forceinline__ Ix off(int c, const DF<T>& f, int j) const {
+        return (Ix)i + (Ix)j * (LAY == kLayOwn ? (Ix)f.s1 : s1[LAY == kLayLoc ? c : 0]);
+    }
+    __device__ __forceinline__ T ld(int c, const DF<T>& f, int j, bool ok) const {
+        return ok ? __ldg(f.p + off(c, f, j)) : T(0);
+    }
+    __device__ __forceinline__ void st(int c, const DF<T>& f, int j, T v) const { f.p[off(c, f, j)] = v; }
 };
 
 // Inputs of one marching step at column i: row j+1 of the vertex-row inputs, row j of the
@@ -621,26 +638,26 @@ struct MarchRow {
     T P, txx, tyy, txo, tyo, fp, rhox, rhoy;  // row j
 };
 
-template <class T, class Ix, bool UNI>
-__device__ __forceinline__ MarchRow<T> march_load(const Fused2D<T>& f, const MAt<T, Ix, UNI>& at, int j, int e1,
+template <class T, class Ix, int LAY>
+__device__ __forceinline__ MarchRow<T> march_load(const Fused2D<T>& f, const MAt<T, Ix, LAY>& at, int j, int e1,
                                                   bool inV, bool inC) {
     MarchRow<T> r;
     const int jn = j + 1;
     const bool vn = inV && jn <= e1 + 1;
-    r.Vx = at.ld(f.Vx_in, jn, vn);
-    r.Vy = at.ld(f.Vy_in, jn, vn);
-    r.ie = at.ld(f.ieta, jn, vn);
-    r.txy = at.ld(f.txy_in, jn, vn);
-    r.txyo = at.ld(f.txy_o, jn, inC && jn <= e1);
+    r.Vx = at.ld(1, f.Vx_in, jn, vn);
+    r.Vy = at.ld(0, f.Vy_in, jn, vn);
+    r.ie = at.ld(0, f.ieta, jn, vn);
+    r.txy = at.ld(1, f.txy_in, jn, vn);
+    r.txyo = at.ld(1, f.txy_o, jn, inC && jn <= e1);
     const bool c = inC && j <= e1;
-    r.P = at.ld(f.P_in, j, c);
-    r.txx = at.ld(f.txx_in, j, c);
-    r.tyy = at.ld(f.tyy_in, j, c);
-    r.txo = at.ld(f.txx_o, j, c);
-    r.tyo = at.ld(f.tyy_o, j, c);
-    r.fp = f.has_fP ? at.ld(f.fP, j, c) : T(0);
-    r.rhox = f.has_rho ? at.ld(f.rhox, j, c) : T(0);
-    r.rhoy = f.has_rho ? at.ld(f.rhoy, j, c) : T(0);
+    r.P = at.ld(0, f.P_in, j, c);
+    r.txx = at.ld(0, f.txx_in, j, c);
+    r.tyy = at.ld(0, f.tyy_in, j, c);
+    r.txo = at.ld(0, f.txx_o, j, c);
+    r.tyo = at.ld(0, f.tyy_o, j, c);
+    r.fp = f.has_fP ? at.ld(0, f.fP, j, c) : T(0);
+    r.rhox = f.has_rho ? at.ld(1, f.rhox, j, c) : T(0);
+    r.rhoy = f.has_rho ? at.ld(0, f.rhoy, j, c) : T(0);
     return r;
 }
 
@@ -728,9 +745,9 @@ __device__ __forceinline__ T march_vertex(const SP<T>& s, T vx0, T vx1, T vyl, T
     return radd(t2, rmul(rmul(stress_res(s, t2, o2, iev, exy), eve), s.dtau_r));
 }
 
-template <class T, class Ix, bool UNI, bool WRITE_RES, int MINB = 1>
+template <class T, class Ix, int LAY, bool WRITE_RES, int MINB = 1>
 __global__ void __launch_bounds__(128, MINB) march2d_kernel(const Fused2D<T> f, const SP<T> s, int e0, int e1,
-                                                            int nstrip, int nwarps, int seg_rows, long s1u) {
+                                                            int nstrip, int nwarps, int seg_rows, const MStr2 str) {
     constexpr unsigned FULL = 0xffffffffu;
     cg_dep_wait();
     cg_dep_release();
@@ -742,7 +759,7 @@ __global__ void __launch_bounds__(128, MINB) march2d_kernel(const Fused2D<T> f, 
     if (js > e1) return;  // whole warp
     const int je = min(js + seg_rows - 1, e1);
     const int i = strip * 30 - 1 + lane;
-    const MAt<T, Ix, UNI> at{i, (Ix)s1u};
+    const MAt<T, Ix, LAY> at(i, str);
     const bool own = lane >= 1 && lane <= 30 && i <= e0;
     const bool inV = i <= e0 + 1;  // V, 1/eta, tau_xy readable
     const bool inC = i <= e0;      // cell inputs, tau_xy_old readable
@@ -760,18 +777,18 @@ __global__ void __launch_bounds__(128, MINB) march2d_kernel(const Fused2D<T> f, 
     MarchRow<T> cur;
     {
         const int jp = js - 1;  // >= -1
-        T vxp = at.ld(f.Vx_in, jp, inV);
-        T vyp = at.ld(f.Vy_in, jp, inV);
-        const T iep = at.ld(f.ieta, jp, inV);
-        const T pp = at.ld(f.P_in, jp, inC);
-        const T typ = at.ld(f.tyy_in, jp, inC);
-        const T tyop = at.ld(f.tyy_o, jp, inC);
-        const T fpp = f.has_fP ? at.ld(f.fP, jp, inC) : T(0);
-        Vx_c = at.ld(f.Vx_in, js, inV);
-        Vy_c = at.ld(f.Vy_in, js, inV);
-        ie_c = at.ld(f.ieta, js, inV);
-        const T t2 = at.ld(f.txy_in, js, inV);
-        const T o2 = at.ld(f.txy_o, js, inC);
+        T vxp = at.ld(1, f.Vx_in, jp, inV);
+        T vyp = at.ld(0, f.Vy_in, jp, inV);
+        const T iep = at.ld(0, f.ieta, jp, inV);
+        const T pp = at.ld(0, f.P_in, jp, inC);
+        const T typ = at.ld(0, f.tyy_in, jp, inC);
+        const T tyop = at.ld(0, f.tyy_o, jp, inC);
+        const T fpp = f.has_fP ? at.ld(0, f.fP, jp, inC) : T(0);
+        Vx_c = at.ld(1, f.Vx_in, js, inV);
+        Vy_c = at.ld(0, f.Vy_in, js, inV);
+        ie_c = at.ld(0, f.ieta, js, inV);
+        const T t2 = at.ld(1, f.txy_in, js, inV);
+        const T o2 = at.ld(1, f.txy_o, js, inC);
         // the first marching step's loads (row js+1) are issued before the prologue computes
         cur = march_load(f, at, js, e1, inV, inC);
         if (yb) {
@@ -802,7 +819,7 @@ __global__ void __launch_bounds__(128, MINB) march2d_kernel(const Fused2D<T> f, 
         const T iepL = __shfl_up_sync(FULL, iep, 1);
         ieL_c = __shfl_up_sync(FULL, ie_c, 1);
         txy_c = (i > e0) ? t2 : march_vertex(s, vxp, Vx_c, vyL, Vy_c, iepL, iep, ieL_c, ie_c, t2, o2);
-        if (own) at.st(f.txy_out, js, txy_c);
+        if (own) at.st(1, f.txy_out, js, txy_c);
         ie_p = iep;
     }
 
@@ -847,17 +864,17 @@ __global__ void __launch_bounds__(128, MINB) march2d_kernel(const Fused2D<T> f, 
                 rx = rsub(rx, cur.rhox);
                 ry = rsub(ry, cur.rhoy);
             }
-            at.st(f.P_out, j, c.P);
-            at.st(f.txx_out, j, c.txx);
-            at.st(f.tyy_out, j, c.tyy);
-            if (j + 1 <= je) at.st(f.txy_out, j + 1, tn);
+            at.st(0, f.P_out, j, c.P);
+            at.st(0, f.txx_out, j, c.txx);
+            at.st(0, f.tyy_out, j, c.tyy);
+            if (j + 1 <= je) at.st(1, f.txy_out, j + 1, tn);
             if (WRITE_RES) {
-                at.st(f.divV, j, c.dvP);
-                at.st(f.rVx, j, rx);
-                at.st(f.rVy, j, ry);
+                at.st(0, f.divV, j, c.dvP);
+                at.st(1, f.rVx, j, rx);
+                at.st(0, f.rVy, j, ry);
             }
-            at.st(f.Vx_out, j, radd(Vx_c, rmul(rx, rmul(s.nu_dtau, radd(fmin(ieL_c, ie_c), s.inv_Gdt)))));
-            at.st(f.Vy_out, j, radd(Vy_c, rmul(ry, rmul(s.nu_dtau, radd(fmin(ie_p, ie_c), s.inv_Gdt)))));
+            at.st(1, f.Vx_out, j, radd(Vx_c, rmul(rx, rmul(s.nu_dtau, radd(fmin(ieL_c, ie_c), s.inv_Gdt)))));
+            at.st(0, f.Vy_out, j, radd(Vy_c, rmul(ry, rmul(s.nu_dtau, radd(fmin(ie_p, ie_c), s.inv_Gdt)))));
         }
         // advance one row
         Vx_c = cur.Vx;
@@ -965,9 +982,9 @@ __device__ __forceinline__ MStep<T> x2_step(const Fused2D<T>& f, const SP<T>& s,
     return o;
 }
 
-template <class T, class Ix, bool UNI, bool WRITE_RES, int MINB = 1>
+template <class T, class Ix, int LAY, bool WRITE_RES, int MINB = 1>
 __global__ void __launch_bounds__(128, MINB) march2d_x2_kernel(const Fused2D<T> f, const SP<T> s, int e0, int e1,
-                                                               int nstrip, int nwarps, int seg_rows, long s1u,
+                                                               int nstrip, int nwarps, int seg_rows, const MStr2 str,
                                                                int fold_a) {
     constexpr unsigned FULL = 0xffffffffu;
     cg_dep_wait();
@@ -980,7 +997,7 @@ __global__ void __launch_bounds__(128, MINB) march2d_x2_kernel(const Fused2D<T> 
     if (js > e1) return;  // whole warp
     const int je = min(js + seg_rows - 1, e1);
     const int i = strip * 28 - 2 + lane;  // >= -2: column -2 lies outside the arrays, never read
-    const MAt<T, Ix, UNI> at{i, (Ix)s1u};
+    const MAt<T, Ix, LAY> at(i, str);
     const bool own = lane >= 2 && lane <= 29 && i <= e0;
     const bool inV = i >= -1 && i <= e0 + 1;  // V, 1/eta, tau_xy readable
     const bool inC = i >= -1 && i <= e0;      // cell inputs, tau_xy_old readable
@@ -1002,9 +1019,9 @@ __global__ void __launch_bounds__(128, MINB) march2d_x2_kernel(const Fused2D<T> 
     {
         const int j0 = js - 2;
         const bool ok = j0 >= -1;
-        a.Vx = at.ld(f.Vx_in, j0, inV && ok);
-        a.Vy = at.ld(f.Vy_in, j0, inV && ok);
-        a.ie = at.ld(f.ieta, j0, inV && ok);
+        a.Vx = at.ld(1, f.Vx_in, j0, inV && ok);
+        a.Vy = at.ld(0, f.Vy_in, j0, inV && ok);
+        a.ie = at.ld(0, f.ieta, j0, inV && ok);
         if (xa && j0 >= 0) {
             a.Vx = fold_x(f.bc, 0, i, a.Vx);
             a.Vy = fold_x(f.bc, 1, i, a.Vy);
@@ -1031,14 +1048,14 @@ __global__ void __launch_bounds__(128, MINB) march2d_x2_kernel(const Fused2D<T> 
         MarchRow<T> cb;
         if (bstep) {
             const int jn = jb + 1;
-            cb.ie = at.ld(f.ieta, jn, inV && jn <= e1 + 1);
-            cb.txyo = at.ld(f.txy_o, jn, inC && jn <= e1);
+            cb.ie = at.ld(0, f.ieta, jn, inV && jn <= e1 + 1);
+            cb.txyo = at.ld(1, f.txy_o, jn, inC && jn <= e1);
             const bool c = inC && jb <= e1;
-            cb.txo = at.ld(f.txx_o, jb, c);
-            cb.tyo = at.ld(f.tyy_o, jb, c);
-            cb.fp = f.has_fP ? at.ld(f.fP, jb, c) : T(0);
-            cb.rhox = f.has_rho ? at.ld(f.rhox, jb, c) : T(0);
-            cb.rhoy = f.has_rho ? at.ld(f.rhoy, jb, c) : T(0);
+            cb.txo = at.ld(0, f.txx_o, jb, c);
+            cb.tyo = at.ld(0, f.tyy_o, jb, c);
+            cb.fp = f.has_fP ? at.ld(0, f.fP, jb, c) : T(0);
+            cb.rhox = f.has_rho ? at.ld(1, f.rhox, jb, c) : T(0);
+            cb.rhoy = f.has_rho ? at.ld(0, f.rhoy, jb, c) : T(0);
         }
         MStep<T> oa;
         if (astep) {
@@ -1054,7 +1071,7 @@ __global__ void __launch_bounds__(128, MINB) march2d_x2_kernel(const Fused2D<T> 
                 b.Vx = fold_x(f.bc, 0, i, b.Vx);
                 b.Vy = fold_x(f.bc, 1, i, b.Vy);
             }
-            b.ie = at.ld(f.ieta, ja, inV);
+            b.ie = at.ld(0, f.ieta, ja, inV);
             b.ieL = __shfl_up_sync(FULL, b.ie, 1);
         }
         if (bstep) {
@@ -1068,19 +1085,19 @@ __global__ void __launch_bounds__(128, MINB) march2d_x2_kernel(const Fused2D<T> 
             const MStep<T> ob = x2_step(f, s, b, cb, oa.vx, oa.vy, i, jb, e0, e1, xb, yb, ylo, yhi);
             if (own) {
                 if (jb >= js) {
-                    at.st(f.P_out, jb, ob.c.P);
-                    at.st(f.txx_out, jb, ob.c.txx);
-                    at.st(f.tyy_out, jb, ob.c.tyy);
-                    if (jb + 1 <= je) at.st(f.txy_out, jb + 1, ob.tn);
+                    at.st(0, f.P_out, jb, ob.c.P);
+                    at.st(0, f.txx_out, jb, ob.c.txx);
+                    at.st(0, f.tyy_out, jb, ob.c.tyy);
+                    if (jb + 1 <= je) at.st(1, f.txy_out, jb + 1, ob.tn);
                     if (WRITE_RES) {
-                        at.st(f.divV, jb, ob.c.dvP);
-                        at.st(f.rVx, jb, ob.rx);
-                        at.st(f.rVy, jb, ob.ry);
+                        at.st(0, f.divV, jb, ob.c.dvP);
+                        at.st(1, f.rVx, jb, ob.rx);
+                        at.st(0, f.rVy, jb, ob.ry);
                     }
-                    at.st(f.Vx_out, jb, ob.vx);
-                    at.st(f.Vy_out, jb, ob.vy);
+                    at.st(1, f.Vx_out, jb, ob.vx);
+                    at.st(0, f.Vy_out, jb, ob.vy);
                 } else {
-                    at.st(f.txy_out, js, ob.tn);  // vertex row js, computed by B's first row
+                    at.st(1, f.txy_out, js, ob.tn);  // vertex row js, computed by B's first row
                 }
             }
         }
@@ -1117,29 +1134,29 @@ inline bool march_fits_int(const Fused2D<T>& f, int e0, int e1) {
     return true;
 }
 
-// The row stride shared by every present array of f, or 0 when they differ.
+// The layout of a view's present arrays and their row strides by location class.
 template <class T>
-inline long march_uniform_stride(const Fused2D<T>& f) {
-    const DF<T>* all[22];
-    fused_arrays(f, all);
-    long s1 = 0;
-    for (const DF<T>* d : all) {
-        if (!d->p) continue;
-        if (s1 == 0) s1 = d->s1;
-        else if (d->s1 != s1) return 0;
-    }
-    return s1;
+inline int march_layout(const Fused2D<T>& f, MStr2* str) {
+    const DF<T>* const c0[15] = {&f.P_in, &f.P_out, &f.txx_in, &f.txx_out, &f.tyy_in, &f.tyy_out, &f.txx_o, &f.tyy_o,
+                                 &f.ieta, &f.fP, &f.Vy_in, &f.Vy_out, &f.rhoy, &f.divV, &f.rVy};
+    const DF<T>* const c1[7] = {&f.Vx_in, &f.Vx_out, &f.txy_in, &f.txy_out, &f.txy_o, &f.rhox, &f.rVx};
+    *str = MStr2{{f.P_in.s1, f.Vx_in.s1}};
+    for (const DF<T>* d : c0)
+        if (d->p && d->s1 != str->s1[0]) return kLayOwn;
+    for (const DF<T>* d : c1)
+        if (d->p && d->s1 != str->s1[1]) return kLayOwn;
+    return str->s1[0] == str->s1[1] ? kLayOne : kLayLoc;
 }
 
 // Rows per warp of the marching kernel: the length at which the strips x segments warps fill
 // every SM once at the kernel's occupancy (one wave), kept within [8, 32] rows. Shorter
 // segments re-read more boundary rows; longer ones leave the memory system fewer warps'
 // worth of loads in flight (measured on 1024^2 to 4096^2 grids).
-template <class T, class Ix, bool UNI, bool WRITE_RES, int MINB = 1>
+template <class T, class Ix, int LAY, bool WRITE_RES, int MINB = 1>
 inline int march_seg_rows(int num_sms, int nstrip, int rows) {
     static const int blocks_per_sm = [] {
         int nb = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, march2d_kernel<T, Ix, UNI, WRITE_RES, MINB>, 128,
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, march2d_kernel<T, Ix, LAY, WRITE_RES, MINB>, 128,
                                                           0) != cudaSuccess)
             nb = 0;
         return nb > 0 ? nb : 4;
@@ -1150,16 +1167,16 @@ inline int march_seg_rows(int num_sms, int nstrip, int rows) {
     return seg < 8 ? 8 : (seg > 32 ? 32 : seg);
 }
 
-template <class T, class Ix, bool UNI, bool WRITE_RES, int MINB = 1>
+template <class T, class Ix, int LAY, bool WRITE_RES, int MINB = 1>
 inline cudaError_t launch_march2d_ix(const Fused2D<T>& f, const SP<T>& s, int n0, int n1, int num_sms, int seg_rows,
-                                     long s1u, cudaStream_t st, bool dep = false) {
+                                     const MStr2& str, cudaStream_t st, bool dep = false) {
     const int e0 = n0 + 1, e1 = n1 + 1;
     const int nstrip = cg_div_up(e0 + 1, 30);
-    if (seg_rows <= 0) seg_rows = march_seg_rows<T, Ix, UNI, WRITE_RES, MINB>(num_sms, nstrip, e1 + 1);
+    if (seg_rows <= 0) seg_rows = march_seg_rows<T, Ix, LAY, WRITE_RES, MINB>(num_sms, nstrip, e1 + 1);
     const int nseg = cg_div_up(e1 + 1, seg_rows);
     const int nwarps = nstrip * nseg;
-    return cg_launch(march2d_kernel<T, Ix, UNI, WRITE_RES, MINB>, dim3(cg_div_up(nwarps, 4)), dim3(128), 0, st, dep, f,
-                     s, e0, e1, nstrip, nwarps, seg_rows, s1u);
+    return cg_launch(march2d_kernel<T, Ix, LAY, WRITE_RES, MINB>, dim3(cg_div_up(nwarps, 4)), dim3(128), 0, st, dep, f,
+                     s, e0, e1, nstrip, nwarps, seg_rows, str);
 }
 
 // Launch of the warp-marching kernel over [0, n0+1] x [0, n1+1]; seg_rows <= 0 picks the
@@ -1167,15 +1184,15 @@ inline cudaError_t launch_march2d_ix(const Fused2D<T>& f, const SP<T>& s, int n0
 template <class T, bool WRITE_RES>
 inline cudaError_t launch_march2d(const Fused2D<T>& f, const SP<T>& s, int n0, int n1, int num_sms, int seg_rows,
                                   cudaStream_t st, bool dep = false) {
-    const long s1u = march_uniform_stride(f);
-    // FP32 with one shared stride fits in 64 registers without spills: 8 blocks (32 warps) per SM
+    MStr2 str;
+    const int lay = march_layout(f, &str);
+    // FP32 with shared or class strides fits in 64 registers without spills: 8 blocks (32 warps) per SM
     constexpr int minb = sizeof(T) == 4 ? 8 : 1;
-    if (march_fits_int(f, n0 + 1, n1 + 1)) {
-        if (s1u) return launch_march2d_ix<T, int, true, WRITE_RES, minb>(f, s, n0, n1, num_sms, seg_rows, s1u, st, dep);
-        return launch_march2d_ix<T, int, false, WRITE_RES>(f, s, n0, n1, num_sms, seg_rows, 0, st, dep);
-    }
-    if (s1u) return launch_march2d_ix<T, long, true, WRITE_RES>(f, s, n0, n1, num_sms, seg_rows, s1u, st, dep);
-    return launch_march2d_ix<T, long, false, WRITE_RES>(f, s, n0, n1, num_sms, seg_rows, 0, st, dep);
+    if (!march_fits_int(f, n0 + 1, n1 + 1))
+        return launch_march2d_ix<T, long, kLayOwn, WRITE_RES>(f, s, n0, n1, num_sms, seg_rows, str, st, dep);
+    if (lay == kLayOne) return launch_march2d_ix<T, int, kLayOne, WRITE_RES, minb>(f, s, n0, n1, num_sms, seg_rows, str, st, dep);
+    if (lay == kLayLoc) return launch_march2d_ix<T, int, kLayLoc, WRITE_RES, minb>(f, s, n0, n1, num_sms, seg_rows, str, st, dep);
+    return launch_march2d_ix<T, int, kLayOwn, WRITE_RES>(f, s, n0, n1, num_sms, seg_rows, str, st, dep);
 }
 
 // Launch of the two-iteration kernel (march2d_x2_kernel) over [0, n0+1] x [0, n1+1]: two PT
@@ -1186,14 +1203,15 @@ inline cudaError_t launch_march2d(const Fused2D<T>& f, const SP<T>& s, int n0, i
 template <class T, bool WRITE_RES, int MINB>
 inline cudaError_t launch_march2d_x2_mb(const Fused2D<T>& f, const SP<T>& s, int n0, int n1, int num_sms, int seg_rows,
                                         bool fold_a, cudaStream_t st, bool dep) {
-    auto kern = march2d_x2_kernel<T, int, true, WRITE_RES, MINB>;
-    const long s1u = march_uniform_stride(f);
+    auto kern = march2d_x2_kernel<T, int, kLayOne, WRITE_RES, MINB>;
+    MStr2 str;
+    march_layout(f, &str);
     const int e0 = n0 + 1, e1 = n1 + 1;
     const int nstrip = cg_div_up(e0 + 1, 28);
     if (seg_rows <= 0) {
         static const int bps = [] {
             int nb = 0;
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, march2d_x2_kernel<T, int, true, WRITE_RES, MINB>, 128,
+            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, march2d_x2_kernel<T, int, kLayOne, WRITE_RES, MINB>, 128,
                                                               0) != cudaSuccess)
                 nb = 0;
             return nb > 0 ? nb : 4;
@@ -1206,7 +1224,7 @@ inline cudaError_t launch_march2d_x2_mb(const Fused2D<T>& f, const SP<T>& s, int
     if (seg_rows < 4) seg_rows = 4;  // no y-plane may lie on a stage's first row
     const int nseg = cg_div_up(e1 + 1, seg_rows);
     const int nwarps = nstrip * nseg;
-    return cg_launch(kern, dim3(cg_div_up(nwarps, 4)), dim3(128), 0, st, dep, f, s, e0, e1, nstrip, nwarps, seg_rows, s1u,
+    return cg_launch(kern, dim3(cg_div_up(nwarps, 4)), dim3(128), 0, st, dep, f, s, e0, e1, nstrip, nwarps, seg_rows, str,
                      (int)fold_a);
 }
 
@@ -1226,7 +1244,8 @@ inline bool march_x2_ok(const Fused2D<T>& f, int n0, int n1) {
         const char* e = std::getenv("CG_MARCH_X2");
         return !(e && e[0] == '0');
     }();
-    return on && march_uniform_stride(f) != 0 && march_fits_int(f, n0 + 1, n1 + 1);
+    MStr2 str;
+    return on && march_layout(f, &str) == kLayOne && march_fits_int(f, n0 + 1, n1 + 1);
 }
 
 }  // namespace cgk
