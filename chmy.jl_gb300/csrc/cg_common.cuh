@@ -37,8 +37,8 @@ struct cg_ctx {
     // slots: 0 thermal partner, 1 SIA D, 2 PT-diffusion partners, 3 SIA ensemble,
     // 4 PT-diffusion defect-correction pool, 5 SIA reverse step, 6 SIA reverse sweep over a tape,
     // 7 SIA ensemble reverse sweep, 8 explicit-diffusion reverse sweep, 9 thermal-step adjoint,
-    // 10 the wait flag of the TMA-fed PT-diffusion iteration
-    static constexpr int kScratchSlots = 11;
+    // 10 the wait flag of the TMA-fed kernels, 11 whether a 2D ping-pong pair's static points differ
+    static constexpr int kScratchSlots = 12;
     void* scratch[kScratchSlots] = {};
     size_t scratch_bytes[kScratchSlots] = {};
 };

@@ -2,6 +2,7 @@
 // examples/stokes_3d_inc_ve_T.jl:23-57, variable-viscosity form) as a z-marching kernel.
 #pragma once
 
+#include "cg_march2d_tile.cuh"
 #include "cg_stokes_kernels.cuh"
 
 namespace cgk {
@@ -15,11 +16,12 @@ struct Fused3D {
     int has_fP, has_rho[3];
 };
 
-// Row and plane strides of a view by location class (kLayOne: class 0 holds them). The class is 0 for cells in x and y (P, tau_dd, 1/eta, V.z), 1 for x faces (V.x, tau_xz), 2
-// for y faces (V.y, tau_yz) and 3 for xy edges (tau_xy). A thread then keeps one offset per class
-// instead of one multiplication pair per access: with own strides the kernel needs more than 80
-// registers and a few hundred integer instructions per plane. Measured at 192 x 160 x 176 FP32 in
-// the dense layout: 381 us per iteration with own strides, 191 us with class strides (8 rows at 3 blocks per SM).
+// Row and plane strides of a view by location class (kLayOne: class 0 holds them). The class is 0
+// for cells in x and y (P, tau_dd, 1/eta, V.z), 1 for x faces (V.x, tau_xz), 2 for y faces (V.y,
+// tau_yz) and 3 for xy edges (tau_xy). A thread then keeps one offset per class instead of one
+// multiplication pair per access: with own strides the kernel needs more than 80 registers and a few
+// hundred integer instructions per plane. Measured at 192 x 160 x 176 FP32 in the dense layout: 381 us
+// per iteration with own strides, 191 us with class strides (8 rows at 3 blocks per SM).
 struct MStr {
     int s1[4], s2[4];
 };
@@ -498,14 +500,14 @@ inline cudaError_t launch_march3d(const Fused3D<T>& f, const SP<T>& s, int n0, i
 // captured. Only the `out` buffers of the ping-pong view are written (the first real iteration
 // writes them again); the residual outputs are not touched. Results are cached per shape,
 // precision and layout for the process.
-// 2D candidates: variant 0 is march2d_kernel (one iteration per launch), variants 1 and 2 the
-// two-iteration march2d_x2_kernel at 4 and 5 blocks per SM (when march_x2_ok); the time
-// compared is per iteration.
+// 2D candidates: variant 0 is march2d_kernel (one iteration per launch, 7 segment lengths), variants
+// 1 and up march2d_tile_kernel's shapes (when march_tile_ok); the time compared is per iteration.
 template <class T>
 inline cg_tune_cfg tune_march2d(const Fused2D<T>& f, const SP<T>& s, int n0, int n1, int nsm, cudaStream_t st) {
     cg_tune_cfg best{0, 0};
+    const bool tile = march_tile_ok(f, n0, n1);
     if (cg_tune_forced(&best)) {
-        if (best.variant > 2 || (best.variant >= 1 && !march_x2_ok(f, n0, n1))) best.variant = 0;
+        if (best.variant > kTileVariants || !tile) best.variant = 0;
         return best;
     }
     if (!cg_autotune_enabled()) return best;
@@ -517,7 +519,7 @@ inline cg_tune_cfg tune_march2d(const Fused2D<T>& f, const SP<T>& s, int n0, int
     cg_key_add(key, march_layout(f, &str));
     cg_key_add(key, str);
     cg_key_add(key, nsm);
-    cg_key_add(key, (int)march_x2_ok(f, n0, n1));
+    cg_key_add(key, (int)tile);
     if (cg_tune_lookup(key, &best)) return best;
     float tbest = 1e30f;
     for (int seg : {0, 8, 16, 24, 32, 48, 64}) {
@@ -530,21 +532,21 @@ inline cg_tune_cfg tune_march2d(const Fused2D<T>& f, const SP<T>& s, int n0, int
             best = cg_tune_cfg{seg, 0};
         }
     }
-    if (march_x2_ok(f, n0, n1))
-        for (int v : {1, 2})
-            for (int seg : {0, 16, 32, 48, 64, 96}) {
-                if (seg > n1 + 2) continue;
-                float t = time_launches(
-                    [&] { return launch_march2d_x2<T, false>(f, s, n0, n1, nsm, seg, true, st, false, v); }, st);
-                if (t >= 0.f) t *= 0.5f;  // per iteration
-                if (cg_tune_verbose())
-                    std::fprintf(stderr, "march2d tune %dx%d: two iterations per pass (variant %d), seg %d: %.1f us per iteration\n",
-                                 n0, n1, v, seg, t >= 0.f ? 1e3f * t / 3 : -1.f);
-                if (t >= 0.f && t < tbest) {
-                    tbest = t;
-                    best = cg_tune_cfg{seg, v};
-                }
+    if constexpr (sizeof(T) == 4) {
+        for (int v = 1; tile && v <= kTileVariants; ++v) {
+            const int kit = kTileIters[v - 1];
+            float t = time_launches(
+                [&] { return launch_march2d_tile<T, false>(f, s, n0, n1, v, kit, true, TileStatic<T>{nullptr, 0}, st); }, st);
+            if (t >= 0.f) t /= (float)kit;
+            if (cg_tune_verbose())
+                std::fprintf(stderr, "march2d tune %dx%d: tiles, variant %d, %d iterations: %.2f us per iteration\n", n0, n1, v, kit,
+                             t >= 0.f ? 1e3f * t / 3 : -1.f);
+            if (t >= 0.f && t < tbest) {
+                tbest = t;
+                best = cg_tune_cfg{0, v};
             }
+        }
+    }
     cudaGetLastError();
     cg_tune_store(key, best);
     return best;

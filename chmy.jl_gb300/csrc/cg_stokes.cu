@@ -776,23 +776,40 @@ int pp_iterations_t(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* a, co
     std::memset(none, 0, sizeof(none));
     for (int d = 0; d < 2; ++d) cg_key_add(key, bc_V ? bc_V[d] : none[d]);
     cg_key_add(key, (int)fold);
-    // two iterations per pass (the tuner's variant 1) where no bc!(V) launch is needed between
-    // iterations: an even number of passes (a -> b, b -> a) leaves at least the last two
-    // iterations to the one-iteration kernel, so that a ends with the state after niter
-    // iterations and b with the state after niter - 1, as in the one-iteration form
-    const bool x2 = tc.variant >= 1 && (fold || !bc_V);
-    const int npass = x2 ? ((niter / 2 - 1) & ~1) : 0;
-    return cg_graph_run(ctx, key, [&](cudaStream_t st) {
-        for (int k = 0; k < npass; ++k) {
-            const Fused2D<T>& fk = (k % 2 == 0) ? fab : fba;
-            const int nsm = ctx->num_sms;
-            const bool last = 2 * k + 2 == niter;
-            const cudaError_t le = (res && last)
-                                       ? launch_march2d_x2<T, true>(fk, s, g->n[0], g->n[1], nsm, tc.seg, k > 0, st, k > 0, tc.variant)
-                                       : launch_march2d_x2<T, false>(fk, s, g->n[0], g->n[1], nsm, tc.seg, k > 0, st, k > 0, tc.variant);
-            if (le != cudaSuccess) return cg_fail(ctx, CG_ERR_CUDA, "fused2d x2 launch: %s", cudaGetErrorString(le));
+    // several iterations per launch (the tuner's variants 1 and up) where no bc!(V) launch is needed
+    // between iterations: an odd number of launches takes niter - 1 iterations a -> b -> a ... -> b
+    // and the one-iteration kernel the last b -> a, so that a ends with the state after niter
+    // iterations and b with the one after niter - 1, as in the one-iteration form
+    const bool tile = tc.variant >= 1 && (fold || !bc_V) && niter > 2;
+    int* differ = nullptr;
+    if constexpr (sizeof(T) == 4) {
+        if (tile) {
+            int rc = CG_OK;
+            differ = static_cast<int*>(cg_scratch(ctx, 11, 256, &rc));
+            if (rc) return rc;
+            static_differ_kernel<T><<<kDifferBlocks, 256, 0, ctx->stream>>>(fab, g->n[0] + 1, g->n[1] + 1, differ);
+            CG_CHECK_LAUNCH(ctx);
         }
-        for (int it = 2 * npass; it < niter; ++it) {
+    }
+    cg_key_add(key, differ);
+    return cg_graph_run(ctx, key, [&](cudaStream_t st) {
+        int first = 0;
+        if constexpr (sizeof(T) == 4) {
+            if (tile) {
+                const int kmax = kTileIters[tc.variant - 1];
+                const int m = cg_div_up(niter - 1, kmax) | 1;
+                for (int k = 0; k < m; ++k) {
+                    const int kit = (niter - 1) / m + (k < (niter - 1) % m ? 1 : 0);
+                    const Fused2D<T>& fk = (k % 2 == 0) ? fab : fba;
+                    const TileStatic<T> ts{differ, (first ^ k) & 1};
+                    const cudaError_t le =
+                        launch_march2d_tile<T, false>(fk, s, g->n[0], g->n[1], tc.variant, kit, k > 0, ts, st, k > 0);
+                    if (le != cudaSuccess) return cg_fail(ctx, CG_ERR_CUDA, "fused2d tile launch: %s", cudaGetErrorString(le));
+                    first += kit;
+                }
+            }
+        }
+        for (int it = first; it < niter; ++it) {
             const Fused2D<T>& fk = it == 0 ? fab0 : (it % 2 == 0) ? fab : fba;
             const int nsm = ctx->num_sms;
             const cudaError_t le = (res && it == niter - 1)

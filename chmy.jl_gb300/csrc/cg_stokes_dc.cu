@@ -541,27 +541,28 @@ int cg_stokes_solve_dc(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f,
     cg_key_add(key, tc);
     const bool staged = nd == 3 && tma.ok && tc.variant >= kM3TmaFirst;
     if (staged) cg_key_add(key, cg_tma_wait_cfg());
-    // two iterations per pass (the tuner's variant 1) where bc!(dV) is folded into the reads:
-    // passes alternate A -> B and B -> A, and an odd count of passes leaves its last two
-    // iterations to the one-iteration kernel, so that the chunk ends in A
-    const bool x2 = nd == 2 && fold && tc.variant >= 1;
-    const int npass = x2 ? (nchunk / 2) - ((nchunk / 2) & 1) : 0;
+    // several iterations per launch (the tuner's variants 1 and up) where bc!(dV) is folded into the
+    // reads: an even number of launches A -> B -> A, so that the chunk ends in A. The buffers of the
+    // pool agree outside the launch range (both are zero where no iteration writes).
+    const bool tile = nd == 2 && fold && tc.variant >= 1;
+    const int npass = tile ? (cg_div_up(nchunk, kTileIters[tc.variant - 1]) + 1) & ~1 : 0;
     auto chunk = [&]() {
         return cg_graph_run(ctx, key, [&](cudaStream_t st) {
             for (int k = 0; k < npass; ++k) {
-                const bool last = 2 * k + 2 == nchunk;
+                const bool last = k == npass - 1;
+                const int kit = nchunk / npass + (k < nchunk % npass ? 1 : 0);
                 const Fused2D<float>& fk = (k % 2 == 0) ? fa : fb;
-                const int nsm = ctx->num_sms;
+                const TileStatic<float> ts{nullptr, 0};
                 const cudaError_t le =
-                    last ? launch_march2d_x2<float, true>(fk, s32, g->n[0], g->n[1], nsm, tc.seg, k > 0, st, k > 0, tc.variant)
-                         : launch_march2d_x2<float, false>(fk, s32, g->n[0], g->n[1], nsm, tc.seg, k > 0, st, k > 0, tc.variant);
-                if (le != cudaSuccess) return cg_fail(ctx, CG_ERR_CUDA, "fused2d x2 launch: %s", cudaGetErrorString(le));
+                    last ? launch_march2d_tile<float, true>(fk, s32, g->n[0], g->n[1], tc.variant, kit, k > 0, ts, st, k > 0)
+                         : launch_march2d_tile<float, false>(fk, s32, g->n[0], g->n[1], tc.variant, kit, k > 0, ts, st, k > 0);
+                if (le != cudaSuccess) return cg_fail(ctx, CG_ERR_CUDA, "fused2d tile launch: %s", cudaGetErrorString(le));
                 if (last) {
                     int r = cg_bc_apply_impl(ctx, g, nd, w.dV, bc0, true);
                     if (r) return r;
                 }
             }
-            for (int it = 2 * npass; it < nchunk; ++it) {
+            for (int it = tile ? nchunk : 0; it < nchunk; ++it) {
                 const bool last = it == nchunk - 1;
                 if (nd == 2) {
                     const Fused2D<float>& fk = it == 0 ? fa0 : (it % 2 == 0) ? fa : fb;
