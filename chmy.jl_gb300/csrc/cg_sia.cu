@@ -9,9 +9,8 @@ namespace {
 
 template <class T>
 struct SiaV {
-    DF<T> H, B, qx, qy, D;
+    DF<T> H, B, qx, qy;
     T Gamma, As, beta, ela, m_max;
-    T Gn2, Asn;  // Gamma (n+2) and As n, for the taped derivatives of D
     T idx, idy;
     int n;
 };
@@ -21,34 +20,13 @@ __device__ __forceinline__ T S_at(const SiaV<T>& v, int i, int j) {
     return v.B(i, j, 0) + v.H(i, j, 0);
 }
 
-// ∇S at the cell's lower faces (a0, b0) and interpolated to the cell (ax, ay) (sia.jl:43-45)
-template <class T>
-__device__ __forceinline__ void grads_at(const SiaV<T>& v, int i, int j, T* a0, T* b0, T* ax, T* ay) {
-    const T s = S_at(v, i, j);
-    *a0 = (s - S_at(v, i - 1, j)) * v.idx;
-    const T a1 = (S_at(v, i + 1, j) - s) * v.idx;
-    *b0 = (s - S_at(v, i, j - 1)) * v.idy;
-    const T b1 = (S_at(v, i, j + 1) - s) * v.idy;
-    *ax = fma(T(0.5), a1 - *a0, *a0);
-    *ay = fma(T(0.5), b1 - *b0, *b0);
-}
-
 // D = (Gamma H^(n+2) + As H^n) vmag(∇S)^(n-1) at cell (i, j) (sia.jl:43-49)
 template <class T>
 __device__ __forceinline__ T D_at(const SiaV<T>& v, int i, int j) {
-    T a0, b0, ax, ay;
-    grads_at(v, i, j, &a0, &b0, &ax, &ay);
+    const T ax = cgsia::slope(S_at(v, i - 1, j), S_at(v, i + 1, j), T(0.5) * v.idx);
+    const T ay = cgsia::slope(S_at(v, i, j - 1), S_at(v, i, j + 1), T(0.5) * v.idy);
     return cgsia::D_cell(v.H(i, j, 0), ax, ay, v.Gamma, v.As, v.n);
 }
-
-// The tape arrays of one step, in H's layout (cgsia::TapeArray; the masks one byte per cell),
-// and its word block.
-template <class T>
-struct TapeV {
-    DF<T> a[cgsia::kArrays];
-    DF<unsigned char> fl;
-    cgsia::TapeWords* w;
-};
 
 using cgsia::bits_of;
 
@@ -72,109 +50,38 @@ __global__ void sia_q_kernel(const SiaV<T> v, int nx, int ny, unsigned long long
     if (dmax_bits) cgsia::block_max_bits(in ? bits_of(dc) : 0ull, dmax_bits);
 }
 
-// D over cells [0, n]^2 into v.D and max over the interior [1, n]^2. TAPE: v.D is the tape's
-// D, and the interior cells also record their lower faces' gradients and D's derivatives.
-template <class T, bool TAPE = false>
-__global__ void sia_D_kernel(const SiaV<T> v, int nx, int ny, unsigned long long* dmax_bits, const TapeV<T> tp) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const bool in = i <= nx && j <= ny;
-    T d = T(0);
-    if (in) {
-        T a0, b0, ax, ay;
-        grads_at(v, i, j, &a0, &b0, &ax, &ay);
-        const T h = v.H(i, j, 0);
-        if (TAPE) {
-            using namespace cgsia;
-            T dh, ex, ey, gf;
-            d = D_and_factors(h, ax, ay, v.Gamma, v.As, v.Gn2, v.Asn, v.n, &dh, &ex, &ey, &gf);
-            if (i >= 1 && j >= 1) {
-                tp.a[kGX](i, j, 0) = a0;
-                tp.a[kGY](i, j, 0) = b0;
-                tp.a[kDH](i, j, 0) = dh;
-                tp.a[kEX](i, j, 0) = ex;
-                tp.a[kEY](i, j, 0) = ey;
-                tp.a[kGF](i, j, 0) = gf;
-            }
-        } else {
-            d = cgsia::D_cell(h, ax, ay, v.Gamma, v.As, v.n);
-        }
-        v.D(i, j, 0) = d;
-    }
-    cgsia::block_max_bits(in && i >= 1 && j >= 1 ? bits_of(d) : 0ull, dmax_bits);
-}
-
-// update_q! from the precomputed D (same arithmetic as sia_q_kernel).
+// The kernels of a time step (cgsia::D_tile, cgsia::H_tile) on one member.
 template <class T>
-__global__ void sia_q_from_D_kernel(const SiaV<T> v, int nx, int ny) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-    if (i > nx || j > ny) return;
-    const T dc = v.D(i, j, 0), dl = v.D(i - 1, j, 0), dd = v.D(i, j - 1, 0);
-    const T Dx = fma(T(0.5), dc - dl, dl);
-    const T Dy = fma(T(0.5), dc - dd, dd);
-    const T sc = S_at(v, i, j);
-    v.qx(i, j, 0) = -Dx * ((sc - S_at(v, i - 1, j)) * v.idx);
-    v.qy(i, j, 0) = -Dy * ((sc - S_at(v, i, j - 1)) * v.idy);
+__global__ void sia_S_kernel(const cgsia::Member<T> v) {
+    cgsia::S_tile(v, blockIdx.x);
+}
+template <class T, bool TAPE>
+__global__ void __launch_bounds__(256) sia_D_kernel(const cgsia::Member<T> v, cgsia::Words* w, int par, char* sb) {
+    cg_dep_wait();
+    cg_dep_release();
+    cgsia::D_tile<T, TAPE>(v, w, blockIdx.x, par, sb);
+}
+template <class T, bool TAPE>
+__global__ void __launch_bounds__(256) sia_step_kernel(const cgsia::Member<T> v, cgsia::Words* w, int par, int last, char* sb) {
+    cg_dep_wait();
+    cg_dep_release();
+    cgsia::H_tile<T, TAPE, false>(v, w, blockIdx.x, par, last != 0, false, sb);
 }
 
-// update_H! over [1, n]^2; dt from a scalar or from device memory. TAPE: also W, the two
-// masks, and the first interior cell where D attains the step's maximum.
-template <class T, bool TAPE = false>
-__global__ void sia_H_kernel(const SiaV<T> v, int nx, int ny, T dt_scalar, const double* dt_dev, const TapeV<T> tp) {
+// update_H! over [1, n]^2.
+template <class T>
+__global__ void sia_H_kernel(const SiaV<T> v, int nx, int ny, T dt) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     if (i > nx || j > ny) return;
-    const T dt = dt_dev ? (T)*dt_dev : dt_scalar;
-    const T h = v.H(i, j, 0);
-    const T x = v.beta * (S_at(v, i, j) - v.ela);
-    const T m = fmin(x, v.m_max);
+    const T m = fmin(v.beta * (S_at(v, i, j) - v.ela), v.m_max);
     T dv = (v.qx(i + 1, j, 0) - v.qx(i, j, 0)) * v.idx;
     dv = dv + (v.qy(i, j + 1, 0) - v.qy(i, j, 0)) * v.idy;
-    const T W = -dv + m;
-    const T u = h + dt * W;
-    v.H(i, j, 0) = fmax(u, T(0.0));
-    if (TAPE) {
-        tp.a[cgsia::kW](i, j, 0) = W;
-        tp.fl(i, j, 0) = (unsigned char)((u > T(0) ? 1 : 0) + (x < v.m_max ? 2 : 0));
-        if (bits_of(v.D(i, j, 0)) == tp.w->dmax) atomicMin(&tp.w->arg, (unsigned long long)((long)j * (nx + 2) + i));
-    }
-}
-
-// Δt = min(min(Δ)^2 / max(D) / cfl, dt_max); t += Δt; reset the max slot for the next step.
-// `tw` (optional): the step's tape words.
-template <class T>
-__global__ void sia_dt_kernel(unsigned long long* dmax_bits, double* dt, double* t, double dx2, double cfl,
-                              double dt_max, cgsia::TapeWords* tw) {
-    const unsigned long long b = *dmax_bits;
-    double dmax;
-    if (sizeof(T) == 8) {
-        dmax = __longlong_as_double((long long)b);
-    } else {
-        dmax = (double)__int_as_float((int)(unsigned)b);
-    }
-    // Julia: Δ^2 / maximum(D) / 4.1 in the grid type
-    const T v = (T)dx2 / (T)dmax / (T)cfl;
-    double d = fmin((double)v, dt_max);
-    bool capped = !((double)v < dt_max);
-    if (!(dmax > 0.0)) {
-        d = dt_max;
-        capped = true;
-    }
-    *dt = d;
-    *t = *t + d;
-    if (tw) {
-        tw->dmax = b;
-        tw->arg = ~0ull;
-        tw->dt = d;
-        tw->capped = capped ? 1.0 : 0.0;
-    }
-    *dmax_bits = 0ull;
+    v.H(i, j, 0) = fmax(v.H(i, j, 0) + dt * (-dv + m), T(0.0));
 }
 
 template <class T>
-SiaV<T> make_view(const cg_grid* g, const cg_field* H, const cg_field* B, const cg_field* q, const cg_sia_params* p,
-                  void* D) {
+SiaV<T> make_view(const cg_grid* g, const cg_field* H, const cg_field* B, const cg_field* q, const cg_sia_params* p) {
     SiaV<T> v;
     std::memset(&v, 0, sizeof(v));
     v.H = cg_view<T>(*H);
@@ -183,17 +90,11 @@ SiaV<T> make_view(const cg_grid* g, const cg_field* H, const cg_field* B, const 
         v.qx = cg_view<T>(q[0]);
         v.qy = cg_view<T>(q[1]);
     }
-    if (D) {
-        v.D = v.H;  // same layout as H
-        v.D.p = static_cast<T*>(D) + cg_origin_offset(*H);
-    }
     v.Gamma = (T)p->Gamma;
     v.As = (T)p->As;
     v.beta = (T)p->beta;
     v.ela = (T)p->ela;
     v.m_max = (T)p->m_max;
-    v.Gn2 = v.Gamma * T(p->n + 2);
-    v.Asn = v.As * T(p->n);
     v.idx = (T)g->inv_spacing[0];
     v.idy = (T)g->inv_spacing[1];
     v.n = p->n;
@@ -227,7 +128,7 @@ void sia_bcs(cg_bc* qb, cg_bc* hb) {
 template <class T>
 int update_q_t(cg_ctx* ctx, const cg_grid* g, const cg_field* q, const cg_field* H, const cg_field* B,
                const cg_sia_params* p, double* dmax) {
-    const SiaV<T> v = make_view<T>(g, H, B, q, p, nullptr);
+    const SiaV<T> v = make_view<T>(g, H, B, q, p);
     const dim3 block(32, 8), grid(cg_div_up(g->n[0], 32), cg_div_up(g->n[1], 8));
     if (dmax) CG_CUDA(ctx, cudaMemsetAsync(ctx->d_red, 0, sizeof(unsigned long long), ctx->stream));
     sia_q_kernel<T><<<grid, block, 0, ctx->stream>>>(v, g->n[0], g->n[1], dmax ? ctx->d_red : nullptr);
@@ -247,9 +148,9 @@ int update_q_t(cg_ctx* ctx, const cg_grid* g, const cg_field* q, const cg_field*
 template <class T>
 int update_H_t(cg_ctx* ctx, const cg_grid* g, const cg_field* H, const cg_field* q, const cg_field* B, double dt,
                const cg_sia_params* p) {
-    const SiaV<T> v = make_view<T>(g, H, B, q, p, nullptr);
+    const SiaV<T> v = make_view<T>(g, H, B, q, p);
     const dim3 block(32, 8), grid(cg_div_up(g->n[0], 32), cg_div_up(g->n[1], 8));
-    sia_H_kernel<T><<<grid, block, 0, ctx->stream>>>(v, g->n[0], g->n[1], (T)dt, nullptr, TapeV<T>{});
+    sia_H_kernel<T><<<grid, block, 0, ctx->stream>>>(v, g->n[0], g->n[1], (T)dt);
     CG_CHECK_LAUNCH(ctx);
     cg_bc qb[2], hb;
     sia_bcs(qb, &hb);
@@ -259,25 +160,19 @@ int update_H_t(cg_ctx* ctx, const cg_grid* g, const cg_field* H, const cg_field*
 template <class T>
 int run_t(cg_ctx* ctx, const cg_grid* g, const cg_field* H, const cg_field* B, const cg_field* q,
           const cg_sia_params* p, int nsteps, double* t_host, char* tape = nullptr) {
-    // scratch: D (same padded layout as H) + 3 words (max bits, dt, t)
-    long cnt = 1;
-    for (int d = 0; d < 2; ++d) cnt *= (H->n[d] + 4L * H->halo[d]);
-    cnt = std::max<long>(cnt, (long)H->stride[1] * (H->n[1] + 4L * H->halo[1]));
+    // scratch: D and the two S buffers (H's padded layout) and the words
+    const size_t ab = cgsia::layout_bytes(*H, sizeof(T));
     int rc = CG_OK;
-    char* base = static_cast<char*>(cg_scratch(ctx, 1, cnt * sizeof(T) + 256 + 64, &rc));
+    char* base = static_cast<char*>(cg_scratch(ctx, 1, 3 * ab + 256, &rc));
     if (rc) return rc;
-    unsigned long long* words = reinterpret_cast<unsigned long long*>(base + ((cnt * sizeof(T) + 255) & ~255L));
-    double* dt = reinterpret_cast<double*>(words + 1);
-    double* t = reinterpret_cast<double*>(words + 2);
-    CG_CUDA(ctx, cudaMemsetAsync(words, 0, 3 * sizeof(unsigned long long), ctx->stream));
-    const SiaV<T> v = make_view<T>(g, H, B, q, p, base);
-    const int nx = g->n[0], ny = g->n[1];
+    cgsia::Words* words = reinterpret_cast<cgsia::Words*>(base + 3 * ab);
+    cgsia::Member<T> v = cgsia::make_member<T>(*g, *H, *B, q, *p, base, base + ab, base + 2 * ab);
+    const cgsia::TapeGeom tg = cgsia::tape_geom(*H, sizeof(T));
+    v.tab = (long long)tg.abytes;
+    v.orig = (long long)cg_origin_offset(*H);
     const dim3 block(32, 8);
-    const dim3 gD(cg_div_up(nx + 1, 32), cg_div_up(ny + 1, 8)), gI(cg_div_up(nx, 32), cg_div_up(ny, 8));
-    const double dx = std::min(g->spacing[0], g->spacing[1]);
-    const double dx2 = (double)((T)dx * (T)dx);
-    cg_bc qb[2], hb;
-    sia_bcs(qb, &hb);
+    const int nS = cg_div_up(v.nx + 2, 32) * cg_div_up(v.ny + 2, 8), nI = cg_div_up(v.nx, 32) * cg_div_up(v.ny, 8);
+    const int nH = cg_div_up(v.nx, cgsia::kHCols) * cg_div_up(v.ny, 8);
     std::string key = "sia_run";
     cg_key_add(key, *g);
     cg_key_add(key, *H);
@@ -288,44 +183,27 @@ int run_t(cg_ctx* ctx, const cg_grid* g, const cg_field* H, const cg_field* B, c
     cg_key_add(key, nsteps);
     cg_key_add(key, base);
     cg_key_add(key, tape);
-    const cgsia::TapeGeom tg = cgsia::tape_geom(*H, sizeof(T));
     rc = cg_graph_run(ctx, key, [&](cudaStream_t st) {
+        CG_CUDA(ctx, cudaMemsetAsync(words, 0, sizeof(cgsia::Words), st));
+        sia_S_kernel<T><<<nS, block, 0, st>>>(v);
+        CG_CHECK_LAUNCH(ctx);
         for (int s = 0; s < nsteps; ++s) {
-            SiaV<T> vs = v;
-            TapeV<T> tp{};
-            if (tape) {
-                char* sb = tape + 256 + (size_t)s * tg.step_bytes;
-                tp.w = reinterpret_cast<cgsia::TapeWords*>(sb);
-                for (int k = 0; k < cgsia::kArrays; ++k) {
-                    tp.a[k] = v.H;
-                    tp.a[k].p = reinterpret_cast<T*>(sb + 256 + (size_t)k * tg.abytes) + cg_origin_offset(*H);
-                }
-                tp.fl.p = reinterpret_cast<unsigned char*>(sb + 256 + (size_t)cgsia::kFL * tg.abytes) + cg_origin_offset(*H);
-                tp.fl.s1 = v.H.s1;
-                tp.fl.s2 = v.H.s2;
-                vs.D = tp.a[cgsia::kD];
-                sia_D_kernel<T, true><<<gD, block, 0, st>>>(vs, nx, ny, words, tp);
-            } else {
-                sia_D_kernel<T><<<gD, block, 0, st>>>(vs, nx, ny, words, tp);
-            }
-            sia_q_from_D_kernel<T><<<gI, block, 0, st>>>(vs, nx, ny);
-            CG_CHECK_LAUNCH(ctx);
-            int r = cg_bc_apply_impl(ctx, g, 2, q, qb);
-            if (r) return r;
-            sia_dt_kernel<T><<<1, 1, 0, st>>>(words, dt, t, dx2, p->cfl, p->dt_max, tp.w);
-            if (tape)
-                sia_H_kernel<T, true><<<gI, block, 0, st>>>(vs, nx, ny, T(0), dt, tp);
-            else
-                sia_H_kernel<T><<<gI, block, 0, st>>>(vs, nx, ny, T(0), dt, tp);
-            CG_CHECK_LAUNCH(ctx);
-            r = cg_bc_apply_impl(ctx, g, 1, H, &hb);
-            if (r) return r;
+            char* sb = tape ? tape + 256 + (size_t)s * tg.step_bytes : nullptr;
+            const int par = s & 1, last = s == nsteps - 1;
+            CG_CUDA(ctx, tape ? cg_launch(sia_D_kernel<T, true>, dim3(nI), block, 0, st, s > 0, v, words, par, sb)
+                              : cg_launch(sia_D_kernel<T, false>, dim3(nI), block, 0, st, s > 0, v, words, par, sb));
+            CG_CUDA(ctx, tape ? cg_launch(sia_step_kernel<T, true>, dim3(nH), block, 0, st, true, v, words, par, last, sb)
+                              : cg_launch(sia_step_kernel<T, false>, dim3(nH), block, 0, st, true, v, words, par, last, sb));
         }
-        return (int)CG_OK;
+        // the tangential points of bc! beyond the ghost layer (index n+2), which no step reads
+        cg_bc bcs[3];
+        sia_bcs(bcs, bcs + 2);
+        const cg_field fs[3] = {q[0], q[1], *H};
+        return cg_bc_apply_impl(ctx, g, 3, fs, bcs);
     });
     if (rc) return rc;
     if (t_host) {
-        CG_CUDA(ctx, cudaMemcpyAsync(t_host, t, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+        CG_CUDA(ctx, cudaMemcpyAsync(t_host, &words->t, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
         CG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     }
     return CG_OK;

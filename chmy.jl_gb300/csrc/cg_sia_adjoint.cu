@@ -65,29 +65,21 @@ __device__ __forceinline__ T S_of(const SiaAdj<T>& v, int i, int j) {
 
 template <class T>
 __device__ __forceinline__ void grads(const SiaAdj<T>& v, int i, int j, T* ax, T* ay) {
-    const T s = S_of(v, i, j);
-    const T a0 = (s - S_of(v, i - 1, j)) * v.idx;
-    const T a1 = (S_of(v, i + 1, j) - s) * v.idx;
-    const T b0 = (s - S_of(v, i, j - 1)) * v.idy;
-    const T b1 = (S_of(v, i, j + 1) - s) * v.idy;
-    *ax = fma(T(0.5), a1 - a0, a0);
-    *ay = fma(T(0.5), b1 - b0, b0);
+    *ax = cgsia::slope(S_of(v, i - 1, j), S_of(v, i + 1, j), T(0.5) * v.idx);
+    *ay = cgsia::slope(S_of(v, i, j - 1), S_of(v, i, j + 1), T(0.5) * v.idy);
 }
 
-// x-face flux at face f of row j, as cg_sia_run leaves it after bc!(q). The product is rounded
-// on its own (rmul), as the forward stores it: fused into the divergence's subtraction it would
-// round differently, and H + dt W could then fall on the other side of the max(., 0) kink.
+// x-face flux at face f of row j, with the forward's arithmetic (cgsia::face_flux): a differently
+// rounded flux could put H + dt W on the other side of the max(., 0) kink.
 template <class T>
 __device__ __forceinline__ T qx_at(const SiaAdj<T>& v, int f, int j) {
     if (f <= 1 || f >= v.nx + 1) return T(0);
-    const T dc = v.D(f, j, 0), dl = v.D(f - 1, j, 0);
-    return cgk::rmul(-fma(T(0.5), dc - dl, dl), (S_of(v, f, j) - S_of(v, f - 1, j)) * v.idx);
+    return cgsia::face_flux(v.D(f - 1, j, 0), v.D(f, j, 0), S_of(v, f - 1, j), S_of(v, f, j), T(0.5) * v.idx);
 }
 template <class T>
 __device__ __forceinline__ T qy_at(const SiaAdj<T>& v, int i, int f) {
     if (f <= 1 || f >= v.ny + 1) return T(0);
-    const T dc = v.D(i, f, 0), dl = v.D(i, f - 1, 0);
-    return cgk::rmul(-fma(T(0.5), dc - dl, dl), (S_of(v, i, f) - S_of(v, i, f - 1)) * v.idy);
+    return cgsia::face_flux(v.D(i, f - 1, 0), v.D(i, f, 0), S_of(v, i, f - 1), S_of(v, i, f), T(0.5) * v.idy);
 }
 
 // D at the interior cells and its maximum (the forward's Dmax)
@@ -171,12 +163,10 @@ __global__ void adj_mu_kernel(const SiaAdj<T> v, SiaWords* w, double* part, int 
     if (in) {
         const T dt = (T)w->dt;
         const T h = v.H(i, j, 0);
-        const T x = v.beta * (S_of(v, i, j) - v.ela);
-        const T m = fmin(x, v.m_max);
-        T dv = (qx_at(v, i + 1, j) - qx_at(v, i, j)) * v.idx;
-        dv = dv + (qy_at(v, i, j + 1) - qy_at(v, i, j)) * v.idy;
-        const T W = -dv + m;
-        const T u = h + dt * W;
+        const T x = cgk::rmul(v.beta, cgk::rsub(S_of(v, i, j), v.ela));
+        const T W = cgsia::rate(qx_at(v, i, j), qx_at(v, i + 1, j), qy_at(v, i, j), qy_at(v, i, j + 1), v.idx, v.idy,
+                                fmin(x, v.m_max));
+        const T u = cgk::rfma(dt, W, h);
         const T mu = u > T(0) ? v.lam(i, j, 0) : T(0);
         const T mM = x < v.m_max ? T(1) : T(0);
         v.mu(i, j, 0) = mu;

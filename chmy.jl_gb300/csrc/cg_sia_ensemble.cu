@@ -6,19 +6,11 @@
 // it is instead ONE persistent cooperative launch with grid barriers between the phases. Both
 // forms give the same bits. The graph is the default: on GB300 the tiles are bound by the FP64
 // pipe, so residency saves nothing, and a grid barrier costs more than a kernel boundary in a
-// replayed graph (64 members of 128^2..1024^2: 2.49 vs 2.41 ms per step; of 32^2..128^2:
-// 70 vs 62 us).
+// replayed graph (64 members of 128^2..1024^2: 1.89 vs 1.77 ms per step; of 32^2..128^2:
+// 49 vs 43 us).
 //
-// Boundary conditions are folded into the kernels with the values of the reference's bc!:
-// q.x => (x = Dirichlet()) writes 0 on the boundary faces i = 1, n+1 (q.y likewise), and
-// H => Neumann() copies the first interior value into the ghost layer, corners taking the
-// value of the diagonal interior cell (the x rule runs last and reads the y ghost).
-//
-// The step is bound by the FP64 pipe, so FP64 work is traded for memory traffic:
-// - S = B + H is kept per cell in a scratch array. The H kernel updates it with the new
-//   thickness, including the ghost layer; the cells beyond it never change.
-// - The D kernel hands its lower-face surface gradients to the q kernel through the q arrays.
-// Every value is the one the direct form computes, with the same operations in the same order.
+// A step is the two tile functions of cg_sia_kernels.cuh (the single-member run's too), with bc! folded
+// into them.
 #include <vector>
 
 #include "cg_common.cuh"
@@ -28,46 +20,8 @@ void* cg_scratch(cg_ctx* ctx, int slot, size_t bytes, int* rc);
 
 namespace {
 
-template <class T>
-struct Member {
-    DF<T> H, B, qx, qy, D, S;
-    T Gamma, As, beta, ela, m_max, idx, idy;
-    T Gn2, Asn;  // Gamma (n+2) and As n, for the taped derivatives of D
-    double dx2, cfl, dt_max;
-    int n, nx, ny;
-    int tiles_D, tiles_I;  // tiles of the [0, n] and [1, n] ranges (32 x blockDim.y each)
-    // taped runs: the member's tape block within a step's block (cgsia layout: 256 bytes of
-    // words, then kArrays arrays of `tab` bytes in H's layout, H's origin at element `orig`)
-    long long toff, tab, orig;
-};
-
-// The member's tape array k (cgsia::TapeArray) of the step whose block starts at `sb`.
-template <class T>
-__device__ __forceinline__ DF<T> tape_arr(const Member<T>& v, char* sb, int k) {
-    DF<T> a = v.H;
-    a.p = reinterpret_cast<T*>(sb + v.toff + 256 + (long long)k * v.tab) + v.orig;
-    return a;
-}
-template <class T>
-__device__ __forceinline__ DF<unsigned char> tape_flags(const Member<T>& v, char* sb) {
-    DF<unsigned char> a;
-    a.p = reinterpret_cast<unsigned char*>(sb + v.toff + 256 + (long long)cgsia::kFL * v.tab) + v.orig;
-    a.s1 = v.H.s1;
-    a.s2 = v.H.s2;
-    return a;
-}
-template <class T>
-__device__ __forceinline__ cgsia::TapeWords* tape_words(const Member<T>& v, char* sb) {
-    return reinterpret_cast<cgsia::TapeWords*>(sb + v.toff);
-}
-
-struct Words {
-    unsigned long long dmax;
-    double dt;
-    double t;
-    double pad;
-};
-
+using cgsia::Member;
+using cgsia::Words;
 using cgsia::bits_of;
 
 // The block's member descriptor, copied once into shared memory (every thread of the block
@@ -96,182 +50,53 @@ __device__ __forceinline__ int find_member(const int* prefix, int nm, int blk) {
     return lo;
 }
 
-template <class T, bool TAPE = false>
-__device__ __forceinline__ void ens_D_tile(const Member<T>* mem, const int* prefix, int nm, Words* w, int blk,
-                                           char* sb = nullptr) {
-    const int m = find_member(prefix, nm, blk);
-    const Member<T>& v = member_of(mem, m);
-    const int t = blk - (m ? prefix[m - 1] : 0);
-    const int tx = (v.nx + 1 + 31) / 32;
-    const int i = (t % tx) * 32 + threadIdx.x;
-    const int j = (t / tx) * (int)blockDim.y + threadIdx.y;
-    const bool in = i <= v.nx && j <= v.ny;
-    T d = T(0);
-    if (in) {
-        // ∇S at the cell's faces, interpolated to the cell; vmag and D (examples/sia.jl:43-49)
-        const T s = v.S(i, j, 0);
-        const T a0 = (s - v.S(i - 1, j, 0)) * v.idx;
-        const T a1 = (v.S(i + 1, j, 0) - s) * v.idx;
-        const T b0 = (s - v.S(i, j - 1, 0)) * v.idy;
-        const T b1 = (v.S(i, j + 1, 0) - s) * v.idy;
-        const T ax = fma(T(0.5), a1 - a0, a0);
-        const T ay = fma(T(0.5), b1 - b0, b0);
-        const T h = v.H(i, j, 0);
-        T dh, ex, ey, gf;
-        if (TAPE)
-            d = cgsia::D_and_factors(h, ax, ay, v.Gamma, v.As, v.Gn2, v.Asn, v.n, &dh, &ex, &ey, &gf);
-        else
-            d = cgsia::D_cell(h, ax, ay, v.Gamma, v.As, v.n);
-        v.D(i, j, 0) = d;
-        if (i >= 1 && j >= 1) {  // the lower faces' gradients, for the q kernel
-            v.qx(i, j, 0) = a0;
-            v.qy(i, j, 0) = b0;
-            if (TAPE) {
-                using namespace cgsia;
-                tape_arr(v, sb, kD)(i, j, 0) = d;
-                tape_arr(v, sb, kGX)(i, j, 0) = a0;
-                tape_arr(v, sb, kGY)(i, j, 0) = b0;
-                tape_arr(v, sb, kDH)(i, j, 0) = dh;
-                tape_arr(v, sb, kEX)(i, j, 0) = ex;
-                tape_arr(v, sb, kEY)(i, j, 0) = ey;
-                tape_arr(v, sb, kGF)(i, j, 0) = gf;
-            }
-        }
-    }
-    cgsia::block_max_bits(in && i >= 1 && j >= 1 ? bits_of(d) : 0ull, &w[m].dmax);
-}
-
-// S = B + H over [-1, n+1]^2 (the D kernel's stencil), once per run
+// A tile function on the tile of block `blk`: its member's descriptor in shared memory, and the
+// member's words. Neither the descriptors nor the prefix tables change within a run, so a kernel
+// launched as a dependent one finds its member (a binary search of dependent loads, 1 to 2 us) while
+// the kernel before it drains, and waits for it only then (DEP).
 template <class T>
 __device__ __forceinline__ void ens_S_tile(const Member<T>* mem, const int* prefix, int nm, int blk) {
     const int m = find_member(prefix, nm, blk);
-    const Member<T>& v = member_of(mem, m);
-    const int t = blk - (m ? prefix[m - 1] : 0);
-    const int tx = (v.nx + 3 + 31) / 32;
-    const int i = (t % tx) * 32 + threadIdx.x - 1;
-    const int j = (t / tx) * (int)blockDim.y + threadIdx.y - 1;
-    if (i > v.nx + 1 || j > v.ny + 1) return;
-    v.S(i, j, 0) = v.B(i, j, 0) + v.H(i, j, 0);
+    cgsia::S_tile(member_of(mem, m), blk - (m ? prefix[m - 1] : 0));
 }
-
-template <class T>
-__device__ __forceinline__ void ens_q_tile(const Member<T>* mem, const int* prefix, int nm, int blk) {
+template <class T, bool TAPE, bool DEP>
+__device__ __forceinline__ void ens_D_tile(const Member<T>* mem, const int* prefix, int nm, Words* w, int blk, int par, char* sb) {
     const int m = find_member(prefix, nm, blk);
     const Member<T>& v = member_of(mem, m);
     const int t = blk - (m ? prefix[m - 1] : 0);
-    const int tx = (v.nx + 31) / 32;
-    const int i = (t % tx) * 32 + threadIdx.x + 1;
-    const int j = (t / tx) * (int)blockDim.y + threadIdx.y + 1;
-    if (i > v.nx || j > v.ny) return;
-    const T dc = v.D(i, j, 0), dl = v.D(i - 1, j, 0), dd = v.D(i, j - 1, 0);
-    const T Dx = fma(T(0.5), dc - dl, dl);
-    const T Dy = fma(T(0.5), dc - dd, dd);
-    // q = -lerp(D) ∂S with ∂S left in q by the D kernel; bc!(q.x => (x = Dirichlet())): the
-    // boundary faces i = 1 and n+1 are 0 (q.y likewise)
-    v.qx(i, j, 0) = i == 1 ? T(0) : -Dx * v.qx(i, j, 0);
-    v.qy(i, j, 0) = j == 1 ? T(0) : -Dy * v.qy(i, j, 0);
-    if (i == v.nx) v.qx(i + 1, j, 0) = T(0);
-    if (j == v.ny) v.qy(i, j + 1, 0) = T(0);
+    if (DEP) cg_dep_wait();
+    cgsia::D_tile<T, TAPE>(v, w + m, t, par, sb);
 }
-
-template <class T, bool TAPE = false>
-__device__ __forceinline__ void ens_dt_member(const Member<T>* mem, Words* w, int m, char* sb = nullptr) {
-    const Member<T>& v = mem[m];
-    const unsigned long long b = w[m].dmax;
-    const double dmax = sizeof(T) == 8 ? __longlong_as_double((long long)b) : (double)__int_as_float((int)(unsigned)b);
-    const T q = (T)v.dx2 / (T)dmax / (T)v.cfl;
-    double d = fmin((double)q, v.dt_max);
-    bool capped = !((double)q < v.dt_max);
-    if (!(dmax > 0.0)) {
-        d = v.dt_max;
-        capped = true;
-    }
-    w[m].dt = d;
-    w[m].t = w[m].t + d;
-    w[m].dmax = 0ull;
-    if (TAPE) {
-        cgsia::TapeWords* tw = tape_words(v, sb);
-        tw->dmax = b;
-        tw->arg = ~0ull;
-        tw->dt = d;
-        tw->capped = capped ? 1.0 : 0.0;
-    }
-}
-
-template <class T, bool TAPE = false>
-__device__ __forceinline__ void ens_H_tile(const Member<T>* mem, const int* prefix, int nm, const Words* w, int blk,
-                                           char* sb = nullptr) {
+template <class T, bool TAPE, bool DEP>
+__device__ __forceinline__ void ens_H_tile(const Member<T>* mem, const int* prefix, int nm, Words* w, int blk, int par, bool last,
+                                           bool dry, char* sb) {
     const int m = find_member(prefix, nm, blk);
     const Member<T>& v = member_of(mem, m);
     const int t = blk - (m ? prefix[m - 1] : 0);
-    const int tx = (v.nx + 31) / 32;
-    const int i = (t % tx) * 32 + threadIdx.x + 1;
-    const int j = (t / tx) * (int)blockDim.y + threadIdx.y + 1;
-    if (i > v.nx || j > v.ny) return;
-    const T dt = (T)w[m].dt;
-    const T h = v.H(i, j, 0);
-    // M = min(beta (S - ela), m_max) and H = max(H + dt (-divg q + M), 0), as std::min/max
-    // (a NaN propagates as in the reference)
-    const T x = v.beta * (v.S(i, j, 0) - v.ela);
-    const T mb = v.m_max < x ? v.m_max : x;
-    T dv = (v.qx(i + 1, j, 0) - v.qx(i, j, 0)) * v.idx;
-    dv = dv + (v.qy(i, j + 1, 0) - v.qy(i, j, 0)) * v.idy;
-    const T W = -dv + mb;
-    const T u = h + dt * W;
-    const T hn = u < T(0.0) ? T(0.0) : u;
-    if (TAPE) {
-        using namespace cgsia;
-        tape_arr(v, sb, kW)(i, j, 0) = W;
-        tape_flags(v, sb)(i, j, 0) = (unsigned char)((u > T(0) ? 1 : 0) + (v.m_max < x ? 0 : 2));
-        cgsia::TapeWords* tw = tape_words(v, sb);
-        if (bits_of(v.D(i, j, 0)) == tw->dmax) atomicMin(&tw->arg, (unsigned long long)((long)j * (v.nx + 2) + i));
-    }
-    v.H(i, j, 0) = hn;
-    v.S(i, j, 0) = v.B(i, j, 0) + hn;
-    // bc!(H => Neumann()): ghost layer and corners from the first interior cells
-    const bool l = i == 1, r = i == v.nx, b = j == 1, tp = j == v.ny;
-    auto ghost = [&](int gi, int gj) {
-        v.H(gi, gj, 0) = hn;
-        v.S(gi, gj, 0) = v.B(gi, gj, 0) + hn;
-    };
-    if (l) ghost(0, j);
-    if (r) ghost(v.nx + 1, j);
-    if (b) ghost(i, 0);
-    if (tp) ghost(i, v.ny + 1);
-    if (l && b) ghost(0, 0);
-    if (r && b) ghost(v.nx + 1, 0);
-    if (l && tp) ghost(0, v.ny + 1);
-    if (r && tp) ghost(v.nx + 1, v.ny + 1);
+    if (DEP) cg_dep_wait();
+    cgsia::H_tile<T, TAPE, true>(v, w + m, t, par, last, dry, sb);
 }
 
-template <class T, bool TAPE = false>
-__global__ void ens_D_kernel(const Member<T>* mem, const int* prefix, int nm, Words* w, char* sb) {
-    ens_D_tile<T, TAPE>(mem, prefix, nm, w, blockIdx.x, sb);
-}
 template <class T>
 __global__ void ens_S_kernel(const Member<T>* mem, const int* prefix, int nm) {
     ens_S_tile(mem, prefix, nm, blockIdx.x);
 }
-template <class T>
-__global__ void ens_q_kernel(const Member<T>* mem, const int* prefix, int nm) {
-    ens_q_tile(mem, prefix, nm, blockIdx.x);
+template <class T, bool TAPE>
+__global__ void ens_D_kernel(const Member<T>* mem, const int* prefix, int nm, Words* w, int par, char* sb) {
+    cg_dep_release();
+    ens_D_tile<T, TAPE, true>(mem, prefix, nm, w, blockIdx.x, par, sb);
 }
-template <class T, bool TAPE = false>
-__global__ void ens_dt_kernel(const Member<T>* mem, int nm, Words* w, char* sb) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m < nm) ens_dt_member<T, TAPE>(mem, w, m, sb);
-}
-template <class T, bool TAPE = false>
-__global__ void ens_H_kernel(const Member<T>* mem, const int* prefix, int nm, const Words* w, char* sb) {
-    ens_H_tile<T, TAPE>(mem, prefix, nm, w, blockIdx.x, sb);
+template <class T, bool TAPE>
+__global__ void ens_H_kernel(const Member<T>* mem, const int* prefix, int nm, Words* w, int par, int last, int dry, char* sb) {
+    cg_dep_release();
+    ens_H_tile<T, TAPE, true>(mem, prefix, nm, w, blockIdx.x, par, last != 0, dry != 0, sb);
 }
 
 // ---- one persistent launch for the whole run ------------------------------------------------
 //
 // The same tiles and arithmetic as the per-phase kernels: the resident blocks of a cooperative
-// launch loop over each phase's tiles, with a grid barrier between the phases. Per step:
-// D and the block maxima; barrier; Δt of every member (block 0) and the fluxes; barrier; the
-// thickness; barrier. The barrier counts arrivals on one monotonic word. Its waits give up
+// launch loop over each phase's tiles, with a grid barrier between the phases. Per step: D and
+// the block maxima; barrier; Δt, the fluxes and the thickness; barrier. The barrier counts arrivals on one monotonic word. Its waits give up
 // after a time limit (two seconds of the GPU's global timer unless the host sets another) and
 // set a timeout flag: the kernel then returns, and the host reports the error. A cooperative
 // launch keeps every block resident, so the waits end.
@@ -312,8 +137,8 @@ __device__ __forceinline__ bool grid_barrier(GridBar* b, unsigned expect, unsign
 }
 
 template <class T>
-__global__ void __launch_bounds__(256, 8) ens_persistent_kernel(const Member<T>* mem, const int* pD, const int* pI,
-                                                             const int* pS, int nm, int totD, int totI, int totS,
+__global__ void __launch_bounds__(256, 4) ens_persistent_kernel(const Member<T>* mem, const int* pI, const int* pH,
+                                                             const int* pS, int nm, int totI, int totH, int totS,
                                                              Words* w, int nsteps, GridBar* bar, unsigned expect,
                                                              unsigned long long limit_ns) {
     const unsigned nb = gridDim.x;
@@ -321,14 +146,9 @@ __global__ void __launch_bounds__(256, 8) ens_persistent_kernel(const Member<T>*
     for (int b = blockIdx.x; b < totS; b += nb) ens_S_tile(mem, pS, nm, b);
     if (!grid_barrier(bar, expect, limit_ns, k)) return;
     for (int s = 0; s < nsteps; ++s) {
-        for (int b = blockIdx.x; b < totD; b += nb) ens_D_tile(mem, pD, nm, w, b);
+        for (int b = blockIdx.x; b < totI; b += nb) ens_D_tile<T, false, false>(mem, pI, nm, w, b, s & 1, nullptr);
         if (!grid_barrier(bar, expect, limit_ns, k)) return;
-        if (blockIdx.x == 0)
-            for (int m = threadIdx.x + blockDim.x * threadIdx.y; m < nm; m += blockDim.x * blockDim.y)
-                ens_dt_member(mem, w, m);
-        for (int b = blockIdx.x; b < totI; b += nb) ens_q_tile(mem, pI, nm, b);
-        if (!grid_barrier(bar, expect, limit_ns, k)) return;
-        for (int b = blockIdx.x; b < totI; b += nb) ens_H_tile(mem, pI, nm, w, b);
+        for (int b = blockIdx.x; b < totH; b += nb) ens_H_tile<T, false, false>(mem, pH, nm, w, b, s & 1, s == nsteps - 1, false, nullptr);
         if (!grid_barrier(bar, expect, limit_ns, k)) return;
     }
 }
@@ -391,13 +211,13 @@ inline unsigned long long ens_tape_hash(int nm, const cg_sia_member* ms, const c
 template <class T>
 int run_t(cg_ctx* ctx, int nm, const cg_sia_member* ms, const cg_sia_params* ps, int nsteps, double* t_host,
           char* tape = nullptr) {
-    // scratch slot 3: [members][prefix D][prefix I][words][D arrays...]
+    // scratch slot 3: [members][prefix I][prefix H][prefix S][words][barrier][D, S, S per member]
     size_t off = 0;
     const size_t mem_off = off;
     off += ((size_t)nm * sizeof(Member<T>) + 255) & ~(size_t)255;
-    const size_t pD_off = off;
-    off += ((size_t)nm * sizeof(int) + 255) & ~(size_t)255;
     const size_t pI_off = off;
+    off += ((size_t)nm * sizeof(int) + 255) & ~(size_t)255;
+    const size_t pH_off = off;
     off += ((size_t)nm * sizeof(int) + 255) & ~(size_t)255;
     const size_t pS_off = off;
     off += ((size_t)nm * sizeof(int) + 255) & ~(size_t)255;
@@ -405,76 +225,47 @@ int run_t(cg_ctx* ctx, int nm, const cg_sia_member* ms, const cg_sia_params* ps,
     off += ((size_t)nm * sizeof(Words) + 255) & ~(size_t)255;
     const size_t bar_off = off;
     off += 256;
-    std::vector<size_t> d_off(nm), s_off(nm);
+    std::vector<size_t> d_off(nm);
     for (int m = 0; m < nm; ++m) {
-        const cg_field& H = ms[m].H;
-        const size_t cnt = (size_t)H.stride[1] * (H.n[1] + 4 * H.halo[1]);
         d_off[m] = off;
-        off += (cnt * sizeof(T) + 255) & ~(size_t)255;
-        s_off[m] = off;
-        off += (cnt * sizeof(T) + 255) & ~(size_t)255;
+        off += 3 * cgsia::layout_bytes(ms[m].H, sizeof(T));
     }
     int rc = CG_OK;
     char* base = static_cast<char*>(cg_scratch(ctx, 3, off, &rc));
     if (rc) return rc;
     std::vector<Member<T>> hm(nm);
-    std::vector<int> pD(nm), pI(nm), pS(nm);
+    std::vector<int> pI(nm), pH(nm), pS(nm);
     const EnsTape et = ens_tape_layout(nm, ms, sizeof(T));
-    int totD = 0, totI = 0, totS = 0;
+    int totI = 0, totH = 0, totS = 0;
     Member<T>* dmem = reinterpret_cast<Member<T>*>(base + mem_off);
-    int* dpD = reinterpret_cast<int*>(base + pD_off);
     int* dpI = reinterpret_cast<int*>(base + pI_off);
+    int* dpH = reinterpret_cast<int*>(base + pH_off);
     int* dpS = reinterpret_cast<int*>(base + pS_off);
     Words* dw = reinterpret_cast<Words*>(base + w_off);
     // members and tile prefix tables for tiles of 32 x ty points, uploaded to the scratch
     auto layout = [&](int ty) -> int {
-        totD = totI = totS = 0;
+        totI = totH = totS = 0;
         for (int m = 0; m < nm; ++m) {
             const cg_sia_member& s = ms[m];
-            const cg_sia_params& p = ps[m];
+            const size_t ab = cgsia::layout_bytes(s.H, sizeof(T));
+            char* sc = base + d_off[m];
             Member<T>& v = hm[m];
-            std::memset(&v, 0, sizeof(v));
-            v.H = cg_view<T>(s.H);
-            v.B = cg_view<T>(s.B);
-            v.qx = cg_view<T>(s.q[0]);
-            v.qy = cg_view<T>(s.q[1]);
-            v.D = v.H;
-            v.D.p = reinterpret_cast<T*>(base + d_off[m]) + cg_origin_offset(s.H);
-            v.S = v.H;
-            v.S.p = reinterpret_cast<T*>(base + s_off[m]) + cg_origin_offset(s.H);
-            v.Gamma = (T)p.Gamma;
-            v.As = (T)p.As;
-            v.beta = (T)p.beta;
-            v.ela = (T)p.ela;
-            v.m_max = (T)p.m_max;
-            v.Gn2 = v.Gamma * T(p.n + 2);
-            v.Asn = v.As * T(p.n);
-            v.idx = (T)s.grid.inv_spacing[0];
-            v.idy = (T)s.grid.inv_spacing[1];
-            const double dx = std::min(s.grid.spacing[0], s.grid.spacing[1]);
-            v.dx2 = (double)((T)dx * (T)dx);
-            v.cfl = p.cfl;
-            v.dt_max = p.dt_max;
-            v.n = p.n;
-            v.nx = s.grid.n[0];
-            v.ny = s.grid.n[1];
-            v.tiles_D = cg_div_up(v.nx + 1, 32) * cg_div_up(v.ny + 1, ty);
-            v.tiles_I = cg_div_up(v.nx, 32) * cg_div_up(v.ny, ty);
+            v = cgsia::make_member<T>(s.grid, s.H, s.B, s.q, ps[m], sc, sc + ab, sc + 2 * ab);
             if (tape) {
                 v.toff = et.toff[m];
                 v.tab = et.tab[m];
                 v.orig = et.orig[m];
             }
-            totD += v.tiles_D;
-            totI += v.tiles_I;
-            totS += cg_div_up(v.nx + 3, 32) * cg_div_up(v.ny + 3, ty);
-            pD[m] = totD;
+            totI += cg_div_up(v.nx, 32) * cg_div_up(v.ny, ty);
+            totH += cg_div_up(v.nx, cgsia::kHCols) * cg_div_up(v.ny, ty);
+            totS += cg_div_up(v.nx + 2, 32) * cg_div_up(v.ny + 2, ty);
             pI[m] = totI;
+            pH[m] = totH;
             pS[m] = totS;
         }
         CG_CUDA(ctx, cudaMemcpyAsync(dmem, hm.data(), nm * sizeof(Member<T>), cudaMemcpyHostToDevice, ctx->stream));
-        CG_CUDA(ctx, cudaMemcpyAsync(dpD, pD.data(), nm * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
         CG_CUDA(ctx, cudaMemcpyAsync(dpI, pI.data(), nm * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
+        CG_CUDA(ctx, cudaMemcpyAsync(dpH, pH.data(), nm * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
         CG_CUDA(ctx, cudaMemcpyAsync(dpS, pS.data(), nm * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
         CG_CUDA(ctx, cudaMemsetAsync(dw, 0, nm * sizeof(Words), ctx->stream));
         // the host tables are read by the copies above before the next layout call rewrites them
@@ -502,9 +293,9 @@ int run_t(cg_ctx* ctx, int nm, const cg_sia_member* ms, const cg_sia_params* ps,
             if (cg_tune_lookup(tkey, &tc)) {
                 ty = tc.variant;
             } else {
-                // time the D and flux phases of one step for each tile height; neither changes
-                // the thickness (D, the face gradients, the fluxes and S = B + H are recomputed
-                // by the run, and the words are cleared by the next layout call)
+                // time one step for each tile height, its second kernel without its stores: the
+                // thickness does not change (D and S = B + H are recomputed by the run, and the
+                // words are cleared by the next layout call)
                 float best = 1e30f;
                 for (int cand : {4, 8, 16}) {
                     if ((rc = layout(cand))) return rc;
@@ -512,8 +303,8 @@ int run_t(cg_ctx* ctx, int nm, const cg_sia_member* ms, const cg_sia_params* ps,
                     const float t = cgk::time_launches(
                         [&] {
                             ens_S_kernel<T><<<totS, bk, 0, ctx->stream>>>(dmem, dpS, nm);
-                            ens_D_kernel<T><<<totD, bk, 0, ctx->stream>>>(dmem, dpD, nm, dw, nullptr);
-                            ens_q_kernel<T><<<totI, bk, 0, ctx->stream>>>(dmem, dpI, nm);
+                            ens_D_kernel<T, false><<<totI, bk, 0, ctx->stream>>>(dmem, dpI, nm, dw, 0, nullptr);
+                            ens_H_kernel<T, false><<<totH, bk, 0, ctx->stream>>>(dmem, dpH, nm, dw, 0, 0, 1, nullptr);
                             return cudaGetLastError();
                         },
                         ctx->stream);
@@ -542,13 +333,13 @@ int run_t(cg_ctx* ctx, int nm, const cg_sia_member* ms, const cg_sia_params* ps,
         GridBar* bar = reinterpret_cast<GridBar*>(base + bar_off);
         CG_CUDA(ctx, cudaMemsetAsync(bar, 0, sizeof(GridBar), ctx->stream));
         const Member<T>* cmem = dmem;
-        const int *cpD = dpD, *cpI = dpI, *cpS = dpS;
-        int anm = nm, atD = totD, atI = totI, atS = totS, ans = nsteps;
+        const int *cpI = dpI, *cpH = dpH, *cpS = dpS;
+        int anm = nm, atI = totI, atH = totH, atS = totS, ans = nsteps;
         const unsigned nblocks = (unsigned)(bps * ctx->num_sms);
         const cg_barrier_cfg bcfg = cg_sia_barrier_cfg();
         unsigned expect = nblocks + (unsigned)bcfg.withheld;
         unsigned long long limit_ns = bcfg.limit_ns;
-        void* args[] = {&cmem, &cpD, &cpI, &cpS, &anm, &atD, &atI, &atS, &dw, &ans, &bar, &expect, &limit_ns};
+        void* args[] = {&cmem, &cpI, &cpH, &cpS, &anm, &atI, &atH, &atS, &dw, &ans, &bar, &expect, &limit_ns};
         CG_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)ens_persistent_kernel<T>, dim3(nblocks), block,
                                                  args, 0, ctx->stream));
         int timed_out = 0;
@@ -566,18 +357,14 @@ int run_t(cg_ctx* ctx, int nm, const cg_sia_member* ms, const cg_sia_params* ps,
     rc = cg_graph_run(ctx, key, [&](cudaStream_t st) {
         ens_S_kernel<T><<<totS, block, 0, st>>>(dmem, dpS, nm);
         for (int s = 0; s < nsteps; ++s) {
-            if (tape) {
-                char* sb = tape + 256 + (size_t)s * et.step_bytes;
-                ens_D_kernel<T, true><<<totD, block, 0, st>>>(dmem, dpD, nm, dw, sb);
-                ens_q_kernel<T><<<totI, block, 0, st>>>(dmem, dpI, nm);
-                ens_dt_kernel<T, true><<<cg_div_up(nm, 64), 64, 0, st>>>(dmem, nm, dw, sb);
-                ens_H_kernel<T, true><<<totI, block, 0, st>>>(dmem, dpI, nm, dw, sb);
-            } else {
-                ens_D_kernel<T><<<totD, block, 0, st>>>(dmem, dpD, nm, dw, nullptr);
-                ens_q_kernel<T><<<totI, block, 0, st>>>(dmem, dpI, nm);
-                ens_dt_kernel<T><<<cg_div_up(nm, 64), 64, 0, st>>>(dmem, nm, dw, nullptr);
-                ens_H_kernel<T><<<totI, block, 0, st>>>(dmem, dpI, nm, dw, nullptr);
-            }
+            const int par = s & 1, last = s == nsteps - 1;
+            char* sb = tape ? tape + 256 + (size_t)s * et.step_bytes : nullptr;
+            const Member<T>* cm = dmem;
+            const int *ci = dpI, *ch = dpH;
+            CG_CUDA(ctx, tape ? cg_launch(ens_D_kernel<T, true>, dim3(totI), block, 0, st, s > 0, cm, ci, nm, dw, par, sb)
+                              : cg_launch(ens_D_kernel<T, false>, dim3(totI), block, 0, st, s > 0, cm, ci, nm, dw, par, sb));
+            CG_CUDA(ctx, tape ? cg_launch(ens_H_kernel<T, true>, dim3(totH), block, 0, st, true, cm, ch, nm, dw, par, last, 0, sb)
+                              : cg_launch(ens_H_kernel<T, false>, dim3(totH), block, 0, st, true, cm, ch, nm, dw, par, last, 0, sb));
             CG_CHECK_LAUNCH(ctx);
         }
         return (int)CG_OK;
@@ -596,8 +383,9 @@ int run_t(cg_ctx* ctx, int nm, const cg_sia_member* ms, const cg_sia_params* ps,
 // ---- reverse sweep over an ensemble tape ----------------------------------------------------
 //
 // The reverse step of cg_sia_adjoint_run applied to every member at once: per step, the cell
-// kernel over all members' interior tiles, one block per member for the ordered sums of its
-// tiles' partials and the dt term at its argmax cell, and the gather kernel over all tiles.
+// kernel over all members' interior tiles and the gather kernel over all tiles, which also adds the
+// dt term at each member's argmax cell. (A launch of its own for the sums of dJ/ddt took 5.9 us of a
+// step's 45 us at 10 members of 64^2 to 224^2.)
 template <class T>
 struct AdjMember {
     DF<T> L, Wk, lo, pax, pay;  // lambda and work (in/out by turns), the step's scratch
@@ -652,7 +440,9 @@ __global__ void __launch_bounds__(256) ens_adj_cell_kernel(const AdjMember<T>* a
                                                            const char* sb, int parity, double* part) {
     using namespace cgsia;
     constexpr unsigned FULL = 0xffffffffu;
-    __shared__ T fdy[8][32], fsy[8][32];
+    __shared__ T fdy[8][32], fsy[8][32], kc[4];
+    __shared__ double sd[8][32];
+    cg_dep_release();
     const int blk = blockIdx.x;
     const int m = find_member(prefix, nm, blk);
     const AdjMember<T>& v = adj_member_of(am, m);
@@ -667,35 +457,59 @@ __global__ void __launch_bounds__(256) ens_adj_cell_kernel(const AdjMember<T>* a
     const DF<unsigned char> FL = adj_flags(v, sb);
     const DF<T> D = adj_tape(v, sb, kD);
     const TapeWords* w = reinterpret_cast<const TapeWords*>(sb + v.toff);
-    const T dt = (T)w->dt;
-    const T dtx = dt * v.idx, dty = dt * v.idy;
-    T muc = T(0), dc = T(0);
-    if (in) {
-        muc = ens_mu(FL, lam, i, j);
-        dc = D(i, j, 0);
+    // the step's constants, once per block: dt beta, 1 + dt beta, and per dimension -dt idx/2 and idx
+    if (lane < 4 && row == 0) {
+        const T dt = (T)w->dt, dtb = dt * v.beta;
+        kc[lane] = lane == 0 ? dtb : lane == 1 ? T(1) + dtb : -T(0.5) * (dt * (lane == 2 ? v.idx : v.idy));
     }
-    // the lower x face (face i, cells i-1 and i) and the lower y face (face j)
+    // the tape does not change within a sweep: its values load while the kernel before this one
+    // drains, and only lambda waits for it
+    T dc = T(0), gx = T(0), gy = T(0), dl = T(0), dd = T(0), cdh = T(0), cex = T(0), cey = T(0), cgf = T(0), cw = T(0);
+    unsigned char flc = 0, fll = 0, fld = 0;
+    if (in) {
+        dc = D(i, j, 0);
+        flc = FL(i, j, 0);
+        if (i >= 2) {
+            dl = D(i - 1, j, 0);
+            fll = FL(i - 1, j, 0);
+            gx = adj_tape(v, sb, kGX)(i, j, 0);
+        }
+        if (j >= 2) {
+            dd = D(i, j - 1, 0);
+            fld = FL(i, j - 1, 0);
+            gy = adj_tape(v, sb, kGY)(i, j, 0);
+        }
+        if (own) {
+            cdh = adj_tape(v, sb, kDH)(i, j, 0);
+            cex = adj_tape(v, sb, kEX)(i, j, 0);
+            cey = adj_tape(v, sb, kEY)(i, j, 0);
+            cgf = adj_tape(v, sb, kGF)(i, j, 0);
+            cw = adj_tape(v, sb, kW)(i, j, 0);
+        }
+    }
+    __syncthreads();
+    cg_dep_wait();
+    const T muc = flc & 1 ? lam(i, j, 0) : T(0);
+    // the lower x face (face i, cells i-1 and i) and the lower y face (face j): with p = -dt idx/2
+    // (mu_upper - mu_lower), dJ/dD of both cells gains p g and dJ/dS of them -/+ (D_l + D_u) p idx
     T tDx = T(0), tSx = T(0), tDy = T(0), tSy = T(0);
     if (in && i >= 2) {
-        const T px = dtx * (muc - ens_mu(FL, lam, i - 1, j));
-        const T dl = D(i - 1, j, 0);
-        tDx = -T(0.5) * px * adj_tape(v, sb, kGX)(i, j, 0);
-        tSx = fma(T(0.5), dc - dl, dl) * px * v.idx;
+        const T px = kc[2] * (muc - (fll & 1 ? lam(i - 1, j, 0) : T(0)));
+        tDx = px * gx;
+        tSx = (dl + dc) * (px * -v.idx);
     }
     if (in && j >= 2) {
-        const T py = dty * (muc - ens_mu(FL, lam, i, j - 1));
-        const T dl = D(i, j - 1, 0);
-        tDy = -T(0.5) * py * adj_tape(v, sb, kGY)(i, j, 0);
-        tSy = fma(T(0.5), dc - dl, dl) * py * v.idy;
+        const T py = kc[3] * (muc - (fld & 1 ? lam(i, j - 1, 0) : T(0)));
+        tDy = py * gy;
+        tSy = (dd + dc) * (py * -v.idy);
     }
     fdy[row][lane] = tDy;
     fsy[row][lane] = tSy;
     T tDu = T(0), tSu = T(0);
     if (row == 7 && in && j + 1 <= v.ny) {  // the face above the tile
-        const T py = dty * (ens_mu(FL, lam, i, j + 1) - muc);
-        const T dr = D(i, j + 1, 0);
-        tDu = -T(0.5) * py * adj_tape(v, sb, kGY)(i, j + 1, 0);
-        tSu = fma(T(0.5), dr - dc, dc) * py * v.idy;
+        const T py = kc[3] * (ens_mu(FL, lam, i, j + 1) - muc);
+        tDu = py * adj_tape(v, sb, kGY)(i, j + 1, 0);
+        tSu = (dc + D(i, j + 1, 0)) * (py * -v.idy);
     }
     const T tDr = __shfl_down_sync(FULL, tDx, 1), tSr = __shfl_down_sync(FULL, tSx, 1);
     __syncthreads();
@@ -724,55 +538,25 @@ __global__ void __launch_bounds__(256) ens_adj_cell_kernel(const AdjMember<T>* a
         }
         // the mass balance's direct terms: d H'/d H = 1 + dt beta and d H'/d ela = -dt beta
         // where it is not capped (the step's constants, once per thread)
-        const bool mM = (FL(i, j, 0) & 2) != 0;
-        const T dtb = dt * v.beta;
-        const T lo = mM ? muc * (T(1) + dtb) : muc;
-        v.lo(i, j, 0) = lo + pD * adj_tape(v, sb, kDH)(i, j, 0) + pS;
-        v.pax(i, j, 0) = pD * adj_tape(v, sb, kEX)(i, j, 0);
-        v.pay(i, j, 0) = pD * adj_tape(v, sb, kEY)(i, j, 0);
-        sdt = (double)(muc * adj_tape(v, sb, kW)(i, j, 0));
-        v.aG(i, j, 0) += (double)(pD * adj_tape(v, sb, kGF)(i, j, 0));
-        if (mM) v.aE(i, j, 0) -= (double)(muc * dtb);
+        const bool mM = (flc & 2) != 0;
+        v.lo(i, j, 0) = fma(pD, cdh, mM ? muc * kc[1] : muc) + pS;
+        v.pax(i, j, 0) = pD * cex;
+        v.pay(i, j, 0) = pD * cey;
+        sdt = (double)(muc * cw);
+        v.aG(i, j, 0) += (double)(pD * cgf);
+        if (mM) v.aE(i, j, 0) -= (double)(muc * kc[0]);
     }
-    const double a = block_sum(sdt);
-    if (threadIdx.x == 0 && threadIdx.y == 0) part[blk] = a;
-}
-
-// Block m (1024 threads): dJ/ddt of member m's step, its tiles' partials summed in a fixed
-// order; then the dt term at its argmax cell (when dt was not capped) into lo, pax, pay and
-// the per-cell dJ/dGamma sum there.
-template <class T>
-__global__ void __launch_bounds__(1024) ens_adj_sum_kernel(const AdjMember<T>* am, const int* prefix, const char* sb,
-                                                           const double* part) {
-    using namespace cgsia;
-    constexpr unsigned FULL = 0xffffffffu;
-    __shared__ double red[32];
-    const int m = blockIdx.x;
-    const int b0 = m ? prefix[m - 1] : 0, b1 = prefix[m];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    double x = 0.0;
-    for (int b = b0 + tid; b < b1; b += blockDim.x) x += part[b];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(FULL, x, o);
-    if (lane == 0) red[warp] = x;
+    // the tile's sum of dJ/ddt in a fixed order: down the rows in one warp, then across its lanes
+    // (a shuffle tree in every warp would cost each five FP64 instructions)
+    sd[row][lane] = sdt;
     __syncthreads();
-    if (warp != 0) return;
-    x = lane < (int)(blockDim.x >> 5) ? red[lane] : 0.0;
+    if (row == 0) {
+        double x = sd[0][lane];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(FULL, x, o);
-    if (lane != 0) return;
-    const AdjMember<T>& v = am[m];
-    const TapeWords* w = reinterpret_cast<const TapeWords*>(sb + v.toff);
-    if (w->capped == 0.0 && w->arg != ~0ull) {
-        const unsigned long long bb = w->dmax;
-        const double dmax = sizeof(T) == 8 ? __longlong_as_double((long long)bb) : (double)__int_as_float((int)(unsigned)bb);
-        const T pD = (T)(-x * w->dt / dmax);
-        const int i = (int)(w->arg % (unsigned long long)(v.nx + 2));
-        const int j = (int)(w->arg / (unsigned long long)(v.nx + 2));
-        v.lo(i, j, 0) = v.lo(i, j, 0) + pD * adj_tape(v, sb, kDH)(i, j, 0);
-        v.pax(i, j, 0) = v.pax(i, j, 0) + pD * adj_tape(v, sb, kEX)(i, j, 0);
-        v.pay(i, j, 0) = v.pay(i, j, 0) + pD * adj_tape(v, sb, kEY)(i, j, 0);
-        v.aG(i, j, 0) += (double)(pD * adj_tape(v, sb, kGF)(i, j, 0));
+        for (int r = 1; r < 8; ++r) x += sd[r][lane];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(FULL, x, o);
+        if (lane == 0) part[blk] = x;
     }
 }
 
@@ -823,29 +607,72 @@ __global__ void __launch_bounds__(1024) ens_adj_final_kernel(const int* prefix, 
 
 // lambda_n of every member from lo and the neighbours' pax, pay (the ghost cells' terms folded
 // into the interior cells they copy); parity 0 writes Wk, 1 writes L. copy: L = Wk instead.
+//
+// The dt term (when dt was not capped) adds pD dD/dh, pD dD/dax, pD dD/day to lo, pax, pay of the one
+// cell where D attains its maximum, with pD = -dJ/ddt dt/Dmax, and pD dD/dGamma to its dJ/dGamma sum.
+// Only the tiles that read that cell need dJ/ddt: they sum the member's tile partials of the cell
+// kernel (cprefix its tile prefix) in a fixed order and add the terms as they read; the tile that owns
+// the cell updates the dJ/dGamma sum.
 template <class T>
-__global__ void __launch_bounds__(256) ens_adj_out_kernel(const AdjMember<T>* am, const int* prefix, int nm, int parity,
-                                                          int copy) {
+__global__ void __launch_bounds__(256) ens_adj_out_kernel(const AdjMember<T>* am, const int* prefix, const int* cprefix, int nm,
+                                                          const char* sb, const double* part, int parity, int copy) {
+    using namespace cgsia;
+    __shared__ double red[8];
+    cg_dep_release();
     const int blk = blockIdx.x;
     const int m = find_member(prefix, nm, blk);
     const AdjMember<T>& v = adj_member_of(am, m);
     const int t = blk - (m ? prefix[m - 1] : 0);
     const int tx = (v.nx + 31) / 32;
-    const int i = (t % tx) * 32 + threadIdx.x + 1;
-    const int j = (t / tx) * 8 + threadIdx.y + 1;
+    const int it = (t % tx) * 32 + 1, jt = (t / tx) * 8 + 1;
+    const int i = it + threadIdx.x, j = jt + threadIdx.y;
+    int ai = -9, aj = -9;  // the argmax cell, where it matters to this tile
+    double pd = 0.0;
+    const TapeWords* w = reinterpret_cast<const TapeWords*>(sb + v.toff);
+    bool near = false;
+    if (!copy && w->capped == 0.0 && w->arg != ~0ull) {
+        const int ci = (int)(w->arg % (unsigned long long)(v.nx + 2)), cj = (int)(w->arg / (unsigned long long)(v.nx + 2));
+        near = ci >= it - 1 && ci <= it + 32 && cj >= jt - 1 && cj <= jt + 8;
+        if (near) {
+            ai = ci;
+            aj = cj;
+        }
+    }
+    cg_dep_wait();
+    if (near) {  // the whole block
+        const int b0 = m ? cprefix[m - 1] : 0, b1 = cprefix[m];
+        const int tid = threadIdx.x + 32 * threadIdx.y;
+        double x = 0.0;
+        for (int b = b0 + tid; b < b1; b += 256) x += part[b];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        if (threadIdx.x == 0) red[threadIdx.y] = x;
+        __syncthreads();
+        x = 0.0;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) x += red[r];
+        const unsigned long long bb = w->dmax;
+        const double dmax = sizeof(T) == 8 ? __longlong_as_double((long long)bb) : (double)__int_as_float((int)(unsigned)bb);
+        pd = (double)(T)(-x * w->dt / dmax);
+    }
     if (i > v.nx || j > v.ny) return;
     if (copy) {
         v.L(i, j, 0) = v.Wk(i, j, 0);
         return;
     }
-    const T hx = T(0.5) * v.idx, hy = T(0.5) * v.idy;
-    auto PX = [&](int a, int b) { return (a >= 1 && a <= v.nx) ? v.pax(a, b, 0) : T(0); };
-    auto PY = [&](int a, int b) { return (b >= 1 && b <= v.ny) ? v.pay(a, b, 0) : T(0); };
-    T r = v.lo(i, j, 0) + hx * (PX(i - 1, j) - PX(i + 1, j)) + hy * (PY(i, j - 1) - PY(i, j + 1));
-    if (i == 1) r += -hx * v.pax(1, j, 0);
-    if (i == v.nx) r += hx * v.pax(v.nx, j, 0);
-    if (j == 1) r += -hy * v.pay(i, 1, 0);
-    if (j == v.ny) r += hy * v.pay(i, v.ny, 0);
+    const T hx = T(0.5) * v.idx, hy = T(0.5) * v.idy, pD = (T)pd;
+    auto at = [&](const DF<T>& f, int k, int a, int b) {  // f's value, with the dt term's at the argmax cell
+        const T x = f(a, b, 0);
+        return a == ai && b == aj ? x + pD * adj_tape(v, sb, k)(a, b, 0) : x;
+    };
+    auto PX = [&](int a, int b) { return (a >= 1 && a <= v.nx) ? at(v.pax, kEX, a, b) : T(0); };
+    auto PY = [&](int a, int b) { return (b >= 1 && b <= v.ny) ? at(v.pay, kEY, a, b) : T(0); };
+    T r = at(v.lo, kDH, i, j) + hx * (PX(i - 1, j) - PX(i + 1, j)) + hy * (PY(i, j - 1) - PY(i, j + 1));
+    if (i == 1) r += -hx * PX(1, j);
+    if (i == v.nx) r += hx * PX(v.nx, j);
+    if (j == 1) r += -hy * PY(i, 1);
+    if (j == v.ny) r += hy * PY(i, v.ny);
+    if (i == ai && j == aj) v.aG(i, j, 0) += (double)(pD * adj_tape(v, sb, kGF)(i, j, 0));
     (parity ? v.L : v.Wk)(i, j, 0) = r;
 }
 
@@ -935,12 +762,13 @@ int adjoint_run_t(cg_ctx* ctx, int nm, const cg_sia_member* ms, const cg_sia_par
         CG_CUDA(ctx, cudaMemsetAsync(base + sums_off, 0, sums_bytes, st));
         for (int r = 0; r < N; ++r) {
             const char* sb = tape + 256 + (size_t)(N - 1 - r) * et.step_bytes;
-            ens_adj_cell_kernel<T><<<totC, block, 0, st>>>(dmem, dpc, nm, sb, r & 1, part);
-            ens_adj_sum_kernel<T><<<nm, 1024, 0, st>>>(dmem, dpc, sb, part);
-            ens_adj_out_kernel<T><<<totI, block, 0, st>>>(dmem, dp, nm, r & 1, 0);
-            CG_CHECK_LAUNCH(ctx);
+            const AdjMember<T>* cm = dmem;
+            const int *ci = dp, *cc = dpc;
+            const double* cpart = part;
+            CG_CUDA(ctx, cg_launch(ens_adj_cell_kernel<T>, dim3(totC), block, 0, st, r > 0, cm, cc, nm, sb, r & 1, part));
+            CG_CUDA(ctx, cg_launch(ens_adj_out_kernel<T>, dim3(totI), block, 0, st, true, cm, ci, cc, nm, sb, cpart, r & 1, 0));
         }
-        if (N & 1) ens_adj_out_kernel<T><<<totI, block, 0, st>>>(dmem, dp, nm, 0, 1);
+        if (N & 1) ens_adj_out_kernel<T><<<totI, block, 0, st>>>(dmem, dp, dpc, nm, tape + 256, part, 0, 1);
         ens_adj_tile_sums_kernel<T><<<totI, block, 0, st>>>(dmem, dp, nm, part, totI);
         ens_adj_final_kernel<<<nm, 1024, 0, st>>>(dp, part, totI, acc);
         CG_CHECK_LAUNCH(ctx);
