@@ -55,7 +55,7 @@ __global__ void update_C_kernel(DF<T> C, DF<T> q0, DF<T> q1, DF<T> q2, T dt, Spa
     C(i, j, k) = rsub(C(i, j, k), rmul(dt, dv));
 }
 
-// Fused compute_q! + update_C! in the reference's flux form: q_d at face I is
+// Fused compute_q! + update_C! (1D and 3D) in the reference's flux form: q_d at face I is
 // -χ ((C[I] - C[I-e_d]) iΔ_d) over the launch range, a face with index n+2 along its dimension is
 // outside compute_q!'s range and reads as zero (fresh q arrays), and C' = C - dt Σ_d (q_d[I+e_d] -
 // q_d[I]) iΔ_d in dim order. Each x-face flux is computed once (a lane's right face is the next
@@ -96,6 +96,94 @@ __global__ void diffusion_step_kernel(DF<T> Co, DF<T> Ci, T mchi, T dt, Spacing<
         dv = radd(dv, rmul(rsub(qzr, qzl), s.i[2]));
     }
     Co(i, j, k) = rsub(c, rmul(dt, dv));
+}
+
+// ---- the 2D step as a march over rows ---------------------------------------------------------
+//
+// FP64 arithmetic bounds the step: 13 instructions per cell (two fluxes of 3, the update of 7; 11
+// where chi is 1) against 16 bytes. A warp owns 31 columns and marches up a segment of rows: a lane
+// takes the flux on the left face of its cell and passes it to the lane below as its right face
+// (lane 31 only supplies lane 30's; owning a 32nd column would cost the warp a second x flux), and
+// carries the upper face's flux to the next row in a register. No flux is computed twice but the
+// lowest of a segment, and there are no barriers; the tile kernel above computes one y flux in nine
+// twice, one x flux per warp twice, and stands at a barrier between its loads and its arithmetic.
+//
+// bc!(C) is folded into the stores (EdgeRules): the thread that updates a cell beside a boundary also
+// writes the ghost cells that follow it, by the rules of cg_bc_apply in their order (y, then x, a
+// corner through its y ghost). A ghost cell under a rule is not computed. Only points at index n+2,
+// which no step reads, are left to one bc! launch at the end of a run.
+//
+// UNIT (chi = 1, the example's): the product by -1 is exact, so the march carries g = -q and takes
+// its differences the other way round, which gives the same bits with two instructions fewer. A face
+// beyond the launch range has q = +0, so g = -0.
+// Measured at 1023 x 769 FP64 (16.4 us at the FP64 pipe's rate with 13 instructions, 13.9 with 11): 27.4 us
+// per step and 2.7 us for bc! before, 21.9 us now (the FP64 pipe is 81 % busy, as it is at 4000^2, where
+// segments of 16 rows take 362 us of 282). A row is a chain of nine dependent FP64 operations, about
+// 0.6 us, so small grids take segments of one or two rows: 126^2 3.4 us per step.
+template <class T>
+struct EdgeRules {
+    int r[2][2];  // [dimension][side]: 0 none, 1 Dirichlet (2 v - C), 2 Neumann (C -/+ h v)
+    T v[2][2], h[2];
+};
+
+template <class T>
+__device__ __forceinline__ T edge_value(const EdgeRules<T>& e, int d, int s, T c) {
+    return e.r[d][s] == 1 ? cgk::rfma(T(2), rsub(e.v[d][s], c), c) : cgk::rfma(e.h[d], e.v[d][s], c);
+}
+
+template <class T, bool UNIT>
+__global__ void __launch_bounds__(128) diffusion_march2d_kernel(DF<T> Co, DF<T> Ci, T mchi, T dt, Spacing<T> s, int e0, int e1,
+                                                                int nstrip, int nwarps, int seg, const EdgeRules<T> er) {
+    constexpr unsigned FULL = 0xffffffffu;
+    cg_dep_wait();
+    cg_dep_release();
+    const int lane = threadIdx.x & 31, gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (gw >= nwarps) return;  // whole warp
+    const int jlo = er.r[1][0] ? 1 : 0, jhi = er.r[1][1] ? e1 - 1 : e1;
+    const int js = jlo + (gw / nstrip) * seg, je = min(js + seg - 1, jhi);
+    const int i = (gw % nstrip) * 31 + lane;
+    const bool in = i <= e0;
+    const bool own = in && lane < 31 && !(i == 0 && er.r[0][0]) && !(i == e0 && er.r[0][1]);
+    const bool gl = own && i == 1 && er.r[0][0], gr = own && i == e0 - 1 && er.r[0][1];
+    const T none = UNIT ? T(-0.0) : T(0);
+    auto flux = [&](T hi, T lo, int d) {
+        const T g = rmul(rsub(hi, lo), s.i[d]);
+        return UNIT ? g : rmul(mchi, g);
+    };
+    auto diff = [&](T ql, T qr) { return UNIT ? rsub(ql, qr) : rsub(qr, ql); };
+    const T* p = Ci.ptr(in ? i : e0, js, 0);
+    const T* pl = Ci.ptr((gw % nstrip) * 31 - 1, js, 0);  // lane 0's left neighbour
+    T c = *p, ql = lane == 0 ? *pl : T(0);
+    T qyl = flux(c, p[-Ci.s1], 1);
+    T* o = Co.ptr(i, js, 0);
+    for (int j = js; j <= je; ++j, o += Co.s1) {
+        p += Ci.s1;
+        pl += Ci.s1;
+        const bool up = j + 1 <= e1;
+        const T cn = up ? *p : T(0);
+        const T qn = lane == 0 && up ? *pl : T(0);
+        T cl = __shfl_up_sync(FULL, c, 1);
+        if (lane == 0) cl = ql;
+        const T qxl = flux(c, cl, 0);
+        T qxr = __shfl_down_sync(FULL, qxl, 1);
+        if (i == e0) qxr = none;
+        const T qyu = up ? flux(cn, c, 1) : none;
+        const T dv = radd(rmul(diff(qxl, qxr), s.i[0]), rmul(diff(qyl, qyu), s.i[1]));
+        const T v = rsub(c, rmul(dt, dv));
+        if (own) {
+            auto put = [&](T* q, T x) {
+                *q = x;
+                if (gl) q[-1] = edge_value(er, 0, 0, x);
+                if (gr) q[1] = edge_value(er, 0, 1, x);
+            };
+            put(o, v);
+            if (j == 1 && er.r[1][0]) put(o - Co.s1, edge_value(er, 1, 0, v));
+            if (j == e1 - 1 && er.r[1][1]) put(o + Co.s1, edge_value(er, 1, 1, v));
+        }
+        qyl = qyu;
+        c = cn;
+        ql = qn;
+    }
 }
 
 // ---- masked operators (src/GridOperators/masked_operators.jl:11-39) --------------------------
@@ -208,35 +296,112 @@ cudaError_t step_launch(const cg_grid* g, const cg_field* Co, const cg_field* Ci
     return cudaGetLastError();
 }
 
-// The step kernel's block shape for this grid and layout: 1D keeps 256 threads; 2D and 3D take
-// the autotuner's choice, timed on C_out = step(C_in) (the first step of a run writes the same
-// points again), or its cached choice when `may_time` is false.
+// The rules of bc! that the 2D march folds into its stores; false where it cannot (periodic sides,
+// per-point values), and then none are set.
+template <class T>
+bool edge_rules(const cg_grid* g, const cg_bc* bc, EdgeRules<T>* er) {
+    std::memset(er, 0, sizeof(*er));
+    if (!bc) return true;
+    EdgeRules<T> e = *er;
+    for (int d = 0; d < 2; ++d) {
+        e.h[d] = (T)g->spacing[d];
+        for (int s = 0; s < 2; ++s) {
+            const int k = bc->kind[d][s];
+            if (bc->values[d][s] || (k != CG_BC_NONE && k != CG_BC_DIRICHLET && k != CG_BC_NEUMANN)) return false;
+            e.r[d][s] = k == CG_BC_DIRICHLET ? 1 : k == CG_BC_NEUMANN ? 2 : 0;
+            const T v = (T)bc->value[d][s];
+            e.v[d][s] = k == CG_BC_NEUMANN && s == 0 ? -v : v;
+        }
+    }
+    *er = e;
+    return true;
+}
+
+template <class T>
+cudaError_t march_launch(const cg_grid* g, const cg_field* Co, const cg_field* Ci, double chi, double dt, int seg,
+                         const EdgeRules<T>& er, cudaStream_t st, bool dep) {
+    const int e0 = g->n[0] + 1, e1 = g->n[1] + 1;
+    const int rows = e1 + 1 - (er.r[1][0] ? 1 : 0) - (er.r[1][1] ? 1 : 0);
+    const int nstrip = cg_div_up(e0 + 1, 31), nwarps = nstrip * cg_div_up(rows, seg);
+    const dim3 grid(cg_div_up(nwarps, 4)), block(128);
+    const DF<T> o = cg_view<T>(*Co), c = cg_view<T>(*Ci);
+    const Spacing<T> s = spacing_of<T>(g);
+    if (chi == 1.0)
+        return cg_launch(diffusion_march2d_kernel<T, true>, grid, block, 0, st, dep, o, c, T(-1), (T)dt, s, e0, e1, nstrip, nwarps, seg, er);
+    return cg_launch(diffusion_march2d_kernel<T, false>, grid, block, 0, st, dep, o, c, -(T)chi, (T)dt, s, e0, e1, nstrip, nwarps, seg, er);
+}
+
+// The layout of the step's launch for this grid, timed on C_out = step(C_in) (the first step of a run
+// writes the same points again), or its cached choice when `may_time` is false: in 2D the march's
+// segment length in x (short segments balance the SMs, long ones recompute fewer y fluxes), in 3D
+// the tile kernel's block; 1D keeps 256 threads.
 template <class T, int ND>
 dim3 step_block(cg_ctx* ctx, const cg_grid* g, const cg_field* Co, const cg_field* Ci, double chi, double dt,
                 bool may_time) {
     if (ND == 1) return block_for<ND>();
-    std::string key = "diffusion_block";
+    std::string key = ND == 2 ? "diffusion_segment" : "diffusion_block";
     cg_key_add(key, *g);
     cg_key_add(key, (int)sizeof(T));
     cg_key_add(key, Ci->stride);
     cg_key_add(key, Co->stride);
     cg_key_add(key, ctx->num_sms);
-    if (!may_time) {
-        dim3 b(32, 8);
-        if (cg_block_forced(&b)) return b;
-        cg_tune_cfg c{0, 0};
-        return cg_tune_lookup(key, &c) ? dim3((unsigned)c.seg, (unsigned)c.variant) : b;
+    if constexpr (ND == 2) {
+        cg_tune_cfg c{8, 1};
+        if (cg_tune_lookup(key, &c) || !may_time || !cg_autotune_enabled()) return dim3((unsigned)c.seg);
+        EdgeRules<T> er;
+        edge_rules<T>(g, nullptr, &er);
+        float best = 1e30f;
+        for (int seg : {1, 2, 3, 4, 6, 8, 12, 16, 24}) {
+            const float t = cgk::time_launches([&] { return march_launch<T>(g, Co, Ci, chi, dt, seg, er, ctx->stream, false); }, ctx->stream);
+            if (cg_tune_verbose())
+                std::fprintf(stderr, "diffusion step tune %dx%d: seg %d: %.1f us\n", g->n[0], g->n[1], seg, t >= 0.f ? 1e3f * t / 3 : -1.f);
+            if (t >= 0.f && t < best) {
+                best = t;
+                c.seg = seg;
+            }
+        }
+        cudaGetLastError();
+        cg_tune_store(key, c);
+        return dim3((unsigned)c.seg);
+    } else {
+        if (!may_time) {
+            dim3 b(32, 8);
+            if (cg_block_forced(&b)) return b;
+            cg_tune_cfg c{0, 0};
+            return cg_tune_lookup(key, &c) ? dim3((unsigned)c.seg, (unsigned)c.variant) : b;
+        }
+        return cgk::tune_block("diffusion step", key,
+                               [&](dim3 b) { return step_launch<T, ND>(g, Co, Ci, chi, dt, b, ctx->stream); }, ctx->stream);
     }
-    return cgk::tune_block("diffusion step", key,
-                           [&](dim3 b) { return step_launch<T, ND>(g, Co, Ci, chi, dt, b, ctx->stream); }, ctx->stream);
 }
 
 template <class T, int ND>
-int step_t(cg_ctx* ctx, const cg_grid* g, const cg_field* Co, const cg_field* Ci, double chi, double dt, bool may_time) {
-    const dim3 block = step_block<T, ND>(ctx, g, Co, Ci, chi, dt, may_time);
-    const cudaError_t e = step_launch<T, ND>(g, Co, Ci, chi, dt, block, ctx->stream);
+int step_t(cg_ctx* ctx, const cg_grid* g, const cg_field* Co, const cg_field* Ci, double chi, double dt) {
+    const dim3 block = step_block<T, ND>(ctx, g, Co, Ci, chi, dt, false);
+    cudaError_t e;
+    if constexpr (ND == 2) {
+        EdgeRules<T> er;
+        edge_rules<T>(g, nullptr, &er);
+        e = march_launch<T>(g, Co, Ci, chi, dt, (int)block.x, er, ctx->stream, false);
+    } else {
+        e = step_launch<T, ND>(g, Co, Ci, chi, dt, block, ctx->stream);
+    }
     if (e != cudaSuccess) return cg_fail(ctx, CG_ERR_CUDA, "diffusion step: %s", cudaGetErrorString(e));
     return CG_OK;
+}
+
+// The steps of a 2D run with bc! folded into them: A -> B -> A ..., and one bc! launch at the end.
+template <class T>
+int folded_steps(cg_ctx* ctx, const cg_grid* g, const cg_field* A, const cg_field* B, double chi, double dt, const cg_bc* bc,
+                 const EdgeRules<T>& er, int seg, int nsteps, cudaStream_t st) {
+    for (int k = 0; k < nsteps; ++k) {
+        const cudaError_t e = march_launch<T>(g, k % 2 ? A : B, k % 2 ? B : A, chi, dt, seg, er, st, k > 0);
+        if (e != cudaSuccess) return cg_fail(ctx, CG_ERR_CUDA, "diffusion step: %s", cudaGetErrorString(e));
+    }
+    if (!bc) return CG_OK;
+    const cg_field fs[2] = {*B, *A};
+    const cg_bc bs[2] = {*bc, *bc};
+    return cg_bc_apply_impl(ctx, g, nsteps > 1 ? 2 : 1, fs, bs);
 }
 
 template <class T>
@@ -321,11 +486,10 @@ extern "C" int cg_diffusion_update_C(cg_ctx* ctx, const cg_grid* grid, const cg_
     return CG_DISPATCH(update_C_t, C->dtype, grid->ndim, ctx, grid, C, q, dt);
 }
 
-// One step and bc!; `may_time`: the block-shape autotuner may time launches (false inside a
-// graph capture, where the cached or default shape is used).
+// One step and bc!, with the launch layout that a run of this shape has tuned, or the default.
 static int step_checked(cg_ctx* ctx, const cg_grid* grid, const cg_field* Co, const cg_field* Ci, double chi,
-                        double dt, const cg_bc* bc, bool may_time) {
-    int rc = CG_DISPATCH(step_t, Ci->dtype, grid->ndim, ctx, grid, Co, Ci, chi, dt, may_time);
+                        double dt, const cg_bc* bc) {
+    int rc = CG_DISPATCH(step_t, Ci->dtype, grid->ndim, ctx, grid, Co, Ci, chi, dt);
     if (rc) return rc;
     if (bc) return cg_bc_apply_impl(ctx, grid, 1, Co, bc);
     return CG_OK;
@@ -346,7 +510,7 @@ extern "C" int cg_diffusion_step(cg_ctx* ctx, const cg_grid* grid, const cg_fiel
     int rc = step_args(ctx, grid, C_out, C_in);
     if (rc) return rc;
     cudaSetDevice(ctx->device);
-    return step_checked(ctx, grid, C_out, C_in, chi, dt, bc, false);
+    return step_checked(ctx, grid, C_out, C_in, chi, dt, bc);
 }
 
 extern "C" int cg_diffusion_run(cg_ctx* ctx, const cg_grid* grid, const cg_field* A, const cg_field* B, double chi,
@@ -366,7 +530,7 @@ extern "C" int cg_diffusion_run(cg_ctx* ctx, const cg_grid* grid, const cg_field
     cg_bc none;
     std::memset(&none, 0, sizeof(none));
     cg_key_add(key, bc ? *bc : none);
-    // the step's block shape, timed on B = step(A) (once per shape) before the graph is captured
+    // the step's launch layout, timed on B = step(A) (once per shape) before the graph is captured
     dim3 blk(256, 1);
     if (grid->ndim > 1) blk = A->dtype == CG_F64
                                   ? (grid->ndim == 2 ? step_block<double, 2>(ctx, grid, B, A, chi, dt, true)
@@ -374,11 +538,19 @@ extern "C" int cg_diffusion_run(cg_ctx* ctx, const cg_grid* grid, const cg_field
                                   : (grid->ndim == 2 ? step_block<float, 2>(ctx, grid, B, A, chi, dt, true)
                                                      : step_block<float, 3>(ctx, grid, B, A, chi, dt, true));
     cg_key_add(key, blk);
-    return cg_graph_run(ctx, key, [&](cudaStream_t) {
+    return cg_graph_run(ctx, key, [&](cudaStream_t st) {
+        if (grid->ndim == 2) {
+            EdgeRules<double> ed;
+            EdgeRules<float> ef;
+            if (A->dtype == CG_F64 && edge_rules(grid, bc, &ed))
+                return folded_steps(ctx, grid, A, B, chi, dt, bc, ed, (int)blk.x, nsteps, st);
+            if (A->dtype == CG_F32 && edge_rules(grid, bc, &ef))
+                return folded_steps(ctx, grid, A, B, chi, dt, bc, ef, (int)blk.x, nsteps, st);
+        }
         for (int s = 0; s < nsteps; ++s) {
             const cg_field* in = (s % 2 == 0) ? A : B;
             const cg_field* out = (s % 2 == 0) ? B : A;
-            int r = step_checked(ctx, grid, out, in, chi, dt, bc, false);
+            int r = step_checked(ctx, grid, out, in, chi, dt, bc);
             if (r) return r;
         }
         return (int)CG_OK;
