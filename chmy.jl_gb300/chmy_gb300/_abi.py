@@ -9,6 +9,7 @@ from __future__ import annotations
 import ctypes as C
 import os
 import re
+import struct
 from pathlib import Path
 
 PKG_DIR = Path(__file__).resolve().parent
@@ -327,6 +328,24 @@ def check(lib: C.CDLL, rc: int, fn: str, ctx=None) -> None:
 # ---- descriptor helpers -------------------------------------------------------------------
 
 
+# Descriptors are packed as bytes in one call: a launch through the Python API builds several of
+# them, and setting a ctypes structure element by element costs about 5 us each.
+_FIELD = struct.Struct("P2i3i3i3ii3q")
+_GRID = struct.Struct("i3i3d3d3d3d")
+_BC = struct.Struct("6i6d6P")
+assert (_FIELD.size, _GRID.size, _BC.size) == (C.sizeof(cg_field), C.sizeof(cg_grid), C.sizeof(cg_bc))
+FIELD_ABSENT = bytes(_FIELD.size)
+
+
+def field_bytes(ptr, dtype_code, n, loc, halo, strides) -> bytes:
+    """The bytes of a cg_field for memory at `ptr` (start of the padded allocation)."""
+    nd = len(n)
+    if nd == 2:
+        return _FIELD.pack(ptr or 0, dtype_code, 2, n[0], n[1], 1, loc[0], loc[1], 0, halo[0], halo[1], 0, 0, strides[0], strides[1], 0)
+    k = 3 - nd
+    return _FIELD.pack(ptr or 0, dtype_code, nd, *n, *(1,) * k, *loc, *(0,) * k, *halo, *(0,) * k, 0, *strides, *(0,) * k)
+
+
 def make_field(
     ptr: int,
     dtype_code: int,
@@ -336,18 +355,17 @@ def make_field(
     strides: tuple[int, ...],
 ) -> cg_field:
     """Build a cg_field for memory at `ptr` (start of the padded allocation)."""
-    nd = len(n)
-    f = cg_field()
-    f.data = ptr
-    f.dtype = dtype_code
-    f.ndim = nd
-    for d in range(3):
-        f.n[d] = n[d] if d < nd else 1
-        f.loc[d] = loc[d] if d < nd else 0
-        f.halo[d] = halo[d] if d < nd else 0
-        f.stride[d] = strides[d] if d < nd else 0
-    f.pad_ = 0
-    return f
+    return cg_field.from_buffer_copy(field_bytes(ptr, dtype_code, n, loc, halo, strides))
+
+
+def bytes_of(f) -> bytes:
+    """The cg_field bytes of anything that describes itself as a field."""
+    return f.desc_bytes() if hasattr(f, "desc_bytes") else bytes(f.desc())
+
+
+def make_bc(kinds, values, pointers) -> cg_bc:
+    """Build a cg_bc from its six kinds, values and value-array addresses, [dimension][side]."""
+    return cg_bc.from_buffer_copy(_BC.pack(*kinds, *values, *pointers))
 
 
 def empty_field() -> cg_field:
@@ -355,13 +373,11 @@ def empty_field() -> cg_field:
 
 
 def make_grid(n, origin, extent, spacing, inv_spacing) -> cg_grid:
-    g = cg_grid()
     nd = len(n)
-    g.ndim = nd
-    for d in range(3):
-        g.n[d] = n[d] if d < nd else 1
-        g.origin[d] = float(origin[d]) if d < nd else 0.0
-        g.extent[d] = float(extent[d]) if d < nd else 0.0
-        g.spacing[d] = float(spacing[d]) if d < nd else 1.0
-        g.inv_spacing[d] = float(inv_spacing[d]) if d < nd else 1.0
-    return g
+    k = 3 - nd
+
+    def pad(v, fill):
+        return [float(x) for x in v] + [fill] * k
+
+    return cg_grid.from_buffer_copy(
+        _GRID.pack(nd, *n, *(1,) * k, *pad(origin, 0.0), *pad(extent, 0.0), *pad(spacing, 1.0), *pad(inv_spacing, 1.0)))

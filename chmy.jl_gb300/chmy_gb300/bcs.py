@@ -216,16 +216,15 @@ def materialize_bc(grid, loc, dtype, spec, device=None, fns=None):
     evaluated on the host. Returns (cg_bc, keep): `keep` holds the arrays, and must stay alive
     while the cg_bc is used."""
     nd = grid.ndim
-    b = _abi.cg_bc()
     keep = []
+    kinds, values, pointers = [_abi.CG_BC_NONE] * 6, [0.0] * 6, [0] * 6
     for d, (l, r) in enumerate(regularise(nd, spec)):
         for s, bc in enumerate((l, r)):
             if bc is None:
-                b.kind[d][s] = _abi.CG_BC_NONE
                 continue
-            b.kind[d][s] = bc.kind
+            kinds[2 * d + s] = bc.kind
             if _constant(bc.value):
-                b.value[d][s] = 0.0 if bc.value is None else float(bc.value)
+                values[2 * d + s] = 0.0 if bc.value is None else float(bc.value)
                 continue
             dfn = device_function_of(bc) if fns is not None else None
             if dfn is not None and bc.kind in (_abi.CG_BC_DIRICHLET, _abi.CG_BC_NEUMANN):
@@ -241,11 +240,11 @@ def materialize_bc(grid, loc, dtype, spec, device=None, fns=None):
 
                 t = torch.from_numpy(arr).to(device)
                 keep.append(t)
-                b.values[d][s] = t.data_ptr()
+                pointers[2 * d + s] = t.data_ptr()
             else:
                 keep.append(arr)
-                b.values[d][s] = arr.ctypes.data
-    return b, keep
+                pointers[2 * d + s] = arr.ctypes.data
+    return _abi.make_bc(kinds, values, pointers), keep
 
 
 class Batch:
@@ -257,13 +256,17 @@ class Batch:
         self.bcs = []
         self.fns = []  # BoundaryFunction sides evaluated by the kernel (cg_bc_fn per field)
         self._keep = []  # per-point value arrays on the fields' device
+        self._varying = False  # some condition's value is not a constant
         for f, spec in pairs:
             dev = getattr(getattr(f, "arch", None), "device", None)
+            sides = regularise(grid.ndim, spec)
+            if all(l is None and r is None for l, r in sides):
+                continue  # prune (batch.jl:235-239)
             fn = _abi.cg_bc_fn() if dev is not None else None
             b, keep = materialize_bc(grid, f.loc, f.dtype, spec, dev, fn)
             self._keep.extend(keep)
-            if all(b.kind[d][s] == _abi.CG_BC_NONE for d in range(grid.ndim) for s in range(2)):
-                continue  # prune (batch.jl:235-239)
+            if not all(bc is None or _constant(bc.value) for lr in sides for bc in lr):
+                self._varying = True
             self.fields.append(f)
             self.bcs.append(b)
             self.fns.append(fn if fn is not None else _abi.cg_bc_fn())
@@ -273,12 +276,12 @@ class Batch:
 
     def descs(self):
         n = len(self.fields)
-        fa = (_abi.cg_field * max(n, 1))(*[f.desc() for f in self.fields])
+        fa = (_abi.cg_field * max(n, 1)).from_buffer_copy(b"".join(_abi.bytes_of(f) for f in self.fields) or _abi.FIELD_ABSENT)
         ba = (_abi.cg_bc * max(n, 1))(*self.bcs)
         return n, fa, ba
 
     def has_functions(self) -> bool:
-        return any(fn.fn[d][s].kind != _abi.CG_FN_NONE for fn in self.fns for d in range(3) for s in range(2))
+        return self._varying and any(fn.fn[d][s].kind != _abi.CG_FN_NONE for fn in self.fns for d in range(3) for s in range(2))
 
 
 def batch(grid, *pairs, exchange=None) -> Batch:
@@ -293,6 +296,9 @@ def apply_batch(arch, grid, b: Batch) -> None:
     n, fa, ba = b.descs()
     g = grid.desc()
     with_fn = b.has_functions()
+    if n <= 8 and not with_fn:
+        arch.call("cg_bc_apply", ctypes.byref(g), n, fa, ba)
+        return
     # the library takes up to 8 fields per launch
     for start in range(0, n, 8):
         cnt = min(8, n - start)

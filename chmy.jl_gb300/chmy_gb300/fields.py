@@ -45,6 +45,7 @@ class Field:
         self.grid = grid
         nd = grid.ndim
         self.loc = expand_loc(nd, loc)
+        self._loc_codes = tuple(l.code for l in self.loc)
         self.dtype = _np_type(dtype if dtype is not None else grid.dtype)
         self.halo = tuple(halo) if isinstance(halo, (tuple, list)) else tuple(int(halo) for _ in range(nd))
         if any(h < 1 for h in self.halo):
@@ -80,20 +81,20 @@ class Field:
     def size(self) -> tuple[int, ...]:
         return self.dims
 
+    def desc_bytes(self) -> bytes:
+        """The bytes of the field's cg_field."""
+        data = self.data
+        return _abi.field_bytes(data.data_ptr(), _CODE[self.dtype], self.dims, self._loc_codes, self.halo, data.stride()[::-1])
+
     def desc(self) -> _abi.cg_field:
-        strides = tuple(reversed(self.data.stride()))
-        return _abi.make_field(
-            self.data.data_ptr(),
-            _CODE[self.dtype],
-            self.dims,
-            tuple(l.code for l in self.loc),
-            self.halo,
-            strides,
-        )
+        return _abi.cg_field.from_buffer_copy(self.desc_bytes())
 
     # -- host transfer helpers (padded array, stored [z, y, x]) --
     def to_numpy(self) -> np.ndarray:
-        return self.data.detach().cpu().numpy().copy()
+        host = self.data.detach().cpu()
+        if self.data.device.type == "cpu":
+            host = host.clone()
+        return np.ascontiguousarray(host.numpy())
 
     def from_numpy(self, arr: np.ndarray) -> None:
         arr = np.asarray(arr, dtype=self.dtype)

@@ -131,6 +131,7 @@ class UniformGrid:
         self.dtype = np.dtype(dtype).type
         self.axes = tuple(UniformAxis(o, e, n, self.dtype) for o, e, n in zip(origin, extent, dims))
         self.dims = dims
+        self._desc = None
 
     @property
     def ndim(self) -> int:
@@ -176,13 +177,15 @@ class UniformGrid:
         return Bounded()
 
     def desc(self) -> _abi.cg_grid:
-        return _abi.make_grid(
-            self.dims,
-            [ax.origin for ax in self.axes],
-            [ax.extent for ax in self.axes],
-            [ax.spacing for ax in self.axes],
-            [ax.inv_spacing for ax in self.axes],
-        )
+        if self._desc is None:  # the axes do not change after construction
+            self._desc = bytes(_abi.make_grid(
+                self.dims,
+                [ax.origin for ax in self.axes],
+                [ax.extent for ax in self.axes],
+                [ax.spacing for ax in self.axes],
+                [ax.inv_spacing for ax in self.axes],
+            ))
+        return _abi.cg_grid.from_buffer_copy(self._desc)
 
     def __repr__(self):
         return f"UniformGrid(dims={self.dims}, dtype={self.dtype.__name__})"

@@ -33,13 +33,11 @@ class CellViscosity:
 
 
 def _vec(fields, n=3):
-    arr = (_abi.cg_field * n)()
-    if fields is None:
-        return arr
-    for i, f in enumerate(fields):
-        if f is not None:
-            arr[i] = f.desc()
-    return arr
+    parts = [_abi.FIELD_ABSENT if f is None else _abi.bytes_of(f) for f in fields] if fields is not None else []
+    if len(parts) > n:
+        raise IndexError(f"{len(parts)} fields where the library takes {n}")
+    parts += [_abi.FIELD_ABSENT] * (n - len(parts))
+    return (_abi.cg_field * n).from_buffer_copy(b"".join(parts))
 
 
 def stokes_fields(
