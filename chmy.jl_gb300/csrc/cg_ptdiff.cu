@@ -311,7 +311,8 @@ struct PDM {
     T* qn[3];
     const T* Co;
     const T* D;
-    int s1, s2;  // row and plane strides shared by every array
+    int s1, s2;        // row and plane strides of C, D, C_old and q.z
+    int s1x, s2x, s2y;  // q.x's, and q.y's plane stride (equal to s1, s2, s2 in a pool layout)
     T idx[3], om, inv_dt, dtc;
 };
 
@@ -434,6 +435,178 @@ __global__ void __launch_bounds__(32 * NW, MINB)
     }
 }
 
+// ---- the iteration with several rows per thread ------------------------------------------------
+//
+// ptd_march3d_kernel and its TMA-fed form spend about 260 instructions per cell: a row computes both
+// its y faces, and every value a thread reads from its neighbours costs an address and a guard. Here a
+// warp owns 30 columns (lane l holds column i0 - 1 + l) by R rows and marches up a z segment with the
+// C and D of its R + 2 rows in registers: x neighbours by shuffle, y neighbours and the shared y faces
+// in registers, each z face carried up. No value is loaded twice but the two halo rows and lanes,
+// every face of the tile is computed once, and there is neither shared memory nor a barrier. Same operations and guards as
+// ptd_march3d_kernel, so the same bits. It reads the strides of q.x and q.y apart from C's, so Chmy's
+// dense layout takes it too.
+//
+// bc!(C) is folded into the stores (PdEdge): the thread that updates a cell beside a boundary writes
+// the ghost cells that follow it, in cg_bc_apply's order (z, then y, then x), and a ghost cell under a
+// rule is not stored by itself.
+// Measured, an iteration with its bc!: 128^3 in the pool layout 32.5 -> 27 us (a solve 18.5 -> 15.7 ms),
+// 60 x 77 x 50 a solve 6.3 -> 2.6 ms, and 191 x 160 x 128 in the dense layout, which ran the flux and
+// update kernels apart, 55.9 -> 47.4 us. From about 200^3 on the TMA-fed kernel is ahead (384^3: 435 us
+// against 504), so it stays a candidate. Three rows per thread (112 registers, 4 blocks per SM) beat four,
+// two are best on the smallest grids; the loads of the next plane are in flight while a plane is
+// computed (without that 37 us at 128^3). Short z segments (3 to 12 planes) fill the SMs of small grids.
+template <class T>
+struct PdEdge {
+    int r[3][2];  // [dimension][side]: 0 none, 1 Dirichlet (2 v - C), 2 Neumann (C -/+ h v)
+    T v[3][2], h[3];
+};
+
+template <class T>
+__device__ __forceinline__ T pd_edge(const PdEdge<T>& e, int d, int s, T c) {
+    return e.r[d][s] == 1 ? cgk::rfma(T(2), cgk::rsub(e.v[d][s], c), c) : cgk::rfma(e.h[d], e.v[d][s], c);
+}
+
+template <class T, int R>
+struct PdPlane {
+    T c[R + 2], d[R + 2], qz[R], qx[R], qy[R + 1], co[R];
+};
+
+template <class T, int R, int MINB>
+__global__ void __launch_bounds__(128, MINB)
+    ptd_rows_kernel(const PDM<T> f, const PdEdge<T> er, int e0, int e1, int e2, int nstrip, int nty, int nwarps, int seg_len) {
+    using namespace cgk;
+    constexpr unsigned FULL = 0xffffffffu;
+    cg_dep_wait();
+    cg_dep_release();
+    const int lane = threadIdx.x & 31, gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (gw >= nwarps) return;  // whole warp
+    const int ks = gw / (nstrip * nty) * seg_len;
+    if (ks > e2) return;  // whole warp
+    const int ke = min(ks + seg_len - 1, e2);
+    const int i = (gw % nstrip) * 30 - 1 + lane, jb = (gw / nstrip) % nty * R;
+    const bool cx = i <= e0;      // C, D, C_old readable
+    const bool lx = i <= e0 + 1;  // column e0+1 passes its stored x flux to the lane below
+    const bool own = lane >= 1 && lane <= 30 && cx;
+    const bool x0 = i == 1 && er.r[0][0], x1 = i == e0 - 1 && er.r[0][1];  // writes an x ghost
+    const bool xg = (i == 0 && er.r[0][0]) || (i == e0 && er.r[0][1]);     // is one
+    int o = i + (jb - 1) * f.s1 + ks * f.s2, ox = i + jb * f.s1x + ks * f.s2x, oy = i + jb * f.s1 + ks * f.s2y;
+    T c[R + 2], d[R + 2], qzl[R];
+#pragma unroll
+    for (int r = 0; r < R + 2; ++r) {
+        const bool ok = cx && jb - 1 + r <= e1;
+        c[r] = ok ? __ldg(f.C + o + r * f.s1) : T(0);
+        d[r] = ok ? __ldg(f.D + o + r * f.s1) : T(0);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int p = o + (r + 1) * f.s1;
+        const bool ok = cx && jb + r <= e1;
+        const T cd = ok ? __ldg(f.C + p - f.s2) : T(0), dd = ok ? __ldg(f.D + p - f.s2) : T(0), q = ok ? __ldg(f.q[2] + p) : T(0);
+        qzl[r] = pd_face(q, dd, d[r + 1], cd, c[r + 1], f.idx[2], f.om);
+    }
+    // plane k's fluxes and C_old, and plane k+1's C, D and z flux, one plane ahead of their use
+    PdPlane<T, R> cur;
+    auto load = [&](PdPlane<T, R>& n, int k) {
+        const bool zu = k + 1 <= e2;
+#pragma unroll
+        for (int r = 0; r < R; ++r) n.qx[r] = lx && jb + r <= e1 ? __ldg(f.q[0] + ox + r * f.s1x) : T(0);
+#pragma unroll
+        for (int r = 0; r < R + 1; ++r) n.qy[r] = cx && jb + r <= e1 + 1 ? __ldg(f.q[1] + oy + r * f.s1) : T(0);
+#pragma unroll
+        for (int r = 0; r < R + 2; ++r) {
+            const bool ok = cx && zu && jb - 1 + r <= e1;
+            n.c[r] = ok ? __ldg(f.C + o + r * f.s1 + f.s2) : T(0);
+            n.d[r] = ok ? __ldg(f.D + o + r * f.s1 + f.s2) : T(0);
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const bool ok = cx && jb + r <= e1;
+            n.qz[r] = ok ? __ldg(f.q[2] + o + (r + 1) * f.s1 + f.s2) : T(0);
+            n.co[r] = ok ? __ldg(f.Co + o + (r + 1) * f.s1) : T(0);
+        }
+    };
+    load(cur, ks);
+    for (int k = ks; k <= ke; ++k) {
+        const bool zu = k + 1 <= e2;
+        PdPlane<T, R> nxt;
+        const int p0 = o, px = ox, py = oy;
+        o += f.s2;
+        ox += f.s2x;
+        oy += f.s2y;
+        if (k < ke) load(nxt, k + 1);
+        T* qy = cur.qy;
+        // a face beyond the launch range keeps its stored value
+#pragma unroll
+        for (int r = 0; r < R + 1; ++r)
+            if (jb + r <= e1) qy[r] = pd_face(qy[r], d[r], d[r + 1], c[r], c[r + 1], f.idx[1], f.om);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int j = jb + r;
+            const T cc = c[r + 1], dc = d[r + 1];
+            const T cl = __shfl_up_sync(FULL, cc, 1), dl = __shfl_up_sync(FULL, dc, 1);
+            const T qxl = cx ? pd_face(cur.qx[r], dl, dc, cl, cc, f.idx[0], f.om) : cur.qx[r];
+            const T qxu = __shfl_down_sync(FULL, qxl, 1);
+            const T qzu = zu ? pd_face(cur.qz[r], dc, cur.d[r + 1], cc, cur.c[r + 1], f.idx[2], f.om) : cur.qz[r];
+            T dv = rmul(rsub(qxu, qxl), f.idx[0]);
+            dv = radd(dv, rmul(rsub(qy[r + 1], qy[r]), f.idx[1]));
+            dv = radd(dv, rmul(rsub(qzu, qzl[r]), f.idx[2]));
+            const T rr = rsub(rmul(-rsub(cc, cur.co[r]), f.inv_dt), dv);
+            const T v = radd(cc, rmul(rr, f.dtc));
+            if (own && j <= e1) {
+                const int p = p0 + (r + 1) * f.s1;
+                f.qn[0][px + r * f.s1x] = qxl;
+                f.qn[1][py + r * f.s1] = qy[r];
+                f.qn[2][p] = qzl[r];
+                const bool ghost = xg || (j == 0 && er.r[1][0]) || (j == e1 && er.r[1][1]) || (k == 0 && er.r[2][0]) ||
+                                   (k == e2 && er.r[2][1]);
+                if (!ghost) {
+                    auto put_x = [&](int q, T x) {
+                        f.Cn[q] = x;
+                        if (x0) f.Cn[q - 1] = pd_edge(er, 0, 0, x);
+                        if (x1) f.Cn[q + 1] = pd_edge(er, 0, 1, x);
+                    };
+                    auto put_y = [&](int q, T x) {
+                        put_x(q, x);
+                        if (j == 1 && er.r[1][0]) put_x(q - f.s1, pd_edge(er, 1, 0, x));
+                        if (j == e1 - 1 && er.r[1][1]) put_x(q + f.s1, pd_edge(er, 1, 1, x));
+                    };
+                    put_y(p, v);
+                    if (k == 1 && er.r[2][0]) put_y(p - f.s2, pd_edge(er, 2, 0, v));
+                    if (k == e2 - 1 && er.r[2][1]) put_y(p + f.s2, pd_edge(er, 2, 1, v));
+                }
+            }
+            qzl[r] = qzu;
+        }
+#pragma unroll
+        for (int r = 0; r < R + 2; ++r) {
+            c[r] = cur.c[r];
+            d[r] = cur.d[r];
+        }
+        cur = nxt;
+    }
+}
+
+// The rules of bc! that ptd_rows_kernel folds into its stores; false (and none set) where it cannot:
+// periodic sides and per-point values.
+template <class T>
+bool pd_edges(const cg_grid* g, const cg_bc* bc, PdEdge<T>* er) {
+    std::memset(er, 0, sizeof(*er));
+    if (!bc) return true;
+    PdEdge<T> e = *er;
+    for (int d = 0; d < 3; ++d) {
+        e.h[d] = (T)g->spacing[d];
+        for (int s = 0; s < 2; ++s) {
+            const int k = bc->kind[d][s];
+            if (bc->values[d][s] || (k != CG_BC_NONE && k != CG_BC_DIRICHLET && k != CG_BC_NEUMANN)) return false;
+            e.r[d][s] = k == CG_BC_DIRICHLET ? 1 : k == CG_BC_NEUMANN ? 2 : 0;
+            const T v = (T)bc->value[d][s];
+            e.v[d][s] = k == CG_BC_NEUMANN && s == 0 ? -v : v;
+        }
+    }
+    *er = e;
+    return true;
+}
+
 // z planes per segment: the count of segments that fills the SMs' resident blocks in whole
 // waves most evenly, with segments of at least 16 planes
 inline int pd_seg_len(long tiles, int planes, long resident) {
@@ -467,6 +640,22 @@ cudaError_t launch_pd_ix(const PDM<T>& f, const cg_grid* g, int num_sms, cudaStr
     const int nseg = cg_div_up(e2 + 1, seg);
     ptd_march3d_kernel<T, NW, MINB><<<(unsigned)(tiles * nseg), 32 * NW, 0, st>>>(f, e0, e1, e2, ntx, nty, seg);
     return cudaGetLastError();
+}
+
+template <class T, int R, int MINB>
+cudaError_t launch_pd_rows(const PDM<T>& f, const PdEdge<T>& er, const cg_grid* g, int num_sms, cudaStream_t st, int seg, bool dep) {
+    const int e0 = g->n[0] + 1, e1 = g->n[1] + 1, e2 = g->n[2] + 1;
+    const int nstrip = cg_div_up(e0 + 1, 30), nty = cg_div_up(e1 + 1, R);
+    static const int bps = [] {
+        int nb = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ptd_rows_kernel<T, R, MINB>, 128, 0) != cudaSuccess) nb = 0;
+        return nb > 0 ? nb : 1;
+    }();
+    const long tiles = (long)nstrip * nty;
+    if (seg <= 0) seg = pd_seg_len(tiles, e2 + 1, (long)num_sms * bps * 4);
+    const int nwarps = (int)(tiles * cg_div_up(e2 + 1, seg));
+    return cg_launch(ptd_rows_kernel<T, R, MINB>, dim3(cg_div_up(nwarps, 4)), dim3(128), 0, st, dep, f, er, e0, e1, e2, nstrip, nty,
+                     nwarps, seg);
 }
 
 }  // namespace
@@ -539,12 +728,17 @@ cudaError_t launch_pd_tma(const PDM<float>& f, const cg_grid* g, int num_sms, cu
 // ptd_tma_kernel (inputs staged by TMA; only with tensor maps for the direction), rings of 4
 // planes with the shared memory of the widest boxes: blocks of 8, 16, 20 and 24 rows (at 512^3
 // 24 rows, 2 blocks per SM, measured fastest; 32 rows, 1 block per SM, 27 % slower).
-constexpr int kPdVariants = 8;
+// Variants 8 and 9, ptd_rows_kernel: 3 rows per thread and 2; the only ones that take a layout whose
+// arrays do not share their strides, and the only ones that fold bc! into their stores.
+constexpr int kPdVariants = 10;
 constexpr int kPdTmaFirst = 4;
+constexpr int kPdRowsFirst = 8;
 
 template <class T>
 cudaError_t launch_pd_march3d(const PDM<T>& f, const cg_grid* g, int num_sms, cudaStream_t st, int variant,
-                              const PdDir& dir = PdDir{}) {
+                              const PdDir& dir = PdDir{}, const PdEdge<T>& er = PdEdge<T>{}, int seg = 0, bool dep = false) {
+    if (variant == kPdRowsFirst) return launch_pd_rows<T, 3, 4>(f, er, g, num_sms, st, seg, dep);
+    if (variant > kPdRowsFirst) return launch_pd_rows<T, 2, 5>(f, er, g, num_sms, st, seg, dep);
     if constexpr (sizeof(T) == 4) {
         if (variant >= kPdTmaFirst && dir.m[0]) {
             const int h = variant - kPdTmaFirst;
@@ -564,7 +758,7 @@ cudaError_t launch_pd_march3d(const PDM<T>& f, const cg_grid* g, int num_sms, cu
     }
 }
 
-// CG_PTD_VARIANT=<0..7> in the environment (read on every call): the fused iteration's layout
+// CG_PTD_VARIANT=<0..9> in the environment (read on every call): the fused iteration's layout
 // instead of the autotuner's (a TMA variant only where its tensor maps exist).
 inline int pd_variant_forced() {
     const char* e = std::getenv("CG_PTD_VARIANT");
@@ -574,35 +768,53 @@ inline int pd_variant_forced() {
 }
 
 // The fastest layout for this grid and layout, timed on the run's own buffers before its graph
-// is captured (the launch writes only the partner buffers) and cached for the process.
-template <class T>
-int tune_pd(const PDM<T>& f, const cg_grid* g, int num_sms, cudaStream_t st, const PdDir& dir = PdDir{}) {
+// is captured (the launches write only the partner buffers) and cached for the process. `after` is the
+// bc! launch that follows an iteration which does not fold it, timed with it.
+template <class T, class F>
+cg_tune_cfg tune_pd(const PDM<T>& f, const cg_grid* g, int num_sms, cudaStream_t st, const PdDir& dir, const PdEdge<T>& er, F&& after) {
     const bool tma = dir.m[0] != nullptr;
+    const bool one = f.s1x == f.s1 && f.s2x == f.s2 && f.s2y == f.s2;
+    const int first = one ? 0 : kPdRowsFirst;
     const int forced = pd_variant_forced();
-    if (forced >= 0) return (forced >= kPdTmaFirst && !tma) ? 0 : forced;
-    if (!cg_autotune_enabled()) return 0;
+    if (forced >= 0) return {0, forced < first ? first : (forced >= kPdTmaFirst && forced < kPdRowsFirst && !tma) ? 0 : forced};
+    if (!cg_autotune_enabled()) return {0, first};
     std::string key = "ptdiff3d";
     for (int d = 0; d < 3; ++d) cg_key_add(key, g->n[d]);
     cg_key_add(key, f.s1);
     cg_key_add(key, f.s2);
+    cg_key_add(key, f.s1x);
     cg_key_add(key, num_sms);
     cg_key_add(key, (int)tma);
-    cg_tune_cfg best{0, 0};
-    if (cg_tune_lookup(key, &best)) return best.variant;
+    cg_tune_cfg best{0, first};
+    if (cg_tune_lookup(key, &best)) return best;
     float tbest = 1e30f;
-    for (int v = 0; v < (tma ? kPdVariants : kPdTmaFirst); ++v) {
-        const float t = cgk::time_launches([&] { return launch_pd_march3d<T>(f, g, num_sms, st, v, dir); }, st);
-        if (cg_tune_verbose())
-            std::fprintf(stderr, "ptdiff3d tune %dx%dx%d: variant %d: %.1f us\n", g->n[0], g->n[1], g->n[2], v,
-                         t >= 0.f ? 1e3f * t / 3 : -1.f);
-        if (t >= 0.f && t < tbest) {
-            tbest = t;
-            best = cg_tune_cfg{0, v};
+    for (int v = first; v < kPdVariants; ++v) {
+        if (v >= kPdTmaFirst && v < kPdRowsFirst && !tma) continue;
+        for (int seg : {0, 3, 6, 12}) {
+            if (seg && (v < kPdRowsFirst || seg > g->n[2] + 2)) continue;
+            const float t = cgk::time_launches(
+                [&] {
+                    const cudaError_t e = launch_pd_march3d<T>(f, g, num_sms, st, v, dir, er, seg);
+                    return e != cudaSuccess || v >= kPdRowsFirst ? e : after();
+                },
+                st);
+            if (cg_tune_verbose())
+                std::fprintf(stderr, "ptdiff3d tune %dx%dx%d: variant %d seg %d: %.1f us\n", g->n[0], g->n[1], g->n[2], v, seg,
+                             t >= 0.f ? 1e3f * t / 3 : -1.f);
+            if (t >= 0.f && t < tbest) {
+                tbest = t;
+                best = cg_tune_cfg{seg, v};
+            }
         }
     }
     cudaGetLastError();
     cg_tune_store(key, best);
-    return best.variant;
+    return best;
+}
+
+// bc! of one field as a launch, for tune_pd.
+inline auto pd_bc_after(cg_ctx* ctx, const cg_grid* g, const cg_field& C, const cg_bc* bc) {
+    return [=] { return !bc || cg_bc_apply_impl(ctx, g, 1, &C, bc) == CG_OK ? cudaSuccess : cudaErrorUnknown; };
 }
 
 template <class T>
@@ -621,6 +833,9 @@ PDM<T> make_pdm(const cg_grid* g, const cg_field& C, const cg_field* q, const cg
     m.D = cg_view<T>(f->D).p;
     m.s1 = (int)C.stride[1];
     m.s2 = (int)C.stride[2];
+    m.s1x = (int)q[0].stride[1];
+    m.s2x = (int)q[0].stride[2];
+    m.s2y = (int)q[1].stride[2];
     m.om = (T)p->omega_q;
     m.inv_dt = T(1) / (T)p->dt;
     m.dtc = (T)p->dtau_C;
@@ -654,10 +869,14 @@ int run_fused3d(cg_ctx* ctx, const cg_grid* g, const cg_ptdiff_fields* f, const 
     if (rc) return rc;
     const PdTma tma = make_pd_tma(f->C, f->q, part[0], part + 1, f->D, f->C_old, err);
     const PdDir dab = pd_dir(tma, true), dba = pd_dir(tma, false);
-    const int variant = tune_pd<T>(ab, g, ctx->num_sms, ctx->stream, dab);
+    PdEdge<T> er;
+    const bool edges = pd_edges(g, bc, &er);
+    const cg_tune_cfg tc = tune_pd<T>(ab, g, ctx->num_sms, ctx->stream, dab, er, pd_bc_after(ctx, g, part[0], bc));
+    const int variant = tc.variant;
+    const bool staged = variant >= kPdTmaFirst && variant < kPdRowsFirst, fold = variant >= kPdRowsFirst && edges;
     cg_key_add(key, base);
-    cg_key_add(key, variant);
-    if (variant >= kPdTmaFirst) {
+    cg_key_add(key, tc);
+    if (staged) {
         // the maps encode this call's pointers, and the wait settings are kernel arguments:
         // both are part of the graph's key
         cg_key_add(key, tma.ab[variant - kPdTmaFirst]);
@@ -670,10 +889,11 @@ int run_fused3d(cg_ctx* ctx, const cg_grid* g, const cg_ptdiff_fields* f, const 
         for (int s = 0; s < nsteps; ++s) {
             CG_CUDA(ctx, cudaMemcpyAsync(f->C_old.data, f->C.data, bytes[0], cudaMemcpyDeviceToDevice, st));
             for (int it = 0; it < npt; ++it) {
-                const cudaError_t le =
-                    launch_pd_march3d<T>(it % 2 == 0 ? ab : ba, g, ctx->num_sms, st, variant, it % 2 == 0 ? dab : dba);
+                const cudaError_t le = launch_pd_march3d<T>(it % 2 == 0 ? ab : ba, g, ctx->num_sms, st, variant,
+                                                            it % 2 == 0 ? dab : dba, er, tc.seg, it > 0 && fold);
                 if (le != cudaSuccess) return cg_fail(ctx, CG_ERR_CUDA, "ptdiff fused launch: %s", cudaGetErrorString(le));
-                if (bc) {
+                // a folded bc! leaves the points at index n+2, which no iteration reads, to one launch
+                if (bc && (!fold || it == npt - 1)) {
                     int r = cg_bc_apply_impl(ctx, g, 1, it % 2 == 0 ? &part[0] : &f->C, bc);
                     if (r) return r;
                 }
@@ -685,20 +905,20 @@ int run_fused3d(cg_ctx* ctx, const cg_grid* g, const cg_ptdiff_fields* f, const 
         return (int)CG_OK;
     });
     if (rc) return rc;
-    return variant >= kPdTmaFirst ? cg_tma_check(ctx, err, "ptdiff fused iteration") : CG_OK;
+    return staged ? cg_tma_check(ctx, err, "ptdiff fused iteration") : CG_OK;
 }
 
-// The fused path needs a 3D FP32 grid, no residual output, and one row and plane stride for
-// C, C_old, D and the three fluxes (a common pitch and plane height, e.g. Field(...,
-// pitch_align, plane_rows)), with every offset in 32 bits.
+// The fused path needs a 3D FP32 grid, no residual output, one row and plane stride for C, C_old, D
+// and q.z, and C's row stride for q.y (Chmy's dense layout, or a common pitch and plane height), with
+// every offset in 32 bits.
 bool fused3d_ok(const cg_grid* g, const cg_ptdiff_fields* f) {
     if (g->ndim != 3 || f->C.dtype != CG_F32 || cg_present(f->R) || !cg_ptdiff_fused_enabled()) return false;
-    const cg_field* all[6] = {&f->C, &f->C_old, &f->D, &f->q[0], &f->q[1], &f->q[2]};
-    for (const cg_field* a : all)
-        for (int d = 1; d < 3; ++d)
-            if (a->stride[d] != f->C.stride[d]) return false;
-    const long last = (long)(g->n[0] + 3) + (long)(g->n[1] + 3) * f->C.stride[1] + (long)(g->n[2] + 3) * f->C.stride[2];
-    return last < 2147483647L;
+    for (const cg_field* a : {&f->C_old, &f->D, &f->q[2]})
+        if (a->stride[1] != f->C.stride[1] || a->stride[2] != f->C.stride[2]) return false;
+    if (f->q[1].stride[1] != f->C.stride[1]) return false;
+    for (const cg_field* a : {&f->C, &f->q[0], &f->q[1]})
+        if ((long)(g->n[0] + 3) + (long)(g->n[1] + 3) * a->stride[1] + (long)(g->n[2] + 3) * a->stride[2] >= 2147483647L) return false;
+    return true;
 }
 
 }  // namespace
@@ -1069,7 +1289,11 @@ int solve_dc(cg_ctx* ctx, const cg_grid* g, const cg_ptdiff_fields* f, const cg_
     if (rc) return rc;
     const PdTma tma = make_pd_tma(dA, qA, dB, qB, D32, co, perr);
     const PdDir dab = pd_dir(tma, true), dba = pd_dir(tma, false);
-    const int variant = tune_pd<float>(ab, g, ctx->num_sms, ctx->stream, dab);
+    PdEdge<float> er;
+    const bool edges = pd_edges(g, &bc0, &er);
+    const cg_tune_cfg tc = tune_pd<float>(ab, g, ctx->num_sms, ctx->stream, dab, er, pd_bc_after(ctx, g, dB, &bc0));
+    const int variant = tc.variant;
+    const bool staged = variant >= kPdTmaFirst && variant < kPdRowsFirst, fold = variant >= kPdRowsFirst && edges;
     const int nchunk = std::max(2, o->ncheck + (o->ncheck & 1));
     std::string key = "ptdiff_dc_chunk";
     cg_key_add(key, *g);
@@ -1077,7 +1301,7 @@ int solve_dc(cg_ctx* ctx, const cg_grid* g, const cg_ptdiff_fields* f, const cg_
     cg_key_add(key, *p);
     cg_key_add(key, bc0);
     cg_key_add(key, nchunk);
-    cg_key_add(key, variant);
+    cg_key_add(key, tc);
     cg_key_add(key, cg_tma_wait_cfg());
     const dim3 ib(32, 8), ig(cg_div_up(g->n[0], 32), cg_div_up(g->n[1], 8), g->n[2]);
     int total = 0;
@@ -1108,8 +1332,9 @@ int solve_dc(cg_ctx* ctx, const cg_grid* g, const cg_ptdiff_fields* f, const cg_
             rc = cg_graph_run(ctx, key, [&](cudaStream_t st) {
                 for (int it = 0; it < nchunk; ++it) {
                     const cudaError_t le = launch_pd_march3d<float>(it % 2 == 0 ? ab : ba, g, ctx->num_sms, st, variant,
-                                                                    it % 2 == 0 ? dab : dba);
+                                                                    it % 2 == 0 ? dab : dba, er, tc.seg, it > 0 && fold);
                     if (le != cudaSuccess) return cg_fail(ctx, CG_ERR_CUDA, "ptdiff fused launch: %s", cudaGetErrorString(le));
+                    if (fold) continue;
                     int r = cg_bc_apply_impl(ctx, g, 1, it % 2 == 0 ? &dB : &dA, &bc0);
                     if (r) return r;
                 }
@@ -1130,7 +1355,7 @@ int solve_dc(cg_ctx* ctx, const cg_grid* g, const cg_ptdiff_fields* f, const cg_
                 break;  // the FP32 floor: back to the FP64 defect
             }
         }
-        if (variant >= kPdTmaFirst && (rc = cg_tma_check(ctx, perr, "ptdiff fused iteration"))) return rc;
+        if (staged && (rc = cg_tma_check(ctx, perr, "ptdiff fused iteration"))) return rc;
         pd_update_kernel<<<ig, ib, 0, ctx->stream>>>(cg_view<double>(f->C), cg_view<float>(dA), g->n[0], g->n[1], g->n[2]);
         CG_CHECK_LAUNCH(ctx);
         if ((rc = cg_bc_apply_impl(ctx, g, 1, &f->C, bc))) return rc;
