@@ -472,8 +472,9 @@ inline cudaError_t launch_march3d_ix(const Fused3D<T>& f, const SP<T>& s, int n0
 // Launch of the z-marching kernel over [0, n+1]^3; seg_len <= 0 picks the z-segment length;
 // dep = true makes it a dependent launch (cg_launch).
 // For FP32 with shared or class strides, variant 0 is 12 rows per block at 2 blocks per SM and
-// variant 1 is 8 rows per block at 3 blocks per SM (80 registers, no spills; the two best measured
-// of 4-16 rows per block and 1-5 blocks per SM at 256^3).
+// variant 1 is 8 rows per block at 3 blocks per SM (80 registers; the two best measured of 4-16 rows
+// per block and 1-5 blocks per SM at 256^3). Variant 4 is 8 rows with 122 registers and no spills, for
+// grids too small to fill the SMs.
 template <class T, bool WRITE_RES>
 inline cudaError_t launch_march3d(const Fused3D<T>& f, const SP<T>& s, int n0, int n1, int n2, int num_sms, int seg_len,
                                   cudaStream_t st, int variant = 0, bool dep = false) {
@@ -484,9 +485,11 @@ inline cudaError_t launch_march3d(const Fused3D<T>& f, const SP<T>& s, int n0, i
     if (lay == kLayOwn) return launch_march3d_ix<T, int, kLayOwn, WRITE_RES, 1>(f, s, n0, n1, n2, num_sms, seg_len, str, st, dep);
     if constexpr (sizeof(T) == 4) {
         if (lay == kLayOne) {
+            if (variant == 4) return launch_march3d_ix<T, int, kLayOne, WRITE_RES, 1, 8>(f, s, n0, n1, n2, num_sms, seg_len, str, st, dep);
             if (variant == 1) return launch_march3d_ix<T, int, kLayOne, WRITE_RES, 3, 8>(f, s, n0, n1, n2, num_sms, seg_len, str, st, dep);
             return launch_march3d_ix<T, int, kLayOne, WRITE_RES, 2, 12>(f, s, n0, n1, n2, num_sms, seg_len, str, st, dep);
         }
+        if (variant == 4) return launch_march3d_ix<T, int, kLayLoc, WRITE_RES, 1, 8>(f, s, n0, n1, n2, num_sms, seg_len, str, st, dep);
         if (variant == 1) return launch_march3d_ix<T, int, kLayLoc, WRITE_RES, 3, 8>(f, s, n0, n1, n2, num_sms, seg_len, str, st, dep);
         return launch_march3d_ix<T, int, kLayLoc, WRITE_RES, 2, 12>(f, s, n0, n1, n2, num_sms, seg_len, str, st, dep);
     } else {

@@ -531,18 +531,18 @@ inline cudaError_t launch_march3d_tma(const Fused3D<float>& f, const SP<float>& 
                      nstrip, nty, seg_len, (int)s1u, (int)s2u, d.xo, d.tx, d.present, wc.limit_ns, wc.withhold, err);
 }
 
-// Variants of the fused 3D iteration: 0 and 1 march3d_kernel (12 rows at 2 blocks per SM, 8 rows
-// at 3); 2 and 3 march3d_tma_kernel (12 rows at 2 blocks per SM, 8 rows at 3, rings of 3 planes),
-// only with the direction's tensor maps and otherwise variant 0.
-constexpr int kM3Variants = 4;
-constexpr int kM3TmaFirst = 2;
+// Variants of the fused 3D iteration: 0, 1 and 4 march3d_kernel (12 rows at 2 blocks per SM, 8 rows
+// at 3, 8 rows at 1); 2 and 3 march3d_tma_kernel (12 rows at 2 blocks per SM, 8 rows at 3, rings of 3
+// planes), only with the direction's tensor maps and otherwise variant 0.
+constexpr int kM3Variants = 5;
+inline bool m3_staged(int variant) { return variant == 2 || variant == 3; }
 
 template <class T, bool WRITE_RES>
 inline cudaError_t launch_march3d_any(const Fused3D<T>& f, const SP<T>& s, int n0, int n1, int n2, int num_sms,
                                       int seg_len, cudaStream_t st, int variant, bool dep, const M3Launch& l) {
     if constexpr (sizeof(T) == 4) {
-        if (variant >= kM3TmaFirst) {
-            const int h = variant - kM3TmaFirst;
+        if (m3_staged(variant)) {
+            const int h = variant - 2;
             MStr str;
             if (h < m3t::kHeights && l.dir[h] && l.dir[h]->ok && l.err && march3_layout(f, &str) == kLayOne &&
                 march3_fits_int(f, n0 + 1, n1 + 1, n2 + 1)) {
@@ -559,7 +559,7 @@ inline cudaError_t launch_march3d_any(const Fused3D<T>& f, const SP<T>& s, int n
             variant = 0;
         }
     }
-    return launch_march3d<T, WRITE_RES>(f, s, n0, n1, n2, num_sms, seg_len, st, variant >= kM3TmaFirst ? 0 : variant, dep);
+    return launch_march3d<T, WRITE_RES>(f, s, n0, n1, n2, num_sms, seg_len, st, m3_staged(variant) ? 0 : variant, dep);
 }
 
 // The autotuner of the fused 3D iteration: segment length and variant (the TMA variants where
@@ -570,7 +570,7 @@ inline cg_tune_cfg tune_march3d(const Fused3D<T>& f, const SP<T>& s, int n0, int
     cg_tune_cfg best{0, 0};
     const bool tma = sizeof(T) == 4 && l.dir[0] && l.dir[0]->ok && l.err;
     if (cg_tune_forced(&best)) {
-        if (best.variant >= kM3TmaFirst && !tma) best.variant = 0;
+        if (m3_staged(best.variant) && !tma) best.variant = 0;
         return best;
     }
     if (!cg_autotune_enabled()) return best;
@@ -586,11 +586,11 @@ inline cg_tune_cfg tune_march3d(const Fused3D<T>& f, const SP<T>& s, int n0, int
     cg_key_add(key, nsm);
     cg_key_add(key, (int)tma);
     if (cg_tune_lookup(key, &best)) return best;
-    const int nvar = (sizeof(T) == 4 && lay != kLayOwn) ? (tma ? kM3Variants : 2) : 1;
+    const int nvar = (sizeof(T) == 4 && lay != kLayOwn) ? kM3Variants : 1;
     float tbest = 1e30f;
     for (int v = 0; v < nvar; ++v)
-        for (int seg : {0, 16, 32, 64}) {
-            if (seg > n2 + 2) continue;
+        for (int seg : {0, 4, 8, 16, 32, 64}) {
+            if (seg > n2 + 2 || (m3_staged(v) && (!tma || (seg && seg < 16)))) continue;
             const float t = time_launches(
                 [&] { return launch_march3d_any<T, false>(f, s, n0, n1, n2, nsm, seg, st, v, false, l); }, st);
             if (cg_tune_verbose())

@@ -717,7 +717,7 @@ int pp_iterations_3d(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* a, c
     }
     const M3Launch lab = m3_launch_of(&tma, true), lba = m3_launch_of(&tma, false);
     const cg_tune_cfg tc = tune_march3d(fab, s, g->n[0], g->n[1], g->n[2], ctx->num_sms, ctx->stream, lab);
-    const bool staged = tma.ok && tc.variant >= kM3TmaFirst;
+    const bool staged = tma.ok && m3_staged(tc.variant);
     std::string key = "stokes_pp3";
     cg_key_add(key, tc);
     if (staged) cg_key_add(key, cg_tma_wait_cfg());

@@ -539,7 +539,7 @@ int cg_stokes_solve_dc(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f,
     const cg_tune_cfg tc = nd == 2 ? tune_march2d(fa, s32, g->n[0], g->n[1], ctx->num_sms, ctx->stream)
                                    : tune_march3d(ga, s32, g->n[0], g->n[1], g->n[2], ctx->num_sms, ctx->stream, lga);
     cg_key_add(key, tc);
-    const bool staged = nd == 3 && tma.ok && tc.variant >= kM3TmaFirst;
+    const bool staged = nd == 3 && tma.ok && m3_staged(tc.variant);
     if (staged) cg_key_add(key, cg_tma_wait_cfg());
     // several iterations per launch (the tuner's variants 1 and up) where bc!(dV) is folded into the
     // reads: an even number of launches A -> B -> A, so that the chunk ends in A. The buffers of the
