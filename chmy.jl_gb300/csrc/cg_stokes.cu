@@ -79,10 +79,10 @@ int check_body(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, const c
     return CG_OK;
 }
 
-// The coefficients of a loop of FP64 PT iterations (PtCoef): scalars, and with a variable
-// viscosity arrays in scratch slot 2 (dense Center layout, halo 1).
+// The coefficients of a loop of FP64 PT iterations with variable viscosity (PtCoef): arrays in
+// scratch slot 2 (dense Center layout, halo 1). base = nullptr: the loop runs stress_kernel and
+// velocity_kernel.
 struct LoopCoef {
-    bool on = false;      // the loop runs stress_loop_kernel and velocity_loop_kernel
     char* base = nullptr;
     long s1 = 0, s2 = 0, count = 0;  // element strides and elements per array
     int own_ieta = 0;                // 1/eta computed here (the caller gave only eta)
@@ -107,13 +107,6 @@ PtCoef<T> loop_coef(const cg_grid* g, const cg_stokes_params* p, const SV<T>& v,
     for (int d = 0; d < 3; ++d) {
         c.idx[d] = s.idx[d];
         c.idx2[d] = T(2) * s.idx[d];
-    }
-    if (!lc.base) {
-        c.ieta_s = T(1) / s.eta;
-        c.cP_s = T(0.5) * (s.eta_ve * s.dtau_Pr);
-        c.cT_s = s.eta_ve * s.dtau_r;
-        c.step_s = s.nu_dtau / s.eta_ve;
-        return c;
     }
     int idx = 0;
     c.ieta = lc.own_ieta ? coef_view<T>(lc, idx++) : v.ieta;
@@ -142,11 +135,7 @@ __global__ void inv_kernel(DF<T> dst, DF<T> src, int lo, int e0, int e1, int e2)
 template <class T, int ND>
 int setup_coef(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p, int niter, LoopCoef* lc) {
     *lc = LoopCoef{};
-    if (sizeof(T) != 8 || niter < 2) return CG_OK;
-    if (!cg_present(f->eta) && !cg_present(f->inv_eta)) {
-        lc->on = true;
-        return CG_OK;
-    }
+    if (sizeof(T) != 8 || niter < 2 || (!cg_present(f->eta) && !cg_present(f->inv_eta))) return CG_OK;
     const long e0 = g->n[0] + 4, e1 = g->n[1] + 4, e2 = ND > 2 ? g->n[2] + 4 : 1;
     lc->s1 = e0;
     lc->s2 = ND > 2 ? e0 * e1 : 0;
@@ -160,7 +149,6 @@ int setup_coef(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, const c
         *lc = LoopCoef{};
         return CG_OK;
     }
-    lc->on = true;
     SV<T> v = views<T>(f, ND);
     const PtCoef<T> c = loop_coef<T, ND>(g, p, v, *lc);
     const dim3 block(32, 8);
@@ -187,63 +175,58 @@ FieldMaskW<T> mask_views(const cg_mask* m) {
     return w;
 }
 
-// update_stress! over [0, n+1]^N with operand reader m, by the loop's kernel where lc is on.
+// update_stress! over [0, n+1]^N with operand reader m, by the loop's kernel where lc has arrays; dep:
+// a dependent launch.
 template <class T, int ND, class M>
 void stress_launch(const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p, bool res, const LoopCoef* lc,
-                   const M& m, dim3 block, cudaStream_t st) {
+                   const M& m, dim3 block, cudaStream_t st, bool dep) {
     const SV<T> v = views<T>(f, ND);
     const dim3 grid = range_grid<ND>(g, block);
     const int e0 = g->n[0] + 1, e1 = g->n[1] + 1;
     if constexpr (sizeof(T) == 8) {
-        if (lc && lc->on) {
+        if (lc && lc->base) {
             const PtCoef<T> c = loop_coef<T, ND>(g, p, v, *lc);
-            if (lc->base && res) stress_loop_kernel<T, ND, true, true, M><<<grid, block, 0, st>>>(v, c, e0, e1, m);
-            else if (lc->base) stress_loop_kernel<T, ND, false, true, M><<<grid, block, 0, st>>>(v, c, e0, e1, m);
-            else if (res) stress_loop_kernel<T, ND, true, false, M><<<grid, block, 0, st>>>(v, c, e0, e1, m);
-            else stress_loop_kernel<T, ND, false, false, M><<<grid, block, 0, st>>>(v, c, e0, e1, m);
+            if (res) cg_launch(stress_loop_kernel<T, ND, true, M>, grid, block, 0, st, dep, v, c, e0, e1, m);
+            else cg_launch(stress_loop_kernel<T, ND, false, M>, grid, block, 0, st, dep, v, c, e0, e1, m);
             return;
         }
     }
     const SP<T> s = scalars<T>(g, p);
-    if (res)
-        stress_kernel<T, ND, true, M><<<grid, block, 0, st>>>(v, s, e0, e1, m);
-    else
-        stress_kernel<T, ND, false, M><<<grid, block, 0, st>>>(v, s, e0, e1, m);
+    const ScalarDiv<T> sd = scalar_divs(s);
+    if (res) cg_launch(stress_kernel<T, ND, true, M>, grid, block, 0, st, dep, v, s, sd, e0, e1, m);
+    else cg_launch(stress_kernel<T, ND, false, M>, grid, block, 0, st, dep, v, s, sd, e0, e1, m);
 }
 
 template <class T, int ND, class M>
 void velocity_launch(const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p, bool res, const LoopCoef* lc,
-                     const M& m, dim3 block, cudaStream_t st) {
+                     const M& m, dim3 block, cudaStream_t st, bool dep) {
     const SV<T> v = views<T>(f, ND);
     const BodyFn<T> bf = body_fns<T>(g, p);
     const dim3 grid = range_grid<ND>(g, block);
     const int e0 = g->n[0] + 1, e1 = g->n[1] + 1;
     if constexpr (sizeof(T) == 8) {
-        if (lc && lc->on) {
+        if (lc && lc->base) {
             const PtCoef<T> c = loop_coef<T, ND>(g, p, v, *lc);
-            if (lc->base && res) velocity_loop_kernel<T, ND, true, true, M><<<grid, block, 0, st>>>(v, c, bf, e0, e1, m);
-            else if (lc->base) velocity_loop_kernel<T, ND, false, true, M><<<grid, block, 0, st>>>(v, c, bf, e0, e1, m);
-            else if (res) velocity_loop_kernel<T, ND, true, false, M><<<grid, block, 0, st>>>(v, c, bf, e0, e1, m);
-            else velocity_loop_kernel<T, ND, false, false, M><<<grid, block, 0, st>>>(v, c, bf, e0, e1, m);
+            if (res) cg_launch(velocity_loop_kernel<T, ND, true, M>, grid, block, 0, st, dep, v, c, bf, e0, e1, m);
+            else cg_launch(velocity_loop_kernel<T, ND, false, M>, grid, block, 0, st, dep, v, c, bf, e0, e1, m);
             return;
         }
     }
     const SP<T> s = scalars<T>(g, p);
-    if (res)
-        velocity_kernel<T, ND, true, M><<<grid, block, 0, st>>>(v, s, bf, e0, e1, m);
-    else
-        velocity_kernel<T, ND, false, M><<<grid, block, 0, st>>>(v, s, bf, e0, e1, m);
+    const ScalarDiv<T> sd = scalar_divs(s);
+    if (res) cg_launch(velocity_kernel<T, ND, true, M>, grid, block, 0, st, dep, v, s, sd, bf, e0, e1, m);
+    else cg_launch(velocity_kernel<T, ND, false, M>, grid, block, 0, st, dep, v, s, sd, bf, e0, e1, m);
 }
 
 // update_stress! over [0, n+1]^N; with `mask`, every strain-rate derivative is the masked
 // operator ∂(V.d, ω, g, I) (src/GridOperators/masked_field_operators.jl:20-57).
 template <class T, int ND>
 cudaError_t stress_any(const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p, bool res,
-                       const LoopCoef* lc, const cg_mask* mask, dim3 block, cudaStream_t st) {
+                       const LoopCoef* lc, const cg_mask* mask, dim3 block, cudaStream_t st, bool dep = false) {
     if (mask)
-        stress_launch<T, ND>(g, f, p, res, lc, mask_views<T>(mask), block, st);
+        stress_launch<T, ND>(g, f, p, res, lc, mask_views<T>(mask), block, st, dep);
     else
-        stress_launch<T, ND>(g, f, p, res, lc, NoMask<T>{}, block, st);
+        stress_launch<T, ND>(g, f, p, res, lc, NoMask<T>{}, block, st, dep);
     return cudaGetLastError();
 }
 
@@ -251,26 +234,28 @@ cudaError_t stress_any(const cg_grid* g, const cg_stokes_fields* f, const cg_sto
 // masked operators.
 template <class T, int ND>
 cudaError_t velocity_any(const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p, bool res,
-                         const LoopCoef* lc, const cg_mask* mask, dim3 block, cudaStream_t st) {
+                         const LoopCoef* lc, const cg_mask* mask, dim3 block, cudaStream_t st, bool dep = false) {
     if (mask)
-        velocity_launch<T, ND>(g, f, p, res, lc, mask_views<T>(mask), block, st);
+        velocity_launch<T, ND>(g, f, p, res, lc, mask_views<T>(mask), block, st, dep);
     else
-        velocity_launch<T, ND>(g, f, p, res, lc, NoMask<T>{}, block, st);
+        velocity_launch<T, ND>(g, f, p, res, lc, NoMask<T>{}, block, st, dep);
     return cudaGetLastError();
 }
 
 template <class T, int ND>
 int launch_stress(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p, bool res,
-                  const LoopCoef* lc = nullptr, const cg_mask* mask = nullptr, dim3 block = dim3(32, 8)) {
-    const cudaError_t e = stress_any<T, ND>(g, f, p, res, lc, mask, block, ctx->stream);
+                  const LoopCoef* lc = nullptr, const cg_mask* mask = nullptr, dim3 block = dim3(32, 8),
+                  bool dep = false) {
+    const cudaError_t e = stress_any<T, ND>(g, f, p, res, lc, mask, block, ctx->stream, dep);
     if (e != cudaSuccess) return cg_fail(ctx, CG_ERR_CUDA, "update_stress: %s", cudaGetErrorString(e));
     return CG_OK;
 }
 
 template <class T, int ND>
 int launch_velocity(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p, bool res,
-                    const LoopCoef* lc = nullptr, const cg_mask* mask = nullptr, dim3 block = dim3(32, 8)) {
-    const cudaError_t e = velocity_any<T, ND>(g, f, p, res, lc, mask, block, ctx->stream);
+                    const LoopCoef* lc = nullptr, const cg_mask* mask = nullptr, dim3 block = dim3(32, 8),
+                  bool dep = false) {
+    const cudaError_t e = velocity_any<T, ND>(g, f, p, res, lc, mask, block, ctx->stream, dep);
     if (e != cudaSuccess) return cg_fail(ctx, CG_ERR_CUDA, "update_velocity: %s", cudaGetErrorString(e));
     return CG_OK;
 }
@@ -301,7 +286,7 @@ int stokes_blocks(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, cons
     cg_key_add(base, (int)sizeof(T));
     cg_key_add(base, f->V[0].stride);
     cg_key_add(base, f->tau[0].stride);
-    cg_key_add(base, (int)cg_present(f->eta) + 2 * (int)cg_present(f->inv_eta) + 4 * (lc && lc->on) + 8 * (mask != nullptr));
+    cg_key_add(base, (int)cg_present(f->eta) + 2 * (int)cg_present(f->inv_eta) + 4 * (lc && lc->base) + 8 * (mask != nullptr));
     cg_key_add(base, ctx->num_sms);
     const std::string ks = base + "stress", kv = base + "velocity";
     cg_tune_cfg c1{0, 0}, c2{0, 0};
@@ -399,7 +384,7 @@ int launch_thermal(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, con
 // Fused thermal step Tin -> Tout (update_thermal_flux! + update_thermal!) over the launch range.
 template <class T, int ND>
 int launch_thermal_step(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p,
-                        const cg_field& Tin, const cg_field& Tout, cudaStream_t st) {
+                        const cg_field& Tin, const cg_field& Tout, bool dep) {
     ThermalStep<T> a;
     std::memset(&a, 0, sizeof(a));
     a.Tin = cg_view<T>(Tin);
@@ -411,22 +396,15 @@ int launch_thermal_step(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f
     }
     a.mlam = -(T)p->lambda_rhoCp;
     a.dt = (T)p->dt;
-    dim3 block(32, 8);
-    thermal_step_kernel<T, ND><<<range_grid<ND>(g, block), block, 0, st>>>(a, g->n[0] + 1, g->n[1] + 1,
-                                                                          ND > 2 ? g->n[2] + 1 : 0);
-    CG_CHECK_LAUNCH(ctx);
+    const dim3 grid(cg_div_up(g->n[0] + 2, kThermalCols), cg_div_up(g->n[1] + 2, 8), ND > 2 ? g->n[2] + 2 : 1);
+    CG_CUDA(ctx, cg_launch(thermal_step_kernel<T, ND>, grid, dim3(32, 8), 0, ctx->stream, dep, a, g->n[0] + 1, g->n[1] + 1,
+                           ND > 2 ? g->n[2] + 1 : 0));
     return CG_OK;
 }
 
 #define SDISPATCH(fn, dtype, nd, ...)                                                              \
     ((dtype) == CG_F64 ? ((nd) == 2 ? fn<double, 2>(__VA_ARGS__) : fn<double, 3>(__VA_ARGS__))    \
                        : ((nd) == 2 ? fn<float, 2>(__VA_ARGS__) : fn<float, 3>(__VA_ARGS__)))
-
-// V boundary conditions of one PT iteration: bc!(V.d => bc_V[d]) as one batch.
-int apply_bc_V(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, const cg_bc* bc_V) {
-    if (!bc_V) return CG_OK;
-    return cg_bc_apply_impl(ctx, g, g->ndim, f->V, bc_V);
-}
 
 // The library's partner buffer of T for the thermal ping-pong (scratch slot 0, T's layout).
 int thermal_partner(cg_ctx* ctx, const cg_field& Tf, cg_field* out) {
@@ -459,7 +437,6 @@ int pt_iterations(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, cons
     std::memset(none, 0, sizeof(none));
     for (int d = 0; d < g->ndim; ++d) cg_key_add(key, bc_V ? bc_V[d] : none[d]);
     cg_key_add(key, lc ? lc->base : nullptr);
-    cg_key_add(key, lc && lc->on ? 1 : 0);
     cg_key_add(key, bc_T ? 1 : 0);
     if (bc_T) {
         cg_key_add(key, *bc_T);
@@ -474,22 +451,24 @@ int pt_iterations(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, cons
     cg_key_add(key, bs);
     cg_key_add(key, bv);
     const size_t tbytes = bc_T ? padded_span_bytes(f->T) : 0;
+    // dependent launches in 2D: 64 x 70 9.5 -> 8.3 us per iteration, 511^2 29.5 -> 28.7 (no difference at
+    // 254^2); in 3D a waiting grid's blocks take the SMs from the one before (32 x 40 x 50: 35 -> 48 us)
+    const bool dep = nd == 2;
     return cg_graph_run(ctx, key, [&](cudaStream_t st) {
         // the partner starts as a copy, so that points no step writes agree in both buffers
         if (bc_T) CG_CUDA(ctx, cudaMemcpyAsync(Tw.data, f->T.data, tbytes, cudaMemcpyDeviceToDevice, st));
         for (int it = 0; it < niter; ++it) {
             const bool last = it == niter - 1;
-            int rc = SDISPATCH(launch_stress, dtype, nd, ctx, g, f, p, last, lc, mask, bs);
+            int rc = SDISPATCH(launch_stress, dtype, nd, ctx, g, f, p, last, lc, mask, bs, dep && it > 0);
             if (rc) return rc;
-            rc = SDISPATCH(launch_velocity, dtype, nd, ctx, g, f, p, last, lc, mask, bv);
+            rc = SDISPATCH(launch_velocity, dtype, nd, ctx, g, f, p, last, lc, mask, bv, dep);
             if (rc) return rc;
-            rc = apply_bc_V(ctx, g, f, bc_V);
-            if (rc) return rc;
+            if (bc_V && (rc = cg_bc_apply_impl(ctx, g, nd, f->V, bc_V, dep))) return rc;
             if (bc_T) {
                 const cg_field& src = (it % 2 == 0) ? f->T : Tw;
                 const cg_field& dst = (it % 2 == 0) ? Tw : f->T;
-                if ((rc = SDISPATCH(launch_thermal_step, dtype, nd, ctx, g, f, p, src, dst, st))) return rc;
-                if ((rc = cg_bc_apply_impl(ctx, g, 1, &dst, bc_T))) return rc;
+                if ((rc = SDISPATCH(launch_thermal_step, dtype, nd, ctx, g, f, p, src, dst, dep))) return rc;
+                if ((rc = cg_bc_apply_impl(ctx, g, 1, &dst, bc_T, dep))) return rc;
             }
         }
         if (bc_T && (niter & 1)) CG_CUDA(ctx, cudaMemcpyAsync(f->T.data, Tw.data, tbytes, cudaMemcpyDeviceToDevice, st));
@@ -989,6 +968,6 @@ extern "C" int cg_stokes_thermal_step(cg_ctx* ctx, const cg_grid* grid, const cg
     if ((rc = cg_check_field(ctx, grid, *T_out, dtype, 0, "T_out"))) return rc;
     if (T_out->data == f->T.data) return cg_fail(ctx, CG_ERR_ARG, "thermal_step: T_out must not be T");
     cudaSetDevice(ctx->device);
-    if ((rc = SDISPATCH(launch_thermal_step, dtype, grid->ndim, ctx, grid, f, p, f->T, *T_out, ctx->stream))) return rc;
+    if ((rc = SDISPATCH(launch_thermal_step, dtype, grid->ndim, ctx, grid, f, p, f->T, *T_out, false))) return rc;
     return bc_T ? cg_bc_apply_impl(ctx, grid, 1, T_out, bc_T) : CG_OK;
 }

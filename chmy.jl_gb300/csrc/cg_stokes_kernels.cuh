@@ -2,6 +2,8 @@
 // entry points (cg_stokes.cu) and the defect-correction solver (cg_stokes_dc.cu).
 #pragma once
 
+#include <cmath>
+
 #include "cg_common.cuh"
 
 namespace cgk {
@@ -113,6 +115,41 @@ BodyFn<T> body_fns(const cg_grid* g, const cg_stokes_params* p) {
     return b;
 }
 
+// x / c for a divisor c that is the same for every point, with the bits of the division. With
+// rc = 1/c correctly rounded, q = x rc, r = x - q c (exact in one fma) and q + r rc is x/c correctly
+// rounded (Markstein; Brisebarre, Muller and Raina, "Accelerating correctly rounded floating-point
+// division when the divisor is known in advance", 2004): three FP64 instructions for about ten of a
+// division. It holds while nothing under- or overflows: for |x| and |c| within 2^+-700 and 2^+-200;
+// zeros, infinities and NaN give x rc, and any other x takes the division.
+template <class T>
+struct ConstDiv {
+    T c, rc;
+    int ok;  // c is within its range
+};
+template <class T>
+inline ConstDiv<T> const_div(T c) {
+    const double m = std::fabs((double)c);
+    return {c, T(1) / c, m > 1e-60 && m < 1e60};
+}
+__device__ __forceinline__ float divide(float x, const ConstDiv<float>& d) { return x / d.c; }
+__device__ __forceinline__ double divide(double x, const ConstDiv<double>& d) {
+    const unsigned hi = (unsigned)__double2hiint(x) & 0x7fffffffu, e = hi >> 20;
+    const double q = __dmul_rn(x, d.rc);
+    if (d.ok && e - 323u < 1400u) return __fma_rn(__fma_rn(-q, d.c, x), d.rc, q);
+    if (d.ok && (e == 0x7ffu || (hi | (unsigned)__double2loint(x)) == 0u)) return q;
+    return x / d.c;
+}
+
+// The divisors of the scalar-viscosity form.
+template <class T>
+struct ScalarDiv {
+    ConstDiv<T> Gdt, eta, eve, three;
+};
+template <class T>
+inline ScalarDiv<T> scalar_divs(const SP<T>& s) {
+    return {const_div<T>(s.G * s.dt), const_div<T>(s.eta), const_div<T>(s.eta_ve), const_div<T>(T(3))};
+}
+
 template <class T>
 __device__ __forceinline__ T eta_ve_of(T eta, T G, T dt) {
     return T(1.0) / (T(1.0) / eta + T(1.0) / (G * dt));
@@ -161,7 +198,9 @@ struct FieldMaskW {
 // M reads the operands of the strain-rate derivatives (NoMask, or FieldMaskW for the masked
 // operators ∂(V.d, ω, g, I) and divg(V, ω, g, I)); V.d sits at location bits 1 << d.
 template <class T, int ND, bool WRITE_RES, class M>
-__global__ void stress_kernel(const SV<T> v, const SP<T> s, int e0, int e1, const M m) {
+__global__ void stress_kernel(const SV<T> v, const SP<T> s, const ScalarDiv<T> sd, int e0, int e1, const M m) {
+    cg_dep_wait();
+    cg_dep_release();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int k = ND > 2 ? blockIdx.z : 0;
@@ -192,7 +231,7 @@ __global__ void stress_kernel(const SV<T> v, const SP<T> s, int e0, int e1, cons
         if (v.has_eta)
             r = -(t - to) * s.inv_Gdt - t * ieta_c + T(2.0) * (edd - dv * s.third);
         else  // examples/stokes_2d_inc_ve_T.jl:28-29, literally
-            r = -(t - to) / (s.G * s.dt) - t / s.eta + T(2.0) * (edd - dv / T(3.0));
+            r = divide(-(t - to), sd.Gdt) - divide(t, sd.eta) + T(2.0) * (edd - divide(dv, sd.three));
         v.tau[c](i, j, k) = t + r * eve_c * s.dtau_r;
     };
     // shear component on the (a, b) edge: 1/eta interpolated with the Linear rule over the 4
@@ -205,7 +244,7 @@ __global__ void stress_kernel(const SV<T> v, const SP<T> s, int e0, int e1, cons
             const T r = -(t - to) * s.inv_Gdt - t * iev + T(2.0) * eod;
             v.tau[c](i, j, k) = t + r * eve * s.dtau_r;
         } else {  // examples/stokes_2d_inc_ve_T.jl:30
-            const T r = -(t - to) / (s.G * s.dt) - t / s.eta + T(2.0) * eod;
+            const T r = divide(-(t - to), sd.Gdt) - divide(t, sd.eta) + T(2.0) * eod;
             v.tau[c](i, j, k) = t + r * s.eta_ve * s.dtau_r;
         }
     };
@@ -234,7 +273,9 @@ __global__ void stress_kernel(const SV<T> v, const SP<T> s, int e0, int e1, cons
 // update_velocity! at one point. M reads the operands of the pressure and stress derivatives
 // (P and τ_dd at location bits 0, τ_xy 3, τ_xz 5, τ_yz 6).
 template <class T, int ND, bool WRITE_RES, class M>
-__global__ void velocity_kernel(const SV<T> v, const SP<T> s, const BodyFn<T> bf, int e0, int e1, const M m) {
+__global__ void velocity_kernel(const SV<T> v, const SP<T> s, const ScalarDiv<T> sd, const BodyFn<T> bf, int e0, int e1, const M m) {
+    cg_dep_wait();
+    cg_dep_release();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int k = ND > 2 ? blockIdx.z : 0;
@@ -282,13 +323,13 @@ __global__ void velocity_kernel(const SV<T> v, const SP<T> s, const BodyFn<T> bf
         if (ND > 2)
             v.V[2](i, j, k) = v.V[2](i, j, k) + rz * (s.nu_dtau * (fmin(v.inv_eta(i, j, k - 1), c) + s.inv_Gdt));
     } else {  // examples/stokes_2d_inc_ve_T.jl:41-42
-        v.V[0](i, j, k) = v.V[0](i, j, k) + rx * s.nu_dtau / s.eta_ve;
-        v.V[1](i, j, k) = v.V[1](i, j, k) + ry * s.nu_dtau / s.eta_ve;
-        if (ND > 2) v.V[2](i, j, k) = v.V[2](i, j, k) + rz * s.nu_dtau / s.eta_ve;
+        v.V[0](i, j, k) = v.V[0](i, j, k) + divide(rx * s.nu_dtau, sd.eve);
+        v.V[1](i, j, k) = v.V[1](i, j, k) + divide(ry * s.nu_dtau, sd.eve);
+        if (ND > 2) v.V[2](i, j, k) = v.V[2](i, j, k) + divide(rz * s.nu_dtau, sd.eve);
     }
 }
 
-// ---- the two kernels of a loop of FP64 PT iterations ------------------------------------------
+// ---- the two kernels of a loop of FP64 PT iterations with variable viscosity ------------------
 //
 // A loop calls update_stress! and update_velocity! many times with the same viscosity, G, dt and
 // PT parameters. FP64 arithmetic bounds both kernels on GB300 (two FP64 instructions per clock and
@@ -297,21 +338,21 @@ __global__ void velocity_kernel(const SV<T> v, const SP<T> s, const BodyFn<T> bf
 // - what depends on the viscosity alone is computed once per loop (coef_kernel), the 1/eta
 //   interpolation and the reciprocals among it: eta_ve dtau_Pr and eta_ve dtau_r at cells, the
 //   interpolated 1/eta and its eta_ve dtau_r at every shear component, and nu_dtau / eta_ve at the
-//   faces (with one scalar viscosity, the same values as scalars);
+//   faces;
 // - strain rates are kept doubled (2 idx is exact), which removes the products by 2 and 1/2;
 // - the stress residual keeps its form (t_old - t)/(G dt) - t/eta + 2 e, evaluated with fused
 //   multiply-adds, and tau += r (eta_ve dtau_r) is one more: the iteration's fixed point is where
 //   the residual itself vanishes, exactly as in stress_kernel.
 // Per 2D cell that leaves 24 + 14 FP64 instructions of 58 + 20 (3D: 48 + 27 of 122 + 36).
 // Measured against a loop of stress_kernel and velocity_kernel: 2D 511^2 stress 29.3 -> 15.2 us,
-// velocity 13.3 -> 10.8 us; 3D 95 x 80 x 112 stress 244 -> 109 us, velocity 90 -> 68 us; 2D 254^2
-// with a scalar viscosity and thermal coupling (the divisions were by scalars) 36.4 -> 23.8 us per
-// iteration.
+// velocity 13.3 -> 10.8 us; 3D 95 x 80 x 112 stress 244 -> 109 us, velocity 90 -> 68 us.
+// With one scalar viscosity the loop keeps stress_kernel and velocity_kernel, whose divisions by
+// scalars are ConstDiv: coupled to the thermal step, whose fixed-point iteration can amplify a last
+// bit of V from one iteration to the next, the loop has to leave the same bits as the kernels apart.
 template <class T>
 struct PtCoef {
-    DF<T> ieta, cP, cT, ievE[3], cE[3], step[3];  // variable viscosity
-    T g;                                          // 1 / (G dt)
-    T ieta_s, cP_s, cT_s, step_s;                 // scalar viscosity
+    DF<T> ieta, cP, cT, ievE[3], cE[3], step[3];
+    T g;  // 1 / (G dt)
     T third, idx[3], idx2[3];
 };
 
@@ -336,9 +377,11 @@ __global__ void coef_kernel(const SV<T> v, const SP<T> s, const PtCoef<T> c, int
         c.step[d](i, j, k) = s.nu_dtau * (fmin(v.inv_eta(i - (d == 0), j - (d == 1), k - (d == 2)), ie) + s.inv_Gdt);
 }
 
-// update_stress! of a PT loop at one point (VAR: the viscosity varies per cell).
-template <class T, int ND, bool WRITE_RES, bool VAR, class M>
+// update_stress! of a PT loop at one point.
+template <class T, int ND, bool WRITE_RES, class M>
 __global__ void stress_loop_kernel(const SV<T> v, const PtCoef<T> c, int e0, int e1, const M m) {
+    cg_dep_wait();
+    cg_dep_release();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int k = ND > 2 ? blockIdx.z : 0;
@@ -356,17 +399,17 @@ __global__ void stress_loop_kernel(const SV<T> v, const PtCoef<T> c, int e0, int
         dv = dv + ezz;
     }
     if (WRITE_RES && v.has_divV) v.divV(i, j, k) = T(0.5) * dv;
-    v.P(i, j, k) = fma(-dv, VAR ? c.cP(i, j, k) : c.cP_s, v.P(i, j, k));
+    v.P(i, j, k) = fma(-dv, c.cP(i, j, k), v.P(i, j, k));
     auto update = [&](int q, T e2, T ie, T ct) {  // e2 = 2 e
         const T t = v.tau[q](i, j, k), to = v.tau_old[q](i, j, k);
         const T r = fma(to - t, c.g, fma(-t, ie, e2));
         v.tau[q](i, j, k) = fma(r, ct, t);
     };
-    const T ie = VAR ? c.ieta(i, j, k) : c.ieta_s, ct = VAR ? c.cT(i, j, k) : c.cT_s;
+    const T ie = c.ieta(i, j, k), ct = c.cT(i, j, k);
     update(0, fma(-dv, c.third, exx), ie, ct);
     update(1, fma(-dv, c.third, eyy), ie, ct);
     if (ND > 2) update(2, fma(-dv, c.third, ezz), ie, ct);
-    auto shear = [&](int q, int e, T e2) { update(q, e2, VAR ? c.ievE[e](i, j, k) : c.ieta_s, VAR ? c.cE[e](i, j, k) : c.cT_s); };
+    auto shear = [&](int q, int e, T e2) { update(q, e2, c.ievE[e](i, j, k), c.cE[e](i, j, k)); };
     shear(ND == 2 ? 2 : 3, 0, fma(vx - m(1, Vx, i, j - 1, k), c.idx[1], (vy - m(2, Vy, i - 1, j, k)) * c.idx[0]));
     if (ND > 2) {
         shear(4, 1, fma(vx - m(1, Vx, i, j, k - 1), c.idx[2], (vz - m(4, Vz, i - 1, j, k)) * c.idx[0]));
@@ -376,8 +419,10 @@ __global__ void stress_loop_kernel(const SV<T> v, const PtCoef<T> c, int e0, int
 
 // update_velocity! of a PT loop at one point. The differences of tau_dd and of P are formed
 // separately (each is small against its operands) and share one product by idx.
-template <class T, int ND, bool WRITE_RES, bool VAR, class M>
+template <class T, int ND, bool WRITE_RES, class M>
 __global__ void velocity_loop_kernel(const SV<T> v, const PtCoef<T> c, const BodyFn<T> bf, int e0, int e1, const M m) {
+    cg_dep_wait();
+    cg_dep_release();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int k = ND > 2 ? blockIdx.z : 0;
@@ -393,7 +438,7 @@ __global__ void velocity_loop_kernel(const SV<T> v, const PtCoef<T> c, const Bod
         if (v.has_rho[d]) r = r - v.rho[d](i, j, k);
         else if (bf.fn[d].kind) r = r - body_fn(bf, d, ND, i, j, k);
         if (WRITE_RES && v.has_rV) v.rV[d](i, j, k) = r;
-        v.V[d](i, j, k) = fma(r, VAR ? c.step[d](i, j, k) : c.step_s, v.V[d](i, j, k));
+        v.V[d](i, j, k) = fma(r, c.step[d](i, j, k), v.V[d](i, j, k));
     };
     const T xy = m(LXY, v.tau[XY], i, j, k);
     T rx = fma(m(LXY, v.tau[XY], i, j + 1, k) - xy, c.idx[1], normal(0));
@@ -463,10 +508,23 @@ __global__ void thermal_kernel(const SV<T> v, const SP<T> s, int e0, int e1) {
 // at the two faces of each cell, over Chmy's launch range. A face flux at index n+2 lies beyond
 // the flux kernel's launch range, so in the two-kernel form it reads the untouched allocation:
 // zero here. Every operation is rounded once in the oracle's order (max/min as std::max/min).
+//
+// FP64 arithmetic bounds it: 7 instructions per face and 7 per cell. Blocks own 31 columns and each
+// x face is computed once (lane 31 only supplies lane 30's), y faces pass through shared memory, and
+// the signs of V are read from its bits: about 22 FP64 instructions per 2D cell for 43.
+// Measured at 254^2: 7.7 -> 4.8 us per launch.
+__device__ __forceinline__ bool is_neg(double v) {  // v < 0
+    const unsigned long long b = bits_of(v);
+    return b > 0x8000000000000000ull && b <= 0xFFF0000000000000ull;
+}
+__device__ __forceinline__ bool is_pos(double v) { return bits_of(v) - 1ull < 0x7FF0000000000000ull; }  // v > 0
+__device__ __forceinline__ bool is_neg(float v) { return v < 0.f; }
+__device__ __forceinline__ bool is_pos(float v) { return 0.f < v; }
+
 template <class T>
 __device__ __forceinline__ T heat_flux(T mlam, T tl, T tr, T v, T idx) {
-    const T vp = v < T(0) ? T(0) : v;  // std::max(v, 0)
-    const T vm = T(0) < v ? T(0) : v;  // std::min(v, 0)
+    const T vp = is_neg(v) ? T(0) : v;  // std::max(v, 0)
+    const T vm = is_pos(v) ? T(0) : v;  // std::min(v, 0)
     return radd(radd(rmul(mlam, rmul(rsub(tr, tl), idx)), rmul(vp, tl)), rmul(vm, tr));
 }
 
@@ -476,19 +534,30 @@ struct ThermalStep {
     T mlam, dt, idx[3];
 };
 
+constexpr int kThermalCols = 31;
+
 template <class T, int ND>
-__global__ void thermal_step_kernel(const ThermalStep<T> a, int e0, int e1, int e2) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = ND > 2 ? blockIdx.z : 0;
-    if (i > e0 || j > e1) return;
-    const T c = a.Tin(i, j, k);
-    const T qx0 = heat_flux(a.mlam, a.Tin(i - 1, j, k), c, a.V[0](i, j, k), a.idx[0]);
-    const T qx1 = i + 1 <= e0 ? heat_flux(a.mlam, c, a.Tin(i + 1, j, k), a.V[0](i + 1, j, k), a.idx[0]) : T(0);
+__global__ void __launch_bounds__(256) thermal_step_kernel(const ThermalStep<T> a, int e0, int e1, int e2) {
+    constexpr unsigned FULL = 0xffffffffu;
+    __shared__ T qy[9][32];
+    cg_dep_wait();
+    cg_dep_release();
+    const int lane = threadIdx.x, row = threadIdx.y;
+    const int i = blockIdx.x * kThermalCols + lane, j = blockIdx.y * 8 + row, k = ND > 2 ? blockIdx.z : 0;
+    const bool in = i <= e0 && j <= e1;
+    T c = T(0), qx0 = T(0), qy0 = T(0);
+    if (in) {
+        c = a.Tin(i, j, k);
+        qx0 = heat_flux(a.mlam, a.Tin(i - 1, j, k), c, a.V[0](i, j, k), a.idx[0]);
+        qy0 = heat_flux(a.mlam, a.Tin(i, j - 1, k), c, a.V[1](i, j, k), a.idx[1]);
+    }
+    qy[row][lane] = qy0;
+    if (row == 7) qy[8][lane] = in && j + 1 <= e1 ? heat_flux(a.mlam, c, a.Tin(i, j + 1, k), a.V[1](i, j + 1, k), a.idx[1]) : T(0);
+    const T qx1 = __shfl_down_sync(FULL, qx0, 1);  // 0 beyond the launch range
+    __syncthreads();
+    if (!in || lane == kThermalCols) return;
     T dq = rmul(rsub(qx1, qx0), a.idx[0]);
-    const T qy0 = heat_flux(a.mlam, a.Tin(i, j - 1, k), c, a.V[1](i, j, k), a.idx[1]);
-    const T qy1 = j + 1 <= e1 ? heat_flux(a.mlam, c, a.Tin(i, j + 1, k), a.V[1](i, j + 1, k), a.idx[1]) : T(0);
-    dq = radd(dq, rmul(rsub(qy1, qy0), a.idx[1]));
+    dq = radd(dq, rmul(rsub(qy[row + 1][lane], qy0), a.idx[1]));
     if (ND > 2) {
         const T qz0 = heat_flux(a.mlam, a.Tin(i, j, k - 1), c, a.V[2](i, j, k), a.idx[2]);
         const T qz1 = k + 1 <= e2 ? heat_flux(a.mlam, c, a.Tin(i, j, k + 1), a.V[2](i, j, k + 1), a.idx[2]) : T(0);

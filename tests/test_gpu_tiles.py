@@ -66,3 +66,22 @@ def test_tiles_with_buffers_that_differ_outside_the_launch_range(arch, monkeypat
                    + [f.to_numpy() for f in other["V"] + other["tau"]])
     for a, b in zip(*out):
         assert np.array_equal(a.view(np.uint8), b.view(np.uint8))
+
+
+@pytest.mark.parametrize("layout", ["0:4", "4:4", "5:1", "8:0"])
+@pytest.mark.parametrize("dims", [(31, 20, 70), (13, 12, 11), (61, 7, 5)])
+@pytest.mark.parametrize("pitch", [0, 512])
+def test_3d_layouts_match_oracle(arch, monkeypatch, layout, dims, pitch):
+    """The 3D march with 122 registers and with short z segments (CG_MARCH_LAYOUT=<segment>:<variant>),
+    in the dense layout (class strides) and in one with shared strides: the oracle's bits."""
+    from test_gpu_stokes import _bc_V
+
+    monkeypatch.setenv("CG_MARCH_LAYOUT", layout)
+    rows = dims[1] + 5 if pitch else 0
+    s, _, _, _ = _pp_run(arch, T, dims, _bc_V(3), 4, seed=71, pitch_align=pitch, plane_rows=rows)
+    for name in ("V", "P", "tau", "divV", "r_V"):
+        hv = s.h[name] if isinstance(s.h[name], list) else [s.h[name]]
+        dv = s.d[name] if isinstance(s.d[name], list) else [s.d[name]]
+        for a, b in zip(dv, hv):
+            if b is not None:
+                assert_close(a, b, 0.0, f"3d {layout} {name}", exact=True)
