@@ -14,6 +14,8 @@
 #include "cg_march3d_tma.cuh"
 #include "cg_stokes_kernels.cuh"
 
+#include <cmath>
+
 int cg_maxabs_enqueue(cg_ctx* ctx, int nfields, const cg_field* fields);
 int cg_maxabs_collect(cg_ctx* ctx, int nfields, const cg_field* fields, double* out, int32_t* nonfinite);
 
@@ -240,79 +242,114 @@ size_t padded_count(const cg_field& f) {
     return (size_t)f.stride[2] * (f.n[2] + 4);
 }
 
-// max |r_tau| of the FP32 correction over the interior of every stress component: the inner
-// loop's constitutive measure, the FP32 counterpart of the outer err_tau. Without it, a state
-// whose momentum and continuity residuals vanish (a uniform stress correction) would end the
-// inner loop at its first check. The maximum is kept as the bits of |r| (a NaN's bits exceed
-// every finite value's, so a non-finite residual is reported).
+// The measures of a check of the inner loop, max |divV|, max |r_V[d]| and max |r_tau| of the FP32
+// correction, in one launch that ends the chunk's graph.
+//
+// - r_V on a normal boundary plane is zero by its Dirichlet condition: those planes are left out
+//   instead of written by a boundary-condition launch (no one else reads r_V).
+// - r_tau is the inner loop's constitutive measure, the FP32 counterpart of the outer err_tau.
+//   Without it, a state whose momentum and continuity residuals vanish (a uniform stress
+//   correction) would end the inner loop at its first check.
+// - Maxima are kept as the bits of |x| (a NaN's bits exceed every finite value's, so a non-finite
+//   residual is reported). The last block to finish hands them, and the wait flag of the TMA-fed
+//   kernels, to the host's pinned words and clears them for the next check: no memset, no copy.
+//
+// Latency bounds a check, which is a chain of small launches: the boundary condition of r_V, the
+// reduction of divV and r_V, the reduction of r_tau, two memsets and a copy took 24 us after a
+// chunk's 48 iterations (66 us) at 191 x 191, this launch 7: the solve 20.0 -> 16.3 ms.
+struct Measure {
+    unsigned* slot;   // device: [0] divV, [1..ND] r_V, [ND + 1] r_tau, [kTicket] blocks done
+    unsigned* host;   // pinned: the same maxima, [kTicket] the wait flag
+    const int* wait;  // the wait flag of the TMA-fed kernels, or nullptr
+    int e0, e1, n[3];
+};
+constexpr int kTicket = 7;
+constexpr int kMeasureAt = 32;  // first 64-bit word of the reduction buffers that the measures use
+
 template <int ND>
-__global__ void tau_res_kernel(const SV<float> v, const SP<float> s, int e0, int e1, int n0, int n1, int n2,
-                               unsigned long long* slot) {
-    // one thread per point of the launch range; the block's maximum goes into the slot, with an
-    // atomic only when it exceeds the slot's current value (one address: atomics from every warp
-    // of the grid would serialise there)
+__global__ void __launch_bounds__(256) measure_kernel(const SV<float> v, const SP<float> s, const Measure ms) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int k = ND > 2 ? blockIdx.z : 0;
-    unsigned m = 0;
-    {
-        if (i <= e0 && j <= e1) {
-            // interior test per location: logical index 1..n (Center) or 1..n+1 (Vertex) along
-            // each dim (0 is the lower ghost layer of the launch range)
-            auto in = [&](int li, int lj, int lk) {
-                return i >= 1 && j >= 1 && i <= n0 + li && j <= n1 + lj && (ND < 3 || (k >= 1 && k <= n2 + lk));
-            };
-            auto take = [&](float r) { m = max(m, __float_as_uint(fabsf(r))); };
-            const float exx = (v.V[0](i + 1, j, k) - v.V[0](i, j, k)) * s.idx[0];
-            const float eyy = (v.V[1](i, j + 1, k) - v.V[1](i, j, k)) * s.idx[1];
-            float ezz = 0.f, dv = exx + eyy;
-            if (ND > 2) {
-                ezz = (v.V[2](i, j, k + 1) - v.V[2](i, j, k)) * s.idx[2];
-                dv = dv + ezz;
-            }
-            const float ie = v.ieta(i, j, k);
-            auto diag = [&](int c, float e) {
-                const float t = v.tau[c](i, j, k);
-                take(-(t - v.tau_old[c](i, j, k)) * s.inv_Gdt - t * ie + 2.f * (e - dv * s.third));
-            };
-            auto shear = [&](int c, float e, int a, int b) {
-                const float t = v.tau[c](i, j, k);
-                const float iev = shear_inv_eta(v, i, j, k, a, b);
-                take(-(t - v.tau_old[c](i, j, k)) * s.inv_Gdt - t * iev + 2.f * e);
-            };
-            const float exy = 0.5f * ((v.V[0](i, j, k) - v.V[0](i, j - 1, k)) * s.idx[1] +
-                                      (v.V[1](i, j, k) - v.V[1](i - 1, j, k)) * s.idx[0]);
-            if (in(0, 0, 0)) {
-                diag(0, exx);
-                diag(1, eyy);
-                if (ND > 2) diag(2, ezz);
-            }
-            if (ND == 2) {
-                if (in(1, 1, 0)) shear(2, exy, 0, 1);
-            } else {
-                const float exz = 0.5f * ((v.V[0](i, j, k) - v.V[0](i, j, k - 1)) * s.idx[2] +
-                                          (v.V[2](i, j, k) - v.V[2](i - 1, j, k)) * s.idx[0]);
-                const float eyz = 0.5f * ((v.V[1](i, j, k) - v.V[1](i, j, k - 1)) * s.idx[2] +
-                                          (v.V[2](i, j, k) - v.V[2](i, j - 1, k)) * s.idx[1]);
-                if (in(1, 1, 0)) shear(3, exy, 0, 1);
-                if (in(1, 0, 1)) shear(4, exz, 0, 2);
-                if (in(0, 1, 1)) shear(5, eyz, 1, 2);
-            }
+    unsigned m[ND + 2];
+#pragma unroll
+    for (int c = 0; c < ND + 2; ++c) m[c] = 0u;
+    cg_dep_wait();
+    if (i <= ms.e0 && j <= ms.e1) {
+        // interior test per location: logical index 1..n (Center) or 1..n+1 (Vertex) along
+        // each dim (0 is the lower ghost layer of the launch range)
+        auto in = [&](int li, int lj, int lk) {
+            return i >= 1 && j >= 1 && i <= ms.n[0] + li && j <= ms.n[1] + lj &&
+                   (ND < 3 || (k >= 1 && k <= ms.n[2] + lk));
+        };
+        auto bits = [](float r) { return __float_as_uint(fabsf(r)); };
+        unsigned& mt = m[ND + 1];
+        auto take = [&](float r) { mt = max(mt, bits(r)); };
+        const float exx = (v.V[0](i + 1, j, k) - v.V[0](i, j, k)) * s.idx[0];
+        const float eyy = (v.V[1](i, j + 1, k) - v.V[1](i, j, k)) * s.idx[1];
+        float ezz = 0.f, dv = exx + eyy;
+        if (ND > 2) {
+            ezz = (v.V[2](i, j, k + 1) - v.V[2](i, j, k)) * s.idx[2];
+            dv = dv + ezz;
+        }
+        const float ie = v.ieta(i, j, k);
+        auto diag = [&](int c, float e) {
+            const float t = v.tau[c](i, j, k);
+            take(-(t - v.tau_old[c](i, j, k)) * s.inv_Gdt - t * ie + 2.f * (e - dv * s.third));
+        };
+        auto shear = [&](int c, float e, int a, int b) {
+            const float t = v.tau[c](i, j, k);
+            const float iev = shear_inv_eta(v, i, j, k, a, b);
+            take(-(t - v.tau_old[c](i, j, k)) * s.inv_Gdt - t * iev + 2.f * e);
+        };
+        const float exy = 0.5f * ((v.V[0](i, j, k) - v.V[0](i, j - 1, k)) * s.idx[1] +
+                                  (v.V[1](i, j, k) - v.V[1](i - 1, j, k)) * s.idx[0]);
+        if (in(0, 0, 0)) {
+            m[0] = bits(v.divV(i, j, k));
+            if (i > 1) m[1] = bits(v.rV[0](i, j, k));
+            if (j > 1) m[2] = bits(v.rV[1](i, j, k));
+            if constexpr (ND > 2)
+                if (k > 1) m[3] = bits(v.rV[2](i, j, k));
+            diag(0, exx);
+            diag(1, eyy);
+            if (ND > 2) diag(2, ezz);
+        }
+        if (ND == 2) {
+            if (in(1, 1, 0)) shear(2, exy, 0, 1);
+        } else {
+            const float exz = 0.5f * ((v.V[0](i, j, k) - v.V[0](i, j, k - 1)) * s.idx[2] +
+                                      (v.V[2](i, j, k) - v.V[2](i - 1, j, k)) * s.idx[0]);
+            const float eyz = 0.5f * ((v.V[1](i, j, k) - v.V[1](i, j, k - 1)) * s.idx[2] +
+                                      (v.V[2](i, j, k) - v.V[2](i, j - 1, k)) * s.idx[1]);
+            if (in(1, 1, 0)) shear(3, exy, 0, 1);
+            if (in(1, 0, 1)) shear(4, exz, 0, 2);
+            if (in(0, 1, 1)) shear(5, eyz, 1, 2);
         }
     }
+    __shared__ unsigned sm[ND + 2][8];
+    const int lane = threadIdx.x & 31, w = threadIdx.y;  // blocks of 32 x 8
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    __shared__ unsigned sm[32];
-    const int t = threadIdx.y * blockDim.x + threadIdx.x, lane = t & 31, w = t >> 5;
-    if (lane == 0) sm[w] = m;
+    for (int c = 0; c < ND + 2; ++c) {
+        const unsigned r = __reduce_max_sync(0xffffffffu, m[c]);
+        if (lane == 0) sm[c][w] = r;
+    }
     __syncthreads();
-    if (w == 0) {
-        const int nwarp = (int)(blockDim.x * blockDim.y) >> 5;
-        m = lane < nwarp ? sm[lane] : 0u;
+    if (w < ND + 2) {
+        const unsigned r = __reduce_max_sync(0xffffffffu, lane < 8 ? sm[w][lane] : 0u);
+        // one address per measure: an atomic only when it would raise the maximum
+        if (lane == 0 && r > *reinterpret_cast<volatile unsigned*>(ms.slot + w)) atomicMax(ms.slot + w, r);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+        __threadfence();
+        const unsigned blocks = gridDim.x * gridDim.y * gridDim.z;
+        if (atomicAdd(ms.slot + kTicket, 1u) == blocks - 1u) {
+            __threadfence();
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if (lane == 0 && m && (unsigned long long)m > *reinterpret_cast<volatile unsigned long long*>(slot))
-            atomicMax(slot, (unsigned long long)m);
+            for (int c = 0; c < ND + 2; ++c) ms.host[c] = atomicExch(ms.slot + c, 0u);
+            ms.host[kTicket] = ms.wait ? (unsigned)*ms.wait : 0u;
+            ms.slot[kTicket] = 0u;
+        }
     }
 }
 
@@ -411,15 +448,10 @@ int cg_stokes_solve_dc(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f,
     // FP64 measures: divV, r_V (the reference's) and the constitutive residuals, read from the
     // FP32 forcing tau_old' = G dt R_tau (the initial guess of a PT solve can have zero divV and
     // r_V while tau is far from its constitutive value)
-    cg_field red64[4 + 6], red32[5];
+    cg_field red64[4 + 6];
     red64[0] = f->divV;
-    red32[0] = w.divV;
-    for (int d = 0; d < nd; ++d) {
-        red64[1 + d] = f->r_V[d];
-        red32[1 + d] = w.rV[d];
-    }
+    for (int d = 0; d < nd; ++d) red64[1 + d] = f->r_V[d];
     for (int c = 0; c < nt; ++c) red64[1 + nd + c] = w.told[c];
-    red32[nd + 1] = w.told[0];  // FP32 slot of the constitutive measure (only its dtype is read)
     cg_bc rbc[3];
     std::memset(rbc, 0, sizeof(rbc));
     for (int d = 0; d < nd; ++d) rbc[d].kind[d][0] = rbc[d].kind[d][1] = CG_BC_DIRICHLET;
@@ -546,6 +578,15 @@ int cg_stokes_solve_dc(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f,
     // pool agree outside the launch range (both are zero where no iteration writes).
     const bool tile = nd == 2 && fold && tc.variant >= 1;
     const int npass = tile ? (cg_div_up(nchunk, kTileIters[tc.variant - 1]) + 1) & ~1 : 0;
+    Measure chk;
+    chk.slot = reinterpret_cast<unsigned*>(ctx->d_red + kMeasureAt);
+    chk.host = reinterpret_cast<unsigned*>(ctx->h_red + kMeasureAt);
+    chk.wait = staged ? terr : nullptr;
+    chk.e0 = e0;
+    chk.e1 = e1;
+    for (int d = 0; d < 3; ++d) chk.n[d] = d < nd ? g->n[d] : 1;
+    CG_CUDA(ctx, cudaMemsetAsync(chk.slot, 0, (kTicket + 1) * sizeof(unsigned), ctx->stream));
+    cg_key_add(key, chk.wait);
     auto chunk = [&]() {
         return cg_graph_run(ctx, key, [&](cudaStream_t st) {
             for (int k = 0; k < npass; ++k) {
@@ -589,6 +630,9 @@ int cg_stokes_solve_dc(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f,
                     if (r) return r;
                 }
             }
+            const cudaError_t le = nd == 2 ? cg_launch(measure_kernel<2>, grid3, block, 0, st, true, v32, s32, chk)
+                                           : cg_launch(measure_kernel<3>, grid3, block, 0, st, !staged, v32, s32, chk);
+            if (le != cudaSuccess) return cg_fail(ctx, CG_ERR_CUDA, "measure launch: %s", cudaGetErrorString(le));
             return (int)CG_OK;
         });
     };
@@ -644,21 +688,18 @@ int cg_stokes_solve_dc(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f,
         int since_best = 0;
         while (total_iter < o->max_iter) {
             if ((rc = chunk())) return rc;
-            if (staged && (rc = cg_tma_check(ctx, terr, "fused3d iteration"))) return rc;
             total_iter += nchunk;
-            if ((rc = cg_bc_apply_impl(ctx, g, nd, f32.r_V, rbc))) return rc;
-            if ((rc = cg_maxabs_enqueue(ctx, nd + 1, red32))) return rc;
-            // the constitutive measure into the next reduction slot
-            CG_CUDA(ctx, cudaMemsetAsync(ctx->d_red + nd + 1, 0, sizeof(unsigned long long), ctx->stream));
-            if (nd == 2)
-                tau_res_kernel<2><<<grid3, block, 0, ctx->stream>>>(v32, s32, e0, e1, g->n[0], g->n[1], 1,
-                                                                     ctx->d_red + nd + 1);
-            else
-                tau_res_kernel<3><<<grid3, block, 0, ctx->stream>>>(v32, s32, e0, e1, g->n[0], g->n[1], g->n[2],
-                                                                     ctx->d_red + nd + 1);
-            CG_CHECK_LAUNCH(ctx);
+            CG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+            if (chk.host[kTicket])
+                return cg_fail(ctx, CG_ERR_TIMEOUT, "fused3d iteration: a wait for staged data timed out");
             double e32[5];
-            if ((rc = cg_maxabs_collect(ctx, nd + 2, red32, e32, &bad))) return rc;
+            bad = 0;
+            for (int c = 0; c < nd + 2; ++c) {
+                float x;
+                std::memcpy(&x, chk.host + c, 4);
+                e32[c] = (double)x;
+                if (!std::isfinite(x)) bad = 1;
+            }
             res->checks++;
             if (bad) {
                 status = CG_ERR_NONFINITE;
