@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
@@ -92,6 +93,10 @@ bool cg_sia_persistent_enabled();
 // CG_SIA_TILE_ROWS=4|8|16: the SIA ensemble's tile height (rows of 32-point tiles) instead of the
 // autotuned one (0 when unset); the results do not depend on it.
 int cg_sia_tile_rows_forced();
+// CG_SIA_STEP_ROWS=0|4|8|13 (read on every call): the tile height of cg_sia_run's one-launch step, 0
+// for two launches per step, instead of the autotuned choice (-1 when unset); the results do not
+// depend on it.
+int cg_sia_step_rows_forced();
 // Grid barriers of the persistent SIA ensemble kernel: the time limit of every wait
 // (CG_SIA_BARRIER_LIMIT_MS, default 2000 ms) and a number of arrivals that the barrier expects
 // beyond the grid's blocks (CG_SIA_BARRIER_WITHHELD, default 0). A withheld arrival never
@@ -158,6 +163,31 @@ __device__ __forceinline__ double rrcp(double x) { return __drcp_rn(x); }
 
 __device__ __forceinline__ unsigned long long bits_of(double d) { return (unsigned long long)__double_as_longlong(d); }
 __device__ __forceinline__ unsigned long long bits_of(float f) { return (unsigned long long)(unsigned)__float_as_int(f); }
+
+// x / c for a divisor c that is the same for every point, with the bits of the division. With
+// rc = 1/c correctly rounded, q = x rc, r = x - q c (exact in one fma) and q + r rc is x/c correctly
+// rounded (Markstein; Brisebarre, Muller and Raina, "Accelerating correctly rounded floating-point
+// division when the divisor is known in advance", 2004): three FP64 instructions for about ten of a
+// division. It holds while nothing under- or overflows: for |x| and |c| within 2^+-700 and 2^+-200;
+// zeros, infinities and NaN give x rc, and any other x takes the division.
+template <class T>
+struct ConstDiv {
+    T c, rc;
+    int ok;  // c is within its range
+};
+template <class T>
+inline ConstDiv<T> const_div(T c) {
+    const double m = std::fabs((double)c);
+    return {c, T(1) / c, m > 1e-60 && m < 1e60};
+}
+__device__ __forceinline__ float divide(float x, const ConstDiv<float>& d) { return x / d.c; }
+__device__ __forceinline__ double divide(double x, const ConstDiv<double>& d) {
+    const unsigned hi = (unsigned)__double2hiint(x) & 0x7fffffffu, e = hi >> 20;
+    const double q = __dmul_rn(x, d.rc);
+    if (d.ok && e - 323u < 1400u) return __fma_rn(__fma_rn(-q, d.c, x), d.rc, q);
+    if (d.ok && (e == 0x7ffu || (hi | (unsigned)__double2loint(x)) == 0u)) return q;
+    return x / d.c;
+}
 
 // Largest of the block's `bits` into *slot with one atomicMax. Every thread of the block
 // calls it. Values are >= 0 (D, or |x|), so the bit patterns order like the values; a NaN orders above every

@@ -148,6 +148,15 @@ int cg_sia_tile_rows_forced() {
     return (r == 4 || r == 8 || r == 16) ? (int)r : 0;
 }
 
+int cg_sia_step_rows_forced() {
+    // read on every call, like CG_SIA_PERSISTENT
+    const char* e = std::getenv("CG_SIA_STEP_ROWS");
+    if (!e) return -1;
+    char* end = nullptr;
+    const long r = std::strtol(e, &end, 10);
+    return end != e && (r == 0 || r == 4 || r == 8 || r == 13) ? (int)r : -1;
+}
+
 cg_barrier_cfg cg_sia_barrier_cfg() {
     // read on every call, like CG_SIA_PERSISTENT
     cg_barrier_cfg c;

@@ -110,6 +110,10 @@ using cgk::bits_of;
 
 using cgk::block_max_bits;
 
+// fmax(u, 0), a NaN's included, from the bits: no FP64 comparison.
+__device__ __forceinline__ double pos_part(double u) { return bits_of(u) <= 0x7FF0000000000000ull ? u : 0.0; }
+__device__ __forceinline__ float pos_part(float u) { return fmaxf(u, 0.f); }
+
 // Sum over the block (valid in thread 0). Every thread calls it; it may be called more than
 // once per kernel (the leading barrier keeps a call's writes after the previous call's reads).
 __device__ __forceinline__ double block_sum(double x) {
@@ -190,8 +194,8 @@ inline TapeGeom tape_geom(const cg_field& H, size_t elem) {
 // two buffers that alternate by step, and the maximum of D two slots. Of D only the interior cells
 // are read: the faces on the boundary carry no flux. Measured against six launches per step (D, q,
 // bc!(q), Δt, H, bc!(H)) and four for an ensemble (D, q, Δt, H): 383 x 255 22.7 -> 14.6 us per step, 64
-// members of 128^2 to 1024^2 (26.3 M cells, 1.3 ms at the FP64 pipe's rate) 2.42 -> 1.77 ms, 64 members
-// of 32^2 to 128^2 62 -> 43 us. Boundary conditions are those of bc!: q.x =>
+// members of 128^2 to 1024^2 (26.3 M cells, 1.3 ms at the FP64 pipe's rate) 2.42 -> 1.71 ms, 64 members
+// of 32^2 to 128^2 62 -> 42 us. Boundary conditions are those of bc!: q.x =>
 // (x = Dirichlet()) is 0 on the faces 1 and n+1 (q.y likewise), and H => Neumann() copies the first
 // interior value into the ghost layer, a corner the diagonal interior cell's.
 template <class T>
@@ -199,7 +203,8 @@ struct Member {
     DF<T> H, B, qx, qy, D, S[2];
     T Gamma, As, beta, ela, m_max, idx, idy, hidx, hidy;
     T Gn2, Asn;  // Gamma (n+2) and As n, for the taped derivatives of D
-    double dx2, cfl, dt_max;
+    double dx2, dt_max;
+    cgk::ConstDiv<T> cfl;
     int n, nx, ny;
     // taped runs: the member's tape block within a step's block (256 bytes of words, then kArrays
     // arrays of `tab` bytes in H's layout, H's origin at element `orig`)
@@ -207,9 +212,8 @@ struct Member {
 };
 
 struct Words {
-    unsigned long long dmax[2];  // the step's maximum of D, by step parity
+    unsigned long long dmax[3];  // the step's maximum of D, by step parity (one launch per step: modulo 3)
     double t;
-    double pad;
 };
 
 // The member's tape array k (TapeArray) of the step whose block starts at `sb`.
@@ -239,6 +243,14 @@ __device__ __forceinline__ void S_tile(const Member<T>& v, int t) {
     const int i = (t % tx) * 32 + threadIdx.x, j = (t / tx) * (int)blockDim.y + threadIdx.y;
     if (i > v.nx + 1 || j > v.ny + 1) return;
     v.S[0](i, j, 0) = v.B(i, j, 0) + v.H(i, j, 0);
+}
+
+// H of the run's start over its interior cells into `dst` (the same tiles).
+template <class T>
+__device__ __forceinline__ void H_copy_tile(const Member<T>& v, const DF<T>& dst, int t) {
+    const int tx = (v.nx + 2 + 31) / 32;
+    const int i = (t % tx) * 32 + threadIdx.x, j = (t / tx) * (int)blockDim.y + threadIdx.y;
+    if (i >= 1 && i <= v.nx && j >= 1 && j <= v.ny) dst(i, j, 0) = v.H(i, j, 0);
 }
 
 // D at the interior cells of tile t and its maximum. TAPE: D goes to the step's tape block, with
@@ -278,7 +290,7 @@ __device__ __forceinline__ void D_tile(const Member<T>& v, Words* w, int t, int 
 template <class T>
 __device__ __forceinline__ double step_dt(const Member<T>& v, unsigned long long b, bool* capped) {
     const double dmax = sizeof(T) == 8 ? __longlong_as_double((long long)b) : (double)__int_as_float((int)(unsigned)b);
-    const T q = (T)v.dx2 / (T)dmax / (T)v.cfl;
+    const T q = cgk::divide((T)v.dx2 / (T)dmax, v.cfl);
     double d = fmin((double)q, v.dt_max);
     *capped = !((double)q < v.dt_max);
     if (!(dmax > 0.0)) {
@@ -352,7 +364,7 @@ __device__ __forceinline__ void H_tile(const Member<T>& v, Words* w, int t, int 
     const T mb = NANMAX ? (v.m_max < x ? v.m_max : x) : fmin(x, v.m_max);
     const T W = rate(qxl, qxr, qyl, qyr, v.idx, v.idy, mb);
     const T u = cgk::rfma(s_dt, W, h);
-    const T hn = NANMAX ? (u < T(0) ? T(0) : u) : fmax(u, T(0));
+    const T hn = NANMAX ? (u < T(0) ? T(0) : u) : pos_part(u);
     if (dry && hn != T(-1)) return;  // hn is never -1: the work is done, nothing is stored
     if (TAPE) {
         tape_arr(v, sb, kW)(i, j, 0) = W;
@@ -411,7 +423,7 @@ inline Member<T> make_member(const cg_grid& g, const cg_field& H, const cg_field
     v.hidy = T(0.5) * v.idy;
     const double dx = std::min(g.spacing[0], g.spacing[1]);
     v.dx2 = (double)((T)dx * (T)dx);
-    v.cfl = p.cfl;
+    v.cfl = cgk::const_div<T>((T)p.cfl);
     v.dt_max = p.dt_max;
     v.n = p.n;
     v.nx = g.n[0];

@@ -115,31 +115,6 @@ BodyFn<T> body_fns(const cg_grid* g, const cg_stokes_params* p) {
     return b;
 }
 
-// x / c for a divisor c that is the same for every point, with the bits of the division. With
-// rc = 1/c correctly rounded, q = x rc, r = x - q c (exact in one fma) and q + r rc is x/c correctly
-// rounded (Markstein; Brisebarre, Muller and Raina, "Accelerating correctly rounded floating-point
-// division when the divisor is known in advance", 2004): three FP64 instructions for about ten of a
-// division. It holds while nothing under- or overflows: for |x| and |c| within 2^+-700 and 2^+-200;
-// zeros, infinities and NaN give x rc, and any other x takes the division.
-template <class T>
-struct ConstDiv {
-    T c, rc;
-    int ok;  // c is within its range
-};
-template <class T>
-inline ConstDiv<T> const_div(T c) {
-    const double m = std::fabs((double)c);
-    return {c, T(1) / c, m > 1e-60 && m < 1e60};
-}
-__device__ __forceinline__ float divide(float x, const ConstDiv<float>& d) { return x / d.c; }
-__device__ __forceinline__ double divide(double x, const ConstDiv<double>& d) {
-    const unsigned hi = (unsigned)__double2hiint(x) & 0x7fffffffu, e = hi >> 20;
-    const double q = __dmul_rn(x, d.rc);
-    if (d.ok && e - 323u < 1400u) return __fma_rn(__fma_rn(-q, d.c, x), d.rc, q);
-    if (d.ok && (e == 0x7ffu || (hi | (unsigned)__double2loint(x)) == 0u)) return q;
-    return x / d.c;
-}
-
 // The divisors of the scalar-viscosity form.
 template <class T>
 struct ScalarDiv {

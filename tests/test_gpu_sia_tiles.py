@@ -37,3 +37,30 @@ def test_run_at_tile_edges(arch, T, n, nsteps):
     for a, b in zip(qg, q):
         assert_close(a, b, rtol_for(T) * nsteps * 10, "q")
     assert abs(t.value - t_ref) <= rtol_for(T) * nsteps * t_ref
+
+
+@pytest.mark.parametrize("T", [np.float32, np.float64])
+@pytest.mark.parametrize("n", [(2, 2), (2, 30), (28, 7), (29, 8), (30, 9), (31, 13), (59, 14), (88, 33), (200, 40)])
+@pytest.mark.parametrize("glen", [3, 4])
+def test_one_launch_per_step_has_the_bits_of_two(arch, monkeypatch, T, n, glen):
+    """A step in one launch (tiles of 29 columns by 4, 8 or 13 rows that repeat their neighbours' cells)
+    against D and the rest apart: thickness with its ghost layer, the last fluxes and the time, byte
+    for byte, for runs of one step, of an even and of an odd number."""
+    grid, H, B, q = setup(T, n=n, seed=7)
+    p = reference_params()
+    p.n = glen
+    g = grid.desc()
+    for nsteps in (1, 2, 7):
+        out = {}
+        for rows in ("0", "4", "8", "13", None):
+            if rows is None:
+                monkeypatch.delenv("CG_SIA_STEP_ROWS")
+            else:
+                monkeypatch.setenv("CG_SIA_STEP_ROWS", rows)
+            Hg, Bg, qg = to_gpu(arch, H), to_gpu(arch, B), [to_gpu(arch, f) for f in q]
+            t = ctypes.c_double()
+            arch.call("cg_sia_run", ctypes.byref(g), ctypes.byref(Hg.desc()), ctypes.byref(Bg.desc()), desc_array(qg, 3),
+                      ctypes.byref(p), nsteps, ctypes.byref(t))
+            out[rows] = [f.to_numpy().tobytes() for f in [Hg] + qg] + [t.value]
+        for rows in ("4", "8", "13", None):
+            assert out[rows] == out["0"], (rows, nsteps)
