@@ -381,10 +381,9 @@ int launch_thermal(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, con
     return CG_OK;
 }
 
-// Fused thermal step Tin -> Tout (update_thermal_flux! + update_thermal!) over the launch range.
 template <class T, int ND>
-int launch_thermal_step(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p,
-                        const cg_field& Tin, const cg_field& Tout, bool dep) {
+ThermalStep<T> thermal_step_of(const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p, const cg_field& Tin,
+                               const cg_field& Tout) {
     ThermalStep<T> a;
     std::memset(&a, 0, sizeof(a));
     a.Tin = cg_view<T>(Tin);
@@ -396,9 +395,47 @@ int launch_thermal_step(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f
     }
     a.mlam = -(T)p->lambda_rhoCp;
     a.dt = (T)p->dt;
+    return a;
+}
+
+// Fused thermal step Tin -> Tout (update_thermal_flux! + update_thermal!) over the launch range.
+template <class T, int ND>
+int launch_thermal_step(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p,
+                        const cg_field& Tin, const cg_field& Tout, bool dep) {
+    const ThermalStep<T> a = thermal_step_of<T, ND>(g, f, p, Tin, Tout);
     const dim3 grid(cg_div_up(g->n[0] + 2, kThermalCols), cg_div_up(g->n[1] + 2, 8), ND > 2 ? g->n[2] + 2 : 1);
     CG_CUDA(ctx, cg_launch(thermal_step_kernel<T, ND>, grid, dim3(32, 8), 0, ctx->stream, dep, a, g->n[0] + 1, g->n[1] + 1,
                            ND > 2 ? g->n[2] + 1 : 0));
+    return CG_OK;
+}
+
+// The thermal step Tin -> Tout and the next iteration's update_stress! (2D).
+template <class T>
+int launch_stress_thermal(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p, bool res,
+                          const LoopCoef* lc, const cg_field& Tin, const cg_field& Tout, bool dep) {
+    const SV<T> v = views<T>(f, 2);
+    const SP<T> s = scalars<T>(g, p);
+    const ScalarDiv<T> sd = scalar_divs(s);
+    const ThermalStep<T> a = thermal_step_of<T, 2>(g, f, p, Tin, Tout);
+    PtCoef<T> c;
+    std::memset(&c, 0, sizeof(c));
+    const int e0 = g->n[0] + 1, e1 = g->n[1] + 1;
+    const int gx = cg_div_up(e0 + 1, 32), ns = gx * cg_div_up(e1 + 1, kPairRows);
+    const int tx = cg_div_up(e0 + 1, kThermalCols), nt = tx * cg_div_up(e1 + 1, kPairRows);
+    auto go = [&](auto kern) {
+        return cg_launch(kern, dim3(ns + nt), dim3(32, kPairRows), 0, ctx->stream, dep, v, s, sd, c, a, e0, e1, gx, ns, tx);
+    };
+    cudaError_t e;
+    bool loop = false;
+    if constexpr (sizeof(T) == 8) {
+        loop = lc && lc->base;
+        if (loop) {
+            c = loop_coef<T, 2>(g, p, v, *lc);
+            e = res ? go(stress_thermal_kernel<T, true, true>) : go(stress_thermal_kernel<T, true, false>);
+        }
+    }
+    if (!loop) e = res ? go(stress_thermal_kernel<T, false, true>) : go(stress_thermal_kernel<T, false, false>);
+    if (e != cudaSuccess) return cg_fail(ctx, CG_ERR_CUDA, "update_stress with the thermal step: %s", cudaGetErrorString(e));
     return CG_OK;
 }
 
@@ -414,6 +451,17 @@ int thermal_partner(cg_ctx* ctx, const cg_field& Tf, cg_field* out) {
     *out = Tf;
     out->data = p;
     return CG_OK;
+}
+
+// Whether the thermal step shares a launch with the next update_stress! (stress_thermal_kernel, blocks of
+// 32 x 4): no forced block shape, T is none of the fields that the stress and velocity updates read, and
+// at most 3500 cells per SM (per iteration 700 x 610 FP32 18.6 us apart, 16.1 paired; 1400 x 1210 FP64
+// 347 and 345, FP32 47.8 and 51.3: large grids fill the chip with each launch).
+bool pairs_thermal(const cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f) {
+    dim3 forced;
+    if (cg_block_forced(&forced) || (long)g->n[0] * g->n[1] > 3500l * ctx->num_sms) return false;
+    const void* T = f->T.data;
+    return T != f->eta.data && T != f->inv_eta.data && T != f->rho_g[0].data && T != f->rho_g[1].data;
 }
 
 // `niter` PT iterations: update_stress!, update_velocity!, bc!(V) and, with bc_T, the thermal
@@ -454,20 +502,33 @@ int pt_iterations(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, cons
     // dependent launches in 2D: 64 x 70 9.5 -> 8.3 us per iteration, 511^2 29.5 -> 28.7 (no difference at
     // 254^2); in 3D a waiting grid's blocks take the SMs from the one before (32 x 40 x 50: 35 -> 48 us)
     const bool dep = nd == 2;
+    const bool pair = bc_T && nd == 2 && !mask && pairs_thermal(ctx, g, f);
+    cg_key_add(key, (int)pair);
     return cg_graph_run(ctx, key, [&](cudaStream_t st) {
         // the partner starts as a copy, so that points no step writes agree in both buffers
         if (bc_T) CG_CUDA(ctx, cudaMemcpyAsync(Tw.data, f->T.data, tbytes, cudaMemcpyDeviceToDevice, st));
+        auto Tbuf = [&](int it) -> const cg_field& { return it % 2 == 0 ? f->T : Tw; };
         for (int it = 0; it < niter; ++it) {
             const bool last = it == niter - 1;
-            int rc = SDISPATCH(launch_stress, dtype, nd, ctx, g, f, p, last, lc, mask, bs, dep && it > 0);
+            int rc;
+            if (pair && it > 0)
+                rc = dtype == CG_F64 ? launch_stress_thermal<double>(ctx, g, f, p, last, lc, Tbuf(it - 1), Tbuf(it), dep)
+                                     : launch_stress_thermal<float>(ctx, g, f, p, last, lc, Tbuf(it - 1), Tbuf(it), dep);
+            else
+                rc = SDISPATCH(launch_stress, dtype, nd, ctx, g, f, p, last, lc, mask, bs, dep && it > 0);
             if (rc) return rc;
             rc = SDISPATCH(launch_velocity, dtype, nd, ctx, g, f, p, last, lc, mask, bv, dep);
             if (rc) return rc;
-            if (bc_V && (rc = cg_bc_apply_impl(ctx, g, nd, f->V, bc_V, dep))) return rc;
-            if (bc_T) {
-                const cg_field& src = (it % 2 == 0) ? f->T : Tw;
-                const cg_field& dst = (it % 2 == 0) ? Tw : f->T;
-                if ((rc = SDISPATCH(launch_thermal_step, dtype, nd, ctx, g, f, p, src, dst, dep))) return rc;
+            // bc!(V), with the T that a paired launch left
+            cg_field fs[4];
+            cg_bc bs4[4];
+            int nf = 0;
+            for (int d = 0; bc_V && d < nd; ++d, ++nf) fs[nf] = f->V[d], bs4[nf] = bc_V[d];
+            if (pair && it > 0) fs[nf] = Tbuf(it), bs4[nf++] = *bc_T;
+            if (nf && (rc = cg_bc_apply_impl(ctx, g, nf, fs, bs4, dep))) return rc;
+            if (bc_T && (!pair || last)) {
+                const cg_field& dst = Tbuf(it + 1);
+                if ((rc = SDISPATCH(launch_thermal_step, dtype, nd, ctx, g, f, p, Tbuf(it), dst, dep))) return rc;
                 if ((rc = cg_bc_apply_impl(ctx, g, 1, &dst, bc_T, dep))) return rc;
             }
         }

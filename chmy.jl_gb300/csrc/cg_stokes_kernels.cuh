@@ -173,13 +173,7 @@ struct FieldMaskW {
 // M reads the operands of the strain-rate derivatives (NoMask, or FieldMaskW for the masked
 // operators ∂(V.d, ω, g, I) and divg(V, ω, g, I)); V.d sits at location bits 1 << d.
 template <class T, int ND, bool WRITE_RES, class M>
-__global__ void stress_kernel(const SV<T> v, const SP<T> s, const ScalarDiv<T> sd, int e0, int e1, const M m) {
-    cg_dep_wait();
-    cg_dep_release();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = ND > 2 ? blockIdx.z : 0;
-    if (i > e0 || j > e1) return;
+__device__ __forceinline__ void stress_point(const SV<T>& v, const SP<T>& s, const ScalarDiv<T>& sd, int i, int j, int k, const M& m) {
     const DF<T>& Vx = v.V[0];
     const DF<T>& Vy = v.V[1];
     // ∂x(V.x) at Center: V.x is Vertex in x -> V.x[i+1] - V.x[i]
@@ -243,6 +237,17 @@ __global__ void stress_kernel(const SV<T> v, const SP<T> s, const ScalarDiv<T> s
         shear(4, exz, 0, 2);
         shear(5, eyz, 1, 2);
     }
+}
+
+template <class T, int ND, bool WRITE_RES, class M>
+__global__ void stress_kernel(const SV<T> v, const SP<T> s, const ScalarDiv<T> sd, int e0, int e1, const M m) {
+    cg_dep_wait();
+    cg_dep_release();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int k = ND > 2 ? blockIdx.z : 0;
+    if (i > e0 || j > e1) return;
+    stress_point<T, ND, WRITE_RES>(v, s, sd, i, j, k, m);
 }
 
 // update_velocity! at one point. M reads the operands of the pressure and stress derivatives
@@ -354,13 +359,7 @@ __global__ void coef_kernel(const SV<T> v, const SP<T> s, const PtCoef<T> c, int
 
 // update_stress! of a PT loop at one point.
 template <class T, int ND, bool WRITE_RES, class M>
-__global__ void stress_loop_kernel(const SV<T> v, const PtCoef<T> c, int e0, int e1, const M m) {
-    cg_dep_wait();
-    cg_dep_release();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = ND > 2 ? blockIdx.z : 0;
-    if (i > e0 || j > e1) return;
+__device__ __forceinline__ void stress_loop_point(const SV<T>& v, const PtCoef<T>& c, int i, int j, int k, const M& m) {
     const DF<T>& Vx = v.V[0];
     const DF<T>& Vy = v.V[1];
     const DF<T>& Vz = v.V[2];
@@ -390,6 +389,17 @@ __global__ void stress_loop_kernel(const SV<T> v, const PtCoef<T> c, int e0, int
         shear(4, 1, fma(vx - m(1, Vx, i, j, k - 1), c.idx[2], (vz - m(4, Vz, i - 1, j, k)) * c.idx[0]));
         shear(5, 2, fma(vy - m(2, Vy, i, j, k - 1), c.idx[2], (vz - m(4, Vz, i, j - 1, k)) * c.idx[1]));
     }
+}
+
+template <class T, int ND, bool WRITE_RES, class M>
+__global__ void stress_loop_kernel(const SV<T> v, const PtCoef<T> c, int e0, int e1, const M m) {
+    cg_dep_wait();
+    cg_dep_release();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int k = ND > 2 ? blockIdx.z : 0;
+    if (i > e0 || j > e1) return;
+    stress_loop_point<T, ND, WRITE_RES>(v, c, i, j, k, m);
 }
 
 // update_velocity! of a PT loop at one point. The differences of tau_dd and of P are formed
@@ -511,14 +521,13 @@ struct ThermalStep {
 
 constexpr int kThermalCols = 31;
 
-template <class T, int ND>
-__global__ void __launch_bounds__(256) thermal_step_kernel(const ThermalStep<T> a, int e0, int e1, int e2) {
+// Tile (bx, by) of plane k, by a block of 32 x ROWS.
+template <class T, int ND, int ROWS>
+__device__ __forceinline__ void thermal_tile(const ThermalStep<T>& a, int bx, int by, int k, int e0, int e1, int e2) {
     constexpr unsigned FULL = 0xffffffffu;
-    __shared__ T qy[9][32];
-    cg_dep_wait();
-    cg_dep_release();
+    __shared__ T qy[ROWS + 1][32];
     const int lane = threadIdx.x, row = threadIdx.y;
-    const int i = blockIdx.x * kThermalCols + lane, j = blockIdx.y * 8 + row, k = ND > 2 ? blockIdx.z : 0;
+    const int i = bx * kThermalCols + lane, j = by * ROWS + row;
     const bool in = i <= e0 && j <= e1;
     T c = T(0), qx0 = T(0), qy0 = T(0);
     if (in) {
@@ -527,7 +536,7 @@ __global__ void __launch_bounds__(256) thermal_step_kernel(const ThermalStep<T> 
         qy0 = heat_flux(a.mlam, a.Tin(i, j - 1, k), c, a.V[1](i, j, k), a.idx[1]);
     }
     qy[row][lane] = qy0;
-    if (row == 7) qy[8][lane] = in && j + 1 <= e1 ? heat_flux(a.mlam, c, a.Tin(i, j + 1, k), a.V[1](i, j + 1, k), a.idx[1]) : T(0);
+    if (row == ROWS - 1) qy[ROWS][lane] = in && j + 1 <= e1 ? heat_flux(a.mlam, c, a.Tin(i, j + 1, k), a.V[1](i, j + 1, k), a.idx[1]) : T(0);
     const T qx1 = __shfl_down_sync(FULL, qx0, 1);  // 0 beyond the launch range
     __syncthreads();
     if (!in || lane == kThermalCols) return;
@@ -539,6 +548,42 @@ __global__ void __launch_bounds__(256) thermal_step_kernel(const ThermalStep<T> 
         dq = radd(dq, rmul(rsub(qz1, qz0), a.idx[2]));
     }
     a.Tout(i, j, k) = rsub(a.Told(i, j, k), rmul(a.dt, dq));
+}
+
+template <class T, int ND>
+__global__ void __launch_bounds__(256) thermal_step_kernel(const ThermalStep<T> a, int e0, int e1, int e2) {
+    cg_dep_wait();
+    cg_dep_release();
+    thermal_tile<T, ND, 8>(a, blockIdx.x, blockIdx.y, ND > 2 ? blockIdx.z : 0, e0, e1, e2);
+}
+
+// The thermal step of one PT iteration and update_stress! of the next in one 2D launch: both read V as
+// bc!(V) left it and neither reads what the other writes. The first ns blocks (gx across) take the
+// stress, the others (tx across) the thermal tiles. LOOP: the stress from a loop's coefficients.
+//
+// A thermal iteration on a small grid is a chain of launches, each with its own latency and with SMs idle
+// in its last wave. With this launch, and bc!(T) beside the next bc!(V), a chain of five becomes one of
+// three. Blocks of 4 rows: the FP64 work is per SM, and at 254^2 blocks of 8 rows put 4 on some SMs
+// where 3.7 is the mean. Measured per iteration, apart -> paired (FP64 scalar viscosity): 62 x 80 16.2
+// -> 10.3 us, 254^2 25.0 -> 21.2 (8 rows 23; 2 rows 20.4, but FP32 511^2 12.3 -> 15.5), 700 x 610 96.4
+// -> 91.9; FP32 254^2 11.9 -> 8.3.
+constexpr int kPairRows = 4;
+
+template <class T, bool LOOP, bool WRITE_RES>
+__global__ void __launch_bounds__(32 * kPairRows)
+    stress_thermal_kernel(const SV<T> v, const SP<T> s, const ScalarDiv<T> sd, const PtCoef<T> c, const ThermalStep<T> a, int e0,
+                          int e1, int gx, int ns, int tx) {
+    cg_dep_wait();
+    cg_dep_release();
+    const int b = blockIdx.x;
+    if (b >= ns) {
+        thermal_tile<T, 2, kPairRows>(a, (b - ns) % tx, (b - ns) / tx, 0, e0, e1, 0);
+        return;
+    }
+    const int i = b % gx * 32 + threadIdx.x, j = b / gx * kPairRows + threadIdx.y;
+    if (i > e0 || j > e1) return;
+    if constexpr (LOOP) stress_loop_point<T, 2, WRITE_RES>(v, c, i, j, 0, NoMask<T>{});
+    else stress_point<T, 2, WRITE_RES>(v, s, sd, i, j, 0, NoMask<T>{});
 }
 
 // ---- bc!(V) folded into the velocity reads of the marching kernels -------------------------
