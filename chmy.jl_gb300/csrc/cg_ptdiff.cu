@@ -442,19 +442,24 @@ __global__ void __launch_bounds__(32 * NW, MINB)
 // warp owns 30 columns (lane l holds column i0 - 1 + l) by R rows and marches up a z segment with the
 // C and D of its R + 2 rows in registers: x neighbours by shuffle, y neighbours and the shared y faces
 // in registers, each z face carried up. No value is loaded twice but the two halo rows and lanes,
-// every face of the tile is computed once, and there is neither shared memory nor a barrier. Same operations and guards as
+// every face of the tile is computed once, and there is neither shared memory nor a barrier. No load has
+// a guard (columns and rows beyond the range are clamped to stored ones). Same operations as
 // ptd_march3d_kernel, so the same bits. It reads the strides of q.x and q.y apart from C's, so Chmy's
 // dense layout takes it too.
 //
 // bc!(C) is folded into the stores (PdEdge): the thread that updates a cell beside a boundary writes
 // the ghost cells that follow it, in cg_bc_apply's order (z, then y, then x), and a ghost cell under a
-// rule is not stored by itself.
-// Measured, an iteration with its bc!: 128^3 in the pool layout 32.5 -> 27 us (a solve 18.5 -> 15.7 ms),
-// 60 x 77 x 50 a solve 6.3 -> 2.6 ms, and 191 x 160 x 128 in the dense layout, which ran the flux and
-// update kernels apart, 55.9 -> 47.4 us. From about 200^3 on the TMA-fed kernel is ahead (384^3: 435 us
-// against 504), so it stays a candidate. Three rows per thread (112 registers, 4 blocks per SM) beat four,
-// two are best on the smallest grids; the loads of the next plane are in flight while a plane is
-// computed (without that 37 us at 128^3). Short z segments (3 to 12 planes) fill the SMs of small grids.
+// rule is not stored by itself; warps with no boundary cell store straight away.
+// Measured, an iteration with its bc!: 128^3 in the pool layout 32.5 -> 27 us (a solve 18.9 -> 16.4 ms),
+// 60 x 77 x 50 a solve 6.7 -> 2.6 ms, and 191 x 160 x 128 in the dense layout, which ran the flux and
+// update kernels apart, 55.7 -> 43.3 us (47.4 with a guard at every load). Reading the same bytes with
+// this access pattern and nothing else takes 17 us at 128^3 and 56 at 192^3 (73 here): instruction issue
+// (190 per warp and row) and the latency of 20 resident warps together hold it there. From about 256^3
+// on the TMA-fed kernel is ahead (384^3: 435 us against 504), so it stays a candidate. Three rows per
+// thread (123 registers, 4 blocks per SM) or two (95, 5) beat four; the loads of the next plane are in
+// flight while a plane is computed (without that 37 us at 128^3); copying two planes ahead to shared
+// memory by cp.async, at 24 to 32 warps per SM, took 30.5. Short z segments (3 to 16 planes) fill the
+// SMs of small grids.
 template <class T>
 struct PdEdge {
     int r[3][2];  // [dimension][side]: 0 none, 1 Dirichlet (2 v - C), 2 Neumann (C -/+ h v)
@@ -484,105 +489,125 @@ __global__ void __launch_bounds__(128, MINB)
     if (ks > e2) return;  // whole warp
     const int ke = min(ks + seg_len - 1, e2);
     const int i = (gw % nstrip) * 30 - 1 + lane, jb = (gw / nstrip) % nty * R;
-    const bool cx = i <= e0;      // C, D, C_old readable
-    const bool lx = i <= e0 + 1;  // column e0+1 passes its stored x flux to the lane below
+    const bool cx = i <= e0;  // column e0+1 passes its stored x flux to the lane below
     const bool own = lane >= 1 && lane <= 30 && cx;
     const bool x0 = i == 1 && er.r[0][0], x1 = i == e0 - 1 && er.r[0][1];  // writes an x ghost
     const bool xg = (i == 0 && er.r[0][0]) || (i == e0 && er.r[0][1]);     // is one
-    int o = i + (jb - 1) * f.s1 + ks * f.s2, ox = i + jb * f.s1x + ks * f.s2x, oy = i + jb * f.s1 + ks * f.s2y;
+    const bool xedge = __any_sync(FULL, own && (x0 || x1 || xg));
+    const bool yedge = (er.r[1][0] && jb <= 1) || (er.r[1][1] && jb + R >= e1);
+    // Offsets of the rows jb - 1 .. jb + R. Columns and rows beyond the launch range read its last stored
+    // ones (index n + 2), whose values no stored result depends on: no load has a guard.
+    const int ic = min(i, e0 + 1);
+    int ro[R + 2], rx[R];
+#pragma unroll
+    for (int r = 0; r < R + 2; ++r) ro[r] = ic + min(jb - 1 + r, e1 + 1) * f.s1;
+#pragma unroll
+    for (int r = 0; r < R; ++r) rx[r] = ic + min(jb + r, e1 + 1) * f.s1x;
+    int zc = ks * f.s2, zx = ks * f.s2x, zy = ks * f.s2y;  // the plane's offsets
     T c[R + 2], d[R + 2], qzl[R];
 #pragma unroll
     for (int r = 0; r < R + 2; ++r) {
-        const bool ok = cx && jb - 1 + r <= e1;
-        c[r] = ok ? __ldg(f.C + o + r * f.s1) : T(0);
-        d[r] = ok ? __ldg(f.D + o + r * f.s1) : T(0);
+        c[r] = __ldg(f.C + ro[r] + zc);
+        d[r] = __ldg(f.D + ro[r] + zc);
     }
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-        const int p = o + (r + 1) * f.s1;
-        const bool ok = cx && jb + r <= e1;
-        const T cd = ok ? __ldg(f.C + p - f.s2) : T(0), dd = ok ? __ldg(f.D + p - f.s2) : T(0), q = ok ? __ldg(f.q[2] + p) : T(0);
-        qzl[r] = pd_face(q, dd, d[r + 1], cd, c[r + 1], f.idx[2], f.om);
+        const int p = ro[r + 1] + zc;
+        qzl[r] = pd_face(__ldg(f.q[2] + p), __ldg(f.D + p - f.s2), d[r + 1], __ldg(f.C + p - f.s2), c[r + 1], f.idx[2], f.om);
     }
-    // plane k's fluxes and C_old, and plane k+1's C, D and z flux, one plane ahead of their use
+    // plane k's fluxes and C_old, and plane k+1's C, D and z flux
     PdPlane<T, R> cur;
-    auto load = [&](PdPlane<T, R>& n, int k) {
-        const bool zu = k + 1 <= e2;
+    int zcs = zc, zxs = zx, zys = zy;  // the next loads' plane
+    auto load = [&](int k) {
+        if (k <= ke) {
 #pragma unroll
-        for (int r = 0; r < R; ++r) n.qx[r] = lx && jb + r <= e1 ? __ldg(f.q[0] + ox + r * f.s1x) : T(0);
+            for (int r = 0; r < R; ++r) cur.qx[r] = __ldg(f.q[0] + rx[r] + zxs);
 #pragma unroll
-        for (int r = 0; r < R + 1; ++r) n.qy[r] = cx && jb + r <= e1 + 1 ? __ldg(f.q[1] + oy + r * f.s1) : T(0);
+            for (int r = 0; r < R + 1; ++r) cur.qy[r] = __ldg(f.q[1] + ro[r + 1] + zys);
 #pragma unroll
-        for (int r = 0; r < R + 2; ++r) {
-            const bool ok = cx && zu && jb - 1 + r <= e1;
-            n.c[r] = ok ? __ldg(f.C + o + r * f.s1 + f.s2) : T(0);
-            n.d[r] = ok ? __ldg(f.D + o + r * f.s1 + f.s2) : T(0);
-        }
+            for (int r = 0; r < R; ++r) cur.co[r] = __ldg(f.Co + ro[r + 1] + zcs);
+            zcs += f.s2;
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const bool ok = cx && jb + r <= e1;
-            n.qz[r] = ok ? __ldg(f.q[2] + o + (r + 1) * f.s1 + f.s2) : T(0);
-            n.co[r] = ok ? __ldg(f.Co + o + (r + 1) * f.s1) : T(0);
+            for (int r = 0; r < R + 2; ++r) {
+                cur.c[r] = __ldg(f.C + ro[r] + zcs);
+                cur.d[r] = __ldg(f.D + ro[r] + zcs);
+            }
+#pragma unroll
+            for (int r = 0; r < R; ++r) cur.qz[r] = __ldg(f.q[2] + ro[r + 1] + zcs);
+            zxs += f.s2x;
+            zys += f.s2y;
         }
     };
-    load(cur, ks);
+    load(ks);
     for (int k = ks; k <= ke; ++k) {
         const bool zu = k + 1 <= e2;
-        PdPlane<T, R> nxt;
-        const int p0 = o, px = ox, py = oy;
-        o += f.s2;
-        ox += f.s2x;
-        oy += f.s2y;
-        if (k < ke) load(nxt, k + 1);
-        T* qy = cur.qy;
+        PdPlane<T, R> n = cur;
+        load(k + 1);
         // a face beyond the launch range keeps its stored value
 #pragma unroll
-        for (int r = 0; r < R + 1; ++r)
-            if (jb + r <= e1) qy[r] = pd_face(qy[r], d[r], d[r + 1], c[r], c[r + 1], f.idx[1], f.om);
+        for (int r = 0; r < R + 1; ++r) {
+            const T q = pd_face(n.qy[r], d[r], d[r + 1], c[r], c[r + 1], f.idx[1], f.om);
+            n.qy[r] = jb + r <= e1 ? q : n.qy[r];
+        }
+        T v[R], qzn[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            const int j = jb + r;
             const T cc = c[r + 1], dc = d[r + 1];
-            const T cl = __shfl_up_sync(FULL, cc, 1), dl = __shfl_up_sync(FULL, dc, 1);
-            const T qxl = cx ? pd_face(cur.qx[r], dl, dc, cl, cc, f.idx[0], f.om) : cur.qx[r];
-            const T qxu = __shfl_down_sync(FULL, qxl, 1);
-            const T qzu = zu ? pd_face(cur.qz[r], dc, cur.d[r + 1], cc, cur.c[r + 1], f.idx[2], f.om) : cur.qz[r];
-            T dv = rmul(rsub(qxu, qxl), f.idx[0]);
-            dv = radd(dv, rmul(rsub(qy[r + 1], qy[r]), f.idx[1]));
-            dv = radd(dv, rmul(rsub(qzu, qzl[r]), f.idx[2]));
-            const T rr = rsub(rmul(-rsub(cc, cur.co[r]), f.inv_dt), dv);
-            const T v = radd(cc, rmul(rr, f.dtc));
-            if (own && j <= e1) {
-                const int p = p0 + (r + 1) * f.s1;
-                f.qn[0][px + r * f.s1x] = qxl;
-                f.qn[1][py + r * f.s1] = qy[r];
-                f.qn[2][p] = qzl[r];
+            const T qf = pd_face(n.qx[r], __shfl_up_sync(FULL, dc, 1), dc, __shfl_up_sync(FULL, cc, 1), cc, f.idx[0], f.om);
+            n.qx[r] = cx ? qf : n.qx[r];
+            const T qxu = __shfl_down_sync(FULL, n.qx[r], 1);
+            const T qz = pd_face(n.qz[r], dc, n.d[r + 1], cc, n.c[r + 1], f.idx[2], f.om);
+            qzn[r] = zu ? qz : n.qz[r];
+            T dv = rmul(rsub(qxu, n.qx[r]), f.idx[0]);
+            dv = radd(dv, rmul(rsub(n.qy[r + 1], n.qy[r]), f.idx[1]));
+            dv = radd(dv, rmul(rsub(qzn[r], qzl[r]), f.idx[2]));
+            const T rr = rsub(rmul(-rsub(cc, n.co[r]), f.inv_dt), dv);
+            v[r] = radd(cc, rmul(rr, f.dtc));
+        }
+        const bool zedge = (er.r[2][0] && k <= 1) || (er.r[2][1] && k + 1 >= e2);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            if (!own || jb + r > e1) continue;
+            f.qn[0][rx[r] + zx] = n.qx[r];
+            f.qn[1][ro[r + 1] + zy] = n.qy[r];
+            f.qn[2][ro[r + 1] + zc] = qzl[r];
+            if (!(xedge || yedge || zedge)) f.Cn[ro[r + 1] + zc] = v[r];
+        }
+        if (xedge || yedge || zedge) {
+#pragma unroll 1
+            for (int r = 0; r < R; ++r) {
+                const int j = jb + r, p = i + j * f.s1 + zc;
                 const bool ghost = xg || (j == 0 && er.r[1][0]) || (j == e1 && er.r[1][1]) || (k == 0 && er.r[2][0]) ||
                                    (k == e2 && er.r[2][1]);
-                if (!ghost) {
-                    auto put_x = [&](int q, T x) {
-                        f.Cn[q] = x;
-                        if (x0) f.Cn[q - 1] = pd_edge(er, 0, 0, x);
-                        if (x1) f.Cn[q + 1] = pd_edge(er, 0, 1, x);
-                    };
-                    auto put_y = [&](int q, T x) {
-                        put_x(q, x);
-                        if (j == 1 && er.r[1][0]) put_x(q - f.s1, pd_edge(er, 1, 0, x));
-                        if (j == e1 - 1 && er.r[1][1]) put_x(q + f.s1, pd_edge(er, 1, 1, x));
-                    };
-                    put_y(p, v);
-                    if (k == 1 && er.r[2][0]) put_y(p - f.s2, pd_edge(er, 2, 0, v));
-                    if (k == e2 - 1 && er.r[2][1]) put_y(p + f.s2, pd_edge(er, 2, 1, v));
-                }
+                if (!own || j > e1 || ghost) continue;
+                T w = v[0];
+#pragma unroll
+                for (int u = 1; u < R; ++u) w = r == u ? v[u] : w;
+                auto put_x = [&](int q, T x) {
+                    f.Cn[q] = x;
+                    if (x0) f.Cn[q - 1] = pd_edge(er, 0, 0, x);
+                    if (x1) f.Cn[q + 1] = pd_edge(er, 0, 1, x);
+                };
+                auto put_y = [&](int q, T x) {
+                    put_x(q, x);
+                    if (j == 1 && er.r[1][0]) put_x(q - f.s1, pd_edge(er, 1, 0, x));
+                    if (j == e1 - 1 && er.r[1][1]) put_x(q + f.s1, pd_edge(er, 1, 1, x));
+                };
+                put_y(p, w);
+                if (k == 1 && er.r[2][0]) put_y(p - f.s2, pd_edge(er, 2, 0, w));
+                if (k == e2 - 1 && er.r[2][1]) put_y(p + f.s2, pd_edge(er, 2, 1, w));
             }
-            qzl[r] = qzu;
         }
 #pragma unroll
+        for (int r = 0; r < R; ++r) qzl[r] = qzn[r];
+#pragma unroll
         for (int r = 0; r < R + 2; ++r) {
-            c[r] = cur.c[r];
-            d[r] = cur.d[r];
+            c[r] = n.c[r];
+            d[r] = n.d[r];
         }
-        cur = nxt;
+        zc += f.s2;
+        zx += f.s2x;
+        zy += f.s2y;
     }
 }
 
@@ -790,11 +815,11 @@ cg_tune_cfg tune_pd(const PDM<T>& f, const cg_grid* g, int num_sms, cudaStream_t
     float tbest = 1e30f;
     for (int v = first; v < kPdVariants; ++v) {
         if (v >= kPdTmaFirst && v < kPdRowsFirst && !tma) continue;
-        for (int seg : {0, 3, 6, 12}) {
+        for (int seg : {0, 3, 5, 7, 9, 12, 16}) {
             if (seg && (v < kPdRowsFirst || seg > g->n[2] + 2)) continue;
             const float t = cgk::time_launches(
                 [&] {
-                    const cudaError_t e = launch_pd_march3d<T>(f, g, num_sms, st, v, dir, er, seg);
+                    const cudaError_t e = launch_pd_march3d<T>(f, g, num_sms, st, v, dir, er, seg, true);
                     return e != cudaSuccess || v >= kPdRowsFirst ? e : after();
                 },
                 st);
