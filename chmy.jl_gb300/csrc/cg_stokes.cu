@@ -160,7 +160,8 @@ int setup_coef(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, const c
         v.ieta = c.ieta;
         v.has_ieta = 1;
     }
-    coef_kernel<T, ND><<<range_grid<ND>(g, block), block, 0, ctx->stream>>>(v, scalars<T>(g, p), c, g->n[0] + 1, g->n[1] + 1);
+    const dim3 flat(256);
+    coef_kernel<T, ND><<<range_grid<ND>(g, flat), flat, 0, ctx->stream>>>(v, scalars<T>(g, p), c, g->n[0] + 1, g->n[1] + 1);
     CG_CHECK_LAUNCH(ctx);
     return CG_OK;
 }
@@ -326,9 +327,9 @@ int stokes_blocks(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, cons
         upd[a]->data = tmp + off[a];
     }
     *bs = cgk::tune_block("update_stress", ks,
-                          [&](dim3 b) { return stress_any<T, ND>(g, &c, p, true, lc, mask, b, ctx->stream); }, ctx->stream);
+                          [&](dim3 b) { return stress_any<T, ND>(g, &c, p, true, lc, mask, b, ctx->stream); }, ctx->stream, true);
     *bv = cgk::tune_block("update_velocity", kv,
-                          [&](dim3 b) { return velocity_any<T, ND>(g, &c, p, true, lc, mask, b, ctx->stream); }, ctx->stream);
+                          [&](dim3 b) { return velocity_any<T, ND>(g, &c, p, true, lc, mask, b, ctx->stream); }, ctx->stream, true);
     cudaStreamSynchronize(ctx->stream);
     cudaFree(tmp);
     return CG_OK;
@@ -420,10 +421,10 @@ int launch_stress_thermal(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields*
     PtCoef<T> c;
     std::memset(&c, 0, sizeof(c));
     const int e0 = g->n[0] + 1, e1 = g->n[1] + 1;
-    const int gx = cg_div_up(e0 + 1, 32), ns = gx * cg_div_up(e1 + 1, kPairRows);
+    const int ns = cg_div_up((long)(e0 + 1) * (e1 + 1), 32 * kPairRows);
     const int tx = cg_div_up(e0 + 1, kThermalCols), nt = tx * cg_div_up(e1 + 1, kPairRows);
     auto go = [&](auto kern) {
-        return cg_launch(kern, dim3(ns + nt), dim3(32, kPairRows), 0, ctx->stream, dep, v, s, sd, c, a, e0, e1, gx, ns, tx);
+        return cg_launch(kern, dim3(ns + nt), dim3(32, kPairRows), 0, ctx->stream, dep, v, s, sd, c, a, e0, e1, ns, tx);
     };
     cudaError_t e;
     bool loop = false;

@@ -133,7 +133,7 @@ __device__ __forceinline__ T eta_ve_of(T eta, T G, T dt) {
 // 2D/3D launch: x, y threads over [0, n+1]; z over blockIdx.z.
 template <int ND>
 inline dim3 range_grid(const cg_grid* g, dim3 block) {
-    return dim3(cg_div_up(g->n[0] + 2, block.x), cg_div_up(g->n[1] + 2, block.y), ND > 2 ? g->n[2] + 2 : 1);
+    return point_grid<ND>(g->n, block);
 }
 
 // 1/eta on the (a, b) shear edge of point I: the Linear rule over the 4 cells around it, dim a
@@ -243,10 +243,8 @@ template <class T, int ND, bool WRITE_RES, class M>
 __global__ void stress_kernel(const SV<T> v, const SP<T> s, const ScalarDiv<T> sd, int e0, int e1, const M m) {
     cg_dep_wait();
     cg_dep_release();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = ND > 2 ? blockIdx.z : 0;
-    if (i > e0 || j > e1) return;
+    int i, j, k;
+    if (!launch_point<ND>(e0, e1, i, j, k)) return;
     stress_point<T, ND, WRITE_RES>(v, s, sd, i, j, k, m);
 }
 
@@ -256,10 +254,8 @@ template <class T, int ND, bool WRITE_RES, class M>
 __global__ void velocity_kernel(const SV<T> v, const SP<T> s, const ScalarDiv<T> sd, const BodyFn<T> bf, int e0, int e1, const M m) {
     cg_dep_wait();
     cg_dep_release();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = ND > 2 ? blockIdx.z : 0;
-    if (i > e0 || j > e1) return;
+    int i, j, k;
+    if (!launch_point<ND>(e0, e1, i, j, k)) return;
     const DF<T>& P = v.P;
     // tensor components: 2D xx=0 yy=1 xy=2; 3D xx=0 yy=1 zz=2 xy=3 xz=4 yz=5
     const int XY = ND == 2 ? 2 : 3;
@@ -325,7 +321,7 @@ __global__ void velocity_kernel(const SV<T> v, const SP<T> s, const ScalarDiv<T>
 //   the residual itself vanishes, exactly as in stress_kernel.
 // Per 2D cell that leaves 24 + 14 FP64 instructions of 58 + 20 (3D: 48 + 27 of 122 + 36).
 // Measured against a loop of stress_kernel and velocity_kernel: 2D 511^2 stress 29.3 -> 15.2 us,
-// velocity 13.3 -> 10.8 us; 3D 95 x 80 x 112 stress 244 -> 109 us, velocity 90 -> 68 us.
+// velocity 13.3 -> 10.8 us; 3D 95 x 80 x 112 stress 244 -> 84 us, velocity 90 -> 53 us.
 // With one scalar viscosity the loop keeps stress_kernel and velocity_kernel, whose divisions by
 // scalars are ConstDiv: coupled to the thermal step, whose fixed-point iteration can amplify a last
 // bit of V from one iteration to the next, the loop has to leave the same bits as the kernels apart.
@@ -339,10 +335,8 @@ struct PtCoef {
 // The viscosity terms over [0, n+1]^N. cP carries a factor 1/2 for the doubled divergence.
 template <class T, int ND>
 __global__ void coef_kernel(const SV<T> v, const SP<T> s, const PtCoef<T> c, int e0, int e1) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = ND > 2 ? blockIdx.z : 0;
-    if (i > e0 || j > e1) return;
+    int i, j, k;
+    if (!launch_point<ND>(e0, e1, i, j, k)) return;
     const T ie = v.inv_eta(i, j, k);
     const T eve = T(1) / (ie + s.inv_Gdt);
     c.cP(i, j, k) = T(0.5) * (eve * s.dtau_Pr);
@@ -395,10 +389,8 @@ template <class T, int ND, bool WRITE_RES, class M>
 __global__ void stress_loop_kernel(const SV<T> v, const PtCoef<T> c, int e0, int e1, const M m) {
     cg_dep_wait();
     cg_dep_release();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = ND > 2 ? blockIdx.z : 0;
-    if (i > e0 || j > e1) return;
+    int i, j, k;
+    if (!launch_point<ND>(e0, e1, i, j, k)) return;
     stress_loop_point<T, ND, WRITE_RES>(v, c, i, j, k, m);
 }
 
@@ -408,10 +400,8 @@ template <class T, int ND, bool WRITE_RES, class M>
 __global__ void velocity_loop_kernel(const SV<T> v, const PtCoef<T> c, const BodyFn<T> bf, int e0, int e1, const M m) {
     cg_dep_wait();
     cg_dep_release();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = ND > 2 ? blockIdx.z : 0;
-    if (i > e0 || j > e1) return;
+    int i, j, k;
+    if (!launch_point<ND>(e0, e1, i, j, k)) return;
     constexpr int XY = ND == 2 ? 2 : 3, XZ = 4, YZ = 5;
     const int LXY = 3, LXZ = 5, LYZ = 6;  // location bits of the shear components
     const T p = m(0, v.P, i, j, k);
@@ -558,8 +548,8 @@ __global__ void __launch_bounds__(256) thermal_step_kernel(const ThermalStep<T> 
 }
 
 // The thermal step of one PT iteration and update_stress! of the next in one 2D launch: both read V as
-// bc!(V) left it and neither reads what the other writes. The first ns blocks (gx across) take the
-// stress, the others (tx across) the thermal tiles. LOOP: the stress from a loop's coefficients.
+// bc!(V) left it and neither reads what the other writes. The first ns blocks take the
+// stress (points in order, as launch_point), the others (tx across) the thermal tiles. LOOP: the stress from a loop's coefficients.
 //
 // A thermal iteration on a small grid is a chain of launches, each with its own latency and with SMs idle
 // in its last wave. With this launch, and bc!(T) beside the next bc!(V), a chain of five becomes one of
@@ -572,7 +562,7 @@ constexpr int kPairRows = 4;
 template <class T, bool LOOP, bool WRITE_RES>
 __global__ void __launch_bounds__(32 * kPairRows)
     stress_thermal_kernel(const SV<T> v, const SP<T> s, const ScalarDiv<T> sd, const PtCoef<T> c, const ThermalStep<T> a, int e0,
-                          int e1, int gx, int ns, int tx) {
+                          int e1, int ns, int tx) {
     cg_dep_wait();
     cg_dep_release();
     const int b = blockIdx.x;
@@ -580,8 +570,9 @@ __global__ void __launch_bounds__(32 * kPairRows)
         thermal_tile<T, 2, kPairRows>(a, (b - ns) % tx, (b - ns) / tx, 0, e0, e1, 0);
         return;
     }
-    const int i = b % gx * 32 + threadIdx.x, j = b / gx * kPairRows + threadIdx.y;
-    if (i > e0 || j > e1) return;
+    const unsigned q = (unsigned)b * (32 * kPairRows) + threadIdx.y * 32 + threadIdx.x, w = (unsigned)e0 + 1u;
+    const int j = (int)(q / w), i = (int)(q - (unsigned)j * w);
+    if (j > e1) return;
     if constexpr (LOOP) stress_loop_point<T, 2, WRITE_RES>(v, c, i, j, 0, NoMask<T>{});
     else stress_point<T, 2, WRITE_RES>(v, s, sd, i, j, 0, NoMask<T>{});
 }
