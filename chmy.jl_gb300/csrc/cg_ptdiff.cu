@@ -441,17 +441,21 @@ __global__ void __launch_bounds__(32 * NW, MINB)
 //
 // bc!(C) is folded into the stores (PdEdge): the thread that updates a cell beside a boundary writes
 // the ghost cells that follow it, in cg_bc_apply's order (z, then y, then x), and a ghost cell under a
-// rule is not stored by itself; warps with no boundary cell store straight away.
-// Measured, an iteration with its bc!: 128^3 in the pool layout 32.5 -> 27 us (a solve 18.9 -> 16.4 ms),
-// 60 x 77 x 50 a solve 6.7 -> 2.6 ms, and 191 x 160 x 128 in the dense layout, which ran the flux and
-// update kernels apart, 55.7 -> 43.3 us (47.4 with a guard at every load). Reading the same bytes with
-// this access pattern and nothing else takes 17 us at 128^3 and 56 at 192^3 (73 here): instruction issue
-// (190 per warp and row) and the latency of 20 resident warps together hold it there. From about 256^3
-// on the TMA-fed kernel is ahead (384^3: 435 us against 504), so it stays a candidate. Three rows per
-// thread (123 registers, 4 blocks per SM) or two (95, 5) beat four; the loads of the next plane are in
-// flight while a plane is computed (without that 37 us at 128^3); copying two planes ahead to shared
-// memory by cp.async, at 24 to 32 warps per SM, took 30.5. Short z segments (3 to 16 planes) fill the
-// SMs of small grids.
+// rule is not stored by itself. Warps at y and z boundaries take a general path, those at x boundaries
+// only add the ghost stores (with five strips across, two are at an x boundary: in the general path
+// they held the launch at 26.7 us, 24 now).
+//
+// Measured, an iteration with its bc!: 128^3 in the pool layout 32.5 -> 21.8 us (a solve 17.5 -> 13.0 ms),
+// 192^3 87 -> 66, 60 x 77 x 50 a solve 6.2 -> 2.4 ms, and 191 x 160 x 128 in the dense layout, which ran
+// the flux and update kernels apart, 55.7 -> 39 us. Reading and writing the same bytes with this access
+// pattern and nothing else takes 17 us at 128^3, 56 at 192^3 and 124 at 256^3 (137 here, 150 by the
+// TMA-fed kernel; 384^3 412 and 436; at 512^3 the TMA-fed kernel's 957 is ahead of 959). Instruction issue bounds it beside
+// memory: 240 instructions per warp and row with a guard at every load, 190 without. Two rows per thread
+// at 6 blocks per SM (80 registers) and three at 5 (96) beat four rows, and the same rows with more
+// registers and fewer blocks (128^3: 23.9 and 24.1) or with 7 or 8 blocks. The loads of the next plane
+// are in flight while a plane is computed (without that 37 us at 128^3). Copying two planes ahead to
+// shared memory by cp.async, at 24 to 32 warps per SM, was slower at equal instructions (30.5 against
+// 27), as was unrolling two planes (31). Short z segments (3 to 22 planes) fill the SMs.
 template <class T>
 struct PdEdge {
     int r[3][2];  // [dimension][side]: 0 none, 1 Dirichlet (2 v - C), 2 Neumann (C -/+ h v)
@@ -556,16 +560,22 @@ __global__ void __launch_bounds__(128, MINB)
             const T rr = rsub(rmul(-rsub(cc, n.co[r]), f.inv_dt), dv);
             v[r] = radd(cc, rmul(rr, f.dtc));
         }
-        const bool zedge = (er.r[2][0] && k <= 1) || (er.r[2][1] && k + 1 >= e2);
+        const bool slow = yedge || (er.r[2][0] && k <= 1) || (er.r[2][1] && k + 1 >= e2);
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             if (!own || jb + r > e1) continue;
             f.qn[0][rx[r] + zx] = n.qx[r];
             f.qn[1][ro[r + 1] + zy] = n.qy[r];
             f.qn[2][ro[r + 1] + zc] = qzl[r];
-            if (!(xedge || yedge || zedge)) f.Cn[ro[r + 1] + zc] = v[r];
+            if (slow) continue;
+            T* const C = f.Cn + (ro[r + 1] + zc);
+            if (!xg) *C = v[r];
+            if (xedge) {
+                if (x0) C[-1] = pd_edge(er, 0, 0, v[r]);
+                if (x1) C[1] = pd_edge(er, 0, 1, v[r]);
+            }
         }
-        if (xedge || yedge || zedge) {
+        if (slow) {
 #pragma unroll 1
             for (int r = 0; r < R; ++r) {
                 const int j = jb + r, p = i + j * f.s1 + zc;
@@ -745,17 +755,19 @@ cudaError_t launch_pd_tma(const PDM<float>& f, const cg_grid* g, int num_sms, cu
 // ptd_tma_kernel (inputs staged by TMA; only with tensor maps for the direction), rings of 4
 // planes with the shared memory of the widest boxes: blocks of 8, 16, 20 and 24 rows (at 512^3
 // 24 rows, 2 blocks per SM, measured fastest; 32 rows, 1 block per SM, 27 % slower).
-// Variants 8 and 9, ptd_rows_kernel: 3 rows per thread and 2; the only ones that take a layout whose
+// Variants 8 to 10, ptd_rows_kernel: 3 rows per thread at 5 blocks per SM, 2 at 6 and 2 at 5 (the last for
+// the smallest grids, 60 x 77 x 50 7.4 -> 6.9 us); the only ones that take a layout whose
 // arrays do not share their strides, and the only ones that fold bc! into their stores.
-constexpr int kPdVariants = 10;
+constexpr int kPdVariants = 11;
 constexpr int kPdTmaFirst = 4;
 constexpr int kPdRowsFirst = 8;
 
 template <class T>
 cudaError_t launch_pd_march3d(const PDM<T>& f, const cg_grid* g, int num_sms, cudaStream_t st, int variant,
                               const PdDir& dir = PdDir{}, const PdEdge<T>& er = PdEdge<T>{}, int seg = 0, bool dep = false) {
-    if (variant == kPdRowsFirst) return launch_pd_rows<T, 3, 4>(f, er, g, num_sms, st, seg, dep);
-    if (variant > kPdRowsFirst) return launch_pd_rows<T, 2, 5>(f, er, g, num_sms, st, seg, dep);
+    if (variant == kPdRowsFirst) return launch_pd_rows<T, 3, 5>(f, er, g, num_sms, st, seg, dep);
+    if (variant == kPdRowsFirst + 1) return launch_pd_rows<T, 2, 6>(f, er, g, num_sms, st, seg, dep);
+    if (variant > kPdRowsFirst + 1) return launch_pd_rows<T, 2, 5>(f, er, g, num_sms, st, seg, dep);
     if constexpr (sizeof(T) == 4) {
         if (variant >= kPdTmaFirst && dir.m[0]) {
             const int h = variant - kPdTmaFirst;
@@ -775,7 +787,7 @@ cudaError_t launch_pd_march3d(const PDM<T>& f, const cg_grid* g, int num_sms, cu
     }
 }
 
-// CG_PTD_VARIANT=<0..9> in the environment (read on every call): the fused iteration's layout
+// CG_PTD_VARIANT=<0..10> in the environment (read on every call): the fused iteration's layout
 // instead of the autotuner's (a TMA variant only where its tensor maps exist).
 inline int pd_variant_forced() {
     const char* e = std::getenv("CG_PTD_VARIANT");
@@ -807,7 +819,7 @@ cg_tune_cfg tune_pd(const PDM<T>& f, const cg_grid* g, int num_sms, cudaStream_t
     float tbest = 1e30f;
     for (int v = first; v < kPdVariants; ++v) {
         if (v >= kPdTmaFirst && v < kPdRowsFirst && !tma) continue;
-        for (int seg : {0, 3, 5, 7, 9, 12, 16}) {
+        for (int seg : {0, 3, 5, 7, 10, 12, 16, 22}) {
             if (seg && (v < kPdRowsFirst || seg > g->n[2] + 2)) continue;
             const float t = cgk::time_launches(
                 [&] {

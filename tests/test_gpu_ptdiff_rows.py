@@ -1,4 +1,4 @@
-"""The PT-diffusion iteration with several rows per thread (ptd_rows_kernel, layouts 8 and 9) with
+"""The PT-diffusion iteration with several rows per thread (ptd_rows_kernel, layouts 8 to 10) with
 bc! folded into its stores, in the pool layout and in Chmy's dense layout."""
 
 import ctypes
@@ -31,7 +31,7 @@ def _desc(fs):
     return s
 
 
-@pytest.mark.parametrize("variant", [8, 9])
+@pytest.mark.parametrize("variant", [8, 9, 10])
 @pytest.mark.parametrize("pitch", [0, 128])
 @pytest.mark.parametrize("dims", [(2, 2, 2), (28, 3, 5), (29, 6, 4), (31, 7, 17), (58, 9, 3), (59, 2, 35)])
 @pytest.mark.parametrize("kind", list(SPECS))
