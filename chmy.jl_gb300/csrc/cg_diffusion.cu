@@ -333,8 +333,11 @@ cudaError_t march_launch(const cg_grid* g, const cg_field* Co, const cg_field* C
 
 // The layout of the step's launch for this grid, timed on C_out = step(C_in) (the first step of a run
 // writes the same points again), or its cached choice when `may_time` is false: in 2D the march's
-// segment length in x (short segments balance the SMs, long ones recompute fewer y fluxes), in 3D
-// the tile kernel's block; 1D keeps 256 threads.
+// segment length in x (short segments balance the SMs, long ones recompute fewer y fluxes) and in y
+// whether a run uses dependent launches, in 3D the tile kernel's block; 1D keeps 256 threads.
+// Dependent launches hide the launch latency (126^2 4.2 -> 2.6 us per step), but where a grid is about one
+// wave the next launch's blocks gather on the SMs that end early (1024^2, segments of 12 rows: 28.7 ->
+// 45.3 us), so both are timed.
 template <class T, int ND>
 dim3 step_block(cg_ctx* ctx, const cg_grid* g, const cg_field* Co, const cg_field* Ci, double chi, double dt,
                 bool may_time) {
@@ -346,23 +349,26 @@ dim3 step_block(cg_ctx* ctx, const cg_grid* g, const cg_field* Co, const cg_fiel
     cg_key_add(key, Co->stride);
     cg_key_add(key, ctx->num_sms);
     if constexpr (ND == 2) {
-        cg_tune_cfg c{8, 1};
-        if (cg_tune_lookup(key, &c) || !may_time || !cg_autotune_enabled()) return dim3((unsigned)c.seg);
+        cg_tune_cfg c{8, (long)g->n[0] * g->n[1] <= 1700l * ctx->num_sms};
+        if (cg_tune_lookup(key, &c) || !may_time || !cg_autotune_enabled()) return dim3((unsigned)c.seg, (unsigned)c.variant);
         EdgeRules<T> er;
         edge_rules<T>(g, nullptr, &er);
         float best = 1e30f;
-        for (int seg : {1, 2, 3, 4, 6, 8, 12, 16, 24}) {
-            const float t = cgk::time_launches([&] { return march_launch<T>(g, Co, Ci, chi, dt, seg, er, ctx->stream, false); }, ctx->stream);
-            if (cg_tune_verbose())
-                std::fprintf(stderr, "diffusion step tune %dx%d: seg %d: %.1f us\n", g->n[0], g->n[1], seg, t >= 0.f ? 1e3f * t / 3 : -1.f);
-            if (t >= 0.f && t < best) {
-                best = t;
-                c.seg = seg;
+        for (int seg : {1, 2, 3, 4, 6, 8, 12, 16, 24})
+            for (int dep = 0; dep < 2; ++dep) {
+                const float t = cgk::time_launches(
+                    [&] { return march_launch<T>(g, Co, Ci, chi, dt, seg, er, ctx->stream, dep != 0); }, ctx->stream);
+                if (cg_tune_verbose())
+                    std::fprintf(stderr, "diffusion step tune %dx%d: seg %d%s: %.1f us\n", g->n[0], g->n[1], seg,
+                                 dep ? ", dependent" : "", t >= 0.f ? 1e3f * t / 3 : -1.f);
+                if (t >= 0.f && t < best) {
+                    best = t;
+                    c = cg_tune_cfg{seg, dep};
+                }
             }
-        }
         cudaGetLastError();
         cg_tune_store(key, c);
-        return dim3((unsigned)c.seg);
+        return dim3((unsigned)c.seg, (unsigned)c.variant);
     } else {
         if (!may_time) {
             dim3 b(32, 8);
@@ -393,9 +399,9 @@ int step_t(cg_ctx* ctx, const cg_grid* g, const cg_field* Co, const cg_field* Ci
 // The steps of a 2D run with bc! folded into them: A -> B -> A ..., and one bc! launch at the end.
 template <class T>
 int folded_steps(cg_ctx* ctx, const cg_grid* g, const cg_field* A, const cg_field* B, double chi, double dt, const cg_bc* bc,
-                 const EdgeRules<T>& er, int seg, int nsteps, cudaStream_t st) {
+                 const EdgeRules<T>& er, int seg, bool dep, int nsteps, cudaStream_t st) {
     for (int k = 0; k < nsteps; ++k) {
-        const cudaError_t e = march_launch<T>(g, k % 2 ? A : B, k % 2 ? B : A, chi, dt, seg, er, st, k > 0);
+        const cudaError_t e = march_launch<T>(g, k % 2 ? A : B, k % 2 ? B : A, chi, dt, seg, er, st, dep && k > 0);
         if (e != cudaSuccess) return cg_fail(ctx, CG_ERR_CUDA, "diffusion step: %s", cudaGetErrorString(e));
     }
     if (!bc) return CG_OK;
@@ -543,9 +549,9 @@ extern "C" int cg_diffusion_run(cg_ctx* ctx, const cg_grid* grid, const cg_field
             EdgeRules<double> ed;
             EdgeRules<float> ef;
             if (A->dtype == CG_F64 && edge_rules(grid, bc, &ed))
-                return folded_steps(ctx, grid, A, B, chi, dt, bc, ed, (int)blk.x, nsteps, st);
+                return folded_steps(ctx, grid, A, B, chi, dt, bc, ed, (int)blk.x, blk.y != 0, nsteps, st);
             if (A->dtype == CG_F32 && edge_rules(grid, bc, &ef))
-                return folded_steps(ctx, grid, A, B, chi, dt, bc, ef, (int)blk.x, nsteps, st);
+                return folded_steps(ctx, grid, A, B, chi, dt, bc, ef, (int)blk.x, blk.y != 0, nsteps, st);
         }
         for (int s = 0; s < nsteps; ++s) {
             const cg_field* in = (s % 2 == 0) ? A : B;

@@ -525,9 +525,11 @@ inline cg_tune_cfg tune_march2d(const Fused2D<T>& f, const SP<T>& s, int n0, int
     cg_key_add(key, (int)tile);
     if (cg_tune_lookup(key, &best)) return best;
     float tbest = 1e30f;
+    // as dependent launches, which a run uses: where a grid is about one wave they can cost a layout half
+    // its speed
     for (int seg : {0, 8, 16, 24, 32, 48, 64}) {
         if (seg > n1 + 2) continue;
-        const float t = time_launches([&] { return launch_march2d<T, false>(f, s, n0, n1, nsm, seg, st); }, st);
+        const float t = time_launches([&] { return launch_march2d<T, false>(f, s, n0, n1, nsm, seg, st, true); }, st);
         if (cg_tune_verbose())
             std::fprintf(stderr, "march2d tune %dx%d: seg %d: %.1f us\n", n0, n1, seg, t >= 0.f ? 1e3f * t / 3 : -1.f);
         if (t >= 0.f && t < tbest) {
@@ -539,7 +541,7 @@ inline cg_tune_cfg tune_march2d(const Fused2D<T>& f, const SP<T>& s, int n0, int
         for (int v = 1; tile && v <= kTileVariants; ++v) {
             const int kit = kTileIters[v - 1];
             float t = time_launches(
-                [&] { return launch_march2d_tile<T, false>(f, s, n0, n1, v, kit, true, TileStatic<T>{nullptr, 0}, st); }, st);
+                [&] { return launch_march2d_tile<T, false>(f, s, n0, n1, v, kit, true, TileStatic<T>{nullptr, 0}, st, true); }, st);
             if (t >= 0.f) t /= (float)kit;
             if (cg_tune_verbose())
                 std::fprintf(stderr, "march2d tune %dx%d: tiles, variant %d, %d iterations: %.2f us per iteration\n", n0, n1, v, kit,

@@ -256,7 +256,7 @@ size_t padded_count(const cg_field& f) {
 //
 // Latency bounds a check, which is a chain of small launches: the boundary condition of r_V, the
 // reduction of divV and r_V, the reduction of r_tau, two memsets and a copy took 24 us after a
-// chunk's 48 iterations (66 us) at 191 x 191, this launch 7: the solve 20.0 -> 16.3 ms.
+// chunk's 48 iterations (66 us) at 191 x 191, this launch 6: the solve 20.0 -> 16.3 ms.
 struct Measure {
     unsigned* slot;   // device: [0] divV, [1..ND] r_V, [ND + 1] r_tau, [kTicket] blocks done
     unsigned* host;   // pinned: the same maxima, [kTicket] the wait flag
