@@ -43,7 +43,9 @@ struct MAt3 {
         return o[c] + (Ix)k * s2[c];
     }
     // c: the array's location class
-    __device__ __forceinline__ T ld(int c, const DF<T>& f, int k, bool ok) const {
+    // ld: an array that the launch before writes; ldc: one that no launch of the chain writes (see MAt)
+    __device__ __forceinline__ T ld(int c, const DF<T>& f, int k, bool ok) const { return ok ? f.p[off(c, f, k)] : T(0); }
+    __device__ __forceinline__ T ldc(int c, const DF<T>& f, int k, bool ok) const {
         return ok ? __ldg(f.p + off(c, f, k)) : T(0);
     }
     __device__ __forceinline__ void st(int c, const DF<T>& f, int k, T v) const { f.p[off(c, f, k)] = v; }
@@ -73,26 +75,26 @@ __device__ __forceinline__ M3Row<T> m3_load(const Fused3D<T>& f, const MAt3<T, I
     r.vx = at.ld(1, f.V_in[0], kn, vn);
     r.vy = at.ld(2, f.V_in[1], kn, vn);
     r.vz = at.ld(0, f.V_in[2], kn, vn);
-    r.ie = at.ld(0, f.ieta, kn, vn);
+    r.ie = at.ldc(0, f.ieta, kn, vn);
     r.txz = at.ld(1, f.tau_in[4], kn, vn && nd.xz);
-    r.txzo = at.ld(1, f.tau_o[4], kn, cn && nd.xz);
+    r.txzo = at.ldc(1, f.tau_o[4], kn, cn && nd.xz);
     r.tyz = at.ld(2, f.tau_in[5], kn, vn && nd.yz);
-    r.tyzo = at.ld(2, f.tau_o[5], kn, cn && nd.yz);
+    r.tyzo = at.ldc(2, f.tau_o[5], kn, cn && nd.yz);
     const bool c = inC && k <= e2;
     const bool v = inV && k <= e2;
     r.P = at.ld(0, f.P_in, k, c && nd.cell_p);
     r.tyy = at.ld(0, f.tau_in[1], k, c && nd.cell_p);
-    r.tyo = at.ld(0, f.tau_o[1], k, c && nd.cell_p);
-    r.fp = f.has_fP ? at.ld(0, f.fP, k, c && nd.cell_p) : T(0);
+    r.tyo = at.ldc(0, f.tau_o[1], k, c && nd.cell_p);
+    r.fp = f.has_fP ? at.ldc(0, f.fP, k, c && nd.cell_p) : T(0);
     r.txx = at.ld(0, f.tau_in[0], k, c && nd.cell_d);
     r.tzz = at.ld(0, f.tau_in[2], k, c && nd.cell_d);
-    r.txo = at.ld(0, f.tau_o[0], k, c && nd.cell_d);
-    r.tzo = at.ld(0, f.tau_o[2], k, c && nd.cell_d);
+    r.txo = at.ldc(0, f.tau_o[0], k, c && nd.cell_d);
+    r.tzo = at.ldc(0, f.tau_o[2], k, c && nd.cell_d);
     r.txy = at.ld(3, f.tau_in[3], k, v && nd.xy);
-    r.txyo = at.ld(3, f.tau_o[3], k, c && nd.xy);
-    r.rhox = f.has_rho[0] ? at.ld(1, f.rho[0], k, c && nd.rho) : T(0);
-    r.rhoy = f.has_rho[1] ? at.ld(2, f.rho[1], k, c && nd.rho) : T(0);
-    r.rhoz = f.has_rho[2] ? at.ld(0, f.rho[2], k, c && nd.rho) : T(0);
+    r.txyo = at.ldc(3, f.tau_o[3], k, c && nd.xy);
+    r.rhox = f.has_rho[0] ? at.ldc(1, f.rho[0], k, c && nd.rho) : T(0);
+    r.rhoy = f.has_rho[1] ? at.ldc(2, f.rho[1], k, c && nd.rho) : T(0);
+    r.rhoz = f.has_rho[2] ? at.ldc(0, f.rho[2], k, c && nd.rho) : T(0);
     return r;
 }
 
@@ -207,16 +209,16 @@ __global__ void __launch_bounds__(32 * NW, MINB)
     {
         const int kp = ks - 1;  // >= -1
         const T vxp = at.ld(1, f.V_in[0], kp, inV), vyp = at.ld(2, f.V_in[1], kp, inV), vzp = at.ld(0, f.V_in[2], kp, inV);
-        const T iep = at.ld(0, f.ieta, kp, inV);
+        const T iep = at.ldc(0, f.ieta, kp, inV);
         const T pp = at.ld(0, f.P_in, kp, inC && !hi), tzp = at.ld(0, f.tau_in[2], kp, inC && !hi);
-        const T tzop = at.ld(0, f.tau_o[2], kp, inC && !hi);
-        const T fpp = f.has_fP ? at.ld(0, f.fP, kp, inC && !hi) : T(0);
+        const T tzop = at.ldc(0, f.tau_o[2], kp, inC && !hi);
+        const T fpp = f.has_fP ? at.ldc(0, f.fP, kp, inC && !hi) : T(0);
         vx_c = at.ld(1, f.V_in[0], ks, inV);
         vy_c = at.ld(2, f.V_in[1], ks, inV);
         vz_c = at.ld(0, f.V_in[2], ks, inV);
-        ie_c = at.ld(0, f.ieta, ks, inV);
-        const T txz0 = at.ld(1, f.tau_in[4], ks, inV && nd.xz), txzo0 = at.ld(1, f.tau_o[4], ks, inC && nd.xz);
-        const T tyz0 = at.ld(2, f.tau_in[5], ks, inV && nd.yz), tyzo0 = at.ld(2, f.tau_o[5], ks, inC && nd.yz);
+        ie_c = at.ldc(0, f.ieta, ks, inV);
+        const T txz0 = at.ld(1, f.tau_in[4], ks, inV && nd.xz), txzo0 = at.ldc(1, f.tau_o[4], ks, inC && nd.xz);
+        const T tyz0 = at.ld(2, f.tau_in[5], ks, inV && nd.yz), tyzo0 = at.ldc(2, f.tau_o[5], ks, inC && nd.yz);
         sm.vx[w][lane] = iep;  // 1/eta at plane ks-1
         sm.vy[w][lane] = vyp;
         sm.vz[w][lane] = vz_c;

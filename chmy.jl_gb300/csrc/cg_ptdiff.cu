@@ -436,7 +436,9 @@ __global__ void __launch_bounds__(32 * NW, MINB)
 // in registers, each z face carried up. No value is loaded twice but the two halo rows and lanes,
 // every face of the tile is computed once, and there is neither shared memory nor a barrier. No load has
 // a guard (columns and rows beyond the range are clamped to stored ones). Same operations as
-// ptd_march3d_kernel, so the same bits. It reads the strides of q.x and q.y apart from C's, so Chmy's
+// ptd_march3d_kernel, so the same bits. As a dependent launch it is resident while the iteration before
+// still writes C and q, so these are read by plain loads (__ldg wants data that does not change during the
+// kernel); D and C_old, which no iteration writes, by __ldg. It reads the strides of q.x and q.y apart from C's, so Chmy's
 // dense layout takes it too.
 //
 // bc!(C) is folded into the stores (PdEdge): the thread that updates a cell beside a boundary writes
@@ -503,13 +505,13 @@ __global__ void __launch_bounds__(128, MINB)
     T c[R + 2], d[R + 2], qzl[R];
 #pragma unroll
     for (int r = 0; r < R + 2; ++r) {
-        c[r] = __ldg(f.C + ro[r] + zc);
+        c[r] = f.C[ro[r] + zc];
         d[r] = __ldg(f.D + ro[r] + zc);
     }
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const int p = ro[r + 1] + zc;
-        qzl[r] = pd_face(__ldg(f.q[2] + p), __ldg(f.D + p - f.s2), d[r + 1], __ldg(f.C + p - f.s2), c[r + 1], f.idx[2], f.om);
+        qzl[r] = pd_face(f.q[2][p], __ldg(f.D + p - f.s2), d[r + 1], f.C[p - f.s2], c[r + 1], f.idx[2], f.om);
     }
     // plane k's fluxes and C_old, and plane k+1's C, D and z flux
     PdPlane<T, R> cur;
@@ -517,19 +519,19 @@ __global__ void __launch_bounds__(128, MINB)
     auto load = [&](int k) {
         if (k <= ke) {
 #pragma unroll
-            for (int r = 0; r < R; ++r) cur.qx[r] = __ldg(f.q[0] + rx[r] + zxs);
+            for (int r = 0; r < R; ++r) cur.qx[r] = f.q[0][rx[r] + zxs];
 #pragma unroll
-            for (int r = 0; r < R + 1; ++r) cur.qy[r] = __ldg(f.q[1] + ro[r + 1] + zys);
+            for (int r = 0; r < R + 1; ++r) cur.qy[r] = f.q[1][ro[r + 1] + zys];
 #pragma unroll
             for (int r = 0; r < R; ++r) cur.co[r] = __ldg(f.Co + ro[r + 1] + zcs);
             zcs += f.s2;
 #pragma unroll
             for (int r = 0; r < R + 2; ++r) {
-                cur.c[r] = __ldg(f.C + ro[r] + zcs);
+                cur.c[r] = f.C[ro[r] + zcs];
                 cur.d[r] = __ldg(f.D + ro[r] + zcs);
             }
 #pragma unroll
-            for (int r = 0; r < R; ++r) cur.qz[r] = __ldg(f.q[2] + ro[r + 1] + zcs);
+            for (int r = 0; r < R; ++r) cur.qz[r] = f.q[2][ro[r + 1] + zcs];
             zxs += f.s2x;
             zys += f.s2y;
         }

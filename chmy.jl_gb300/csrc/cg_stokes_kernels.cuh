@@ -704,7 +704,11 @@ struct MAt {  // column i of a lane
     __device__ __forceinline__ Ix off(int c, const DF<T>& f, int j) const {
         return (Ix)i + (Ix)j * (LAY == kLayOwn ? (Ix)f.s1 : s1[LAY == kLayLoc ? c : 0]);
     }
-    __device__ __forceinline__ T ld(int c, const DF<T>& f, int j, bool ok) const {
+    // ld: an array that the launch before writes (V, P, tau); ldc: one that no launch of the chain
+    // writes. A dependent launch is resident while the one before it still writes, and a
+    // non-coherent load is only defined where the data does not change during the kernel.
+    __device__ __forceinline__ T ld(int c, const DF<T>& f, int j, bool ok) const { return ok ? f.p[off(c, f, j)] : T(0); }
+    __device__ __forceinline__ T ldc(int c, const DF<T>& f, int j, bool ok) const {
         return ok ? __ldg(f.p + off(c, f, j)) : T(0);
     }
     __device__ __forceinline__ void st(int c, const DF<T>& f, int j, T v) const { f.p[off(c, f, j)] = v; }
@@ -726,18 +730,18 @@ __device__ __forceinline__ MarchRow<T> march_load(const Fused2D<T>& f, const MAt
     const bool vn = inV && jn <= e1 + 1;
     r.Vx = at.ld(1, f.Vx_in, jn, vn);
     r.Vy = at.ld(0, f.Vy_in, jn, vn);
-    r.ie = at.ld(0, f.ieta, jn, vn);
+    r.ie = at.ldc(0, f.ieta, jn, vn);
     r.txy = at.ld(1, f.txy_in, jn, vn);
-    r.txyo = at.ld(1, f.txy_o, jn, inC && jn <= e1);
+    r.txyo = at.ldc(1, f.txy_o, jn, inC && jn <= e1);
     const bool c = inC && j <= e1;
     r.P = at.ld(0, f.P_in, j, c);
     r.txx = at.ld(0, f.txx_in, j, c);
     r.tyy = at.ld(0, f.tyy_in, j, c);
-    r.txo = at.ld(0, f.txx_o, j, c);
-    r.tyo = at.ld(0, f.tyy_o, j, c);
-    r.fp = f.has_fP ? at.ld(0, f.fP, j, c) : T(0);
-    r.rhox = f.has_rho ? at.ld(1, f.rhox, j, c) : T(0);
-    r.rhoy = f.has_rho ? at.ld(0, f.rhoy, j, c) : T(0);
+    r.txo = at.ldc(0, f.txx_o, j, c);
+    r.tyo = at.ldc(0, f.tyy_o, j, c);
+    r.fp = f.has_fP ? at.ldc(0, f.fP, j, c) : T(0);
+    r.rhox = f.has_rho ? at.ldc(1, f.rhox, j, c) : T(0);
+    r.rhoy = f.has_rho ? at.ldc(0, f.rhoy, j, c) : T(0);
     return r;
 }
 
@@ -859,16 +863,16 @@ __global__ void __launch_bounds__(128, MINB) march2d_kernel(const Fused2D<T> f, 
         const int jp = js - 1;  // >= -1
         T vxp = at.ld(1, f.Vx_in, jp, inV);
         T vyp = at.ld(0, f.Vy_in, jp, inV);
-        const T iep = at.ld(0, f.ieta, jp, inV);
+        const T iep = at.ldc(0, f.ieta, jp, inV);
         const T pp = at.ld(0, f.P_in, jp, inC);
         const T typ = at.ld(0, f.tyy_in, jp, inC);
-        const T tyop = at.ld(0, f.tyy_o, jp, inC);
-        const T fpp = f.has_fP ? at.ld(0, f.fP, jp, inC) : T(0);
+        const T tyop = at.ldc(0, f.tyy_o, jp, inC);
+        const T fpp = f.has_fP ? at.ldc(0, f.fP, jp, inC) : T(0);
         Vx_c = at.ld(1, f.Vx_in, js, inV);
         Vy_c = at.ld(0, f.Vy_in, js, inV);
-        ie_c = at.ld(0, f.ieta, js, inV);
+        ie_c = at.ldc(0, f.ieta, js, inV);
         const T t2 = at.ld(1, f.txy_in, js, inV);
-        const T o2 = at.ld(1, f.txy_o, js, inC);
+        const T o2 = at.ldc(1, f.txy_o, js, inC);
         // the first marching step's loads (row js+1) are issued before the prologue computes
         cur = march_load(f, at, js, e1, inV, inC);
         if (yb) {
