@@ -813,11 +813,15 @@ cg_tune_cfg tune_pd(const PDM<T>& f, const cg_grid* g, int num_sms, cudaStream_t
     for (int d = 0; d < 3; ++d) cg_key_add(key, g->n[d]);
     cg_key_add(key, f.s1);
     cg_key_add(key, f.s2);
+    // q's own strides too: the layouts below `first` address every array with C's
     cg_key_add(key, f.s1x);
+    cg_key_add(key, f.s2x);
+    cg_key_add(key, f.s2y);
     cg_key_add(key, num_sms);
     cg_key_add(key, (int)tma);
     cg_tune_cfg best{0, first};
-    if (cg_tune_lookup(key, &best)) return best;
+    if (cg_tune_lookup(key, &best) && best.variant >= first) return best;
+    best = cg_tune_cfg{0, first};
     float tbest = 1e30f;
     for (int v = first; v < kPdVariants; ++v) {
         if (v >= kPdTmaFirst && v < kPdRowsFirst && !tma) continue;
