@@ -47,6 +47,10 @@ struct cg_ctx {
 // Device scratch buffer `slot` of at least `bytes` (reallocated when too small; contents are
 // not preserved across growth). Sets *rc on failure and returns NULL.
 void* cg_scratch(cg_ctx* ctx, int slot, size_t bytes, int* rc);
+// Scratch that a call can do without: nullptr, and no error, where it finds no room (`what` names the
+// arrays in the verbose output). CG_SCRATCH_LIMIT=<bytes> in the environment (read on every call) fails
+// every larger scratch request.
+void* cg_scratch_optional(cg_ctx* ctx, int slot, size_t bytes, const char* what);
 // The wait flag of the TMA-fed kernels (scratch slot 10), cleared on the context's stream: a
 // kernel whose bounded wait for staged data ran out sets it. cg_tma_check reads it after a run
 // (synchronising the stream) and reports CG_ERR_TIMEOUT for `what` when it is set.

@@ -223,10 +223,25 @@ int cg_tma_check(cg_ctx* ctx, int* flag, const char* what) {
     return CG_OK;
 }
 
+namespace {
+size_t cg_scratch_limit() {
+    // CG_SCRATCH_LIMIT, read on every call, so that a process can compare runs with and without it
+    const char* e = std::getenv("CG_SCRATCH_LIMIT");
+    if (!e || !e[0]) return ~(size_t)0;
+    char* end = nullptr;
+    const unsigned long long v = std::strtoull(e, &end, 10);
+    return end != e ? (size_t)v : ~(size_t)0;
+}
+}  // namespace
+
 void* cg_scratch(cg_ctx* ctx, int slot, size_t bytes, int* rc) {
     *rc = CG_OK;
     if (slot < 0 || slot >= cg_ctx::kScratchSlots) {
         *rc = cg_fail(ctx, CG_ERR_ARG, "scratch slot %d out of range", slot);
+        return nullptr;
+    }
+    if (bytes > cg_scratch_limit()) {
+        *rc = cg_fail(ctx, CG_ERR_CUDA, "scratch allocation of %zu bytes: more than CG_SCRATCH_LIMIT", bytes);
         return nullptr;
     }
     if (ctx->scratch_bytes[slot] >= bytes) return ctx->scratch[slot];
@@ -243,6 +258,18 @@ void* cg_scratch(cg_ctx* ctx, int slot, size_t bytes, int* rc) {
     }
     ctx->scratch_bytes[slot] = bytes;
     return ctx->scratch[slot];
+}
+
+void* cg_scratch_optional(cg_ctx* ctx, int slot, size_t bytes, const char* what) {
+    char err[sizeof(ctx->err)];
+    std::memcpy(err, ctx->err, sizeof(err));
+    int rc = CG_OK;
+    void* p = cg_scratch(ctx, slot, bytes, &rc);
+    if (!rc) return p;
+    cudaGetLastError();
+    std::memcpy(ctx->err, err, sizeof(err));  // the call goes on: no error to report
+    if (cg_tune_verbose()) std::fprintf(stderr, "%s: no room for %zu bytes of scratch\n", what, bytes);
+    return nullptr;
 }
 
 extern "C" int cg_set_stream(cg_ctx* ctx, void* stream) {

@@ -879,10 +879,11 @@ PDM<T> make_pdm(const cg_grid* g, const cg_field& C, const cg_field* q, const cg
 
 // cg_ptdiff_run on the fused kernel (3D): partner buffers for C and q in scratch slot 2, with
 // the caller's layouts and contents (so the points no iteration writes agree), ping-pong
-// between the two sets, and the result copied back after an odd number of iterations.
+// between the two sets, and the result copied back after an odd number of iterations. *ran = false: the
+// partner buffers found no room and nothing was done.
 template <class T>
 int run_fused3d(cg_ctx* ctx, const cg_grid* g, const cg_ptdiff_fields* f, const cg_ptdiff_params* p, const cg_bc* bc,
-                int nsteps, int npt, std::string key) {
+                int nsteps, int npt, std::string key, bool* ran) {
     size_t bytes[4], off[4], total = 0;
     const cg_field* src[4] = {&f->C, &f->q[0], &f->q[1], &f->q[2]};
     for (int a = 0; a < 4; ++a) {
@@ -891,8 +892,9 @@ int run_fused3d(cg_ctx* ctx, const cg_grid* g, const cg_ptdiff_fields* f, const 
         total += (bytes[a] + 255) & ~(size_t)255;
     }
     int rc = CG_OK;
-    char* base = static_cast<char*>(cg_scratch(ctx, 2, total, &rc));
-    if (rc) return rc;
+    char* base = static_cast<char*>(cg_scratch_optional(ctx, 2, total, "ptdiff partner buffers"));
+    *ran = base != nullptr;
+    if (!base) return CG_OK;
     cg_field part[4];
     for (int a = 0; a < 4; ++a) {
         part[a] = *src[a];
@@ -992,7 +994,12 @@ extern "C" int cg_ptdiff_run(cg_ctx* ctx, const cg_grid* grid, const cg_ptdiff_f
     cg_key_add(key, bc ? *bc : none);
     cg_key_add(key, nsteps);
     cg_key_add(key, npt);
-    if (fused3d_ok(grid, f)) return run_fused3d<float>(ctx, grid, f, p, bc, nsteps, npt, key + "fused3d");
+    if (fused3d_ok(grid, f)) {
+        // without room for the partner buffers the flux and update kernels run in place
+        bool ran = false;
+        rc = run_fused3d<float>(ctx, grid, f, p, bc, nsteps, npt, key + "fused3d", &ran);
+        if (rc || ran) return rc;
+    }
     const size_t cbytes = padded_bytes(f->C);
     const int dtype = f->C.dtype, nd = grid->ndim;
     LoopCoef lc;
