@@ -151,13 +151,19 @@ PdCoef<T> coef_views(const LoopCoef& lc, int nd) {
     return c;
 }
 
+// Whether a run writes D: the caller passes C (a diffusivity that follows the solution), C_old or R for it.
+inline bool D_changes(const cg_ptdiff_fields* f) {
+    const void* D = f->D.data;
+    return D == f->C.data || D == f->C_old.data || (cg_present(f->R) && D == f->R.data);
+}
+
 // Fill the coefficients for a loop of `iters` FP64 iterations. From four iterations on they cost less
 // than they save (one pass over D against three face products per iteration); FP32 is bound by
-// memory and keeps ptdiff_q_kernel, as does a loop whose arrays find no room.
+// memory and keeps ptdiff_q_kernel, as does a loop whose arrays find no room and one that changes D.
 template <class T, int ND>
 int setup_coef(cg_ctx* ctx, const cg_grid* g, const cg_ptdiff_fields* f, const cg_ptdiff_params* p, long iters, LoopCoef* lc) {
     *lc = LoopCoef{};
-    if (sizeof(T) != 8 || iters < 4) return CG_OK;
+    if (sizeof(T) != 8 || iters < 4 || D_changes(f)) return CG_OK;
     const long e0 = g->n[0] + 2, e1 = ND > 1 ? g->n[1] + 2 : 1, e2 = ND > 2 ? g->n[2] + 2 : 1;
     int rc = CG_OK;
     char* base = static_cast<char*>(cg_scratch(ctx, 2, (size_t)(ND * e0 * e1 * e2) * sizeof(T), &rc));
@@ -947,9 +953,11 @@ int run_fused3d(cg_ctx* ctx, const cg_grid* g, const cg_ptdiff_fields* f, const 
 
 // The fused path needs a 3D FP32 grid, no residual output, one row and plane stride for C, C_old, D
 // and q.z, and C's row stride for q.y (Chmy's dense layout, or a common pitch and plane height), with
-// every offset in 32 bits.
+// every offset in 32 bits. D and C_old may not be C itself: the iterations read C from two buffers by
+// turns, these from one.
 bool fused3d_ok(const cg_grid* g, const cg_ptdiff_fields* f) {
     if (g->ndim != 3 || f->C.dtype != CG_F32 || cg_present(f->R) || !cg_ptdiff_fused_enabled()) return false;
+    if (f->D.data == f->C.data || f->C_old.data == f->C.data) return false;
     for (const cg_field* a : {&f->C_old, &f->D, &f->q[2]})
         if (a->stride[1] != f->C.stride[1] || a->stride[2] != f->C.stride[2]) return false;
     if (f->q[1].stride[1] != f->C.stride[1]) return false;
