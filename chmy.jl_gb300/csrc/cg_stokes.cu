@@ -542,7 +542,9 @@ int pt_iterations(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, cons
 int pt_loop(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p, const cg_bc* bc_V,
             int niter, int dtype, const cg_bc* bc_T, const cg_mask* mask) {
     LoopCoef lc;
-    const int rc = SDISPATCH(setup_coef, dtype, g->ndim, ctx, g, f, p, niter, &lc);
+    // a viscosity that is the temperature's array changes within the loop
+    const bool changes = bc_T && (f->eta.data == f->T.data || f->inv_eta.data == f->T.data);
+    const int rc = changes ? CG_OK : SDISPATCH(setup_coef, dtype, g->ndim, ctx, g, f, p, niter, &lc);
     if (rc) return rc;
     return pt_iterations(ctx, g, f, p, bc_V, niter, dtype, &lc, bc_T, mask);
 }
