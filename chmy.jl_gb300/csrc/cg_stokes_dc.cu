@@ -567,6 +567,7 @@ int cg_stokes_solve_dc(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f,
     const bool fold = nd == 2 && cg_bc_fold_enabled() && make_vfold(g, bc0, &vf);
     if (fold) fa.bc = fb.bc = vf;
     cg_key_add(key, (int)fold);
+    for (int d = 0; d < nd; ++d) cg_key_add(key, bc0[d]);  // the kinds that the chunk's launches apply
     // launch layout of the fused kernel, timed on the work buffers (A -> B) before capture
     const cg_tune_cfg tc = nd == 2 ? tune_march2d(fa, s32, g->n[0], g->n[1], ctx->num_sms, ctx->stream)
                                    : tune_march3d(ga, s32, g->n[0], g->n[1], g->n[2], ctx->num_sms, ctx->stream, lga);
