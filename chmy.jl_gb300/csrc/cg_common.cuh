@@ -4,11 +4,13 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <chrono>
 #include <cmath>
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <vector>
 #include <utility>
 
 #include "../../include/chmy_gb300.h"
@@ -220,35 +222,109 @@ __device__ __forceinline__ void block_max_bits(unsigned long long bits, unsigned
     }
 }
 
-// Time (ms) of three launches after one untimed launch, with CUDA events on `st`; -1 if a launch
-// fails (the autotuners' measurement). Where three take less than 0.15 ms, a few microseconds of
-// event and launch noise would decide between candidates (a 254^2 loop took 1.6 or 1.9 ms by the
-// block shapes it drew), so 24 launches are timed then and their time divided by 8.
+// Keeps the stream busy for `ns` (at most a few milliseconds), so that the launches queued behind it run
+// without host gaps.
+template <int>
+__global__ void tune_delay_kernel(unsigned ns) {
+    unsigned long long t0, t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+    for (int it = 0; it < 100000; ++it) {
+        __nanosleep(500);
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+        if (t - t0 >= ns) break;
+    }
+}
+
+// Times (us) of the candidates 0..n-1 of an autotuner, each enqueued on `st` by launch(c) and divided by
+// per[c] (the iterations that one launch of it takes); -1 where one fails or was left out. A user pays for
+// this at the first call of a shape, so it takes few launches: every candidate once, which drops those
+// behind the best, and the others a few times back to back. The launches queue behind a delay kernel, so
+// that the events see the kernels and not the rate at which the host launches them (a pair of events around
+// three bare launches of 3 us varies by more than the candidates differ). A first 50-step run of explicit
+// diffusion takes 1.0 ms at 120^2, 1.6 at 500^2 and 2.8 at 1000^2 this way, 4.7, 7.0 and 16.9 ms with 28 launches
+// of every candidate and a synchronisation after each.
+template <class F>
+inline std::vector<float> time_candidates(int n, F&& launch, cudaStream_t st, std::vector<int> per = {}) {
+    per.resize(n, 1);
+    std::vector<float> us(n, -1.f);
+    std::vector<cudaEvent_t> ev(2 * n, nullptr);
+    bool good = n > 0;
+    for (auto& e : ev) good = good && cudaEventCreate(&e) == cudaSuccess;
+    std::vector<int> todo;
+    // the host's time for one candidate, once its code is loaded (the first launch of a kernel loads it)
+    double host = 8.;
+    bool loaded = false;
+    auto delay = [&](double us_) { tune_delay_kernel<0><<<1, 1, 0, st>>>((unsigned)(1e3 * std::min(us_, 2e3))); };
+    if (good) delay(host * n);
+    for (int c = 0; good && c < n; ++c)
+        for (int again = 0; again < 2; ++again) {
+            const auto h0 = std::chrono::steady_clock::now();
+            cudaEventRecord(ev[2 * c], st);
+            const bool ok = launch(c) == cudaSuccess;
+            cudaEventRecord(ev[2 * c + 1], st);
+            const double took = std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - h0).count();
+            if (!ok) {
+                cudaGetLastError();
+                break;
+            }
+            if (again == 0) todo.push_back(c);
+            if (took < 50.) {
+                host = took;
+                break;
+            }
+            loaded = true;  // launched again
+        }
+    good = good && cudaStreamSynchronize(st) == cudaSuccess;
+    float best = 1e30f;
+    for (int c : todo) {
+        float ms = 0.f;
+        if (good && cudaEventElapsedTime(&ms, ev[2 * c], ev[2 * c + 1]) == cudaSuccess) us[c] = 1e3f * ms / per[c];
+        if (us[c] >= 0.f) best = std::min(best, us[c]);
+    }
+    if (good && todo.size() > 1) {
+        const float bound = 1.25f * best + (loaded ? 12.f : 2.f);
+        todo.erase(std::remove_if(todo.begin(), todo.end(), [&](int c) { return us[c] < 0.f || us[c] > bound; }), todo.end());
+        constexpr size_t kFinal = 8;  // as many are timed again
+        if (todo.size() > kFinal) {
+            std::nth_element(todo.begin(), todo.begin() + kFinal, todo.end(), [&](int a, int b) { return us[a] < us[b]; });
+            todo.resize(kFinal);
+            std::sort(todo.begin(), todo.end());
+        }
+        std::fill(us.begin(), us.end(), -1.f);
+        const int reps = best < 6.f ? 8 : best < 25.f ? 4 : best < 200.f ? 2 : 1;
+        if (best < 25.f) delay(host * (1 + reps * (double)todo.size()));
+        launch(todo[0]);
+        for (int c : todo) {
+            cudaEventRecord(ev[2 * c], st);
+            bool ok = true;
+            for (int r = 0; r < reps && ok; ++r) ok = launch(c) == cudaSuccess;
+            cudaEventRecord(ev[2 * c + 1], st);
+        }
+        good = cudaStreamSynchronize(st) == cudaSuccess;
+        for (int c : todo) {
+            float ms = 0.f;
+            if (good && cudaEventElapsedTime(&ms, ev[2 * c], ev[2 * c + 1]) == cudaSuccess) us[c] = 1e3f * ms / (reps * per[c]);
+        }
+    }
+    for (auto& e : ev)
+        if (e) cudaEventDestroy(e);
+    cudaGetLastError();
+    return us;
+}
+
+// The index of the shortest time in `us`, or -1 where every candidate failed.
+inline int fastest(const std::vector<float>& us) {
+    int b = -1;
+    for (int c = 0; c < (int)us.size(); ++c)
+        if (us[c] >= 0.f && (b < 0 || us[c] < us[b])) b = c;
+    return b;
+}
+
+// Time (us) of one launch, of a few back to back; -1 if a launch fails.
 template <class F>
 inline float time_launches(F&& launch, cudaStream_t st) {
-    cudaEvent_t a, b;
-    if (cudaEventCreate(&a) != cudaSuccess) return -1.f;
-    if (cudaEventCreate(&b) != cudaSuccess) {
-        cudaEventDestroy(a);
-        return -1.f;
-    }
-    float ms = -1.f;
-    auto timed = [&](int n) {
-        if (cudaEventRecord(a, st) != cudaSuccess) return false;
-        for (int r = 0; r < n; ++r)
-            if (launch() != cudaSuccess) return false;
-        return cudaEventRecord(b, st) == cudaSuccess && cudaEventSynchronize(b) == cudaSuccess &&
-               cudaEventElapsedTime(&ms, a, b) == cudaSuccess;
-    };
-    bool ok = launch() == cudaSuccess && timed(3);
-    if (ok && ms < 0.15f) {
-        ok = timed(24);
-        ms /= 8.f;
-    }
-    if (!ok) ms = -1.f;
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
-    return ms;
+    const std::vector<float> us = time_candidates(2, [&](int) { return launch(); }, st);
+    return us[0] >= 0.f && us[1] >= 0.f ? std::min(us[0], us[1]) : std::max(us[0], us[1]);
 }
 
 // A device FunctionField (cg_function) in the field precision.
@@ -315,8 +391,9 @@ inline dim3 point_grid(const int* n, dim3 block) {
 // Block shapes (threads along x, along y) the per-point kernels are timed over. Each thread
 // computes one point whatever the shape, so every shape gives the same bits. 32 x 2 spreads a small
 // FP64 grid evenly (update_stress! at 254^2: 9.7 -> 8.8 us; 256 threads put 2 blocks on most SMs and 1 on
-// the others). kFlatBlocks: the threads of launch_point's in-order blocks.
-constexpr int kBlockShapes[8][2] = {{32, 8}, {32, 4}, {32, 2}, {64, 4}, {128, 2}, {32, 16}, {64, 8}, {128, 4}};
+// the others). kFlatBlocks: the threads of launch_point's in-order blocks; beside these the last three
+// shapes never won (2D and 3D Stokes and PT-diffusion kernels, FP32 and FP64) and are not timed.
+constexpr int kBlockShapes[8][2] = {{32, 8}, {32, 4}, {32, 2}, {128, 2}, {32, 16}, {64, 4}, {64, 8}, {128, 4}};
 constexpr int kFlatBlocks[3] = {64, 128, 256};
 
 // The block shape of a per-point kernel: CG_BLOCK when set, else the fastest of kBlockShapes for
@@ -330,20 +407,14 @@ inline dim3 tune_block(const char* name, const std::string& key, F&& launch, cud
     if (!cg_autotune_enabled()) return b;
     cg_tune_cfg c{0, 0};
     if (cg_tune_lookup(key, &c)) return dim3((unsigned)c.seg, (unsigned)c.variant);
-    float best = 1e30f;
-    auto time = [&](int x, int y) {
-        const dim3 cand((unsigned)x, (unsigned)y);
-        const float t = time_launches([&] { return launch(cand); }, st);
-        if (cg_tune_verbose())
-            std::fprintf(stderr, "%s tune: block %dx%d: %.1f us\n", name, x, y, t >= 0.f ? 1e3f * t / 3 : -1.f);
-        if (t >= 0.f && t < best) {
-            best = t;
-            b = cand;
-        }
-    };
-    for (const auto& sh : kBlockShapes) time(sh[0], sh[1]);
+    std::vector<dim3> cand;
+    for (int q = 0; q < (flat ? 5 : 8); ++q) cand.push_back(dim3((unsigned)kBlockShapes[q][0], (unsigned)kBlockShapes[q][1]));
     for (int x : kFlatBlocks)
-        if (flat) time(x, 1);
+        if (flat) cand.push_back(dim3((unsigned)x, 1));
+    const std::vector<float> us = time_candidates((int)cand.size(), [&](int q) { return launch(cand[q]); }, st);
+    for (size_t q = 0; cg_tune_verbose() && q < cand.size(); ++q)
+        std::fprintf(stderr, "%s tune: block %ux%u: %.1f us\n", name, cand[q].x, cand[q].y, us[q]);
+    if (fastest(us) >= 0) b = cand[fastest(us)];
     cudaGetLastError();
     cg_tune_store(key, cg_tune_cfg{(int)b.x, (int)b.y});
     return b;

@@ -353,19 +353,30 @@ dim3 step_block(cg_ctx* ctx, const cg_grid* g, const cg_field* Co, const cg_fiel
         if (cg_tune_lookup(key, &c) || !may_time || !cg_autotune_enabled()) return dim3((unsigned)c.seg, (unsigned)c.variant);
         EdgeRules<T> er;
         edge_rules<T>(g, nullptr, &er);
-        float best = 1e30f;
+        // the segments as dependent launches, then the three best of them as ordinary ones
+        std::vector<cg_tune_cfg> cand;
         for (int seg : {1, 2, 3, 4, 6, 8, 12, 16, 24})
-            for (int dep = 0; dep < 2; ++dep) {
-                const float t = cgk::time_launches(
-                    [&] { return march_launch<T>(g, Co, Ci, chi, dt, seg, er, ctx->stream, dep != 0); }, ctx->stream);
-                if (cg_tune_verbose())
-                    std::fprintf(stderr, "diffusion step tune %dx%d: seg %d%s: %.1f us\n", g->n[0], g->n[1], seg,
-                                 dep ? ", dependent" : "", t >= 0.f ? 1e3f * t / 3 : -1.f);
-                if (t >= 0.f && t < best) {
-                    best = t;
-                    c = cg_tune_cfg{seg, dep};
-                }
-            }
+            if (seg == 1 || seg <= g->n[1] + 2) cand.push_back(cg_tune_cfg{seg, 1});
+        auto time = [&](const std::vector<cg_tune_cfg>& v) {
+            return cgk::time_candidates(
+                (int)v.size(), [&](int q) { return march_launch<T>(g, Co, Ci, chi, dt, v[q].seg, er, ctx->stream, v[q].variant != 0); },
+                ctx->stream);
+        };
+        std::vector<float> us = time(cand);
+        std::vector<cg_tune_cfg> plain;
+        std::vector<float> left = us;
+        for (int k = 0; k < 3 && cgk::fastest(left) >= 0; ++k) {
+            const int q = cgk::fastest(left);
+            plain.push_back(cg_tune_cfg{cand[q].seg, 0});
+            left[q] = -1.f;
+        }
+        const std::vector<float> up = time(plain);
+        cand.insert(cand.end(), plain.begin(), plain.end());
+        us.insert(us.end(), up.begin(), up.end());
+        for (size_t q = 0; cg_tune_verbose() && q < cand.size(); ++q)
+            std::fprintf(stderr, "diffusion step tune %dx%d: seg %d%s: %.1f us\n", g->n[0], g->n[1], cand[q].seg,
+                         cand[q].variant ? ", dependent" : "", us[q]);
+        if (cgk::fastest(us) >= 0) c = cand[cgk::fastest(us)];
         cudaGetLastError();
         cg_tune_store(key, c);
         return dim3((unsigned)c.seg, (unsigned)c.variant);

@@ -505,7 +505,7 @@ inline cudaError_t launch_march3d(const Fused3D<T>& f, const SP<T>& s, int n0, i
 // captured. Only the `out` buffers of the ping-pong view are written (the first real iteration
 // writes them again); the residual outputs are not touched. Results are cached per shape,
 // precision and layout for the process.
-// 2D candidates: variant 0 is march2d_kernel (one iteration per launch, 7 segment lengths), variants
+// 2D candidates: variant 0 is march2d_kernel (one iteration per launch, 5 to 7 segment lengths), variants
 // 1 and up march2d_tile_kernel's shapes (when march_tile_ok); the time compared is per iteration.
 template <class T>
 inline cg_tune_cfg tune_march2d(const Fused2D<T>& f, const SP<T>& s, int n0, int n1, int nsm, cudaStream_t st) {
@@ -526,34 +526,27 @@ inline cg_tune_cfg tune_march2d(const Fused2D<T>& f, const SP<T>& s, int n0, int
     cg_key_add(key, nsm);
     cg_key_add(key, (int)tile);
     if (cg_tune_lookup(key, &best)) return best;
-    float tbest = 1e30f;
+    std::vector<cg_tune_cfg> cand;
+    for (int seg : {0, 8, 16, 24, 32, 48, 64})
+        if (seg <= n1 + 2 && !(tile && seg % 16 == 8)) cand.push_back(cg_tune_cfg{seg, 0});
+    for (int v = 1; tile && v <= kTileVariants; ++v) cand.push_back(cg_tune_cfg{0, v});
+    std::vector<int> iters;
+    for (const cg_tune_cfg& c : cand) iters.push_back(c.variant ? kTileIters[c.variant - 1] : 1);
     // as dependent launches, which a run uses: where a grid is about one wave they can cost a layout half
     // its speed
-    for (int seg : {0, 8, 16, 24, 32, 48, 64}) {
-        if (seg > n1 + 2) continue;
-        const float t = time_launches([&] { return launch_march2d<T, false>(f, s, n0, n1, nsm, seg, st, true); }, st);
-        if (cg_tune_verbose())
-            std::fprintf(stderr, "march2d tune %dx%d: seg %d: %.1f us\n", n0, n1, seg, t >= 0.f ? 1e3f * t / 3 : -1.f);
-        if (t >= 0.f && t < tbest) {
-            tbest = t;
-            best = cg_tune_cfg{seg, 0};
-        }
-    }
-    if constexpr (sizeof(T) == 4) {
-        for (int v = 1; tile && v <= kTileVariants; ++v) {
-            const int kit = kTileIters[v - 1];
-            float t = time_launches(
-                [&] { return launch_march2d_tile<T, false>(f, s, n0, n1, v, kit, true, TileStatic<T>{nullptr, 0}, st, true); }, st);
-            if (t >= 0.f) t /= (float)kit;
-            if (cg_tune_verbose())
-                std::fprintf(stderr, "march2d tune %dx%d: tiles, variant %d, %d iterations: %.2f us per iteration\n", n0, n1, v, kit,
-                             t >= 0.f ? 1e3f * t / 3 : -1.f);
-            if (t >= 0.f && t < tbest) {
-                tbest = t;
-                best = cg_tune_cfg{0, v};
-            }
-        }
-    }
+    const std::vector<float> us = time_candidates(
+        (int)cand.size(),
+        [&](int q) {
+            if constexpr (sizeof(T) == 4)
+                if (cand[q].variant)
+                    return launch_march2d_tile<T, false>(f, s, n0, n1, cand[q].variant, iters[q], true, TileStatic<T>{nullptr, 0}, st, true);
+            return launch_march2d<T, false>(f, s, n0, n1, nsm, cand[q].seg, st, true);
+        },
+        st, iters);
+    for (size_t q = 0; cg_tune_verbose() && q < cand.size(); ++q)
+        std::fprintf(stderr, "march2d tune %dx%d: variant %d (%d iterations per launch), seg %d: %.2f us per iteration\n", n0, n1,
+                     cand[q].variant, iters[q], cand[q].seg, us[q]);
+    if (fastest(us) >= 0) best = cand[fastest(us)];
     cudaGetLastError();
     cg_tune_store(key, best);
     return best;

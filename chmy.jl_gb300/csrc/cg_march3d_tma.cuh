@@ -587,20 +587,16 @@ inline cg_tune_cfg tune_march3d(const Fused3D<T>& f, const SP<T>& s, int n0, int
     cg_key_add(key, (int)tma);
     if (cg_tune_lookup(key, &best)) return best;
     const int nvar = (sizeof(T) == 4 && lay != kLayOwn) ? kM3Variants : 1;
-    float tbest = 1e30f;
+    std::vector<cg_tune_cfg> cand;
     for (int v = 0; v < nvar; ++v)
-        for (int seg : {0, 4, 8, 16, 32, 64}) {
-            if (seg > n2 + 2 || (m3_staged(v) && (!tma || (seg && seg < 16)))) continue;
-            const float t = time_launches(
-                [&] { return launch_march3d_any<T, false>(f, s, n0, n1, n2, nsm, seg, st, v, false, l); }, st);
-            if (cg_tune_verbose())
-                std::fprintf(stderr, "march3d tune %dx%dx%d: seg %d variant %d: %.1f us\n", n0, n1, n2, seg, v,
-                             t >= 0.f ? 1e3f * t / 3 : -1.f);
-            if (t >= 0.f && t < tbest) {
-                tbest = t;
-                best = cg_tune_cfg{seg, v};
-            }
-        }
+        for (int seg : {0, 4, 8, 16, 32, 64})
+            if ((seg < 32 ? seg <= n2 + 2 : 2 * seg <= n2 + 2) && !(m3_staged(v) && (!tma || (seg && seg < 16)))) cand.push_back(cg_tune_cfg{seg, v});
+    const std::vector<float> us = time_candidates(
+        (int)cand.size(),
+        [&](int q) { return launch_march3d_any<T, false>(f, s, n0, n1, n2, nsm, cand[q].seg, st, cand[q].variant, false, l); }, st);
+    for (size_t q = 0; cg_tune_verbose() && q < cand.size(); ++q)
+        std::fprintf(stderr, "march3d tune %dx%dx%d: seg %d variant %d: %.1f us\n", n0, n1, n2, cand[q].seg, cand[q].variant, us[q]);
+    if (fastest(us) >= 0) best = cand[fastest(us)];
     cudaGetLastError();
     cg_tune_store(key, best);
     return best;

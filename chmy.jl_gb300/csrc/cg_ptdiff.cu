@@ -828,26 +828,25 @@ cg_tune_cfg tune_pd(const PDM<T>& f, const cg_grid* g, int num_sms, cudaStream_t
     cg_tune_cfg best{0, first};
     if (cg_tune_lookup(key, &best) && best.variant >= first) return best;
     best = cg_tune_cfg{0, first};
-    float tbest = 1e30f;
+    // every segment length for every rows layout: their blocks per SM differ, and with them the lengths that
+    // fill whole waves (128^3 in the pool: 3 rows best with 5 planes, 2 rows with 12)
+    std::vector<cg_tune_cfg> cand;
     for (int v = first; v < kPdVariants; ++v) {
         if (v >= kPdTmaFirst && v < kPdRowsFirst && !tma) continue;
-        for (int seg : {0, 3, 5, 7, 10, 12, 16, 22}) {
-            if (seg && (v < kPdRowsFirst || seg > g->n[2] + 2)) continue;
-            const float t = cgk::time_launches(
-                [&] {
-                    const cudaError_t e = launch_pd_march3d<T>(f, g, num_sms, st, v, dir, er, seg, true);
-                    return e != cudaSuccess || v >= kPdRowsFirst ? e : after();
-                },
-                st);
-            if (cg_tune_verbose())
-                std::fprintf(stderr, "ptdiff3d tune %dx%dx%d: variant %d seg %d: %.1f us\n", g->n[0], g->n[1], g->n[2], v, seg,
-                             t >= 0.f ? 1e3f * t / 3 : -1.f);
-            if (t >= 0.f && t < tbest) {
-                tbest = t;
-                best = cg_tune_cfg{seg, v};
-            }
-        }
+        for (int seg : {0, 3, 5, 7, 10, 12, 16, 22})
+            if (!seg || (v >= kPdRowsFirst && seg <= g->n[2] + 2)) cand.push_back(cg_tune_cfg{seg, v});
     }
+    const std::vector<float> us = cgk::time_candidates(
+        (int)cand.size(),
+        [&](int q) {
+            const cudaError_t e = launch_pd_march3d<T>(f, g, num_sms, st, cand[q].variant, dir, er, cand[q].seg, true);
+            return e != cudaSuccess || cand[q].variant >= kPdRowsFirst ? e : after();
+        },
+        st);
+    for (size_t q = 0; cg_tune_verbose() && q < cand.size(); ++q)
+        std::fprintf(stderr, "ptdiff3d tune %dx%dx%d: variant %d seg %d: %.1f us\n", g->n[0], g->n[1], g->n[2], cand[q].variant,
+                     cand[q].seg, us[q]);
+    if (cgk::fastest(us) >= 0) best = cand[cgk::fastest(us)];
     cudaGetLastError();
     cg_tune_store(key, best);
     return best;

@@ -328,17 +328,12 @@ int step_rows(cg_ctx* ctx, const cg_grid* g, const cg_field* H, const cgsia::Mem
                    ? cg_launch(sia_step_kernel<T, false>, dim3(nH), block, 0, st, true, v, words, 0, 0, 1, (char*)nullptr)
                    : e;
     };
-    float best = cgk::time_launches(two, st);
-    if (cg_tune_verbose()) std::fprintf(stderr, "sia step tune: two launches: %.1f us\n", 1e3f * best / 3);
     const StepBufs<T> f{Hb[0], Db[0], v.S[0], Hb[1], Db[1], v.S[1]};
-    for (int cand : kStepRows) {
-        const float t = cgk::time_launches([&] { return launch_whole_step(cand, v, f, words, 0, 0, st); }, st);
-        if (cg_tune_verbose()) std::fprintf(stderr, "sia step tune: one launch, %d rows: %.1f us\n", cand, 1e3f * t / 3);
-        if (t >= 0.f && (best < 0.f || t < best)) {
-            best = t;
-            rows = cand;
-        }
-    }
+    const std::vector<float> us = cgk::time_candidates(
+        4, [&](int c) { return c == 0 ? two() : launch_whole_step(kStepRows[c - 1], v, f, words, 0, 0, st); }, st);
+    for (int c = 0; cg_tune_verbose() && c < 4; ++c)
+        std::fprintf(stderr, "sia step tune: %s, %d rows: %.1f us\n", c ? "one launch" : "two launches", c ? kStepRows[c - 1] : 8, us[c]);
+    if (cgk::fastest(us) > 0) rows = kStepRows[cgk::fastest(us) - 1];
     cudaGetLastError();
     rows = std::max(rows, 0);
     cg_tune_store(key, cg_tune_cfg{rows, 0});

@@ -310,7 +310,7 @@ int run_t(cg_ctx* ctx, int nm, const cg_sia_member* ms, const cg_sia_params* ps,
                         ctx->stream);
                     if (cg_tune_verbose())
                         std::fprintf(stderr, "sia ensemble tune (%d members): 32x%d tiles: %.1f us\n", nm, cand,
-                                     t >= 0.f ? 1e3f * t / 3 : -1.f);
+                                     t);
                     if (t >= 0.f && t < best) {
                         best = t;
                         ty = cand;
