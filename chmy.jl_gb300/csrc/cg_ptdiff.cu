@@ -806,9 +806,11 @@ inline int pd_variant_forced() {
 
 // The fastest layout for this grid and layout, timed on the run's own buffers before its graph
 // is captured (the launches write only the partner buffers) and cached for the process. `after` is the
-// bc! launch that follows an iteration which does not fold it, timed with it.
+// bc! launch that follows an iteration which does not fold it, timed with it; fold: the rows layouts fold
+// the call's rules (without it the launches are the ordinary ones that the run then takes).
 template <class T, class F>
-cg_tune_cfg tune_pd(const PDM<T>& f, const cg_grid* g, int num_sms, cudaStream_t st, const PdDir& dir, const PdEdge<T>& er, F&& after) {
+cg_tune_cfg tune_pd(const PDM<T>& f, const cg_grid* g, int num_sms, cudaStream_t st, const PdDir& dir, const PdEdge<T>& er, bool fold,
+                    bool bc, F&& after) {
     const bool tma = dir.m[0] != nullptr;
     const bool one = f.s1x == f.s1 && f.s2x == f.s2 && f.s2y == f.s2;
     const int first = one ? 0 : kPdRowsFirst;
@@ -825,6 +827,7 @@ cg_tune_cfg tune_pd(const PDM<T>& f, const cg_grid* g, int num_sms, cudaStream_t
     cg_key_add(key, f.s2y);
     cg_key_add(key, num_sms);
     cg_key_add(key, (int)tma);
+    cg_key_add(key, (int)fold + 2 * (int)bc);
     cg_tune_cfg best{0, first};
     if (cg_tune_lookup(key, &best) && best.variant >= first) return best;
     best = cg_tune_cfg{0, first};
@@ -839,8 +842,8 @@ cg_tune_cfg tune_pd(const PDM<T>& f, const cg_grid* g, int num_sms, cudaStream_t
     const std::vector<float> us = cgk::time_candidates(
         (int)cand.size(),
         [&](int q) {
-            const cudaError_t e = launch_pd_march3d<T>(f, g, num_sms, st, cand[q].variant, dir, er, cand[q].seg, true);
-            return e != cudaSuccess || cand[q].variant >= kPdRowsFirst ? e : after();
+            const cudaError_t e = launch_pd_march3d<T>(f, g, num_sms, st, cand[q].variant, dir, er, cand[q].seg, fold);
+            return e != cudaSuccess || (fold && cand[q].variant >= kPdRowsFirst) ? e : after();
         },
         st);
     for (size_t q = 0; cg_tune_verbose() && q < cand.size(); ++q)
@@ -913,7 +916,7 @@ int run_fused3d(cg_ctx* ctx, const cg_grid* g, const cg_ptdiff_fields* f, const 
     const PdDir dab = pd_dir(tma, true), dba = pd_dir(tma, false);
     PdEdge<T> er;
     const bool edges = pd_edges(g, bc, &er);
-    const cg_tune_cfg tc = tune_pd<T>(ab, g, ctx->num_sms, ctx->stream, dab, er, pd_bc_after(ctx, g, part[0], bc));
+    const cg_tune_cfg tc = tune_pd<T>(ab, g, ctx->num_sms, ctx->stream, dab, er, edges, bc != nullptr, pd_bc_after(ctx, g, part[0], bc));
     const int variant = tc.variant;
     const bool staged = variant >= kPdTmaFirst && variant < kPdRowsFirst, fold = variant >= kPdRowsFirst && edges;
     cg_key_add(key, base);
@@ -1340,7 +1343,7 @@ int solve_dc(cg_ctx* ctx, const cg_grid* g, const cg_ptdiff_fields* f, const cg_
     const PdDir dab = pd_dir(tma, true), dba = pd_dir(tma, false);
     PdEdge<float> er;
     const bool edges = pd_edges(g, &bc0, &er);
-    const cg_tune_cfg tc = tune_pd<float>(ab, g, ctx->num_sms, ctx->stream, dab, er, pd_bc_after(ctx, g, dB, &bc0));
+    const cg_tune_cfg tc = tune_pd<float>(ab, g, ctx->num_sms, ctx->stream, dab, er, edges, true, pd_bc_after(ctx, g, dB, &bc0));
     const int variant = tc.variant;
     const bool staged = variant >= kPdTmaFirst && variant < kPdRowsFirst, fold = variant >= kPdRowsFirst && edges;
     const int nchunk = std::max(2, o->ncheck + (o->ncheck & 1));

@@ -1,6 +1,7 @@
 """Layouts fixed by the environment are taken without timing the candidates."""
 
 import os
+import re
 import subprocess
 import sys
 from pathlib import Path
@@ -34,3 +35,36 @@ def test_march_layouts(arch, dims, layouts):
     assert any(name in l for l in tuned(script))
     for layout in layouts:
         assert not any(name in l for l in tuned(script, CG_MARCH_LAYOUT=layout)), layout
+
+
+PTD = """
+from chmy_gb300 import Field, _abi
+from chmy_gb300.bcs import Neumann, Periodic, to_cg_bc
+from chmy_gb300.configs import ptdiff_params
+from chmy_gb300.grids import Center, UniformGrid, Vertex
+T, dims = np.float32, (66, 40, 30)
+grid = UniformGrid(origin=(T(-0.5),) * 3, extent=(T(1),) * 3, dims=dims, dtype=T)
+C, C_old, D = (Field(arch, grid, Center(), T) for _ in range(3))
+q = [Field(arch, grid, tuple(Vertex() if e == d else Center() for e in range(3)), T) for d in range(3)]
+D.data.fill_(1.0)
+s = _abi.cg_ptdiff_fields()
+s.C, s.C_old, s.D = C.desc(), C_old.desc(), D.desc()
+s.q = (_abi.cg_field * 3)(*[f.desc() for f in q])
+p = ptdiff_params(grid, dt=1e-3, Dmax=1.0)
+for spec in ({"x": Neumann(), "y": Neumann(), "z": Neumann()}, {"x": Periodic(), "y": Neumann(), "z": Neumann()}, None):
+    print("--- tune", spec, file=sys.stderr, flush=True)
+    bc = to_cg_bc(3, spec) if spec else None
+    arch.call("cg_ptdiff_run", ctypes.byref(grid.desc()), ctypes.byref(s), ctypes.byref(p), ctypes.byref(bc) if bc else None, 1, 8)
+"""
+
+
+def test_ptdiff_layouts_are_timed_with_the_launches_of_the_run(arch):
+    """Rules that the rows layouts fold, rules that they do not (a bc! launch follows every iteration) and
+    no rules are three runs, each timed for itself: with the launch an iteration takes longer."""
+    lines = tuned(PTD)
+    runs, best = " ".join(lines).split("--- tune")[1:], []
+    for log in runs:
+        us = [float(w) for w in re.findall(r"seg \d+: ([\d.]+) us", log)]
+        assert us, "a layout timed under other rules was taken"
+        best.append(min(us))
+    assert best[1] > best[0] + 1.0 and best[1] > best[2] + 1.0, best
