@@ -506,11 +506,12 @@ inline cudaError_t launch_march3d(const Fused3D<T>& f, const SP<T>& s, int n0, i
 // writes them again); the residual outputs are not touched. Results are cached per shape,
 // precision and layout for the process.
 // 2D candidates: variant 0 is march2d_kernel (one iteration per launch, 5 to 7 segment lengths), variants
-// 1 and up march2d_tile_kernel's shapes (when march_tile_ok); the time compared is per iteration.
+// 1 and up march2d_tile_kernel's shapes (when march_tile_ok, and `tiles`: the call takes several iterations
+// without a bc! launch between them); the time compared is per iteration.
 template <class T>
-inline cg_tune_cfg tune_march2d(const Fused2D<T>& f, const SP<T>& s, int n0, int n1, int nsm, cudaStream_t st) {
+inline cg_tune_cfg tune_march2d(const Fused2D<T>& f, const SP<T>& s, int n0, int n1, int nsm, bool tiles, cudaStream_t st) {
     cg_tune_cfg best{0, 0};
-    const bool tile = march_tile_ok(f, n0, n1);
+    const bool tile = tiles && march_tile_ok(f, n0, n1);
     if (cg_tune_forced(&best)) {
         if (best.variant > kTileVariants || !tile) best.variant = 0;
         return best;

@@ -807,7 +807,8 @@ int pp_iterations_t(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* a, co
     if (fold) fab.bc = fba.bc = vf;
     const SP<T> s = scalars<T>(g, p);
     const bool res = cg_present(a->divV) && cg_present(a->r_V[0]);
-    const cg_tune_cfg tc = tune_march2d(fab, s, g->n[0], g->n[1], ctx->num_sms, ctx->stream);
+    const bool tiles = (fold || !bc_V) && niter > 2;
+    const cg_tune_cfg tc = tune_march2d(fab, s, g->n[0], g->n[1], ctx->num_sms, tiles, ctx->stream);
     std::string key = "stokes_pp";
     cg_key_add(key, tc);
     cg_key_add(key, *g);
@@ -823,7 +824,7 @@ int pp_iterations_t(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* a, co
     // between iterations: an odd number of launches takes niter - 1 iterations a -> b -> a ... -> b
     // and the one-iteration kernel the last b -> a, so that a ends with the state after niter
     // iterations and b with the one after niter - 1, as in the one-iteration form
-    const bool tile = tc.variant >= 1 && (fold || !bc_V) && niter > 2;
+    const bool tile = tc.variant >= 1;
     int* differ = nullptr;
     if constexpr (sizeof(T) == 4) {
         if (tile) {

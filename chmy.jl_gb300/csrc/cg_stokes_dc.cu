@@ -569,7 +569,7 @@ int cg_stokes_solve_dc(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f,
     cg_key_add(key, (int)fold);
     for (int d = 0; d < nd; ++d) cg_key_add(key, bc0[d]);  // the kinds that the chunk's launches apply
     // launch layout of the fused kernel, timed on the work buffers (A -> B) before capture
-    const cg_tune_cfg tc = nd == 2 ? tune_march2d(fa, s32, g->n[0], g->n[1], ctx->num_sms, ctx->stream)
+    const cg_tune_cfg tc = nd == 2 ? tune_march2d(fa, s32, g->n[0], g->n[1], ctx->num_sms, fold, ctx->stream)
                                    : tune_march3d(ga, s32, g->n[0], g->n[1], g->n[2], ctx->num_sms, ctx->stream, lga);
     cg_key_add(key, tc);
     const bool staged = nd == 3 && tma.ok && m3_staged(tc.variant);
@@ -577,7 +577,7 @@ int cg_stokes_solve_dc(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f,
     // several iterations per launch (the tuner's variants 1 and up) where bc!(dV) is folded into the
     // reads: an even number of launches A -> B -> A, so that the chunk ends in A. The buffers of the
     // pool agree outside the launch range (both are zero where no iteration writes).
-    const bool tile = nd == 2 && fold && tc.variant >= 1;
+    const bool tile = nd == 2 && tc.variant >= 1;
     const int npass = tile ? (cg_div_up(nchunk, kTileIters[tc.variant - 1]) + 1) & ~1 : 0;
     Measure chk;
     chk.slot = reinterpret_cast<unsigned*>(ctx->d_red + kMeasureAt);

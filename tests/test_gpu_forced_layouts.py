@@ -68,3 +68,22 @@ def test_ptdiff_layouts_are_timed_with_the_launches_of_the_run(arch):
         assert us, "a layout timed under other rules was taken"
         best.append(min(us))
     assert best[1] > best[0] + 1.0 and best[1] > best[2] + 1.0, best
+
+
+PP2D = """
+from test_gpu_stokes import _bc_V, _pp_run
+from chmy_gb300.bcs import Neumann, Periodic, to_cg_bc
+for bcs, niter in ((_bc_V(2), 6), ([to_cg_bc(2, {"x": Periodic(), "y": Neumann()}) for _ in range(2)], 6), (_bc_V(2), 2)):
+    print("--- tune", file=sys.stderr, flush=True)
+    _pp_run(arch, np.float32, (150, 131), bcs, niter)
+"""
+
+
+def test_tiles_are_timed_only_where_the_call_can_take_them(arch):
+    """Ping-pong iterations whose rules fold, with periodic sides (a bc! launch between iterations), and two
+    iterations: only the first can take the tile kernel. The others time the one-iteration kernel's segments
+    and run the best of these."""
+    runs = " ".join(tuned(PP2D)).split("--- tune")[1:]
+    assert len(runs) == 3 and re.search(r"variant [123] ", runs[0])
+    for log in runs[1:]:
+        assert not re.search(r"variant [123] ", log) and (log is runs[2] or "variant 0 " in log)
