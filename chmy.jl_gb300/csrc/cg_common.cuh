@@ -78,6 +78,10 @@ void cg_tune_store(const std::string& key, const cg_tune_cfg& cfg);
 // valid shape (x a multiple of 32, x * y from 64 to 1024).
 bool cg_block_forced(dim3* out);
 
+// CG_DIFFUSION_LAYOUT=<rows per segment>:<0|1, dependent launches> in the environment (read on every call):
+// the layout of the 2D explicit diffusion march; the results do not depend on it.
+bool cg_diffusion_forced(cg_tune_cfg* out);
+
 // Programmatic dependent launch. A kernel launched by cg_launch(..., dep = true) may be
 // scheduled while the kernel before it on the stream is still running; it calls cg_dep_wait()
 // before its first global-memory access, which returns once that kernel has completed and its

@@ -110,6 +110,16 @@ bool cg_block_forced(dim3* out) {
     return true;
 }
 
+bool cg_diffusion_forced(cg_tune_cfg* out) {
+    // read on every call, like CG_BLOCK
+    const char* e = std::getenv("CG_DIFFUSION_LAYOUT");
+    if (!e || !e[0]) return false;
+    int seg = 0, dep = 0;
+    if (std::sscanf(e, "%d:%d", &seg, &dep) != 2 || seg < 1 || dep < 0 || dep > 1) return false;
+    *out = cg_tune_cfg{seg, dep};
+    return true;
+}
+
 bool cg_pdl_enabled() {
     static const bool on = [] {
         const char* e = std::getenv("CG_PDL");

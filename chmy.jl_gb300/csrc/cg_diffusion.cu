@@ -350,7 +350,7 @@ dim3 step_block(cg_ctx* ctx, const cg_grid* g, const cg_field* Co, const cg_fiel
     cg_key_add(key, ctx->num_sms);
     if constexpr (ND == 2) {
         cg_tune_cfg c{8, (long)g->n[0] * g->n[1] <= 1700l * ctx->num_sms};
-        if (cg_tune_lookup(key, &c) || !may_time || !cg_autotune_enabled()) return dim3((unsigned)c.seg, (unsigned)c.variant);
+        if (cg_diffusion_forced(&c) || cg_tune_lookup(key, &c) || !may_time || !cg_autotune_enabled()) return dim3((unsigned)c.seg, (unsigned)c.variant);
         EdgeRules<T> er;
         edge_rules<T>(g, nullptr, &er);
         // the segments as dependent launches, then the three best of them as ordinary ones

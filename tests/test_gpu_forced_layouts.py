@@ -87,3 +87,18 @@ def test_tiles_are_timed_only_where_the_call_can_take_them(arch):
     assert len(runs) == 3 and re.search(r"variant [123] ", runs[0])
     for log in runs[1:]:
         assert not re.search(r"variant [123] ", log) and (log is runs[2] or "variant 0 " in log)
+
+
+DIFFUSION = """
+from chmy_gb300 import Field
+from chmy_gb300.grids import Center, UniformGrid
+grid = UniformGrid(origin=(-1.0, -1.0), extent=(2.0, 2.0), dims=(70, 60))
+A, B = (Field(arch, grid, Center()) for _ in range(2))
+arch.call("cg_diffusion_run", ctypes.byref(grid.desc()), ctypes.byref(A.desc()), ctypes.byref(B.desc()), 1.0, 1e-6, None, 4)
+"""
+
+
+def test_diffusion_layouts(arch):
+    assert any("diffusion step tune" in l for l in tuned(DIFFUSION))
+    for layout in ("1:0", "8:1"):
+        assert not tuned(DIFFUSION, CG_DIFFUSION_LAYOUT=layout)
