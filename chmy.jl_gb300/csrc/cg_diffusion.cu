@@ -349,7 +349,11 @@ dim3 step_block(cg_ctx* ctx, const cg_grid* g, const cg_field* Co, const cg_fiel
     cg_key_add(key, Co->stride);
     cg_key_add(key, ctx->num_sms);
     if constexpr (ND == 2) {
-        cg_tune_cfg c{8, (long)g->n[0] * g->n[1] <= 1700l * ctx->num_sms};
+        // untimed: segments that leave an SM about 20 warps, of 1 to 8 rows. A row is a chain of 0.6 us in FP64: a
+        // step at 126^2 takes 4.2 us with one row and 8.3 with 8; at 1022^2 31.0 and 30.8 (FP32 4.1 and 6.2, 12.3
+        // and 7.1), at 2040 x 1500 82.0 and 73.8.
+        const long warps = (long)cg_div_up(g->n[0] + 2, 31) * (g->n[1] + 2);
+        cg_tune_cfg c{std::min(std::max(cg_div_up(warps, 20l * ctx->num_sms), 1), 8), (long)g->n[0] * g->n[1] <= 1700l * ctx->num_sms};
         if (cg_diffusion_forced(&c) || cg_tune_lookup(key, &c) || !may_time || !cg_autotune_enabled()) return dim3((unsigned)c.seg, (unsigned)c.variant);
         EdgeRules<T> er;
         edge_rules<T>(g, nullptr, &er);
