@@ -259,6 +259,7 @@ inline std::vector<float> time_candidates(int n, F&& launch, cudaStream_t st, st
     double host = 8.;
     bool loaded = false;
     auto delay = [&](double us_) { tune_delay_kernel<0><<<1, 1, 0, st>>>((unsigned)(1e3 * std::min(us_, 2e3))); };
+    if (good && launch(0) != cudaSuccess) cudaGetLastError();  // untimed: most candidates share its code
     if (good) delay(host * n);
     for (int c = 0; good && c < n; ++c)
         for (int again = 0; again < 2; ++again) {

@@ -334,13 +334,14 @@ cudaError_t march_launch(const cg_grid* g, const cg_field* Co, const cg_field* C
 // The layout of the step's launch for this grid, timed on C_out = step(C_in) (the first step of a run
 // writes the same points again), or its cached choice when `may_time` is false: in 2D the march's
 // segment length in x (short segments balance the SMs, long ones recompute fewer y fluxes) and in y
-// whether a run uses dependent launches, in 3D the tile kernel's block; 1D keeps 256 threads.
+// whether a run uses dependent launches (chain: its steps follow each other; with a bc! launch between them,
+// or one step, only ordinary launches are timed), in 3D the tile kernel's block; 1D keeps 256 threads.
 // Dependent launches hide the launch latency (126^2 4.2 -> 2.6 us per step), but where a grid is about one
 // wave the next launch's blocks gather on the SMs that end early (1024^2, segments of 12 rows: 28.7 ->
 // 45.3 us), so both are timed.
 template <class T, int ND>
 dim3 step_block(cg_ctx* ctx, const cg_grid* g, const cg_field* Co, const cg_field* Ci, double chi, double dt,
-                bool may_time) {
+                bool may_time, bool chain) {
     if (ND == 1) return block_for<ND>();
     std::string key = ND == 2 ? "diffusion_segment" : "diffusion_block";
     cg_key_add(key, *g);
@@ -349,18 +350,28 @@ dim3 step_block(cg_ctx* ctx, const cg_grid* g, const cg_field* Co, const cg_fiel
     cg_key_add(key, Co->stride);
     cg_key_add(key, ctx->num_sms);
     if constexpr (ND == 2) {
-        // untimed: segments that leave an SM about 20 warps, of 1 to 8 rows. A row is a chain of 0.6 us in FP64: a
+        // Untimed: segments that leave an SM about 20 warps, of 1 to 8 rows. A row is a chain of 0.6 us in FP64: a
         // step at 126^2 takes 4.2 us with one row and 8.3 with 8; at 1022^2 31.0 and 30.8 (FP32 4.1 and 6.2, 12.3
         // and 7.1), at 2040 x 1500 82.0 and 73.8.
+        // Up to 32 (FP64) and 128 (FP32) warps per SM a step is shorter than about 5 us, which launches on a
+        // stream cannot tell apart (each takes 4); there the rule with at most 3 rows stands, timed in graphs of 40
+        // steps: FP64 130 x 128 2.5 us with one row, 3.2 with two; 380 x 370 6.2 and 5.4; FP32 254^2 2.1, 2.4;
+        // 513 x 400 2.9, 3.2 and 2.8 with three; 760 x 720 5.6, 4.4, 3.8 and 4.5 with six.
         const long warps = (long)cg_div_up(g->n[0] + 2, 31) * (g->n[1] + 2);
-        cg_tune_cfg c{std::min(std::max(cg_div_up(warps, 20l * ctx->num_sms), 1), 8), (long)g->n[0] * g->n[1] <= 1700l * ctx->num_sms};
-        if (cg_diffusion_forced(&c) || cg_tune_lookup(key, &c) || !may_time || !cg_autotune_enabled()) return dim3((unsigned)c.seg, (unsigned)c.variant);
+        const bool small = warps <= (sizeof(T) == 8 ? 32l : 128l) * ctx->num_sms;
+        cg_tune_cfg c{std::min(std::max(cg_div_up(warps, 20l * ctx->num_sms), 1), small ? 3 : 8),
+                      chain && (small || (long)g->n[0] * g->n[1] <= 1700l * ctx->num_sms)};
+        const std::string other = key + (chain ? '0' : '1');
+        key += chain ? '1' : '0';
+        if (cg_diffusion_forced(&c) || cg_tune_lookup(key, &c) || (!may_time && cg_tune_lookup(other, &c)) || !may_time ||
+            small || !cg_autotune_enabled())
+            return dim3((unsigned)c.seg, (unsigned)c.variant);
         EdgeRules<T> er;
         edge_rules<T>(g, nullptr, &er);
-        // the segments as dependent launches, then the three best of them as ordinary ones
+        // the segments, for a chain of steps as dependent launches and then the three best as ordinary ones
         std::vector<cg_tune_cfg> cand;
         for (int seg : {1, 2, 3, 4, 6, 8, 12, 16, 24})
-            if (seg == 1 || seg <= g->n[1] + 2) cand.push_back(cg_tune_cfg{seg, 1});
+            if (seg == 1 || seg <= g->n[1] + 2) cand.push_back(cg_tune_cfg{seg, chain});
         auto time = [&](const std::vector<cg_tune_cfg>& v) {
             return cgk::time_candidates(
                 (int)v.size(), [&](int q) { return march_launch<T>(g, Co, Ci, chi, dt, v[q].seg, er, ctx->stream, v[q].variant != 0); },
@@ -369,7 +380,7 @@ dim3 step_block(cg_ctx* ctx, const cg_grid* g, const cg_field* Co, const cg_fiel
         std::vector<float> us = time(cand);
         std::vector<cg_tune_cfg> plain;
         std::vector<float> left = us;
-        for (int k = 0; k < 3 && cgk::fastest(left) >= 0; ++k) {
+        for (int k = 0; chain && k < 3 && cgk::fastest(left) >= 0; ++k) {
             const int q = cgk::fastest(left);
             plain.push_back(cg_tune_cfg{cand[q].seg, 0});
             left[q] = -1.f;
@@ -398,7 +409,7 @@ dim3 step_block(cg_ctx* ctx, const cg_grid* g, const cg_field* Co, const cg_fiel
 
 template <class T, int ND>
 int step_t(cg_ctx* ctx, const cg_grid* g, const cg_field* Co, const cg_field* Ci, double chi, double dt) {
-    const dim3 block = step_block<T, ND>(ctx, g, Co, Ci, chi, dt, false);
+    const dim3 block = step_block<T, ND>(ctx, g, Co, Ci, chi, dt, false, false);
     cudaError_t e;
     if constexpr (ND == 2) {
         EdgeRules<T> er;
@@ -553,11 +564,13 @@ extern "C" int cg_diffusion_run(cg_ctx* ctx, const cg_grid* grid, const cg_field
     cg_key_add(key, bc ? *bc : none);
     // the step's launch layout, timed on B = step(A) (once per shape) before the graph is captured
     dim3 blk(256, 1);
+    EdgeRules<double> any;
+    const bool chain = nsteps > 1 && grid->ndim == 2 && edge_rules(grid, bc, &any);
     if (grid->ndim > 1) blk = A->dtype == CG_F64
-                                  ? (grid->ndim == 2 ? step_block<double, 2>(ctx, grid, B, A, chi, dt, true)
-                                                     : step_block<double, 3>(ctx, grid, B, A, chi, dt, true))
-                                  : (grid->ndim == 2 ? step_block<float, 2>(ctx, grid, B, A, chi, dt, true)
-                                                     : step_block<float, 3>(ctx, grid, B, A, chi, dt, true));
+                                  ? (grid->ndim == 2 ? step_block<double, 2>(ctx, grid, B, A, chi, dt, true, chain)
+                                                     : step_block<double, 3>(ctx, grid, B, A, chi, dt, true, chain))
+                                  : (grid->ndim == 2 ? step_block<float, 2>(ctx, grid, B, A, chi, dt, true, chain)
+                                                     : step_block<float, 3>(ctx, grid, B, A, chi, dt, true, chain));
     cg_key_add(key, blk);
     return cg_graph_run(ctx, key, [&](cudaStream_t st) {
         if (grid->ndim == 2) {

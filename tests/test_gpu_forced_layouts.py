@@ -92,7 +92,7 @@ def test_tiles_are_timed_only_where_the_call_can_take_them(arch):
 DIFFUSION = """
 from chmy_gb300 import Field
 from chmy_gb300.grids import Center, UniformGrid
-grid = UniformGrid(origin=(-1.0, -1.0), extent=(2.0, 2.0), dims=(70, 60))
+grid = UniformGrid(origin=(-1.0, -1.0), extent=(2.0, 2.0), dims=(700, 600))
 A, B = (Field(arch, grid, Center()) for _ in range(2))
 arch.call("cg_diffusion_run", ctypes.byref(grid.desc()), ctypes.byref(A.desc()), ctypes.byref(B.desc()), 1.0, 1e-6, None, 4)
 """
@@ -102,3 +102,24 @@ def test_diffusion_layouts(arch):
     assert any("diffusion step tune" in l for l in tuned(DIFFUSION))
     for layout in ("1:0", "8:1"):
         assert not tuned(DIFFUSION, CG_DIFFUSION_LAYOUT=layout)
+
+
+DIFFUSION_BC = """
+from chmy_gb300 import Field
+from chmy_gb300.bcs import Neumann, Periodic, to_cg_bc
+from chmy_gb300.grids import Center, UniformGrid
+grid = UniformGrid(origin=(-1.0, -1.0), extent=(2.0, 2.0), dims=(700, 610))
+A, B = (Field(arch, grid, Center()) for _ in range(2))
+for spec, n in ((Neumann(), 8), ({"x": Periodic(), "y": Neumann()}, 8), (Neumann(), 1)):
+    print("--- tune", file=sys.stderr, flush=True)
+    arch.call("cg_diffusion_run", ctypes.byref(grid.desc()), ctypes.byref(A.desc()), ctypes.byref(B.desc()), 1.0, 1e-6,
+              ctypes.byref(to_cg_bc(2, spec)), n)
+"""
+
+
+def test_diffusion_steps_apart_are_timed_as_ordinary_launches(arch):
+    """Steps that follow each other are dependent launches; steps with a bc! launch between them (periodic
+    sides) and a single step are not, and take a layout timed without."""
+    runs = " ".join(tuned(DIFFUSION_BC)).split("--- tune")[1:]
+    assert len(runs) == 3 and "dependent" in runs[0]
+    assert "seg" in runs[1] and "dependent" not in runs[1] and "dependent" not in runs[2]
