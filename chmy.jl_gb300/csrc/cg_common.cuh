@@ -366,30 +366,34 @@ __device__ __forceinline__ T fn_eval(const FnDev<T>& f, int nd, const T* x) {
 }
 
 // The thread's point of the launch range [0, e0] x [0, e1] (x [0, gridDim.z)) in a per-point kernel;
-// false: none. Blocks of one row of threads take the points of a plane in order, without a row's ragged
-// end: a warp costs the FP64 pipe the same for one point as for 32, and an x extent of 97 leaves a quarter
-// of the lanes of row-wise blocks idle. Measured, row-wise -> in order: FP64 update_stress! at 95 x 80 x 112
-// 110 -> 84 us, update_velocity! 68 -> 53; PT diffusion at 191 x 160 x 128 update_q! 81 -> 70 us, update_C!
-// 84 -> 73. Kernels bound by memory gain nothing, so both kinds are timed.
-template <int ND>
+// false: none. FLAT (in_order, blocks of one row of threads): a block takes the points of a plane in order,
+// without a row's ragged end: a warp costs the FP64 pipe the same for one point as for 32, and an x extent of
+// 97 leaves a quarter of the lanes of row-wise blocks idle. Measured, row-wise -> in order: FP64
+// update_stress! at 95 x 80 x 112 110 -> 84 us, update_velocity! 68 -> 53; PT diffusion at 191 x 160 x 128
+// update_q! 81 -> 70 us, update_C! 84 -> 73. Kernels bound by memory gain less, so both kinds are timed.
+// FLAT is a template parameter: a branch on the block's shape in one kernel cost the FP32 kernels, which
+// memory bounds, up to a third (update_velocity! at 160 x 150 x 140 80 -> 105 us).
+template <int ND, bool FLAT>
 __device__ __forceinline__ bool launch_point(int e0, int e1, int& i, int& j, int& k) {
     i = blockIdx.x * blockDim.x + threadIdx.x;
-    j = 0;
+    j = ND > 1 && !FLAT ? blockIdx.y * blockDim.y + threadIdx.y : 0;
     k = ND > 2 ? blockIdx.z : 0;
-    if (ND > 1 && blockDim.y == 1) {
+    if (ND > 1 && FLAT) {
         const unsigned w = (unsigned)e0 + 1u;
         j = (int)((unsigned)i / w);
         i -= j * (int)w;
-    } else if (ND > 1) {
-        j = blockIdx.y * blockDim.y + threadIdx.y;
     }
     return i <= e0 && j <= e1;
+}
+template <int ND>
+inline bool in_order(dim3 block) {
+    return ND > 1 && block.y == 1;
 }
 // The grid of such a kernel over [0, n+1]^ND.
 template <int ND>
 inline dim3 point_grid(const int* n, dim3 block) {
     const unsigned w = n[0] + 2, h = ND > 1 ? n[1] + 2 : 1, z = ND > 2 ? n[2] + 2 : 1;
-    if (ND > 1 && block.y == 1) return dim3((unsigned)(((size_t)w * h + block.x - 1) / block.x), 1, z);
+    if (in_order<ND>(block)) return dim3((unsigned)(((size_t)w * h + block.x - 1) / block.x), 1, z);
     return dim3((w + block.x - 1) / block.x, (h + block.y - 1) / block.y, z);
 }
 

@@ -44,10 +44,10 @@ inline dim3 block_for() {
 }
 
 // q_d += (-(lerp(D -> face_d) * ∂_d C) - q_d) * omega_q at I in [0, n+1]^N
-template <class T, int ND>
+template <class T, int ND, bool FLAT>
 __global__ void ptdiff_q_kernel(const PV<T> v, int e0, int e1) {
     int i, j, k;
-    if (!cgk::launch_point<ND>(e0, e1, i, j, k)) return;
+    if (!cgk::launch_point<ND, FLAT>(e0, e1, i, j, k)) return;
     const T c = v.C(i, j, k), dc = v.D(i, j, k);
 #pragma unroll
     for (int d = 0; d < ND; ++d) {
@@ -75,7 +75,7 @@ struct PdCoef {
 template <class T, int ND>
 __global__ void ptdiff_coef_kernel(const PV<T> v, const PdCoef<T> c, int e0, int e1) {
     int i, j, k;
-    if (!cgk::launch_point<ND>(e0, e1, i, j, k)) return;
+    if (!cgk::launch_point<ND, true>(e0, e1, i, j, k)) return;
     const T dc = v.D(i, j, k);
 #pragma unroll
     for (int d = 0; d < ND; ++d) {
@@ -84,10 +84,10 @@ __global__ void ptdiff_coef_kernel(const PV<T> v, const PdCoef<T> c, int e0, int
     }
 }
 
-template <class T, int ND>
+template <class T, int ND, bool FLAT>
 __global__ void ptdiff_qk_kernel(const PV<T> v, const PdCoef<T> c, int e0, int e1) {
     int i, j, k;
-    if (!cgk::launch_point<ND>(e0, e1, i, j, k)) return;
+    if (!cgk::launch_point<ND, FLAT>(e0, e1, i, j, k)) return;
     const T cc = v.C(i, j, k);
 #pragma unroll
     for (int d = 0; d < ND; ++d) {
@@ -98,10 +98,10 @@ __global__ void ptdiff_qk_kernel(const PV<T> v, const PdCoef<T> c, int e0, int e
 }
 
 // R = -(C - C_old)/dt - divg(q); C += R dtau_C at I in [0, n+1]^N
-template <class T, int ND>
+template <class T, int ND, bool FLAT>
 __global__ void ptdiff_C_kernel(const PV<T> v, int e0, int e1) {
     int i, j, k;
-    if (!cgk::launch_point<ND>(e0, e1, i, j, k)) return;
+    if (!cgk::launch_point<ND, FLAT>(e0, e1, i, j, k)) return;
     T dv = (v.q[0](i + 1, j, k) - v.q[0](i, j, k)) * v.idx[0];
     if (ND > 1) dv = dv + (v.q[1](i, j + 1, k) - v.q[1](i, j, k)) * v.idx[1];
     if (ND > 2) dv = dv + (v.q[2](i, j, k + 1) - v.q[2](i, j, k)) * v.idx[2];
@@ -179,16 +179,28 @@ int setup_coef(cg_ctx* ctx, const cg_grid* g, const cg_ptdiff_fields* f, const c
     return CG_OK;
 }
 
-template <class T, int ND>
-void enqueue_q(const cg_grid* g, const PV<T>& v, const LoopCoef* lc, dim3 b, cudaStream_t st) {
+template <class T, int ND, bool FLAT>
+void enqueue_q_by(const cg_grid* g, const PV<T>& v, const LoopCoef* lc, dim3 b, cudaStream_t st) {
     const int e0 = g->n[0] + 1, e1 = ND > 1 ? g->n[1] + 1 : 0;
     if constexpr (sizeof(T) == 8) {
         if (lc && lc->base) {
-            ptdiff_qk_kernel<T, ND><<<range_grid<ND>(g, b), b, 0, st>>>(v, coef_views<T>(*lc, ND), e0, e1);
+            ptdiff_qk_kernel<T, ND, FLAT><<<range_grid<ND>(g, b), b, 0, st>>>(v, coef_views<T>(*lc, ND), e0, e1);
             return;
         }
     }
-    ptdiff_q_kernel<T, ND><<<range_grid<ND>(g, b), b, 0, st>>>(v, e0, e1);
+    ptdiff_q_kernel<T, ND, FLAT><<<range_grid<ND>(g, b), b, 0, st>>>(v, e0, e1);
+}
+
+template <class T, int ND>
+void enqueue_q(const cg_grid* g, const PV<T>& v, const LoopCoef* lc, dim3 b, cudaStream_t st) {
+    cgk::in_order<ND>(b) ? enqueue_q_by<T, ND, true>(g, v, lc, b, st) : enqueue_q_by<T, ND, false>(g, v, lc, b, st);
+}
+
+template <class T, int ND>
+void enqueue_C(const cg_grid* g, const PV<T>& v, dim3 b, cudaStream_t st) {
+    const int e0 = g->n[0] + 1, e1 = ND > 1 ? g->n[1] + 1 : 0;
+    if (cgk::in_order<ND>(b)) ptdiff_C_kernel<T, ND, true><<<range_grid<ND>(g, b), b, 0, st>>>(v, e0, e1);
+    else ptdiff_C_kernel<T, ND, false><<<range_grid<ND>(g, b), b, 0, st>>>(v, e0, e1);
 }
 
 template <class T, int ND>
@@ -202,8 +214,7 @@ int launch_q(cg_ctx* ctx, const cg_grid* g, const cg_ptdiff_fields* f, const cg_
 template <class T, int ND>
 int launch_C(cg_ctx* ctx, const cg_grid* g, const cg_ptdiff_fields* f, const cg_ptdiff_params* p,
              dim3 b = block_for<ND>()) {
-    ptdiff_C_kernel<T, ND><<<range_grid<ND>(g, b), b, 0, ctx->stream>>>(make_pv<T>(g, f, p), g->n[0] + 1,
-                                                                         ND > 1 ? g->n[1] + 1 : 0);
+    enqueue_C<T, ND>(g, make_pv<T>(g, f, p), b, ctx->stream);
     CG_CHECK_LAUNCH(ctx);
     return CG_OK;
 }
@@ -263,7 +274,6 @@ int ptdiff_blocks(cg_ctx* ctx, const cg_grid* g, const cg_ptdiff_fields* f, cons
         upd[a]->data = tmp + off[a];
     }
     const PV<T> v = make_pv<T>(g, &c, p);
-    const int e0 = g->n[0] + 1, e1 = ND > 1 ? g->n[1] + 1 : 0;
     *bq = cgk::tune_block("ptdiff update_q", kq,
                           [&](dim3 b) {
                               enqueue_q<T, ND>(g, v, lc, b, ctx->stream);
@@ -272,7 +282,7 @@ int ptdiff_blocks(cg_ctx* ctx, const cg_grid* g, const cg_ptdiff_fields* f, cons
                           ctx->stream, true);
     *bc = cgk::tune_block("ptdiff update_C", kc,
                           [&](dim3 b) {
-                              ptdiff_C_kernel<T, ND><<<range_grid<ND>(g, b), b, 0, ctx->stream>>>(v, e0, e1);
+                              enqueue_C<T, ND>(g, v, b, ctx->stream);
                               return cudaGetLastError();
                           },
                           ctx->stream, true);

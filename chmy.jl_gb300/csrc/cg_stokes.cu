@@ -178,7 +178,7 @@ FieldMaskW<T> mask_views(const cg_mask* m) {
 
 // update_stress! over [0, n+1]^N with operand reader m, by the loop's kernel where lc has arrays; dep:
 // a dependent launch.
-template <class T, int ND, class M>
+template <class T, int ND, bool FLAT, class M>
 void stress_launch(const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p, bool res, const LoopCoef* lc,
                    const M& m, dim3 block, cudaStream_t st, bool dep) {
     const SV<T> v = views<T>(f, ND);
@@ -187,18 +187,18 @@ void stress_launch(const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_
     if constexpr (sizeof(T) == 8) {
         if (lc && lc->base) {
             const PtCoef<T> c = loop_coef<T, ND>(g, p, v, *lc);
-            if (res) cg_launch(stress_loop_kernel<T, ND, true, M>, grid, block, 0, st, dep, v, c, e0, e1, m);
-            else cg_launch(stress_loop_kernel<T, ND, false, M>, grid, block, 0, st, dep, v, c, e0, e1, m);
+            if (res) cg_launch(stress_loop_kernel<T, ND, true, M, FLAT>, grid, block, 0, st, dep, v, c, e0, e1, m);
+            else cg_launch(stress_loop_kernel<T, ND, false, M, FLAT>, grid, block, 0, st, dep, v, c, e0, e1, m);
             return;
         }
     }
     const SP<T> s = scalars<T>(g, p);
     const ScalarDiv<T> sd = scalar_divs(s);
-    if (res) cg_launch(stress_kernel<T, ND, true, M>, grid, block, 0, st, dep, v, s, sd, e0, e1, m);
-    else cg_launch(stress_kernel<T, ND, false, M>, grid, block, 0, st, dep, v, s, sd, e0, e1, m);
+    if (res) cg_launch(stress_kernel<T, ND, true, M, FLAT>, grid, block, 0, st, dep, v, s, sd, e0, e1, m);
+    else cg_launch(stress_kernel<T, ND, false, M, FLAT>, grid, block, 0, st, dep, v, s, sd, e0, e1, m);
 }
 
-template <class T, int ND, class M>
+template <class T, int ND, bool FLAT, class M>
 void velocity_launch(const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p, bool res, const LoopCoef* lc,
                      const M& m, dim3 block, cudaStream_t st, bool dep) {
     const SV<T> v = views<T>(f, ND);
@@ -208,15 +208,15 @@ void velocity_launch(const cg_grid* g, const cg_stokes_fields* f, const cg_stoke
     if constexpr (sizeof(T) == 8) {
         if (lc && lc->base) {
             const PtCoef<T> c = loop_coef<T, ND>(g, p, v, *lc);
-            if (res) cg_launch(velocity_loop_kernel<T, ND, true, M>, grid, block, 0, st, dep, v, c, bf, e0, e1, m);
-            else cg_launch(velocity_loop_kernel<T, ND, false, M>, grid, block, 0, st, dep, v, c, bf, e0, e1, m);
+            if (res) cg_launch(velocity_loop_kernel<T, ND, true, M, FLAT>, grid, block, 0, st, dep, v, c, bf, e0, e1, m);
+            else cg_launch(velocity_loop_kernel<T, ND, false, M, FLAT>, grid, block, 0, st, dep, v, c, bf, e0, e1, m);
             return;
         }
     }
     const SP<T> s = scalars<T>(g, p);
     const ScalarDiv<T> sd = scalar_divs(s);
-    if (res) cg_launch(velocity_kernel<T, ND, true, M>, grid, block, 0, st, dep, v, s, sd, bf, e0, e1, m);
-    else cg_launch(velocity_kernel<T, ND, false, M>, grid, block, 0, st, dep, v, s, sd, bf, e0, e1, m);
+    if (res) cg_launch(velocity_kernel<T, ND, true, M, FLAT>, grid, block, 0, st, dep, v, s, sd, bf, e0, e1, m);
+    else cg_launch(velocity_kernel<T, ND, false, M, FLAT>, grid, block, 0, st, dep, v, s, sd, bf, e0, e1, m);
 }
 
 // update_stress! over [0, n+1]^N; with `mask`, every strain-rate derivative is the masked
@@ -224,10 +224,9 @@ void velocity_launch(const cg_grid* g, const cg_stokes_fields* f, const cg_stoke
 template <class T, int ND>
 cudaError_t stress_any(const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p, bool res,
                        const LoopCoef* lc, const cg_mask* mask, dim3 block, cudaStream_t st, bool dep = false) {
-    if (mask)
-        stress_launch<T, ND>(g, f, p, res, lc, mask_views<T>(mask), block, st, dep);
-    else
-        stress_launch<T, ND>(g, f, p, res, lc, NoMask<T>{}, block, st, dep);
+    auto go = [&](auto flat, const auto& m) { stress_launch<T, ND, decltype(flat)::value>(g, f, p, res, lc, m, block, st, dep); };
+    auto with = [&](auto flat) { mask ? go(flat, mask_views<T>(mask)) : go(flat, NoMask<T>{}); };
+    in_order<ND>(block) ? with(std::true_type{}) : with(std::false_type{});
     return cudaGetLastError();
 }
 
@@ -236,10 +235,9 @@ cudaError_t stress_any(const cg_grid* g, const cg_stokes_fields* f, const cg_sto
 template <class T, int ND>
 cudaError_t velocity_any(const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p, bool res,
                          const LoopCoef* lc, const cg_mask* mask, dim3 block, cudaStream_t st, bool dep = false) {
-    if (mask)
-        velocity_launch<T, ND>(g, f, p, res, lc, mask_views<T>(mask), block, st, dep);
-    else
-        velocity_launch<T, ND>(g, f, p, res, lc, NoMask<T>{}, block, st, dep);
+    auto go = [&](auto flat, const auto& m) { velocity_launch<T, ND, decltype(flat)::value>(g, f, p, res, lc, m, block, st, dep); };
+    auto with = [&](auto flat) { mask ? go(flat, mask_views<T>(mask)) : go(flat, NoMask<T>{}); };
+    in_order<ND>(block) ? with(std::true_type{}) : with(std::false_type{});
     return cudaGetLastError();
 }
 

@@ -239,23 +239,23 @@ __device__ __forceinline__ void stress_point(const SV<T>& v, const SP<T>& s, con
     }
 }
 
-template <class T, int ND, bool WRITE_RES, class M>
+template <class T, int ND, bool WRITE_RES, class M, bool FLAT>
 __global__ void stress_kernel(const SV<T> v, const SP<T> s, const ScalarDiv<T> sd, int e0, int e1, const M m) {
     cg_dep_wait();
     cg_dep_release();
     int i, j, k;
-    if (!launch_point<ND>(e0, e1, i, j, k)) return;
+    if (!launch_point<ND, FLAT>(e0, e1, i, j, k)) return;
     stress_point<T, ND, WRITE_RES>(v, s, sd, i, j, k, m);
 }
 
 // update_velocity! at one point. M reads the operands of the pressure and stress derivatives
 // (P and τ_dd at location bits 0, τ_xy 3, τ_xz 5, τ_yz 6).
-template <class T, int ND, bool WRITE_RES, class M>
+template <class T, int ND, bool WRITE_RES, class M, bool FLAT>
 __global__ void velocity_kernel(const SV<T> v, const SP<T> s, const ScalarDiv<T> sd, const BodyFn<T> bf, int e0, int e1, const M m) {
     cg_dep_wait();
     cg_dep_release();
     int i, j, k;
-    if (!launch_point<ND>(e0, e1, i, j, k)) return;
+    if (!launch_point<ND, FLAT>(e0, e1, i, j, k)) return;
     const DF<T>& P = v.P;
     // tensor components: 2D xx=0 yy=1 xy=2; 3D xx=0 yy=1 zz=2 xy=3 xz=4 yz=5
     const int XY = ND == 2 ? 2 : 3;
@@ -332,11 +332,11 @@ struct PtCoef {
     T third, idx[3], idx2[3];
 };
 
-// The viscosity terms over [0, n+1]^N. cP carries a factor 1/2 for the doubled divergence.
+// The viscosity terms over [0, n+1]^N, by blocks of one row. cP carries a factor 1/2 for the doubled divergence.
 template <class T, int ND>
 __global__ void coef_kernel(const SV<T> v, const SP<T> s, const PtCoef<T> c, int e0, int e1) {
     int i, j, k;
-    if (!launch_point<ND>(e0, e1, i, j, k)) return;
+    if (!launch_point<ND, true>(e0, e1, i, j, k)) return;
     const T ie = v.inv_eta(i, j, k);
     const T eve = T(1) / (ie + s.inv_Gdt);
     c.cP(i, j, k) = T(0.5) * (eve * s.dtau_Pr);
@@ -385,23 +385,23 @@ __device__ __forceinline__ void stress_loop_point(const SV<T>& v, const PtCoef<T
     }
 }
 
-template <class T, int ND, bool WRITE_RES, class M>
+template <class T, int ND, bool WRITE_RES, class M, bool FLAT>
 __global__ void stress_loop_kernel(const SV<T> v, const PtCoef<T> c, int e0, int e1, const M m) {
     cg_dep_wait();
     cg_dep_release();
     int i, j, k;
-    if (!launch_point<ND>(e0, e1, i, j, k)) return;
+    if (!launch_point<ND, FLAT>(e0, e1, i, j, k)) return;
     stress_loop_point<T, ND, WRITE_RES>(v, c, i, j, k, m);
 }
 
 // update_velocity! of a PT loop at one point. The differences of tau_dd and of P are formed
 // separately (each is small against its operands) and share one product by idx.
-template <class T, int ND, bool WRITE_RES, class M>
+template <class T, int ND, bool WRITE_RES, class M, bool FLAT>
 __global__ void velocity_loop_kernel(const SV<T> v, const PtCoef<T> c, const BodyFn<T> bf, int e0, int e1, const M m) {
     cg_dep_wait();
     cg_dep_release();
     int i, j, k;
-    if (!launch_point<ND>(e0, e1, i, j, k)) return;
+    if (!launch_point<ND, FLAT>(e0, e1, i, j, k)) return;
     constexpr int XY = ND == 2 ? 2 : 3, XZ = 4, YZ = 5;
     const int LXY = 3, LXZ = 5, LYZ = 6;  // location bits of the shear components
     const T p = m(0, v.P, i, j, k);
