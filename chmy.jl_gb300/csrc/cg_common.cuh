@@ -385,15 +385,17 @@ __device__ __forceinline__ bool launch_point(int e0, int e1, int& i, int& j, int
     }
     return i <= e0 && j <= e1;
 }
+// Whether blocks of this shape take the points in order; a plane whose points an int cannot count is taken
+// row by row.
 template <int ND>
-inline bool in_order(dim3 block) {
-    return ND > 1 && block.y == 1;
+inline bool in_order(const int* n, dim3 block) {
+    return ND > 1 && block.y == 1 && ((long)n[0] + 2) * ((long)n[1] + 2) <= 2147483647l - 1024;
 }
 // The grid of such a kernel over [0, n+1]^ND.
 template <int ND>
 inline dim3 point_grid(const int* n, dim3 block) {
     const unsigned w = n[0] + 2, h = ND > 1 ? n[1] + 2 : 1, z = ND > 2 ? n[2] + 2 : 1;
-    if (in_order<ND>(block)) return dim3((unsigned)(((size_t)w * h + block.x - 1) / block.x), 1, z);
+    if (in_order<ND>(n, block)) return dim3((unsigned)(((size_t)w * h + block.x - 1) / block.x), 1, z);
     return dim3((w + block.x - 1) / block.x, (h + block.y - 1) / block.y, z);
 }
 

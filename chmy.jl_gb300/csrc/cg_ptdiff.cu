@@ -72,10 +72,10 @@ struct PdCoef {
     DF<T> k[3];
 };
 
-template <class T, int ND>
+template <class T, int ND, bool FLAT>
 __global__ void ptdiff_coef_kernel(const PV<T> v, const PdCoef<T> c, int e0, int e1) {
     int i, j, k;
-    if (!cgk::launch_point<ND, true>(e0, e1, i, j, k)) return;
+    if (!cgk::launch_point<ND, FLAT>(e0, e1, i, j, k)) return;
     const T dc = v.D(i, j, k);
 #pragma unroll
     for (int d = 0; d < ND; ++d) {
@@ -172,9 +172,12 @@ int setup_coef(cg_ctx* ctx, const cg_grid* g, const cg_ptdiff_fields* f, const c
         return CG_OK;
     }
     *lc = LoopCoef{base, ND > 1 ? e0 : 0, ND > 2 ? e0 * e1 : 0, e0 * e1 * e2};
-    const dim3 b(256);
-    ptdiff_coef_kernel<T, ND><<<range_grid<ND>(g, b), b, 0, ctx->stream>>>(make_pv<T>(g, f, p), coef_views<T>(*lc, ND),
-                                                                           g->n[0] + 1, ND > 1 ? g->n[1] + 1 : 0);
+    const PV<T> v = make_pv<T>(g, f, p);
+    const PdCoef<T> c = coef_views<T>(*lc, ND);
+    const int l0 = g->n[0] + 1, l1 = ND > 1 ? g->n[1] + 1 : 0;
+    const dim3 flat(256), rows = block_for<ND>();
+    if (cgk::in_order<ND>(g->n, flat)) ptdiff_coef_kernel<T, ND, true><<<range_grid<ND>(g, flat), flat, 0, ctx->stream>>>(v, c, l0, l1);
+    else ptdiff_coef_kernel<T, ND, false><<<range_grid<ND>(g, rows), rows, 0, ctx->stream>>>(v, c, l0, l1);
     CG_CHECK_LAUNCH(ctx);
     return CG_OK;
 }
@@ -193,13 +196,13 @@ void enqueue_q_by(const cg_grid* g, const PV<T>& v, const LoopCoef* lc, dim3 b, 
 
 template <class T, int ND>
 void enqueue_q(const cg_grid* g, const PV<T>& v, const LoopCoef* lc, dim3 b, cudaStream_t st) {
-    cgk::in_order<ND>(b) ? enqueue_q_by<T, ND, true>(g, v, lc, b, st) : enqueue_q_by<T, ND, false>(g, v, lc, b, st);
+    cgk::in_order<ND>(g->n, b) ? enqueue_q_by<T, ND, true>(g, v, lc, b, st) : enqueue_q_by<T, ND, false>(g, v, lc, b, st);
 }
 
 template <class T, int ND>
 void enqueue_C(const cg_grid* g, const PV<T>& v, dim3 b, cudaStream_t st) {
     const int e0 = g->n[0] + 1, e1 = ND > 1 ? g->n[1] + 1 : 0;
-    if (cgk::in_order<ND>(b)) ptdiff_C_kernel<T, ND, true><<<range_grid<ND>(g, b), b, 0, st>>>(v, e0, e1);
+    if (cgk::in_order<ND>(g->n, b)) ptdiff_C_kernel<T, ND, true><<<range_grid<ND>(g, b), b, 0, st>>>(v, e0, e1);
     else ptdiff_C_kernel<T, ND, false><<<range_grid<ND>(g, b), b, 0, st>>>(v, e0, e1);
 }
 

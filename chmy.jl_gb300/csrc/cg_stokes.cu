@@ -160,8 +160,12 @@ int setup_coef(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, const c
         v.ieta = c.ieta;
         v.has_ieta = 1;
     }
+    const int l0 = g->n[0] + 1, l1 = g->n[1] + 1;
     const dim3 flat(256);
-    coef_kernel<T, ND><<<range_grid<ND>(g, flat), flat, 0, ctx->stream>>>(v, scalars<T>(g, p), c, g->n[0] + 1, g->n[1] + 1);
+    if (in_order<ND>(g->n, flat))
+        coef_kernel<T, ND, true><<<range_grid<ND>(g, flat), flat, 0, ctx->stream>>>(v, scalars<T>(g, p), c, l0, l1);
+    else
+        coef_kernel<T, ND, false><<<range_grid<ND>(g, block), block, 0, ctx->stream>>>(v, scalars<T>(g, p), c, l0, l1);
     CG_CHECK_LAUNCH(ctx);
     return CG_OK;
 }
@@ -226,7 +230,7 @@ cudaError_t stress_any(const cg_grid* g, const cg_stokes_fields* f, const cg_sto
                        const LoopCoef* lc, const cg_mask* mask, dim3 block, cudaStream_t st, bool dep = false) {
     auto go = [&](auto flat, const auto& m) { stress_launch<T, ND, decltype(flat)::value>(g, f, p, res, lc, m, block, st, dep); };
     auto with = [&](auto flat) { mask ? go(flat, mask_views<T>(mask)) : go(flat, NoMask<T>{}); };
-    in_order<ND>(block) ? with(std::true_type{}) : with(std::false_type{});
+    in_order<ND>(g->n, block) ? with(std::true_type{}) : with(std::false_type{});
     return cudaGetLastError();
 }
 
@@ -237,7 +241,7 @@ cudaError_t velocity_any(const cg_grid* g, const cg_stokes_fields* f, const cg_s
                          const LoopCoef* lc, const cg_mask* mask, dim3 block, cudaStream_t st, bool dep = false) {
     auto go = [&](auto flat, const auto& m) { velocity_launch<T, ND, decltype(flat)::value>(g, f, p, res, lc, m, block, st, dep); };
     auto with = [&](auto flat) { mask ? go(flat, mask_views<T>(mask)) : go(flat, NoMask<T>{}); };
-    in_order<ND>(block) ? with(std::true_type{}) : with(std::false_type{});
+    in_order<ND>(g->n, block) ? with(std::true_type{}) : with(std::false_type{});
     return cudaGetLastError();
 }
 

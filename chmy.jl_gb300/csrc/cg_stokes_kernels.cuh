@@ -332,11 +332,11 @@ struct PtCoef {
     T third, idx[3], idx2[3];
 };
 
-// The viscosity terms over [0, n+1]^N, by blocks of one row. cP carries a factor 1/2 for the doubled divergence.
-template <class T, int ND>
+// The viscosity terms over [0, n+1]^N. cP carries a factor 1/2 for the doubled divergence.
+template <class T, int ND, bool FLAT>
 __global__ void coef_kernel(const SV<T> v, const SP<T> s, const PtCoef<T> c, int e0, int e1) {
     int i, j, k;
-    if (!launch_point<ND, true>(e0, e1, i, j, k)) return;
+    if (!launch_point<ND, FLAT>(e0, e1, i, j, k)) return;
     const T ie = v.inv_eta(i, j, k);
     const T eve = T(1) / (ie + s.inv_Gdt);
     c.cP(i, j, k) = T(0.5) * (eve * s.dtau_Pr);
