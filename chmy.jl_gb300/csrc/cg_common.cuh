@@ -94,6 +94,9 @@ bool cg_pdl_enabled();
 // bc!(V) folded into the velocity reads of the 2D marching kernel (one boundary-condition
 // launch per run of PT iterations); CG_BC_FOLD=0 in the environment launches it every iteration.
 bool cg_bc_fold_enabled();
+// CG_LOOP_COEF=0|1 in the environment (read on every call): FP64 loops never, or always, compute the
+// coefficients that do not change within them once (-1 when unset: by the loop's size and length).
+int cg_loop_coef_forced();
 // The fused single-pass PT-diffusion iteration (3D FP32); CG_PTDIFF_FUSED=0 keeps the
 // two-kernel form.
 bool cg_ptdiff_fused_enabled();

@@ -136,6 +136,12 @@ bool cg_bc_fold_enabled() {
     return on;
 }
 
+int cg_loop_coef_forced() {
+    // read on every call, like CG_BLOCK
+    const char* e = std::getenv("CG_LOOP_COEF");
+    return !e || !e[0] ? -1 : e[0] != '0';
+}
+
 bool cg_ptdiff_fused_enabled() {
     static const bool on = [] {
         const char* e = std::getenv("CG_PTDIFF_FUSED");

@@ -157,13 +157,25 @@ inline bool D_changes(const cg_ptdiff_fields* f) {
     return D == f->C.data || D == f->C_old.data || (cg_present(f->R) && D == f->R.data);
 }
 
-// Fill the coefficients for a loop of `iters` FP64 iterations. From four iterations on they cost less
-// than they save (one pass over D against three face products per iteration); FP32 is bound by
+// Whether a loop of `iters` FP64 iterations is long enough for its coefficients: filling them costs a launch
+// (2 to 3 us on a small grid), and below about 150 cells per SM, where latency bounds an iteration, they save
+// nothing. Measured without and with them, in us: 24^3, 16 iterations 137 and 148; 126^2, 16 105 and 109;
+// 160^2, 8 76.0 and 76.1; 32^3, 16 152 and 154, 24 226 and 225; 40^3, 6 67.9 and 67.8; 300 x 260, 4 41.2 and 40.2;
+// 96^3, 4 230 and 186.
+inline bool coef_pays(const cg_grid* g, int nd, int num_sms, long iters) {
+    const int forced = cg_loop_coef_forced();
+    if (forced >= 0) return forced == 1;
+    long cells = 1;
+    for (int d = 0; d < nd; ++d) cells *= g->n[d];
+    return cells >= 150l * num_sms && iters >= (cells >= 500l * num_sms ? 4 : 16);
+}
+
+// Fill the coefficients for a loop of `iters` FP64 iterations where these pay; FP32 is bound by
 // memory and keeps ptdiff_q_kernel, as does a loop whose arrays find no room and one that changes D.
 template <class T, int ND>
 int setup_coef(cg_ctx* ctx, const cg_grid* g, const cg_ptdiff_fields* f, const cg_ptdiff_params* p, long iters, LoopCoef* lc) {
     *lc = LoopCoef{};
-    if (sizeof(T) != 8 || iters < 4 || D_changes(f)) return CG_OK;
+    if (sizeof(T) != 8 || !coef_pays(g, ND, ctx->num_sms, iters) || D_changes(f)) return CG_OK;
     const long e0 = g->n[0] + 2, e1 = ND > 1 ? g->n[1] + 2 : 1, e2 = ND > 2 ? g->n[2] + 2 : 1;
     int rc = CG_OK;
     char* base = static_cast<char*>(cg_scratch(ctx, 2, (size_t)(ND * e0 * e1 * e2) * sizeof(T), &rc));

@@ -128,14 +128,26 @@ __global__ void inv_kernel(DF<T> dst, DF<T> src, int lo, int e0, int e1, int e2)
     for (int k = e2 < 0 ? 0 : lo; k <= (e2 < 0 ? 0 : e2); ++k) dst(i, j, k) = T(1) / src(i, j, k);
 }
 
-// Set up `lc` for a loop of PT iterations over the field set `f` and fill its arrays. The loop's
-// kernels run for FP64 from two iterations on: for a single one, filling the arrays costs what
-// they save. FP32 loops are bound by HBM (the arrays would add traffic) and keep stress_kernel and
+// Whether a loop of niter FP64 PT iterations is long enough for its coefficients. For a single one, filling
+// the arrays costs what they save; on small grids it is a launch of 2 to 4 us that a few iterations do not
+// repay. Measured without and with them, in us: 2D 64^2 and 126^2, 2 iterations 22.8 and 24.9 to 26.9, 5 49.4 to
+// 51.5 and 47.4 to 51.5; 254^2, 2 33.0 and 33.1, 4 61.7 and 55.2; 3D 24^3, 2 39.2 and 39.1, 3 55.5 and 51.3; 48^3, 2
+// 84 and 72.
+inline bool coef_pays(const cg_grid* g, int nd, int num_sms, int niter) {
+    const int forced = cg_loop_coef_forced();
+    if (forced >= 0) return forced == 1;
+    long cells = 1;
+    for (int d = 0; d < nd; ++d) cells *= g->n[d];
+    return niter >= (cells >= 256l * num_sms ? 2 : nd == 2 ? 5 : 3);
+}
+
+// Set up `lc` for a loop of PT iterations over the field set `f` and fill its arrays, for FP64 where they
+// pay. FP32 loops are bound by HBM (the arrays would add traffic) and keep stress_kernel and
 // velocity_kernel, as does a loop whose arrays find no room.
 template <class T, int ND>
 int setup_coef(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, const cg_stokes_params* p, int niter, LoopCoef* lc) {
     *lc = LoopCoef{};
-    if (sizeof(T) != 8 || niter < 2 || (!cg_present(f->eta) && !cg_present(f->inv_eta))) return CG_OK;
+    if (sizeof(T) != 8 || !coef_pays(g, ND, ctx->num_sms, niter) || (!cg_present(f->eta) && !cg_present(f->inv_eta))) return CG_OK;
     const long e0 = g->n[0] + 4, e1 = g->n[1] + 4, e2 = ND > 2 ? g->n[2] + 4 : 1;
     lc->s1 = e0;
     lc->s2 = ND > 2 ? e0 * e1 : 0;
