@@ -37,8 +37,8 @@ struct cg_ctx {
     void* dc_pool = nullptr;
     size_t dc_pool_bytes = 0;
     // numbered scratch buffers of the time-stepping loops (grown on demand, freed by cg_destroy)
-    // slots: 0 thermal partner, 1 SIA D, 2 PT-diffusion partners, 3 SIA ensemble,
-    // 4 PT-diffusion defect-correction pool, 5 SIA reverse step, 6 SIA reverse sweep over a tape,
+    // slots: 0 thermal partner, 1 the arrays of a SIA run (D, S twice, a second D and H), 2 PT-diffusion
+    // partners and the coefficients of FP64 Stokes and PT-diffusion loops, 3 SIA ensemble, 4 PT-diffusion defect-correction pool, 5 SIA reverse step, 6 SIA reverse sweep over a tape,
     // 7 SIA ensemble reverse sweep, 8 explicit-diffusion reverse sweep, 9 thermal-step adjoint,
     // 10 the wait flag of the TMA-fed kernels, 11 whether a 2D ping-pong pair's static points differ
     static constexpr int kScratchSlots = 12;
@@ -50,9 +50,12 @@ struct cg_ctx {
 // not preserved across growth). Sets *rc on failure and returns NULL.
 void* cg_scratch(cg_ctx* ctx, int slot, size_t bytes, int* rc);
 // Scratch that a call can do without: nullptr, and no error, where it finds no room (`what` names the
-// arrays in the verbose output). CG_SCRATCH_LIMIT=<bytes> in the environment (read on every call) fails
-// every larger scratch request.
-void* cg_scratch_optional(cg_ctx* ctx, int slot, size_t bytes, const char* what);
+// arrays in the verbose output). spare: it must also leave the caller as much free memory as it takes, since
+// a context keeps its scratch. CG_SCRATCH_LIMIT=<bytes> in the environment (read on every call) fails every
+// larger scratch request.
+void* cg_scratch_optional(cg_ctx* ctx, int slot, size_t bytes, const char* what, bool spare = true);
+// Whether a slot that holds `have` bytes may grow to `bytes` for optional arrays with `free` bytes unused.
+inline bool cg_scratch_spares(size_t bytes, size_t have, size_t free) { return bytes <= have || bytes <= (free + have) / 2; }
 // The wait flag of the TMA-fed kernels (scratch slot 10), cleared on the context's stream: a
 // kernel whose bounded wait for staged data ran out sets it. cg_tma_check reads it after a run
 // (synchronising the stream) and reports CG_ERR_TIMEOUT for `what` when it is set.

@@ -276,14 +276,18 @@ void* cg_scratch(cg_ctx* ctx, int slot, size_t bytes, int* rc) {
     return ctx->scratch[slot];
 }
 
-void* cg_scratch_optional(cg_ctx* ctx, int slot, size_t bytes, const char* what) {
-    char err[sizeof(ctx->err)];
-    std::memcpy(err, ctx->err, sizeof(err));
-    int rc = CG_OK;
-    void* p = cg_scratch(ctx, slot, bytes, &rc);
-    if (!rc) return p;
+void* cg_scratch_optional(cg_ctx* ctx, int slot, size_t bytes, const char* what, bool spare) {
+    size_t free = 0, total = 0;
+    if (!spare || bytes <= ctx->scratch_bytes[slot] ||
+        (cudaMemGetInfo(&free, &total) == cudaSuccess && cg_scratch_spares(bytes, ctx->scratch_bytes[slot], free))) {
+        char err[sizeof(ctx->err)];
+        std::memcpy(err, ctx->err, sizeof(err));
+        int rc = CG_OK;
+        void* p = cg_scratch(ctx, slot, bytes, &rc);
+        if (!rc) return p;
+        std::memcpy(ctx->err, err, sizeof(err));  // the call goes on: no error to report
+    }
     cudaGetLastError();
-    std::memcpy(ctx->err, err, sizeof(err));  // the call goes on: no error to report
     if (cg_tune_verbose()) std::fprintf(stderr, "%s: no room for %zu bytes of scratch\n", what, bytes);
     return nullptr;
 }

@@ -177,12 +177,8 @@ int setup_coef(cg_ctx* ctx, const cg_grid* g, const cg_ptdiff_fields* f, const c
     *lc = LoopCoef{};
     if (sizeof(T) != 8 || !coef_pays(g, ND, ctx->num_sms, iters) || D_changes(f)) return CG_OK;
     const long e0 = g->n[0] + 2, e1 = ND > 1 ? g->n[1] + 2 : 1, e2 = ND > 2 ? g->n[2] + 2 : 1;
-    int rc = CG_OK;
-    char* base = static_cast<char*>(cg_scratch(ctx, 2, (size_t)(ND * e0 * e1 * e2) * sizeof(T), &rc));
-    if (rc) {
-        cudaGetLastError();
-        return CG_OK;
-    }
+    char* base = static_cast<char*>(cg_scratch_optional(ctx, 2, (size_t)(ND * e0 * e1 * e2) * sizeof(T), "ptdiff coefficients"));
+    if (!base) return CG_OK;
     *lc = LoopCoef{base, ND > 1 ? e0 : 0, ND > 2 ? e0 * e1 : 0, e0 * e1 * e2};
     const PV<T> v = make_pv<T>(g, f, p);
     const PdCoef<T> c = coef_views<T>(*lc, ND);
@@ -910,10 +906,19 @@ PDM<T> make_pdm(const cg_grid* g, const cg_field& C, const cg_field* q, const cg
     return m;
 }
 
+// Whether every array has C's row and plane strides (a pool layout).
+inline bool one_layout(const cg_ptdiff_fields* f) {
+    bool one = true;
+    for (const cg_field* a : {&f->q[0], &f->q[1]})
+        one = one && a->stride[1] == f->C.stride[1] && a->stride[2] == f->C.stride[2];
+    return one;
+}
+
 // cg_ptdiff_run on the fused kernel (3D): partner buffers for C and q in scratch slot 2, with
 // the caller's layouts and contents (so the points no iteration writes agree), ping-pong
 // between the two sets, and the result copied back after an odd number of iterations. *ran = false: the
-// partner buffers found no room and nothing was done.
+// partner buffers found no room (a pool layout takes what there is, the dense one leaves as much free) and
+// nothing was done.
 template <class T>
 int run_fused3d(cg_ctx* ctx, const cg_grid* g, const cg_ptdiff_fields* f, const cg_ptdiff_params* p, const cg_bc* bc,
                 int nsteps, int npt, std::string key, bool* ran) {
@@ -925,7 +930,7 @@ int run_fused3d(cg_ctx* ctx, const cg_grid* g, const cg_ptdiff_fields* f, const 
         total += (bytes[a] + 255) & ~(size_t)255;
     }
     int rc = CG_OK;
-    char* base = static_cast<char*>(cg_scratch_optional(ctx, 2, total, "ptdiff partner buffers"));
+    char* base = static_cast<char*>(cg_scratch_optional(ctx, 2, total, "ptdiff partner buffers", !one_layout(f)));
     *ran = base != nullptr;
     if (!base) return CG_OK;
     cg_field part[4];
@@ -1000,10 +1005,7 @@ bool fused3d_ok(const cg_grid* g, const cg_ptdiff_fields* f) {
 // 3 120 and 107; of 4 118 and 138; eight steps of 1 453 and 308, of 2 422 and 565, of 3 767 and 827. A pool
 // layout (one pitch and plane height) or a layout fixed by CG_PTD_VARIANT is fused whatever the counts.
 inline bool fused3d_pays(const cg_ptdiff_fields* f, long nsteps, long npt) {
-    bool one = true;
-    for (const cg_field* a : {&f->q[0], &f->q[1]})
-        one = one && a->stride[1] == f->C.stride[1] && a->stride[2] == f->C.stride[2];
-    if (one || pd_variant_forced() >= 0) return true;
+    if (one_layout(f) || pd_variant_forced() >= 0) return true;
     return 8 + nsteps * (10 * npt + 8 * (npt & 1)) < 14 * nsteps * npt;
 }
 

@@ -348,11 +348,8 @@ int run_t(cg_ctx* ctx, const cg_grid* g, const cg_field* H, const cg_field* B, c
     const size_t ab = cgsia::layout_bytes(*H, sizeof(T));
     int rc = CG_OK;
     bool whole = !tape && (cg_sia_step_rows_forced() > 0 || whole_step_fits<T>(ctx, g));
-    char* base = whole ? static_cast<char*>(cg_scratch(ctx, 1, 5 * ab + 256, &rc)) : nullptr;
-    if (rc) {  // no room for the second buffers
-        cudaGetLastError();
-        whole = false;
-    }
+    char* base = whole ? static_cast<char*>(cg_scratch_optional(ctx, 1, 5 * ab + 256, "sia second buffers")) : nullptr;
+    whole = base != nullptr;
     if (!whole) base = static_cast<char*>(cg_scratch(ctx, 1, 3 * ab + 256, &rc));
     if (rc) return rc;
     cgsia::Words* words = reinterpret_cast<cgsia::Words*>(base + (whole ? 5 : 3) * ab);

@@ -154,10 +154,8 @@ int setup_coef(cg_ctx* ctx, const cg_grid* g, const cg_stokes_fields* f, const c
     lc->count = e0 * e1 * e2;
     lc->own_ieta = !cg_present(f->inv_eta);
     const int narr = lc->own_ieta + 2 + 2 * (ND == 2 ? 1 : 3) + ND;
-    int rc = CG_OK;
-    lc->base = static_cast<char*>(cg_scratch(ctx, 2, (size_t)narr * lc->count * sizeof(T), &rc));
-    if (rc) {
-        cudaGetLastError();
+    lc->base = static_cast<char*>(cg_scratch_optional(ctx, 2, (size_t)narr * lc->count * sizeof(T), "Stokes coefficients"));
+    if (!lc->base) {
         *lc = LoopCoef{};
         return CG_OK;
     }

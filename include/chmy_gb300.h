@@ -347,7 +347,12 @@ CG_API int cg_stokes_update_thermal(cg_ctx* ctx, const cg_grid* grid, const cg_s
 
 /* `niter` PT iterations: update_stress!, update_velocity!, bc!(V => bc_V[d]) each, captured
  * into a CUDA graph per (fields, niter) and replayed. divV and r_V are written only on the
- * last iteration (they are only read by the convergence check). */
+ * last iteration (they are only read by the convergence check).
+ * With variable viscosity in FP64, a loop long enough for it (2 iterations, 3 or 5 on small grids)
+ * computes the viscosity terms once, into 6 or 7 (2D) or 11 or 12 (3D) arrays of scratch, where these
+ * leave as much device memory free as they take. It then rounds otherwise than its launches one by one,
+ * in the last places: N calls of one iteration and one call of N agree to rounding, and so do two
+ * calls of which one found no room. CG_LOOP_COEF=0 in the environment gives the launches' bits always. */
 CG_API int cg_stokes_pt_iterations(cg_ctx* ctx, const cg_grid* grid, const cg_stokes_fields* f,
                             const cg_stokes_params* p, const cg_bc* bc_V, int niter);
 
@@ -506,7 +511,16 @@ CG_API int cg_ptdiff_update_C(cg_ctx* ctx, const cg_grid* grid, const cg_ptdiff_
                               const cg_ptdiff_params* p);
 /* `nsteps` implicit steps of `npt` PT iterations each (C_old <- C at the start of every step;
  * bc!(C => bc) after every iteration), replayed from one CUDA graph. R (if given) holds the
- * residual of the last iteration. */
+ * residual of the last iteration.
+ * Scratch, kept by the context: FP64 runs long enough for it (4 iterations in all, 16 on small grids)
+ * compute the face diffusivities once, into ndim arrays; 3D FP32 runs without R take a fused iteration
+ * with partner buffers of C and q (in Chmy's dense layout where the run is long enough for the copies).
+ * These are taken where they leave as much device memory free as they take (a pool layout's partner
+ * buffers where they fit), and a run without them works in place. The forms round differently: results
+ * agree to rounding, not in every bit, between a run and its launches one by one, between one run of N
+ * iterations and N of one, and between a run that found room and one that did not (CG_LOOP_COEF=0 and
+ * CG_PTDIFF_FUSED=0 in the environment give the launches' bits). D may be C, C_old or R: it is then read
+ * as it changes. */
 CG_API int cg_ptdiff_run(cg_ctx* ctx, const cg_grid* grid, const cg_ptdiff_fields* f,
                          const cg_ptdiff_params* p, const cg_bc* bc, int nsteps, int npt);
 
@@ -570,7 +584,9 @@ CG_API int cg_sia_update_H(cg_ctx* ctx, const cg_grid* grid, const cg_field* H, 
                            const cg_field* B, double dt, const cg_sia_params* p);
 /* `nsteps` SIA time steps with the adaptive Δt computed on the device every step (no host
  * synchronisation), replayed from one CUDA graph. q is the flux work array (its final
- * values are those of the last step). `t_host` (optional) receives the simulated time. */
+ * values are those of the last step). `t_host` (optional) receives the simulated time.
+ * Scratch, kept by the context: three arrays in H's layout, or five where a step may be one launch and
+ * they leave as much device memory free as they take; the results do not depend on it. */
 CG_API int cg_sia_run(cg_ctx* ctx, const cg_grid* grid, const cg_field* H, const cg_field* B,
                       const cg_field* q, const cg_sia_params* p, int nsteps, double* t_host);
 

@@ -53,3 +53,39 @@ def test_ptdiff_run_without_room(arch, monkeypatch, T, pitch, npt):
         assert_close(d[k], h[k], rtol_for(T) * 2 * npt, k)
     for a, b in zip(d["q"], h["q"]):
         assert_close(a, b, rtol_for(T) * 2 * npt, "q")
+
+
+@pytest.mark.parametrize("dims", [(60, 50), (16, 14, 12)])
+def test_stokes_loop_without_room(arch, monkeypatch, dims):
+    """An FP64 loop without its viscosity terms has the bits of its launches one by one."""
+    from test_gpu_loop_coef import stokes
+
+    monkeypatch.setenv("CG_SCRATCH_LIMIT", SMALL)
+    for a, b in zip(stokes(arch, dims, [20]), stokes(arch, dims, [0] * 20)):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("T", [np.float32, np.float64])
+def test_sia_run_without_room_for_second_buffers(arch, monkeypatch, T):
+    """Three arrays of scratch instead of five: two launches a step, the same bits; one array less is an
+    error that says so."""
+    from chmy_gb300 import ChmyError
+    from test_gpu_sia import reference_params, setup
+    from _oracle import desc_array
+
+    grid, H, B, q = setup(T, n=(66, 41), seed=7)
+    p, out = reference_params(), []
+    array = H.a.nbytes + 255 & ~255
+    for limit in (None, 4 * array):
+        if limit:
+            monkeypatch.setenv("CG_SCRATCH_LIMIT", str(limit))
+        Hg, Bg, qg = to_gpu(arch, H), to_gpu(arch, B), [to_gpu(arch, f) for f in q]
+        g, t = grid.desc(), ctypes.c_double()
+        call = lambda: arch.call("cg_sia_run", ctypes.byref(g), ctypes.byref(Hg.desc()), ctypes.byref(Bg.desc()), desc_array(qg, 3),
+                                 ctypes.byref(p), 7, ctypes.byref(t))
+        call()
+        out.append([f.to_numpy().tobytes() for f in [Hg] + qg] + [t.value])
+    assert out[0] == out[1]
+    monkeypatch.setenv("CG_SCRATCH_LIMIT", str(2 * array))
+    with pytest.raises(ChmyError, match="scratch"):
+        call()
