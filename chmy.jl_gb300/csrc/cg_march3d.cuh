@@ -482,8 +482,10 @@ inline cudaError_t launch_march3d(const Fused3D<T>& f, const SP<T>& s, int n0, i
                                   cudaStream_t st, int variant = 0, bool dep = false) {
     MStr str;
     const int lay = march3_layout(f, &str);
-    if (!march3_fits_int(f, n0 + 1, n1 + 1, n2 + 1))
-        return launch_march3d_ix<T, long, kLayOwn, WRITE_RES, 1>(f, s, n0, n1, n2, num_sms, seg_len, str, st, dep);
+    if (!march3_fits_int(f, n0 + 1, n1 + 1, n2 + 1)) {
+        if (lay == kLayOwn) return launch_march3d_ix<T, long, kLayOwn, WRITE_RES, 1>(f, s, n0, n1, n2, num_sms, seg_len, str, st, dep);
+        return launch_march3d_ix<T, long, kLayLoc, WRITE_RES, 1>(f, s, n0, n1, n2, num_sms, seg_len, str, st, dep);
+    }
     if (lay == kLayOwn) return launch_march3d_ix<T, int, kLayOwn, WRITE_RES, 1>(f, s, n0, n1, n2, num_sms, seg_len, str, st, dep);
     if constexpr (sizeof(T) == 4) {
         if (lay == kLayOne) {

@@ -59,3 +59,11 @@ def test_every_point_of_a_plane_has_a_thread(tmp_path):
                 assert ay == 1 and w * h <= ax * bx < 2**31
             else:
                 assert (ax, ay) == (-(-w // bx), -(-h // by))
+
+
+def test_large_layouts_keep_their_shared_strides():
+    """Views whose offsets need 64 bits run the marching kernels with the layout that their strides have: with
+    every array's own strides a 2D iteration took 15 % longer."""
+    for name, launch in (("cg_stokes_kernels.cuh", "launch_march2d_ix"), ("cg_march3d.cuh", "launch_march3d_ix")):
+        layouts = re.findall(launch + r"<T, long, (\w+),", _code(name))
+        assert "kLayOwn" in layouts and "kLayLoc" in layouts, (name, layouts)
