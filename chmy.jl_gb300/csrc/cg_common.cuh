@@ -251,8 +251,8 @@ __global__ void tune_delay_kernel(unsigned ns) {
 // behind the best, and the others a few times back to back. The launches queue behind a delay kernel, so
 // that the events see the kernels and not the rate at which the host launches them (a pair of events around
 // three bare launches of 3 us varies by more than the candidates differ). A first 50-step run of explicit
-// diffusion takes 1.0 ms at 120^2, 1.6 at 500^2 and 2.8 at 1000^2 this way, 4.7, 7.0 and 16.9 ms with 28 launches
-// of every candidate and a synchronisation after each.
+// diffusion takes 1.6 ms at 500^2 and 2.6 at 1000^2 this way, 7.0 and 16.9 ms with 28 launches of every candidate and
+// a synchronisation after each; a first FP32 PT-diffusion run of 20 iterations at 128^3 2.5 ms, and 17.8.
 template <class F>
 inline std::vector<float> time_candidates(int n, F&& launch, cudaStream_t st, std::vector<int> per = {}) {
     per.resize(n, 1);
@@ -261,31 +261,27 @@ inline std::vector<float> time_candidates(int n, F&& launch, cudaStream_t st, st
     bool good = n > 0;
     for (auto& e : ev) good = good && cudaEventCreate(&e) == cudaSuccess;
     std::vector<int> todo;
-    // the host's time for one candidate, once its code is loaded (the first launch of a kernel loads it)
-    double host = 8.;
-    bool loaded = false;
+    double host = 8.;  // the host's time for one candidate
     auto delay = [&](double us_) { tune_delay_kernel<0><<<1, 1, 0, st>>>((unsigned)(1e3 * std::min(us_, 2e3))); };
-    if (good && launch(0) != cudaSuccess) cudaGetLastError();  // untimed: most candidates share its code
-    if (good) delay(host * n);
-    for (int c = 0; good && c < n; ++c)
-        for (int again = 0; again < 2; ++again) {
+    // a first launch of a kernel loads its code and holds up the host: the pass is repeated then
+    for (int pass = 0; good && pass < 2; ++pass) {
+        bool loaded = false;
+        todo.clear();
+        delay(host * n);
+        for (int c = 0; c < n; ++c) {
             const auto h0 = std::chrono::steady_clock::now();
             cudaEventRecord(ev[2 * c], st);
             const bool ok = launch(c) == cudaSuccess;
             cudaEventRecord(ev[2 * c + 1], st);
             const double took = std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - h0).count();
-            if (!ok) {
-                cudaGetLastError();
-                break;
-            }
-            if (again == 0) todo.push_back(c);
-            if (took < 50.) {
-                host = took;
-                break;
-            }
-            loaded = true;  // launched again
+            if (ok) todo.push_back(c);
+            else cudaGetLastError();
+            if (took < 50.) host = took;
+            loaded = loaded || took >= 50.;
         }
-    good = good && cudaStreamSynchronize(st) == cudaSuccess;
+        good = cudaStreamSynchronize(st) == cudaSuccess;
+        if (!loaded) break;
+    }
     float best = 1e30f;
     for (int c : todo) {
         float ms = 0.f;
@@ -293,16 +289,16 @@ inline std::vector<float> time_candidates(int n, F&& launch, cudaStream_t st, st
         if (us[c] >= 0.f) best = std::min(best, us[c]);
     }
     if (good && todo.size() > 1) {
-        const float bound = 1.25f * best + (loaded ? 12.f : 2.f);
+        const float bound = 1.25f * best + 2.f;
         todo.erase(std::remove_if(todo.begin(), todo.end(), [&](int c) { return us[c] < 0.f || us[c] > bound; }), todo.end());
-        constexpr size_t kFinal = 8;  // as many are timed again
-        if (todo.size() > kFinal) {
-            std::nth_element(todo.begin(), todo.begin() + kFinal, todo.end(), [&](int a, int b) { return us[a] < us[b]; });
-            todo.resize(kFinal);
+        const size_t final = std::max(5, n / 3);  // as many are timed again
+        if (todo.size() > final) {
+            std::nth_element(todo.begin(), todo.begin() + final, todo.end(), [&](int a, int b) { return us[a] < us[b]; });
+            todo.resize(final);
             std::sort(todo.begin(), todo.end());
         }
         std::fill(us.begin(), us.end(), -1.f);
-        const int reps = best < 6.f ? 8 : best < 25.f ? 4 : best < 200.f ? 2 : 1;
+        const int reps = best < 6.f ? 8 : best < 25.f ? (n > 16 ? 4 : 6) : best < 200.f ? 2 : 1;
         if (best < 25.f) delay(host * (1 + reps * (double)todo.size()));
         launch(todo[0]);
         for (int c : todo) {
