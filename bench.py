@@ -521,9 +521,9 @@ def run_ours(args, rank, world, dist):
             "e2e": {"value": e2e_value, "unit": "GB/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h, "steps": e2e_steps},
             "gpu_launches": launches,
             "roofline": {
-                "bound": "hbm",
+                "bound": "instruction issue",
                 "kernel": "march2d_tile_kernel<float> (update_stress! + update_velocity!, 4 PT iterations per launch)",
-                "note": "bytes and time of one PT iteration; a launch moves them once for several, so frac can exceed 1",
+                "note": "bytes and time of one PT iteration against the HBM rate: an effective rate, since a launch moves them once for several iterations (profiles/loop_kernels.md)",
                 "achieved": achieved,
                 "peak": peak,
                 "unit": "GB/s",

@@ -304,11 +304,11 @@ __global__ void __launch_bounds__(256) static_differ_kernel(const Fused2D<T> f, 
 }
 
 // The tile shapes (the 2D layouts' variants 1 and up), W x R and K. Measured per iteration against
-// the one-iteration kernel's best segment length (its launches alone, without the overlap of a run):
-//   97^2      1.7 us (variant 2), 11.1 us     1023^2        11.3 us (variant 1), 20.7 us
-//   192^2     1.7 us (variant 2), 11.1 us     2047 x 1535   30.3 us (variant 1), 42.7 us
-//   384^2     3.3 us (variant 3), 11.8 us     4000^2         141 us (variant 1), 184 us
-//   768 x 700 6.9 us (variant 3), 14.5 us
+// the one-iteration kernel's best segment length, in runs of 50 iterations:
+//   97^2      1.7 us (variant 2), 8.3 us      1023^2        10.8 us (variant 1), 17.3 us
+//   192^2     1.9 us (variant 2), 8.4 us      2047 x 1535   29.0 us (variant 1), 41.1 us
+//   384^2     3.0 us (variant 3), 8.9 us      4000^2         137 us (variant 1), 190 us
+//   768 x 700 6.5 us (variant 3), 11.0 us
 // 32 x 32 tiles of 8 warps with 4 iterations (56 % of the points owned, two blocks per SM) are bound
 // by instruction issue from 1023^2 on; up to about 256^2 the grid does not fill the SMs, and 16 warps
 // of 2 rows with 8 iterations shorten the chain; 64-row tiles own 66 % but leave one block per SM.

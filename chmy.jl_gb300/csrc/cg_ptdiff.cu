@@ -465,8 +465,8 @@ __global__ void __launch_bounds__(32 * NW, MINB)
 // a guard (columns and rows beyond the range are clamped to stored ones). Same operations as
 // ptd_march3d_kernel, so the same bits. As a dependent launch it is resident while the iteration before
 // still writes C and q, so these are read by plain loads (__ldg wants data that does not change during the
-// kernel); D and C_old, which no iteration writes, by __ldg. It reads the strides of q.x and q.y apart from C's, so Chmy's
-// dense layout takes it too.
+// kernel); D and C_old, which no iteration writes, by __ldg. It reads the strides of q.x and q.y apart
+// from C's, so Chmy's dense layout takes it too.
 //
 // bc!(C) is folded into the stores (PdEdge): the thread that updates a cell beside a boundary writes
 // the ghost cells that follow it, in cg_bc_apply's order (z, then y, then x), and a ghost cell under a
@@ -478,8 +478,9 @@ __global__ void __launch_bounds__(32 * NW, MINB)
 // 192^3 87 -> 66, 60 x 77 x 50 a solve 6.2 -> 2.4 ms, and 191 x 160 x 128 in the dense layout, which ran
 // the flux and update kernels apart, 55.7 -> 39 us. Reading and writing the same bytes with this access
 // pattern and nothing else takes 17 us at 128^3, 56 at 192^3 and 124 at 256^3 (137 here, 150 by the
-// TMA-fed kernel; 384^3 412 and 436; at 512^3 the TMA-fed kernel's 957 is ahead of 959). Instruction issue bounds it beside
-// memory: 240 instructions per warp and row with a guard at every load, 190 without. Two rows per thread
+// TMA-fed kernel; 384^3 412 and 436; at 512^3 the TMA-fed kernel's 957 is ahead of 959). Memory latency and
+// instruction issue bound it together: 152 instructions per warp and row at two rows per thread, issue slots 49 %
+// and DRAM 46 % busy at 192 x 160 x 128. Two rows per thread
 // at 6 blocks per SM (80 registers) and three at 5 (96) beat four rows, and the same rows with more
 // registers and fewer blocks (128^3: 23.9 and 24.1) or with 7 or 8 blocks. The loads of the next plane
 // are in flight while a plane is computed (without that 37 us at 128^3). Copying two planes ahead to

@@ -142,7 +142,7 @@ __device__ __forceinline__ double block_sum(double x) {
 // Layout: a 256-byte header, then per step a 256-byte word block and kArrays arrays of `cnt`
 // elements in H's padded layout (each rounded up to 256 bytes).
 enum TapeArray {
-    kD = 0,   // D over cells [0, n]^2
+    kD = 0,   // D over the interior cells [1, n]^2
     kGX = 1,  // dS/dx at the cell's lower x face ((S_i - S_i-1)/dx)
     kGY = 2,  // dS/dy at the lower y face
     kDH = 3,  // dD/dh

@@ -378,10 +378,11 @@ CG_API int cg_stokes_pt_iterations_masked(cg_ctx* ctx, const cg_grid* grid, cons
  * that marches over rows (2D) or planes (3D). It reads V, P, tau from `a` and writes them to
  * `b`, then from `b` to `a`, and each launch is followed by bc!(V). `niter` must be even (the
  * result is in `a`; `b` holds the state one iteration earlier). Points outside the launch range
- * [0, n+1]^N are never written: `a` and `b` must agree there (b a copy of a, for instance), as
- * the in-place reference loop keeps one value per point. In 2D the autotuner may take two
- * iterations per launch (a kernel that keeps the intermediate state in registers) where no
- * bc!(V) launch is needed between iterations; the results are the same bits. All other fields (tau_old, inv_eta, rho_g, divV, r_V) are taken from
+ * [0, n+1]^N are never written; each iteration reads them from the buffer whose turn it is, so `a`
+ * and `b` should agree there (b a copy of a, for instance), as the in-place reference loop keeps one
+ * value per point. In 2D FP32 the autotuner may take four or eight iterations per launch (a kernel that
+ * keeps tiles in registers) where no bc!(V) launch is needed between iterations; the results are the
+ * same bits, also where the buffers differ outside the launch range. All other fields (tau_old, inv_eta, rho_g, divV, r_V) are taken from
  * `a`; inv_eta is required. divV and r_V are written on the last iteration. Every operation
  * is rounded once, in the order of the reference kernels, with no contraction into FMA: the
  * values are those of a CPU evaluation with -ffp-contract=off. */
